@@ -126,7 +126,7 @@ typedef struct lelph_gpu_stats
     double finish_ms;            /* device time of the finish kernel (profiling on) */
     long long pairs_done;        /* (k, q) pairs computed */
     size_t device_bytes;         /* device memory held by the context */
-    int product_grid[3];         /* grid of the real-space sandwich and wavefunction FFTs */
+    int product_grid[3];         /* plain product grid (the grid in use may be a smaller one: lelph_gpu_grid) */
     int chunk_points;            /* grid points per K chunk of the tensor-core sandwich (mixed form) */
     double dmats_ms;             /* device time of the Dmat kernels (index maps + contraction, profiling on) */
     double dmats_host_ms;        /* host time spent building Dmat jobs (always measured) */
@@ -335,6 +335,14 @@ int lelph_gpu_set_profiling(lelph_gpu* h, int on);
  * a test exercise that path.) */
 int lelph_gpu_set_wait_limit(lelph_gpu* h, unsigned long long ns);
 int lelph_gpu_stats_get(lelph_gpu* h, lelph_gpu_stats* s);
+/* Product grid in use: out = N_x, N_y, N_z, nsub, a_x, a_y, a_z -- nsub
+ * interleaved copies of an N_x x N_y x N_z grid, copy j shifted by
+ * j a_i / (nsub N_i) of the cell along axis i (no counterpart in the
+ * reference, which works on its FFT box).  Plain grid: nsub = 1.  The one-call
+ * stage (compute_elphq, compute_elphq_star) of the mixed form keeps the plain
+ * product grid, so that its complex128 results keep their digits; batch runs
+ * take the smallest grid that is exact for the spheres. */
+int lelph_gpu_grid(lelph_gpu* h, int out[7]);
 /* the CUDA stream (cudaStream_t) every kernel of the context runs on */
 void* lelph_gpu_stream(lelph_gpu* h);
 const char* lelph_gpu_strerror(int status);

@@ -263,12 +263,13 @@ __global__ void __launch_bounds__(256) k_fft_x_split(const float2* __restrict__ 
     float2* tws = b + (size_t)ich * p.L;
     for (int t = threadIdx.x; t < p.L; t += blockDim.x) tws[t] = tw[t];
     const int inner = gd.Ny * gd.Nz;
-    const long long N = (long long)gd.Nx * inner;
+    const long long Ns = (long long)gd.Nx * inner;  // points of one copy of the grid
+    const long long N = gd.nsub * Ns;
     int o = blockIdx.x / nchunk;
     int c = blockIdx.x - o * nchunk;
     int i0 = c * ich;
     const int ic = NLC > 0 ? NLC : min(ich, inner - i0);
-    const float2* g = boxes + (size_t)o * N + i0;
+    const float2* g = boxes + (size_t)o * Ns + i0;
     int n = p.L * ic;
     // x planes that the sphere of this k-point does not reach are zero: not read
     const uint8_t* xpl = mk.xpl ? mk.xpl + (size_t)(o / mk.nbox_per_k) * gd.Nx : nullptr;
@@ -306,9 +307,11 @@ __global__ void __launch_bounds__(256) k_fft_x_split(const float2* __restrict__ 
         r = ct_fft<float2, float, CTL, 0, 1, true, NLC>(a, b, ic, ic, 1, nullptr, ic, 1, tws, sign);
     else
         r = fft_smem<float2, float>(a, b, ic, ic, 1, p, tws, sign);
-    // box o -> (kslot, spin, band, spinor)
-    int sp = o % gd.nspinor;
-    int t = o / gd.nspinor;
+    // box o -> (kslot, spin, band, spinor, copy of the grid)
+    int t = o / gd.nsub;
+    const int cpy = o - t * gd.nsub;
+    int sp = t % gd.nspinor;
+    t /= gd.nspinor;
     int band = t % gd.nbnds;
     t /= gd.nbnds;
     int spin = t % gd.nspin;
@@ -329,7 +332,7 @@ __global__ void __launch_bounds__(256) k_fft_x_split(const float2* __restrict__ 
     uint32_t* const Blo = Bhi + nkb * NT * 32;
     const uint32_t rot = (uint32_t)gd.nbp * 32;  // (-Im, Re) rows
     float2* const P = psi32 + pg * npb * gd.nbp * 16 + (size_t)band * 16;
-    const uint32_t kbase = (uint32_t)((long long)sp * N) + (uint32_t)i0;  // K index of (x = 0, column 0)
+    const uint32_t kbase = (uint32_t)((long long)sp * N + cpy * Ns) + (uint32_t)i0;  // K index of (x = 0, column 0)
     if constexpr (NLC > 0)
     {
         // two adjacent points per thread: kc is even, so both sit in one
@@ -475,7 +478,7 @@ __global__ void __launch_bounds__(256) k_scatter(int k0, const KPointSym* __rest
                                                  const long long* __restrict__ coef_off, GeomDev gd,
                                                  T2* __restrict__ boxes, double2* __restrict__ chat,
                                                  float2* __restrict__ chat32, const long long* __restrict__ chat_off,
-                                                 BoxMask mk)
+                                                 const double2* __restrict__ sub_tw, BoxMask mk)
 {
     const int kslot = blockIdx.y;
     const int kbz = k0 + kslot;
@@ -484,7 +487,8 @@ __global__ void __launch_bounds__(256) k_scatter(int k0, const KPointSym* __rest
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= npw) return;
     const int* mil = miller + 3 * pw_off[s.ik];
-    const long long N = (long long)gd.Nx * gd.Ny * gd.Nz;
+    const long long N = lelph_sub_points(gd);
+    const int nsub = gd.nsub;
     const int nsets = gd.nspin * gd.nbnds;
     const int n0 = mil[3 * g], n1 = mil[3 * g + 1], n2 = mil[3 * g + 2];
     const int G0 = s.W[0] * n0 + s.W[1] * n1 + s.W[2] * n2;
@@ -513,7 +517,24 @@ __global__ void __launch_bounds__(256) k_scatter(int k0, const KPointSym* __rest
     // the unfolded coefficients in FP64, or in FP32 (chat32) for the tensor-core projections
     double2* chb = chat32 ? nullptr : chat + chat_off[kbz];
     float2* chb32 = chat32 ? chat32 + chat_off[kbz] : nullptr;
-    T2* bxb = boxes ? boxes + (size_t)kslot * nsets * gd.nspinor * N : nullptr;
+    T2* bxb = boxes ? boxes + (size_t)kslot * nsets * gd.nspinor * nsub * N : nullptr;
+    // e^{i G.delta} of the shift of copy 1 (its powers: the other copies'), from exact
+    // tables of the rational angles
+    double2 sh = make_double2(1.0, 0.0);
+    if (nsub > 1 && bxb)
+    {
+        const double2* tw = sub_tw;
+        const int Ga[3] = {gd.sa[0] * G0, gd.sa[1] * G1, gd.sa[2] * G2}, Na[3] = {gd.Nx, gd.Ny, gd.Nz};
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+        {
+            const int L = nsub * Na[x];
+            int e = Ga[x] % L;
+            if (e < 0) e += L;
+            sh = cmul(sh, tw[e]);
+            tw += L;
+        }
+    }
     for (int set = 0; set < nsets; ++set)
     {
         const double2* c = cbase + (size_t)set * gd.nspinor * npw;
@@ -535,7 +556,17 @@ __global__ void __launch_bounds__(256) k_scatter(int k0, const KPointSym* __rest
             if (s.trev) w.y = -w.y;
             if (chb32) chb32[co + (size_t)sp * npw + g] = make_float2((float)w.x, (float)w.y);
             else chb[co + (size_t)sp * npw + g] = w;
-            if (bxb) bxb[((size_t)set * gd.nspinor + sp) * N + bidx] = mk2<T2>(w.x, w.y);
+            if (bxb)
+            {
+                T2* b = bxb + ((size_t)set * gd.nspinor + sp) * nsub * N + bidx;
+                *b = mk2<T2>(w.x, w.y);
+                for (int j = 1; j < nsub; ++j)
+                {
+                    w = cmul(w, sh);
+                    b += N;
+                    *b = mk2<T2>(w.x, w.y);
+                }
+            }
         }
     }
 }
@@ -570,7 +601,27 @@ static int ich_for(int L, int inner, int elems)
 }
 
 // Line lengths with a compile-time FFT instance (FP32 passes of the mixed form)
-#define LELPH_CT_SIZES(X) X(24) X(36) X(48) X(60) X(64) X(72) X(96)
+// the original ones, and those of the interleaved grids' copies
+#define LELPH_CT_SIZES0(X) X(24) X(36) X(48) X(60) X(64) X(72) X(96)
+#define LELPH_CT_SIZES(X) LELPH_CT_SIZES0(X) X(10) X(12) X(16) X(18) X(20) X(30) X(32) X(40) X(45) X(54)
+
+bool lelph_fft_fixed(int L, int all)
+{
+#define LELPH_CT_CASE(N) case N:
+    switch (L)
+    {
+        LELPH_CT_SIZES0(LELPH_CT_CASE)
+        return true;
+    default: break;
+    }
+    switch (L)
+    {
+        LELPH_CT_SIZES(LELPH_CT_CASE)
+        return all != 0;
+    default: return false;
+    }
+#undef LELPH_CT_CASE
+}
 
 template <typename T2, typename T, int CTL>
 static void launch_contig_l(T2* data, long long nlines, const FftPlan1D& p, const T2* tw, int sign, cudaStream_t st,
@@ -629,7 +680,7 @@ static void launch_contig(T2* data, long long nlines, const FftPlan1D& p, const 
 {
     if constexpr (sizeof(T) == 4)
     {
-        switch (p.L)
+        if (lelph_fft_fixed(p.L, p.allct)) switch (p.L)
         {
 #define LELPH_CT_CASE(N) \
     case N: launch_contig_l<T2, T, N>(data, nlines, p, tw, sign, st, mk); return;
@@ -647,7 +698,7 @@ static void launch_strided(T2* data, long long nouter, int inner, const FftPlan1
 {
     if constexpr (sizeof(T) == 4)
     {
-        switch (p.L)
+        if (lelph_fft_fixed(p.L, p.allct)) switch (p.L)
         {
 #define LELPH_CT_CASE(N) \
     case N: launch_strided_l<T2, T, N>(data, nouter, inner, p, tw, sign, st, mk); return;
@@ -709,15 +760,28 @@ static void launch_x_split_l(unsigned nb, size_t smem, const float2* boxes, int 
                              const float* band_scale, uint16_t* Bsplit, float2* psi32, cudaStream_t st,
                              const BoxMask& mk)
 {
-    // an even count: the compile-time form works on column pairs
-    constexpr int NLC = (CTL > 0 && x_split_nlc(CTL) % 2 == 0) ? x_split_nlc(CTL) : 0;
+    // compile-time column counts that tile the plane: the block's usual count, or
+    // one of three others of at most 2560 elements (24-point lines: 96 columns of a
+    // 24 x 24 plane); even, since the compile-time form works on column pairs
     const int inner = g.Ny * g.Nz;
-    if (NLC > 0 && ich == NLC && inner % NLC == 0 && 256 / NLC >= 1)
-        launch_x_split_n<BF16, CTL, NLC>(nb, smem, boxes, nbox, k0, ich, nchunk, p, tw, sign, g, band_scale, Bsplit,
-                                         psi32, st, mk);
-    else
-        launch_x_split_n<BF16, CTL, 0>(nb, smem, boxes, nbox, k0, ich, nchunk, p, tw, sign, g, band_scale, Bsplit,
-                                       psi32, st, mk);
+    constexpr int NLC = (CTL > 0 && x_split_nlc(CTL) % 2 == 0) ? x_split_nlc(CTL) : 0;
+#define LELPH_XS_TRY(C)                                                                                            \
+    if constexpr (CTL > 0 && (C) > 0 && (C) * CTL <= 2560 && (C) <= 512)                                           \
+        if (inner % (C) == 0)                                                                                      \
+        {                                                                                                          \
+            const size_t sm = (size_t)(2 * (C) * CTL + CTL) * sizeof(float2);                                      \
+            const unsigned blocks = (unsigned)(nb / nchunk) * (unsigned)(inner / (C));                             \
+            launch_x_split_n<BF16, CTL, (C)>(blocks, sm, boxes, nbox, k0, (C), inner / (C), p, tw, sign, g,        \
+                                             band_scale, Bsplit, psi32, st, mk);                                   \
+            return;                                                                                                \
+        }
+    LELPH_XS_TRY(NLC)
+    LELPH_XS_TRY(96)
+    LELPH_XS_TRY(64)
+    LELPH_XS_TRY(48)
+#undef LELPH_XS_TRY
+    launch_x_split_n<BF16, CTL, 0>(nb, smem, boxes, nbox, k0, ich, nchunk, p, tw, sign, g, band_scale, Bsplit, psi32,
+                                   st, mk);
 }
 
 template <int BF16>
@@ -725,7 +789,7 @@ static void launch_x_split(unsigned nb, size_t smem, const float2* boxes, int nb
                            const FftPlan1D& p, const float2* tw, int sign, const GeomDev& g, const float* band_scale,
                            uint16_t* Bsplit, float2* psi32, cudaStream_t st, const BoxMask& mk)
 {
-    switch (p.L)
+    if (lelph_fft_fixed(p.L, p.allct)) switch (p.L)
     {
 #define LELPH_CT_CASE(N)                                                                                         \
     case N:                                                                                                      \
@@ -751,7 +815,7 @@ void lelph_launch_fft_x_to_split(const float2* boxes, int nbox_k, int k0, const 
     int ich = ich_for(p.L, inner, 2048);
     int nchunk = (inner + ich - 1) / ich;
     size_t smem = (size_t)(2 * ich * p.L + p.L) * sizeof(float2);
-    long long nbox = (long long)nbox_k * g.nspin * g.nbnds * g.nspinor;
+    long long nbox = (long long)nbox_k * g.nspin * g.nbnds * g.nspinor * g.nsub;
     unsigned nb = (unsigned)(nbox * nchunk);
     if (ab_bf16)
         launch_x_split<1>(nb, smem, boxes, (int)nbox, k0, ich, nchunk, p, tw, sign, g, band_scale, Bsplit, psi32, st,
@@ -764,15 +828,15 @@ void lelph_launch_fft_x_to_split(const float2* boxes, int nbox_k, int k0, const 
 void lelph_launch_scatter(int k0, int nk, const KPointSym* ksym_dev, const int* miller, const long long* pw_off,
                           const int* npw, int npw_max, const double2* coef, const long long* coef_off,
                           const GeomDev& g, int box_fp64, void* boxes, double2* chat, const long long* chat_off,
-                          cudaStream_t st, const BoxMask& mk, float2* chat32)
+                          const double2* sub_tw, cudaStream_t st, const BoxMask& mk, float2* chat32)
 {
     dim3 grid((unsigned)((npw_max + 255) / 256), nk);
     if (box_fp64)
         k_scatter<double2><<<grid, 256, 0, st>>>(k0, ksym_dev, miller, pw_off, npw, coef, coef_off, g,
-                                                 (double2*)boxes, chat, chat32, chat_off, mk);
+                                                 (double2*)boxes, chat, chat32, chat_off, sub_tw, mk);
     else
         k_scatter<float2><<<grid, 256, 0, st>>>(k0, ksym_dev, miller, pw_off, npw, coef, coef_off, g,
-                                                (float2*)boxes, chat, chat32, chat_off, mk);
+                                                (float2*)boxes, chat, chat32, chat_off, sub_tw, mk);
 }
 
 void lelph_launch_gmap(const KPointSym* ks, int kbz, const int* miller, const long long* pw_off, const int* npw,

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_plane(const T2* __restrict__ 
     const int nu = nu0 + nul;
     for (int t = threadIdx.x; t < Ny; t += blockDim.x) ty[t] = twy[t];
     for (int t = threadIdx.x; t < Nz; t += blockDim.x) tz[t] = twz[t];
-    const long long M = (long long)gg.Nx * NP;
+    const long long M = (long long)gg.nsub * gg.Nx * NP;
     const size_t xoff = (size_t)x * NP;
     const T2* pm = psi + (size_t)m * gg.nspinor * M + xoff;           // psi_k, band m, spinor 0, plane x
     const T2* dv = win + (size_t)nu * gg.nmag * M + xoff;             // window of mode nu, component 0, plane x
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_plane(const T2* __restrict__ 
         T2* r = fft_smem<T2, T>(a, b, Ny, 1, Nz, pz, tz, -1);       // z lines
         T2* o = r == a ? b : a;
         r = fft_smem<T2, T>(r, o, Nz, Nz, 1, py, ty, -1);           // y lines
-        T2* dst = out + (((size_t)(nul * gg.nb + m) * gg.nspinor + s) * gg.Nx + x) * ncol;
+        T2* dst = out + (((size_t)(nul * gg.nb + m) * gg.nspinor + s) * gg.nsub * gg.Nx + x) * ncol;
         for (int c = threadIdx.x; c < ncol; c += blockDim.x) dst[c] = r[cols[c]];
         __syncthreads();
     }
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_plane_ct(const T2* __restrict
     for (int t = threadIdx.x; t < NZ; t += blockDim.x) tz[t] = twz[t];
     for (int t = threadIdx.x; t < nzl; t += blockDim.x) szl[t] = zl[t];
     constexpr int NPL = NY * NZ;      // points of a plane in global memory
-    const long long M = (long long)gg.Nx * NPL;
+    const long long M = (long long)gg.nsub * gg.Nx * NPL;
     const size_t xoff = (size_t)x * NPL;
     const T2* pm = psi + (size_t)m * gg.nspinor * M + xoff;
     const T2* dv = win + (size_t)nu * gg.nmag * M + xoff;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_plane_ct(const T2* __restrict
         T2* r = ct_fft<T2, T, NZ, 0, 1, true, NY>(a, b, NY, 1, NZP, nullptr, 1, NZP, tz, -1);
         T2* o = r == a ? b : a;
         r = ct_fft<T2, T, NY, 0, 1, true, 0>(r, o, nzl, NZP, 1, szl, nzl, 1, ty, -1);
-        T2* dst = out + (((size_t)(nul * gg.nb + m) * gg.nspinor + s) * gg.Nx + x) * ncol;
+        T2* dst = out + (((size_t)(nul * gg.nb + m) * gg.nspinor + s) * gg.nsub * gg.Nx + x) * ncol;
         for (int c = threadIdx.x; c < ncol; c += GS_THREADS) dst[c] = r[cols2[c]];
         __syncthreads();
     }
@@ -162,51 +162,76 @@ __device__ __forceinline__ void gs_store(float2* hi, float2* lo, int K, float2 v
     lo[K] = make_float2(tf32_rn(v.x - h.x), tf32_rn(v.y - h.y));
 }
 
+// Sphere point K: the copies' values summed with their phases e^{-i G.delta_j} = shph[K]^j.
+template <typename T2>
+__device__ __forceinline__ T2 gs_sum_copies(const T2* r, int cb, int nsub, const T2* __restrict__ shph, int K)
+{
+    T2 v = r[0];
+    if (nsub > 1)
+    {
+        const T2 w = shph[K];
+        T2 p = w;
+        for (int j = 1; j < nsub; ++j)
+        {
+            v = cadd(v, cmul(r[j * cb], p));
+            p = cmul(p, w);
+        }
+    }
+    return v;
+}
+
 // -------------------------------------------------------------------- x pass
 // grid: (ceil(ncol / GS_CB), rows of the block x nspinor); the tile [x][column]
 // is read along the columns (coalesced), transformed along x, and the sphere
 // points of the block's columns -- a contiguous K range, sorted by (column, x)
-// -- are written in order.
+// -- are written in order.  On an interleaved grid a tile holds the block's
+// columns of every copy (line j cb + c: column c of copy j), and a sphere
+// point is the sum of the copies' values times e^{-i G.delta_j}, the powers of
+// its shph[K].
 template <typename T2, typename T>
 __global__ void __launch_bounds__(GS_THREADS) k_gs_xpass(const T2* __restrict__ in, int Nx, int ncol,
                                                          FftPlan1D px, const T2* __restrict__ twx,
                                                          const int* __restrict__ cst, const int* __restrict__ kcx,
-                                                         int npad, T2* __restrict__ A, T2* __restrict__ A_lo)
+                                                         const T2* __restrict__ shph, int nsub, int npad,
+                                                         T2* __restrict__ A, T2* __restrict__ A_lo)
 {
     extern __shared__ __align__(16) unsigned char gsx_smem[];
     T2* a = reinterpret_cast<T2*>(gsx_smem);
     T2* b = a + Nx * GS_CB;
     T2* tx = b + Nx * GS_CB;
-    const int c0 = blockIdx.x * GS_CB;
+    const int cb = GS_CB / nsub;  // columns of the tile
+    const int c0 = blockIdx.x * cb;
     const int rb = blockIdx.y;
     for (int t = threadIdx.x; t < Nx; t += blockDim.x) tx[t] = twx[t];
-    const T2* src = in + (size_t)rb * Nx * ncol;
+    const T2* src = in + (size_t)rb * nsub * Nx * ncol;
     for (int e = threadIdx.x; e < Nx * GS_CB; e += blockDim.x)
     {
-        const int x = e / GS_CB, cc = e - x * GS_CB;
-        const int c = c0 + cc;
-        a[e] = c < ncol ? src[(size_t)x * ncol + c] : mk2<T2>(0.0, 0.0);
+        const int x = e / GS_CB, l = e - x * GS_CB;
+        const int j = l / cb, c = c0 + l - j * cb;
+        a[e] = (j < nsub && c < ncol) ? src[((size_t)j * Nx + x) * ncol + c] : mk2<T2>(0.0, 0.0);
     }
     __syncthreads();
     T2* r = fft_smem<T2, T>(a, b, GS_CB, GS_CB, 1, px, tx, -1);
-    const int k0 = cst[c0], k1 = cst[min(c0 + GS_CB, ncol)];
+    const int k0 = cst[c0], k1 = cst[min(c0 + cb, ncol)];
     T2* dst = A + (size_t)rb * npad;
     for (int K = k0 + threadIdx.x; K < k1; K += blockDim.x)
     {
         const int v = kcx[K];
         const int c = v / Nx, x = v - c * Nx;
-        gs_store(dst, A_lo ? A_lo + (size_t)rb * npad : nullptr, K, r[x * GS_CB + (c - c0)]);
+        gs_store(dst, A_lo ? A_lo + (size_t)rb * npad : nullptr, K,
+                 gs_sum_copies(r + x * GS_CB + (c - c0), cb, nsub, shph, K));
     }
 }
 
-// x pass for the compile-time sizes: CB columns per CTA, every load of the
-// tile issued before the first is used (the generic pass waits on each), the
-// x transform with the compile-time schedule, consecutive threads on
-// consecutive columns (conflict-free).
+// x pass for the compile-time sizes: CB lines per CTA (CB / nsub columns of
+// every copy), every load of the tile issued before the first is used (the
+// generic pass waits on each), the x transform with the compile-time
+// schedule, consecutive threads on consecutive lines (conflict-free).
 template <typename T2, typename T, int NX, int CB>
 __global__ void __launch_bounds__(GS_THREADS) k_gs_xpass_ct(const T2* __restrict__ in, int ncol,
                                                             const T2* __restrict__ twx, const int* __restrict__ cst,
-                                                            const int* __restrict__ kcx, int npad,
+                                                            const int* __restrict__ kcx,
+                                                            const T2* __restrict__ shph, int nsub, int npad,
                                                             T2* __restrict__ A, T2* __restrict__ A_lo)
 {
     constexpr int NE = NX * CB;
@@ -215,17 +240,19 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_xpass_ct(const T2* __restrict
     T2* a = reinterpret_cast<T2*>(gsxc_smem);
     T2* b = a + NE;
     T2* tx = b + NE;
-    const int c0 = blockIdx.x * CB;
+    const int cb = CB / nsub;  // columns of the tile
+    const int c0 = blockIdx.x * cb;
     const int rb = blockIdx.y;
     for (int t = threadIdx.x; t < NX; t += blockDim.x) tx[t] = twx[t];
-    const T2* src = in + (size_t)rb * NX * ncol + c0;
+    const T2* src = in + (size_t)rb * nsub * NX * ncol + c0;
     T2 v[PER];
 #pragma unroll
     for (int i = 0; i < PER; ++i)
     {
         const int e = threadIdx.x + i * GS_THREADS;
-        const int x = e / CB, cc = e - x * CB;
-        v[i] = (e < NE && c0 + cc < ncol) ? src[(size_t)x * ncol + cc] : mk2<T2>(0.0, 0.0);
+        const int x = e / CB, l = e - x * CB;
+        const int j = l / cb, cc = l - j * cb;
+        v[i] = (e < NE && j < nsub && c0 + cc < ncol) ? src[((size_t)j * NX + x) * ncol + cc] : mk2<T2>(0.0, 0.0);
     }
 #pragma unroll
     for (int i = 0; i < PER; ++i)
@@ -235,14 +262,14 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_xpass_ct(const T2* __restrict
     }
     __syncthreads();
     T2* r = ct_fft<T2, T, NX, 0, 1, true, CB>(a, b, CB, CB, 1, nullptr, CB, 1, tx, -1);
-    const int k0 = cst[c0], k1 = cst[min(c0 + CB, ncol)];
+    const int k0 = cst[c0], k1 = cst[min(c0 + cb, ncol)];
     T2* dst = A + (size_t)rb * npad;
     T2* dlo = A_lo ? A_lo + (size_t)rb * npad : nullptr;
     for (int K = k0 + threadIdx.x; K < k1; K += blockDim.x)
     {
         const int w = kcx[K];
         const int c = w / NX, x = w - c * NX;
-        gs_store(dst, dlo, K, r[x * CB + (c - c0)]);
+        gs_store(dst, dlo, K, gs_sum_copies(r + x * CB + (c - c0), cb, nsub, shph, K));
     }
 }
 
@@ -544,7 +571,7 @@ __global__ void __launch_bounds__(GS_THREADS, 3) k_gs_plane_ct1(const float2* __
     for (int t = threadIdx.x; t < NY; t += blockDim.x) ty[t] = twy[t];
     for (int t = threadIdx.x; t < NZ; t += blockDim.x) tz[t] = twz[t];
     for (int t = threadIdx.x; t < nzl; t += blockDim.x) szl[t] = zl[t];
-    const long long M = (long long)gg.Nx * NPL;
+    const long long M = (long long)gg.nsub * gg.Nx * NPL;
     const size_t xoff = (size_t)x * NPL;
     const float2* pm = psi + (size_t)m * M + xoff;
     const int comp = gg.nmag == 2 ? gg.spin : 0;
@@ -568,7 +595,7 @@ __global__ void __launch_bounds__(GS_THREADS, 3) k_gs_plane_ct1(const float2* __
         float2* r = ct_fft<float2, float, NZ, 0, 1, true, NY>(a, b, NY, 1, NZP, nullptr, 1, NZP, tz, -1);
         float2* o = r == a ? b : a;
         r = ct_fft<float2, float, NY, 0, 1, true, 0>(r, o, nzl, NZP, 1, szl, nzl, 1, ty, -1);
-        float2* dst = out + ((size_t)(nul * gg.nb + m) * gg.Nx + x) * ncol;
+        float2* dst = out + ((size_t)(nul * gg.nb + m) * gg.nsub * gg.Nx + x) * ncol;
         for (int c = threadIdx.x; c < ncol; c += GS_THREADS) dst[c] = r[cols2[c]];
         __syncthreads();
     }
@@ -585,7 +612,7 @@ static int gs_plane_ct(const GsGeom& gg, const void* psi, const void* win, int n
         if (gg.nspinor == 1)
         {
             constexpr int NUC = 8;
-            dim3 g1((unsigned)((nub + NUC - 1) / NUC), (unsigned)gg.nb, (unsigned)gg.Nx);
+            dim3 g1((unsigned)((nub + NUC - 1) / NUC), (unsigned)gg.nb, (unsigned)(gg.nsub * gg.Nx));
             static bool attr1 = false;
             if (!attr1)
             {
@@ -608,7 +635,7 @@ static int gs_plane_ct(const GsGeom& gg, const void* psi, const void* win, int n
             return -1;
         attr = true;
     }
-    dim3 grid((unsigned)nub, (unsigned)gg.nb, (unsigned)gg.Nx);
+    dim3 grid((unsigned)nub, (unsigned)gg.nb, (unsigned)(gg.nsub * gg.Nx));
     k_gs_plane_ct<T2, T, N, N><<<grid, GS_THREADS, smem, st>>>((const T2*)psi, (const T2*)win, gg, nu0,
                                                                (const T2*)twy, (const T2*)twz, cols2, ncol, zl, nzl,
                                                                (T2*)out);
@@ -621,6 +648,7 @@ bool lelph_gs_plane_fixed(const GsGeom& gg, int fp64)
     switch (gg.Ny)
     {
     case 36: case 48: case 60: case 64: case 72: case 80: return true;
+    case 24: case 30: case 32: case 40: case 45: return gg.allct != 0;
     case 96: return !fp64;  // two FP64 96 x 96 planes exceed shared memory
     default: return false;
     }
@@ -631,13 +659,18 @@ int lelph_launch_gs_plane(const GsGeom& gg, int fp64, const void* psi, const voi
                           int ncol, const int* cols2, const int* zl, int nzl, void* out, cudaStream_t st)
 {
     const size_t smem = lelph_gs_plane_smem(gg, fp64);
-    if (smem > 220 * 1024 || nub > 65535 || gg.nb > 65535 || gg.Nx > 65535) return -1;
+    if (smem > 220 * 1024 || nub > 65535 || gg.nb > 65535 || gg.nsub * gg.Nx > 65535) return -1;
     if (lelph_gs_plane_fixed(gg, fp64) && cols2 && zl)
     {
 #define GS_CT(N)                                                                                                       case N:                                                                                                                return fp64 ? gs_plane_ct<double2, double, N>(gg, psi, win, nu0, nub, twy, twz, cols2, ncol, zl, nzl, out, st)                     : gs_plane_ct<float2, float, N>(gg, psi, win, nu0, nub, twy, twz, cols2, ncol, zl, nzl, out, st);
         switch (gg.Ny)
         {
+            GS_CT(24)
+            GS_CT(30)
+            GS_CT(32)
             GS_CT(36)
+            GS_CT(40)
+            GS_CT(45)
             GS_CT(48)
             GS_CT(60)
             GS_CT(64)
@@ -651,7 +684,7 @@ int lelph_launch_gs_plane(const GsGeom& gg, int fp64, const void* psi, const voi
         }
 #undef GS_CT
     }
-    dim3 grid((unsigned)nub, (unsigned)gg.nb, (unsigned)gg.Nx);
+    dim3 grid((unsigned)nub, (unsigned)gg.nb, (unsigned)(gg.nsub * gg.Nx));
     if (fp64)
     {
         if (cudaFuncSetAttribute(k_gs_plane<double2, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -674,8 +707,8 @@ int lelph_launch_gs_plane(const GsGeom& gg, int fp64, const void* psi, const voi
 }
 
 template <typename T2, typename T, int NX, int CB>
-static int gs_xpass_ct(int nrb, int ncol, const void* twx, const int* cst, const int* kcx, int npad, const void* in,
-                       void* A, void* A_lo, cudaStream_t st)
+static int gs_xpass_ct(int nrb, int ncol, int nsub, const void* twx, const int* cst, const int* kcx,
+                       const void* shph, int npad, const void* in, void* A, void* A_lo, cudaStream_t st)
 {
     const size_t smem = sizeof(T2) * (2 * (size_t)NX * CB + NX);
     static bool attr = false;
@@ -686,26 +719,35 @@ static int gs_xpass_ct(int nrb, int ncol, const void* twx, const int* cst, const
             return -1;
         attr = true;
     }
-    dim3 grid((unsigned)((ncol + CB - 1) / CB), (unsigned)nrb);
-    k_gs_xpass_ct<T2, T, NX, CB><<<grid, GS_THREADS, smem, st>>>((const T2*)in, ncol, (const T2*)twx, cst, kcx, npad,
-                                                                (T2*)A, (T2*)A_lo);
+    const int cb = CB / nsub;
+    dim3 grid((unsigned)((ncol + cb - 1) / cb), (unsigned)nrb);
+    k_gs_xpass_ct<T2, T, NX, CB><<<grid, GS_THREADS, smem, st>>>((const T2*)in, ncol, (const T2*)twx, cst, kcx,
+                                                                (const T2*)shph, nsub, npad, (T2*)A, (T2*)A_lo);
     return 0;
 }
 
 int lelph_launch_gs_xpass(const GsGeom& gg, int fp64, const void* in, int nrb, int ncol, const FftPlan1D& px,
-                          const void* twx, const int* cst, const int* kcx, int npad, void* A, cudaStream_t st,
-                          void* A_lo)
+                          const void* twx, const int* cst, const int* kcx, const void* shph, int npad, void* A,
+                          cudaStream_t st, void* A_lo)
 {
     if (fp64) A_lo = nullptr;
     const size_t smem = lelph_gs_xpass_smem(gg, fp64);
     if (smem > 220 * 1024 || nrb > 65535) return -1;
 #define GS_XC(N)                                                                                            \
     case N:                                                                                                 \
-        return fp64 ? gs_xpass_ct<double2, double, N, 32>(nrb, ncol, twx, cst, kcx, npad, in, A, A_lo, st)  \
-                    : gs_xpass_ct<float2, float, N, 64>(nrb, ncol, twx, cst, kcx, npad, in, A, A_lo, st);
+        return fp64 ? gs_xpass_ct<double2, double, N, 32>(nrb, ncol, gg.nsub, twx, cst, kcx, shph, npad, in, A,   \
+                                                          A_lo, st)                                         \
+                    : gs_xpass_ct<float2, float, N, 64>(nrb, ncol, gg.nsub, twx, cst, kcx, shph, npad, in, A, A_lo, \
+                                                        st);
+    if (gg.allct || gg.Nx == 36 || gg.Nx == 48 || gg.Nx == 60 || gg.Nx == 64 || gg.Nx == 72 || gg.Nx == 80 || gg.Nx == 96)
     switch (gg.Nx)
     {
+        GS_XC(24)
+        GS_XC(30)
+        GS_XC(32)
         GS_XC(36)
+        GS_XC(40)
+        GS_XC(45)
         GS_XC(48)
         GS_XC(60)
         GS_XC(64)
@@ -716,14 +758,16 @@ int lelph_launch_gs_xpass(const GsGeom& gg, int fp64, const void* in, int nrb, i
         break;
     }
 #undef GS_XC
-    dim3 grid((unsigned)((ncol + GS_CB - 1) / GS_CB), (unsigned)nrb);
+    const int cb = GS_CB / gg.nsub;
+    dim3 grid((unsigned)((ncol + cb - 1) / cb), (unsigned)nrb);
     if (fp64)
     {
         if (cudaFuncSetAttribute(k_gs_xpass<double2, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem) != cudaSuccess)
             return -1;
         k_gs_xpass<double2, double><<<grid, GS_THREADS, smem, st>>>((const double2*)in, gg.Nx, ncol, px,
-                                                                    (const double2*)twx, cst, kcx, npad,
+                                                                    (const double2*)twx, cst, kcx,
+                                                                    (const double2*)shph, gg.nsub, npad,
                                                                     (double2*)A, nullptr);
     }
     else
@@ -732,7 +776,8 @@ int lelph_launch_gs_xpass(const GsGeom& gg, int fp64, const void* in, int nrb, i
                                  (int)smem) != cudaSuccess)
             return -1;
         k_gs_xpass<float2, float><<<grid, GS_THREADS, smem, st>>>((const float2*)in, gg.Nx, ncol, px,
-                                                                  (const float2*)twx, cst, kcx, npad, (float2*)A,
+                                                                  (const float2*)twx, cst, kcx,
+                                                                  (const float2*)shph, gg.nsub, npad, (float2*)A,
                                                                   (float2*)A_lo);
     }
     return 0;

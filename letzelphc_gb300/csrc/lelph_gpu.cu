@@ -46,7 +46,68 @@ struct QSlot
     int dmin[3];            // first G' - G1 of the window of differences this q needs
 };
 
-struct lelph_gpu
+// A product grid and its cost (points, weighted by how well the kernels take it).
+struct GridChoice
+{
+    int n[3] = {0, 0, 0};
+    int nsub = 1;
+    int sa[3] = {0, 0, 0};
+    bool sphere = false;
+    double cost = 0;
+    long long points() const { return (long long)nsub * n[0] * n[1] * n[2]; }
+};
+
+// What a context holds on one product grid: psi(r) of every full-BZ k, the dV
+// windows of the q slots, and the tables of both.  The mixed form has two where
+// pick_grid finds a grid smaller than the plain one: batch runs (run,
+// run_device and the allocation-free form) use the smaller one, the one-call
+// entry points (compute_elphq, compute_elphq_star) the plain one, whose
+// complex128 results thereby keep their digits.  use_grid makes one of them
+// active (the base of lelph_gpu) and sets it up when it is first needed.
+struct GridState
+{
+    int which = 0;  // 0: batch runs, 1: one-call stage
+    GeomDev g{};
+    bool set_up = false;
+    bool prepared = false;
+    FftPlan1D plan[3];   // one copy of the product grid (g.Nx, g.Ny, g.Nz)
+    FftPlan1D planN[3];  // the reference's FFT box
+    DevBuf d_tw64[3], d_tw32[3];
+    bool sphere_window = false;   // dV windows hold the differences nearest to -q (see k_dv_window)
+    DevBuf d_subtw64, d_subtw32;  // e^{+2 pi i t / (nsub N_i)} per axis (interleaved grids)
+    DevBuf d_psi64, d_bsplit, d_psi32;
+    CUtensorMap tmapB, tmapP, tmapV;
+    void* tmapV_base = nullptr;
+    int tmapV_rows = 0;
+    int chunk_pts = 0, nchunks = 0;
+    DevBuf d_win64, d_win32, d_winscale;  // dV windows, per (slot, umklapp)
+    std::vector<int> win_base;  // first window entry of each q slot
+    int nwin = 0;
+    bool windows_ok = false;
+    DevBuf d_colmask;  // box occupancy of every full-BZ k (z-columns of all k, then x planes of all k)
+    DevBuf d_collist, d_colcnt;  // occupied z-columns of every k as lists
+    bool boxmask_ready = false;  // occupancy and lists built (geometry only: they stay valid)
+    long long box_columns = 0;
+    // G-space route: every full-BZ k's sphere (its k+q role) sorted by
+    // ((y, z) column, x) on the product grid, and the k+q coefficients stored
+    // in that order (Bp)
+    std::vector<int> gs_npad, gs_ncol, gs_nzl;
+    std::vector<long long> gs_perm_off, gs_col_off, gs_cst_off, gs_bp_off, gs_zl_off;
+    int gs_npad_max = 0, gs_ncol_max = 0;
+    long long gs_bp_total = 0;
+    DevBuf d_gs_perm, d_gs_kcx, d_gs_cols, d_gs_cst, d_gs_npw, d_gs_npad, d_gs_permoff, d_gs_bpoff, d_gs_bp;
+    DevBuf d_gs_shph;  // e^{-i G.delta} of copy 1 of an interleaved grid, per sphere point (sorted order)
+    DevBuf d_gs_zl, d_gs_cols2;  // z lines holding a column of the sphere; column index into the pruned plane
+    std::vector<DevBuf*> buffers()
+    {
+        return {&d_tw64[0], &d_tw64[1], &d_tw64[2], &d_tw32[0], &d_tw32[1], &d_tw32[2], &d_subtw64, &d_subtw32,
+                &d_psi64, &d_bsplit, &d_psi32, &d_win64, &d_win32, &d_winscale, &d_colmask, &d_collist, &d_colcnt,
+                &d_gs_perm, &d_gs_kcx, &d_gs_cols, &d_gs_cst, &d_gs_npw, &d_gs_npad, &d_gs_permoff, &d_gs_bpoff,
+                &d_gs_bp, &d_gs_shph, &d_gs_zl, &d_gs_cols2};
+    }
+};
+
+struct lelph_gpu : GridState
 {
     lelph_gpu_desc d;
     int device = 0;
@@ -62,13 +123,11 @@ struct lelph_gpu
     bool profiling = false;
     std::string err;
     lelph_gpu_stats stats;
-    GeomDev g;
     int nltimesj = 0, ntype = 0;
     int nproj_max = 0;
     int ab_bf16 = 0;
     unsigned long long wait_ns = 0;  // limit of each pipeline wait of the tensor-core sandwich (0: default)
     bool mixed = false;
-    bool prepared = false;
     bool gspace = false;  // G-space route of the local sandwich
     bool proj_tc = false;  // KB projections on the tensor cores (mixed form)
     // host copies
@@ -83,30 +142,24 @@ struct lelph_gpu
     // device buffers
     std::vector<DevBuf*> owned;
     DevBuf d_miller, d_pwoff, d_npw, d_coef, d_coefoff, d_gvec, d_fk, d_fkoff, d_ksym, d_chat, d_chatoff;
-    DevBuf d_psi64, d_boxes32, d_bsplit, d_psi32, d_band_scale, d_proj;
+    DevBuf d_boxes32, d_band_scale, d_proj;
     DevBuf d_atype, d_apos, d_pp, d_fsign, d_fcoef, d_fcoefoff;
-    DevBuf d_tw64[3], d_tw32[3], d_twN[3], d_twN32[3];
+    DevBuf d_twN[3], d_twN32[3];
     DevBuf d_dvr, d_eig, d_maxabs;                 // per q slot: dV_scf on the reference box (FP64), eigVec
-    DevBuf d_win64, d_win32, d_winscale, d_wtmpN, d_wtmpM;  // dV windows on the product grid, per (slot, umklapp)
+    DevBuf d_wtmpN, d_wtmpM;
     DevBuf d_pairs, d_glocal, d_partials, d_gout, d_status, d_tmp;
     std::vector<int> ulms_all;  // every q slot's umklapp list, the host side of one upload
-    FftPlan1D plan[3];   // product grid (g.Nx, g.Ny, g.Nz)
-    FftPlan1D planN[3];  // the reference's FFT box
     int Nbox[3] = {0, 0, 0};
     double Rc[3] = {0, 0, 0};  // largest |k+G| component (crystal units) over every rotated sphere
-    std::vector<int> win_base;  // first window entry of each q slot
-    int nwin = 0;
-    bool windows_ok = false;
-    CUtensorMap tmapB, tmapP, tmapV;
-    void* tmapV_base = nullptr;
-    int tmapV_rows = 0;
+    double Gc = 0;             // largest |k+G| (cartesian, no 2 pi)
+    int box_grid[3] = {0, 0, 0};  // plain product grid; the one in use (g) may be interleaved
+    bool ran = false;             // a run has picked the active grid
+    GridChoice choice[2];         // product grids: batch runs, one-call stage (GridState::which)
+    bool two_grids = false;
+    GridState other;              // the inactive one (two_grids)
     int nslots_alloc = 0;
-    int chunk_pts = 0, nchunks = 0;
     // local bare potential: V_loc(|G|) table and its spline slopes per species
     DevBuf d_vl_v, d_vl_dv, d_vl_in, d_vloc;
-    DevBuf d_colmask;  // box occupancy of every full-BZ k (z-columns of all k, then x planes of all k)
-    DevBuf d_collist, d_colcnt;  // occupied z-columns of every k as lists
-    bool boxmask_ready = false;  // occupancy and lists built (geometry only: they stay valid)
     // Dmats: Miller -> position tables of the iBZ lists, the job table and the
     // last block of representation matrices (jobs dm_first .. dm_first + dm_count - 1)
     DevBuf d_dmgtab, d_dmjobs, d_dmats, d_dmmap, d_dmcoef32, d_dmstar, d_gstar, d_qsitems;
@@ -125,18 +178,10 @@ struct lelph_gpu
     int vl_npts = 0, vl_dim2 = 0;
     double vl_dg = 0, vl_volume = 0;
     std::vector<double> vl_zval;
-    // G-space route: every full-BZ k's sphere (its k+q role) sorted by
-    // ((y, z) column, x) on the product grid, and the k+q coefficients stored
-    // in that order (Bp); psi(r) of one k at a time and the pass buffers
-    std::vector<int> gs_npad, gs_ncol, gs_nzl;
-    std::vector<long long> gs_perm_off, gs_col_off, gs_cst_off, gs_bp_off, gs_zl_off;
-    int gs_npad_max = 0, gs_ncol_max = 0;
-    long long gs_bp_total = 0;
-    DevBuf d_gs_perm, d_gs_kcx, d_gs_cols, d_gs_cst, d_gs_npw, d_gs_npad, d_gs_permoff, d_gs_bpoff, d_gs_bp;
+    // G-space route: psi(r) of one k at a time and the pass buffers
     DevBuf d_gs_psi, d_gs_out1, d_gs_A, d_gs_part;
     DevBuf d_gs_bq;      // mixed form on the tensor cores: the pair's k+q operand split into TF32 hi / lo
     bool gs_tc = false;  // mixed G-space GEMM on the tensor cores (gspace_tc.cu)
-    DevBuf d_gs_zl, d_gs_cols2;  // z lines holding a column of the sphere; column index into the pruned plane
 };
 
 namespace
@@ -673,10 +718,22 @@ extern "C" int lelph_gpu_stats_get(lelph_gpu* h, lelph_gpu_stats* s)
     size_t tot = 0;
     for (DevBuf* b : h->owned) tot += b->n;
     s->device_bytes = tot;
-    s->product_grid[0] = h->g.Nx;
-    s->product_grid[1] = h->g.Ny;
-    s->product_grid[2] = h->g.Nz;
+    for (int x = 0; x < 3; ++x) s->product_grid[x] = h->box_grid[x];
     s->chunk_points = h->chunk_pts;
+    s->box_columns = h->box_columns;
+    return LELPH_GPU_OK;
+}
+
+extern "C" int lelph_gpu_grid(lelph_gpu* h, int out[7])
+{
+    if (!h || !out) return LELPH_GPU_ERR_INVALID;
+    const GridChoice& c = h->choice[h->which];
+    for (int x = 0; x < 3; ++x)
+    {
+        out[x] = c.n[x];
+        out[4 + x] = c.sa[x];
+    }
+    out[3] = c.nsub;
     return LELPH_GPU_OK;
 }
 
@@ -741,7 +798,7 @@ static int upload_wfc(lelph_gpu* h, const double* const* wfc)
     int rc = upload(h, h->d_band_scale, h->band_scale.data(), sizeof(float) * h->band_scale.size());
     if (rc) return rc;
     CUDA_TRY(h, cudaStreamSynchronize(h->st));
-    h->prepared = false;
+    h->prepared = h->other.prepared = false;
     h->dm_coef32_ready = false;
     h->dm_coefT_ready = false;
     return LELPH_GPU_OK;
@@ -760,6 +817,7 @@ static int gs_tables(lelph_gpu* h)
     const GeomDev& g = h->g;
     const int nk = d.nkpts_BZ;
     std::vector<std::vector<int>> perm(nk), kcx(nk), cols(nk), cst(nk), zls(nk), cols2(nk);
+    std::vector<std::vector<double2>> shph(nk);
     std::vector<int> bad(nk, 0);
     auto one = [&](int k) {
         const KPointSym& ks = h->ksym[k];
@@ -800,6 +858,25 @@ static int gs_tables(lelph_gpu* h)
             kc[K] = (int)(cl.size() - 1) * g.Nx + x;
         }
         cs.push_back(npw);
+        if (g.nsub > 1)
+        {
+            // phase of copy 1 at each sphere point (K order)
+            shph[k].resize(npw);
+            for (int K = 0; K < npw; ++K)
+            {
+                const int* n = mil + 3 * pm[K];
+                const int N3[3] = {g.Nx, g.Ny, g.Nz};
+                double t = 0;
+                for (int r = 0; r < 3; ++r)
+                {
+                    const int G = ks.W[3 * r] * n[0] + ks.W[3 * r + 1] * n[1] + ks.W[3 * r + 2] * n[2];
+                    t += (double)(g.sa[r] * G) / (double)(g.nsub * N3[r]);
+                }
+                t -= std::rint(t);
+                const double ang = -6.283185307179586476925287 * t;
+                shph[k][K] = make_double2(std::cos(ang), std::sin(ang));
+            }
+        }
         // z lines of the sphere's columns, and each column's place in the
         // result of the y transform run on those lines only
         std::vector<int>& zl = zls[k];
@@ -866,6 +943,24 @@ static int gs_tables(lelph_gpu* h)
         std::copy(zls[k].begin(), zls[k].end(), zall.begin() + h->gs_zl_off[k]);
     }
     int rc;
+    if (g.nsub > 1)
+    {
+        // in the type of the pass that applies them
+        std::vector<double2> s64(po, make_double2(0, 0));
+        for (int k = 0; k < nk; ++k) std::copy(shph[k].begin(), shph[k].end(), s64.begin() + h->gs_perm_off[k]);
+        if (h->mixed)
+        {
+            std::vector<float2> s32(po);
+            for (long long i = 0; i < po; ++i) s32[i] = make_float2((float)s64[i].x, (float)s64[i].y);
+            if ((rc = upload(h, h->d_gs_shph, s32.data(), sizeof(float2) * po))) return rc;
+            CUDA_TRY(h, cudaStreamSynchronize(h->st));  // the vector is read until the copy is done
+        }
+        else
+        {
+            if ((rc = upload(h, h->d_gs_shph, s64.data(), sizeof(double2) * po))) return rc;
+            CUDA_TRY(h, cudaStreamSynchronize(h->st));
+        }
+    }
     if ((rc = upload(h, h->d_gs_perm, pall.data(), sizeof(int) * pall.size()))) return rc;
     if ((rc = upload(h, h->d_gs_kcx, kall.data(), sizeof(int) * kall.size()))) return rc;
     if ((rc = upload(h, h->d_gs_cols, call.data(), sizeof(int) * call.size()))) return rc;
@@ -877,6 +972,287 @@ static int gs_tables(lelph_gpu* h)
     if ((rc = upload(h, h->d_gs_permoff, h->gs_perm_off.data(), sizeof(long long) * nk))) return rc;
     if ((rc = upload(h, h->d_gs_bpoff, h->gs_bp_off.data(), sizeof(long long) * nk))) return rc;
     return LELPH_GPU_OK;
+}
+
+// K chunk of the tensor-core sandwich for M grid points and kp-point stages: a
+// multiple of the stage dividing M (so a chunk stays within one spinor
+// component), as large as possible up to 8192 points (each chunk's FP32 sum is
+// one term of the finish kernel).
+static long long tc_chunk_points(long long M, int kp)
+{
+    const long long units = M / kp;
+    long long best = 1;
+    for (long long c = 1; c <= units && c * kp <= 8192; ++c)
+        if (units % c == 0) best = c;
+    return best * kp;
+}
+
+static int upload_twiddles(lelph_gpu* h, int L, DevBuf& b64, DevBuf& b32)
+{
+    std::vector<double2> t64(L);
+    std::vector<float2> t32(L);
+    for (int t = 0; t < L; ++t)
+    {
+        const long double ang = 6.283185307179586476925286766559005768L * (long double)t / (long double)L;
+        t64[t] = make_double2((double)cosl(ang), (double)sinl(ang));
+        t32[t] = make_float2((float)cosl(ang), (float)sinl(ang));
+    }
+    int rc = upload(h, b64, t64.data(), sizeof(double2) * L);
+    if (!rc) rc = upload(h, b32, t32.data(), sizeof(float2) * L);
+    return rc;
+}
+
+// Bytes of the tensor-core sandwich's operands of every full-BZ k on N grid points.
+static void tc_operand_bytes(const lelph_gpu* h, long long N, size_t* bsplit, size_t* psi32)
+{
+    const lelph_gpu_desc& d = h->d;
+    const size_t Kr = 2 * (size_t)d.nspinor * N;
+    *bsplit = sizeof(uint16_t) * Kr * ((size_t)d.nkpts_BZ * d.nspin * 2 * 2 * h->g.nbp);
+    *psi32 = sizeof(float) * Kr * ((size_t)d.nkpts_BZ * d.nspin * h->g.nbp);
+}
+
+// The active grid's operand buffers and their tensor maps (mixed form,
+// real-space route).  Where the device has no room for a second grid's, the
+// inactive grid gives up its own and is prepared again when it is next used.
+static int grid_operands(lelph_gpu* h)
+{
+    const lelph_gpu_desc& d = h->d;
+    const GeomDev& g = h->g;
+    const long long N = lelph_grid_points(g);
+    size_t bb, pb;
+    tc_operand_bytes(h, N, &bb, &pb);
+    if (h->two_grids && !h->d_bsplit.p && !h->other.prepared)
+    {
+        // buffers that hold nothing yet (made at creation, large enough for either grid)
+        std::swap(h->d_bsplit, h->other.d_bsplit);
+        std::swap(h->d_psi32, h->other.d_psi32);
+        h->other.set_up = false;
+    }
+    int rc = ensure(h, h->d_bsplit, bb);
+    if (!rc) rc = ensure(h, h->d_psi32, pb);
+    if (rc && h->two_grids && h->other.d_bsplit.p)
+    {
+        for (DevBuf* b : {&h->d_bsplit, &h->d_psi32})
+        {
+            if (b->p) cudaFree(b->p);
+            *b = DevBuf();
+        }
+        std::swap(h->d_bsplit, h->other.d_bsplit);
+        std::swap(h->d_psi32, h->other.d_psi32);
+        h->other.prepared = false;
+        h->other.set_up = false;
+        rc = ensure(h, h->d_bsplit, bb);
+        if (!rc) rc = ensure(h, h->d_psi32, pb);
+    }
+    if (rc) return rc;
+    CUDA_TRY(h, cudaMemsetAsync(h->d_bsplit.p, 0, bb, h->st));
+    CUDA_TRY(h, cudaMemsetAsync(h->d_psi32.p, 0, pb, h->st));
+    const size_t Kr = 2 * (size_t)d.nspinor * N;
+    const size_t rows = (size_t)d.nkpts_BZ * d.nspin * 2 * 2 * g.nbp;
+    // split rows, tile-major: blocks (k, spin, hi|lo, 32-point K block) of 2*nbp rows x 64 halves
+    rc = make_tmap3(h, &h->tmapB, h->d_bsplit.p, false, 64, 2 * g.nbp, rows / (2 * g.nbp) * (Kr / 64), 2 * g.nbp, 1,
+                    true);
+    if (rc) return rc;
+    // FP32 psi(r) of the k role, tile-major: blocks (k, spin, 16-point block) of nbp rows x 32 floats,
+    // four blocks (one 64-point stage) per box, 128-byte swizzled
+    return make_tmap3(h, &h->tmapP, h->d_psi32.p, true, 32, g.nbp, (size_t)d.nkpts_BZ * d.nspin * (Kr / 32), g.nbp,
+                      (unsigned)(g.kpts / 16), true);
+}
+
+// Sets the active grid up from its choice: plans, twiddles, K chunks, operand
+// buffers or sphere tables.
+static int grid_setup(lelph_gpu* h)
+{
+    const GridChoice& c = h->choice[h->which];
+    GeomDev& g = h->g;
+    g.Nx = c.n[0];
+    g.Ny = c.n[1];
+    g.Nz = c.n[2];
+    g.nsub = c.nsub;
+    h->sphere_window = c.sphere;
+    h->tmapV_base = nullptr;
+    int rc;
+    for (int x = 0; x < 3; ++x)
+    {
+        g.sa[x] = c.sa[x];
+        if (!plan_1d(c.n[x], h->plan[x]) || !plan_1d(h->Nbox[x], h->planN[x]))
+            return fail(h, LELPH_GPU_ERR_UNSUPPORTED, "product grid");
+        h->plan[x].allct = h->planN[x].allct = c.sphere;
+        rc = upload_twiddles(h, c.n[x], h->d_tw64[x], h->d_tw32[x]);
+        if (rc) return rc;
+    }
+    if (g.nsub > 1)
+    {
+        // shifts of the copies: e^{+2 pi i t / (nsub N_i)}, the axes in sequence
+        std::vector<double2> t64;
+        std::vector<float2> t32;
+        for (int x = 0; x < 3; ++x)
+        {
+            const int L = g.nsub * c.n[x];
+            for (int t = 0; t < L; ++t)
+            {
+                const long double ang = 6.283185307179586476925286766559005768L * (long double)t / (long double)L;
+                t64.push_back(make_double2((double)cosl(ang), (double)sinl(ang)));
+                t32.push_back(make_float2((float)cosl(ang), (float)sinl(ang)));
+            }
+        }
+        rc = upload(h, h->d_subtw64, t64.data(), sizeof(double2) * t64.size());
+        if (!rc) rc = upload(h, h->d_subtw32, t32.data(), sizeof(float2) * t32.size());
+        if (rc) return rc;
+    }
+    if (h->gspace)
+    {
+        rc = gs_tables(h);
+        if (rc) return rc;
+    }
+    else if (h->mixed)
+    {
+        const long long N = lelph_grid_points(g);
+        if (N % g.kpts != 0) g.kpts = 32;
+        h->chunk_pts = (int)tc_chunk_points(N, g.kpts);
+        // tuning override: LELPH_TC_CHUNK = grid points per K chunk (multiple of the stage dividing N)
+        if (const char* e = getenv("LELPH_TC_CHUNK"))
+        {
+            long long k = atoll(e);
+            if (k > 0 && k % g.kpts == 0 && N % k == 0) h->chunk_pts = (int)k;
+        }
+        h->nchunks = (int)(h->d.nspinor * N / h->chunk_pts);
+        rc = grid_operands(h);
+        if (rc) return rc;
+    }
+    h->set_up = true;
+    return LELPH_GPU_OK;
+}
+
+// Makes grid `which` the active one.
+static int use_grid(lelph_gpu* h, int which)
+{
+    if (!h->two_grids) return LELPH_GPU_OK;
+    if (h->which != which) std::swap(static_cast<GridState&>(*h), h->other);
+    return h->set_up ? LELPH_GPU_OK : grid_setup(h);
+}
+
+// Metric of the reciprocal lattice (crystal units, no 2 pi): |v|^2 = v^T gm v,
+// gm packed (xx, yy, zz, xy, xz, yz).
+static void recip_metric(const lelph_gpu* h, double gm[6])
+{
+    const double* B = h->blat.data();
+    auto dot = [&](int i, int j) {
+        return (B[i] * B[j] + B[3 + i] * B[3 + j] + B[6 + i] * B[6 + j]) / (4 * PI_T * PI_T);
+    };
+    gm[0] = dot(0, 0);
+    gm[1] = dot(1, 1);
+    gm[2] = dot(2, 2);
+    gm[3] = dot(0, 1);
+    gm[4] = dot(0, 2);
+    gm[5] = dot(1, 2);
+}
+static double metric_norm2(const double gm[6], const double v[3])
+{
+    return gm[0] * v[0] * v[0] + gm[1] * v[1] * v[1] + gm[2] * v[2] * v[2] +
+           2 * (gm[3] * v[0] * v[1] + gm[4] * v[0] * v[2] + gm[5] * v[1] * v[2]);
+}
+
+// Smallest product grid that uses the spheres' shape.  Every difference D that
+// a pair needs satisfies |D + q| <= 2 Gc (D + q = S'(k'+G') - S(k+G)), a ball
+// rather than the box the plain grid covers, so a grid is exact as soon as no
+// two points of that ball coincide on it: as soon as every nonzero vector of
+// its reciprocal lattice is longer than 4 Gc (margin 1e-4: k_dv_window picks
+// the representative of each class in FP32).  Candidates are plain grids and
+// nsub interleaved copies of a smaller one (GeomDev), e.g. the body-centred
+// sampling of a cubic cell, whose reciprocal lattice is the densest packing of
+// balls: 2 x 24^3 points instead of 36^3 for the 4-atom cell at npw 2500, and
+// 3 x 10 x 10 x 96 instead of 24 x 24 x 120 for the hexagonal slab at npw 2600.
+// The work of the sandwich (and of the transforms and windows) is proportional
+// to the points.  Measured, plain grid -> this one: 4-atom cell, 8 q x 512 k,
+// mixed, 77.3 -> 47.5 ms a batch (sandwich 60 -> 35.6 ms); its FP64 form, 64
+// pairs, 314 -> 187 ms; slab, 4 q x 144 k, 16.8 -> 6.9 ms.  c holds the plain grid on entry and is replaced by any
+// cheaper one; the interleaved copies must hold every sphere without
+// overlap (n > ext), the tensor-core sandwich wants a multiple of 32 points (64
+// for its wider stages) and no more K chunks than before (its scratch).
+static void pick_grid(const lelph_gpu* h, const double gm[6], const int ext[3], bool gspace, GridChoice& c)
+{
+    const lelph_gpu_desc& d = h->d;
+    const bool tc = h->mixed && !gspace;
+    auto friendly = [](int n) {
+        for (int p : {2, 3, 5})
+            while (n % p == 0) n /= p;
+        return n == 1;
+    };
+    auto kp_of = [&](long long M) { return h->g.kpts == 64 && M % 64 == 0 ? 64 : 32; };
+    auto weight = [&](const GridChoice& g) {
+        const long long M = g.points();
+        double w = (double)M;
+        // 32-point stages of the sandwich cost about a tenth more; lengths without a
+        // compile-time transform only touch the preparation
+        if (tc && h->g.kpts == 64 && M % 64 != 0) w *= 1.1;
+        if (h->mixed)
+            for (int x = 0; x < 3; ++x)
+                if (!lelph_fft_fixed(g.n[x], g.sphere)) w *= gspace ? 1.1 : 1.02;
+        if (gspace)
+        {
+            GsGeom gg{g.n[0], g.n[1], g.n[2], g.nsub, d.nbnds, d.nspinor, d.nmag, 0, !h->mixed || g.sphere};
+            if (!lelph_gs_plane_fixed(gg, !h->mixed)) w *= 1.4;
+        }
+        return w;
+    };
+    const GridChoice plain = c;
+    c.cost = weight(c);
+    const long long nch_plain = tc ? plain.points() / tc_chunk_points(plain.points(), kp_of(plain.points())) : 0;
+    const double lim2 = 16.0 * h->Gc * h->Gc * (1.0 + 2e-4);
+    // |v_i| <= |v| |a_i| in crystal units bounds the short vectors' components
+    double alen[3];
+    std::vector<int> cand[3];
+    for (int r = 0; r < 3; ++r)
+    {
+        const double* A = h->alat.data();
+        alen[r] = std::sqrt(A[r] * A[r] + A[3 + r] * A[3 + r] + A[6 + r] * A[6 + r]);
+        for (int n = ext[r] + 1; n <= 4 * ext[r] + 8; ++n)
+            if (friendly(n)) cand[r].push_back(n);
+    }
+    auto exact = [&](const int* n, int p, const int* a) {
+        int mm[3];
+        for (int r = 0; r < 3; ++r) mm[r] = (int)std::floor(std::sqrt(lim2) * alen[r] / n[r] + 1e-6);
+        for (int x = 0; x <= mm[0]; ++x)
+            for (int y = (x == 0 ? 0 : -mm[1]); y <= mm[1]; ++y)
+                for (int z = (x == 0 && y == 0 ? 1 : -mm[2]); z <= mm[2]; ++z)
+                {
+                    if ((x * a[0] + y * a[1] + z * a[2]) % p != 0) continue;
+                    const double v[3] = {(double)x * n[0], (double)y * n[1], (double)z * n[2]};
+                    if (metric_norm2(gm, v) <= lim2) return false;
+                }
+        return true;
+    };
+    for (int p = 1; p <= LELPH_MAX_SUB; ++p)
+        for (int code = 0; code < p * p * p; ++code)
+        {
+            GridChoice t;
+            t.nsub = p;
+            t.sa[0] = code / (p * p);
+            t.sa[1] = code / p % p;
+            t.sa[2] = code % p;
+            t.sphere = true;
+            // a generator of order p; one code of each pair a, -a
+            const int first = t.sa[0] ? t.sa[0] : (t.sa[1] ? t.sa[1] : t.sa[2]);
+            if (p > 1 && (2 * first > p || (p == 4 && t.sa[0] % 2 == 0 && t.sa[1] % 2 == 0 && t.sa[2] % 2 == 0)))
+                continue;
+            if (p > 1 && first == 0) continue;
+            for (int a : cand[0])
+                for (int b : cand[1])
+                    for (int e : cand[2])
+                    {
+                        t.n[0] = a;
+                        t.n[1] = b;
+                        t.n[2] = e;
+                        const long long M = t.points();
+                        if ((double)M >= c.cost) break;  // ascending lengths: the rest cost more
+                        if (M >= plain.points() || (tc && M % (d.tile_points == 64 ? 64 : 32) != 0)) continue;
+                        t.cost = weight(t);
+                        if (t.cost >= c.cost || !exact(t.n, p, t.sa)) continue;
+                        if (tc && M / tc_chunk_points(M, kp_of(M)) > nch_plain) continue;
+                        c = t;
+                    }
+        }
 }
 
 extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
@@ -1027,6 +1403,8 @@ extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
     for (int i = 0; i < 9; ++i) B[i] = d.blat_vec[i] / (2 * PI_T);
     h->ksym.resize(d.nkpts_BZ);
     int ext[3] = {0, 0, 0};  // largest extent (max - min) of a rotated sphere on each axis
+    double gm[6], gc2 = 0;   // metric of the reciprocal lattice; largest |k+G|^2
+    recip_metric(h, gm);
     for (int i = 0; i < d.nkpts_BZ; ++i)
     {
         KPointSym& ks = h->ksym[i];
@@ -1088,13 +1466,16 @@ extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
         for (int g = 0; g < h->npw[ks.ik]; ++g)
         {
             const int* n = &h->miller[3 * (h->pw_off[ks.ik] + g)];
+            double u[3];
             for (int r = 0; r < 3; ++r)
             {
-                double u = (double)(ks.W[3 * r] * n[0] + ks.W[3 * r + 1] * n[1] + ks.W[3 * r + 2] * n[2]) + krot[r];
-                h->Rc[r] = std::max(h->Rc[r], std::fabs(u));
+                u[r] = (double)(ks.W[3 * r] * n[0] + ks.W[3 * r + 1] * n[1] + ks.W[3 * r + 2] * n[2]) + krot[r];
+                h->Rc[r] = std::max(h->Rc[r], std::fabs(u[r]));
             }
+            gc2 = std::max(gc2, metric_norm2(gm, u));
         }
     }
+    h->Gc = std::sqrt(gc2);
     for (int r = 0; r < 3; ++r)
         if (ext[r] >= d.fft_dims[r]) return bad(LELPH_GPU_ERR_GEOMETRY, "FFT box too small for the plane-wave sphere");
     // Product grid.  For a pair, D = G' - G1 (k+q sphere, shift G0 included,
@@ -1104,7 +1485,9 @@ extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
     // real-space sandwich with the dV window of each q (k_dv_window) gives the
     // reference's sum over G exactly.  Smallest 2^a 3^b 5^c sizes, never above
     // the reference's box (which is always exact); the mixed form also wants
-    // a multiple of 32 points.
+    // a multiple of 32 points.  pick_grid then looks for a smaller grid that
+    // uses the spheres' shape.
+    bool keep_plain = false;
     {
         auto friendly = [](int n) {
             for (int p : {2, 3, 5})
@@ -1134,15 +1517,27 @@ extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
                         bm[2] = c;
                     }
                 }
+        bool plain = false;  // keep the plain grid (tests)
         if (const char* e = getenv("LELPH_FULL_BOX"))
-            if (atoi(e) != 0) bm[0] = d.fft_dims[0], bm[1] = d.fft_dims[1], bm[2] = d.fft_dims[2];
-        h->g.Nx = bm[0];
-        h->g.Ny = bm[1];
-        h->g.Nz = bm[2];
+            if (atoi(e) != 0) bm[0] = d.fft_dims[0], bm[1] = d.fft_dims[1], bm[2] = d.fft_dims[2], plain = true;
+        if (const char* e = getenv("LELPH_PLAIN_GRID"))
+            if (atoi(e) != 0) plain = true;
         for (int r = 0; r < 3; ++r)
+        {
+            h->box_grid[r] = bm[r];
             if (!plan_1d(bm[r], h->plan[r])) return bad(LELPH_GPU_ERR_UNSUPPORTED, "product grid");
+        }
+        if (h->gspace)
+        {
+            GsGeom gg{bm[0], bm[1], bm[2], 1, d.nbnds, d.nspinor, d.nmag, 0, 0};
+            if (lelph_gs_plane_smem(gg, !h->mixed) > 220 * 1024 || lelph_gs_xpass_smem(gg, !h->mixed) > 220 * 1024)
+                return bad(LELPH_GPU_ERR_UNSUPPORTED, "G-space route: a (y, z) plane of the product grid exceeds shared memory");
+        }
+        else if (h->mixed && ((long long)bm[0] * bm[1] * bm[2]) % 32 != 0)
+            return bad(LELPH_GPU_ERR_UNSUPPORTED, "grid size must be a multiple of 32");
+        keep_plain = plain;
     }
-    const long long N = (long long)h->g.Nx * h->g.Ny * h->g.Nz;
+    const long long N = (long long)h->box_grid[0] * h->box_grid[1] * h->box_grid[2];
     if (d.route == LELPH_GPU_ROUTE_AUTO && !h->gspace)
     {
         // the real-space route keeps psi(r) of every full-BZ k resident (split
@@ -1179,13 +1574,12 @@ extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
     }
     if (h->gspace)
     {
-        GsGeom gg{h->g.Nx, h->g.Ny, h->g.Nz, d.nbnds, d.nspinor, d.nmag, 0};
+        GsGeom gg{h->box_grid[0], h->box_grid[1], h->box_grid[2], 1, d.nbnds, d.nspinor, d.nmag, 0, 0};
         if (lelph_gs_plane_smem(gg, !h->mixed) > 220 * 1024 || lelph_gs_xpass_smem(gg, !h->mixed) > 220 * 1024)
             return bad(LELPH_GPU_ERR_UNSUPPORTED, "G-space route: a (y, z) plane of the product grid exceeds shared memory");
     }
     if (h->mixed && !h->gspace)
     {
-        if (N % 32 != 0) return bad(LELPH_GPU_ERR_UNSUPPORTED, "grid size must be a multiple of 32");
         if (N % h->g.kpts != 0) h->g.kpts = 32;
         // the descriptor's stage size (a tuned choice), or LELPH_TC_STAGE = 32 (tests)
         if (d.tile_points == 32) h->g.kpts = 32;
@@ -1196,6 +1590,16 @@ extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
         if (const char* e = getenv("LELPH_TC_STAGE"))
             if (atoi(e) == 32) h->g.kpts = 32;
         if (lelph_local_tc_smem_bytes(h->g) > 227 * 1024) return bad(LELPH_GPU_ERR_UNSUPPORTED, "shared memory");
+    }
+    // product grids (the plain one has passed every check above)
+    {
+        GridChoice& c = h->choice[0];
+        for (int r = 0; r < 3; ++r) c.n[r] = h->box_grid[r];
+        h->choice[1] = c;
+        if (!keep_plain) pick_grid(h, gm, ext, h->gspace, c);
+        h->two_grids = h->mixed && c.sphere;
+        h->other.which = 1;
+        h->other.g = h->g;
     }
     // chat offsets per full-BZ k
     h->chat_off.resize(d.nkpts_BZ);
@@ -1218,21 +1622,17 @@ extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
     cudaEventCreate(&h->evg0);
     cudaEventCreate(&h->evg1);
     DevBuf* bufs[] = {&h->d_miller, &h->d_pwoff, &h->d_npw, &h->d_coef, &h->d_coefoff, &h->d_gvec, &h->d_fk,
-                      &h->d_fkoff, &h->d_ksym, &h->d_chat, &h->d_chatoff, &h->d_psi64, &h->d_boxes32, &h->d_bsplit,
-                      &h->d_psi32, &h->d_band_scale, &h->d_proj, &h->d_atype, &h->d_apos, &h->d_pp, &h->d_fsign, &h->d_fcoef,
-                      &h->d_fcoefoff, &h->d_tw64[0], &h->d_tw64[1], &h->d_tw64[2], &h->d_tw32[0], &h->d_tw32[1],
-                      &h->d_tw32[2], &h->d_twN[0], &h->d_twN[1], &h->d_twN[2], &h->d_twN32[0], &h->d_twN32[1],
-                      &h->d_twN32[2], &h->d_dvr, &h->d_eig,
-                      &h->d_maxabs, &h->d_win64, &h->d_win32, &h->d_winscale, &h->d_wtmpN, &h->d_wtmpM,
-                      &h->d_pairs, &h->d_glocal, &h->d_partials, &h->d_gout, &h->d_status, &h->d_tmp,
-                      &h->d_vl_v, &h->d_vl_dv, &h->d_vl_in, &h->d_vloc, &h->d_colmask, &h->d_collist, &h->d_colcnt,
-                      &h->d_dmgtab,
-                      &h->d_dmjobs, &h->d_dmats, &h->d_dmmap, &h->d_dmcoef32, &h->d_dmstar, &h->d_gstar,
-                      &h->d_dmgroups, &h->d_dmperm, &h->d_dmcoefT,
-                      &h->d_qsitems, &h->d_dvraw, &h->d_gs_perm, &h->d_gs_kcx, &h->d_gs_cols, &h->d_gs_cst,
-                      &h->d_gs_npw, &h->d_gs_npad, &h->d_gs_permoff, &h->d_gs_bpoff, &h->d_gs_bp, &h->d_gs_psi,
-                      &h->d_gs_out1, &h->d_gs_A, &h->d_gs_part, &h->d_gs_zl, &h->d_gs_cols2, &h->d_gs_bq};
+                      &h->d_fkoff, &h->d_ksym, &h->d_chat, &h->d_chatoff, &h->d_boxes32, &h->d_band_scale,
+                      &h->d_proj, &h->d_atype, &h->d_apos, &h->d_pp, &h->d_fsign, &h->d_fcoef, &h->d_fcoefoff,
+                      &h->d_twN[0], &h->d_twN[1], &h->d_twN[2], &h->d_twN32[0], &h->d_twN32[1], &h->d_twN32[2],
+                      &h->d_dvr, &h->d_eig, &h->d_maxabs, &h->d_wtmpN, &h->d_wtmpM, &h->d_pairs, &h->d_glocal,
+                      &h->d_partials, &h->d_gout, &h->d_status, &h->d_tmp, &h->d_vl_v, &h->d_vl_dv, &h->d_vl_in,
+                      &h->d_vloc, &h->d_dmgtab, &h->d_dmjobs, &h->d_dmats, &h->d_dmmap, &h->d_dmcoef32, &h->d_dmstar,
+                      &h->d_gstar, &h->d_dmgroups, &h->d_dmperm, &h->d_dmcoefT, &h->d_qsitems, &h->d_dvraw,
+                      &h->d_gs_psi, &h->d_gs_out1, &h->d_gs_A, &h->d_gs_part, &h->d_gs_bq};
     for (DevBuf* b : bufs) h->owned.push_back(b);
+    for (DevBuf* b : h->buffers()) h->owned.push_back(b);
+    for (DevBuf* b : h->other.buffers()) h->owned.push_back(b);
     int rc = 0;
 #define UP(buf, ptr, bytes)                              \
     do                                                   \
@@ -1275,28 +1675,11 @@ extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
         if (pack.size() == 2) h->d_fcoef.n = 16;  // marks "no coefficients"
         UP(h->d_fcoefoff, off.data(), sizeof(int) * off.size());
     }
-    // twiddles e^{+2 pi i t / L}: product grid and reference box, FP64 and FP32
-    for (int x = 0; x < 6; ++x)
+    // twiddles e^{+2 pi i t / L} of the reference box, FP64 and FP32
+    for (int x = 0; x < 3; ++x)
     {
-        int L = x < 3 ? (x == 0 ? h->g.Nx : (x == 1 ? h->g.Ny : h->g.Nz)) : d.fft_dims[x - 3];
-        std::vector<double2> t64(L);
-        std::vector<float2> t32(L);
-        for (int t = 0; t < L; ++t)
-        {
-            long double ang = 6.283185307179586476925286766559005768L * (long double)t / (long double)L;
-            t64[t] = make_double2((double)cosl(ang), (double)sinl(ang));
-            t32[t] = make_float2((float)cosl(ang), (float)sinl(ang));
-        }
-        if (x < 3)
-        {
-            UP(h->d_tw64[x], t64.data(), sizeof(double2) * L);
-            UP(h->d_tw32[x], t32.data(), sizeof(float2) * L);
-        }
-        else
-        {
-            UP(h->d_twN[x - 3], t64.data(), sizeof(double2) * L);
-            UP(h->d_twN32[x - 3], t32.data(), sizeof(float2) * L);
-        }
+        rc = upload_twiddles(h, d.fft_dims[x], h->d_twN[x], h->d_twN32[x]);
+        if (rc) return bad(rc, h->err);
     }
     rc = ensure(h, h->d_coef, sizeof(double2) * (size_t)ctot);
     if (rc) return bad(rc, h->err);
@@ -1308,48 +1691,19 @@ extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
     rc = ensure(h, h->d_status, 64);
     if (rc) return bad(rc, h->err);
     if (cudaMemsetAsync(h->d_status.p, 0, 64, h->st) != cudaSuccess) return bad(LELPH_GPU_ERR_CUDA, "memset");
-    if (h->gspace)
-    {
-        rc = gs_tables(h);
-        if (rc) return bad(rc, h->err);
-    }
     if (h->mixed && !h->gspace)
     {
-        const size_t Kr = 2 * (size_t)d.nspinor * N;
-        const size_t rows = (size_t)d.nkpts_BZ * d.nspin * 2 * 2 * h->g.nbp;
-        rc = ensure(h, h->d_bsplit, sizeof(uint16_t) * Kr * rows);
+        // the operands of the plain grid, which holds those of any smaller one
+        size_t bb, pb;
+        tc_operand_bytes(h, N, &bb, &pb);
+        rc = ensure(h, h->d_bsplit, bb);
+        if (!rc) rc = ensure(h, h->d_psi32, pb);
         if (rc) return bad(rc, h->err);
-        if (cudaMemsetAsync(h->d_bsplit.p, 0, h->d_bsplit.n, h->st) != cudaSuccess) return bad(LELPH_GPU_ERR_CUDA, "memset");
-        // split rows, tile-major: blocks (k, spin, hi|lo, 32-point K block) of 2*nbp rows x 64 halves
-        rc = make_tmap3(h, &h->tmapB, h->d_bsplit.p, false, 64, 2 * h->g.nbp, rows / (2 * h->g.nbp) * (Kr / 64),
-                        2 * h->g.nbp, 1, true);
+    }
+    if (!h->two_grids)  // else the first preparation or run sets up the grid that it uses
+    {
+        rc = grid_setup(h);
         if (rc) return bad(rc, h->err);
-        // FP32 psi(r) of the k role, tile-major: blocks (k, spin, 16-point block) of nbp rows x 32 floats,
-        // four blocks (one 64-point stage) per box, 128-byte swizzled
-        const size_t prow = (size_t)d.nkpts_BZ * d.nspin * h->g.nbp;
-        rc = ensure(h, h->d_psi32, sizeof(float) * Kr * prow);
-        if (rc) return bad(rc, h->err);
-        if (cudaMemsetAsync(h->d_psi32.p, 0, h->d_psi32.n, h->st) != cudaSuccess) return bad(LELPH_GPU_ERR_CUDA, "memset");
-        rc = make_tmap3(h, &h->tmapP, h->d_psi32.p, true, 32, h->g.nbp, (size_t)d.nkpts_BZ * d.nspin * (Kr / 32),
-                        h->g.nbp, (unsigned)(h->g.kpts / 16), true);
-        if (rc) return bad(rc, h->err);
-        // K chunk per work unit: a multiple of the stage dividing N (so a chunk stays
-        // within one spinor component), as large as possible up to 8192 points: each
-        // chunk's FP32 sum is one FP64 term of the finish kernel
-        const int kp = h->g.kpts;
-        long long Ktot = (long long)d.nspinor * N;
-        long long units = N / kp;
-        long long best = 1;
-        for (long long c = 1; c <= units; ++c)
-            if (units % c == 0 && c * kp <= 8192) best = c;
-        h->chunk_pts = (int)(best * kp);
-        // tuning override: LELPH_TC_CHUNK = grid points per K chunk (multiple of the stage dividing N)
-        if (const char* e = getenv("LELPH_TC_CHUNK"))
-        {
-            long long c = atoll(e);
-            if (c > 0 && c % kp == 0 && N % c == 0) h->chunk_pts = (int)c;
-        }
-        h->nchunks = (int)(Ktot / h->chunk_pts);
     }
     rc = upload_wfc(h, d.wfc);
     if (rc) return bad(rc, h->err);
@@ -1369,14 +1723,16 @@ extern "C" int lelph_gpu_set_wavefunctions(lelph_gpu* h, const double* const* wf
 
 static int build_windows(lelph_gpu* h);
 
-extern "C" int lelph_gpu_prepare(lelph_gpu* h)
+// The q-independent stage on the active grid.
+static int prepare_grid(lelph_gpu* h)
 {
-    if (!h) return LELPH_GPU_ERR_INVALID;
-    CUDA_TRY(h, cudaSetDevice(h->device));
     const lelph_gpu_desc& d = h->d;
     const GeomDev& g = h->g;
-    const long long N = (long long)g.Nx * g.Ny * g.Nz;
-    const int nbox_per_k = d.nspin * d.nbnds * d.nspinor;
+    // boxes: one copy of the (interleaved) product grid each, nsub per (spin, band, spinor)
+    const long long N = lelph_sub_points(g);
+    const int nset_per_k = d.nspin * d.nbnds * d.nspinor;
+    const int nbox_per_k = nset_per_k * g.nsub;
+    const double2* sub_tw = (const double2*)h->d_subtw64.p;
     const int npw_max = *std::max_element(h->npw.begin(), h->npw.end());
     tstart(h);
     int rc;
@@ -1392,14 +1748,14 @@ extern "C" int lelph_gpu_prepare(lelph_gpu* h)
         lelph_launch_scatter(0, d.nkpts_BZ, (const KPointSym*)h->d_ksym.p, (const int*)h->d_miller.p,
                              (const long long*)h->d_pwoff.p, (const int*)h->d_npw.p, npw_max,
                              (const double2*)h->d_coef.p, (const long long*)h->d_coefoff.p, g, !h->mixed, nullptr,
-                             (double2*)h->d_chat.p, (const long long*)h->d_chatoff.p, h->st);
+                             (double2*)h->d_chat.p, (const long long*)h->d_chatoff.p, sub_tw, h->st);
         const size_t e = h->mixed ? sizeof(float2) : sizeof(double2);
         rc = ensure(h, h->d_gs_bp, e * (size_t)h->gs_bp_total);
         if (rc) return rc;
         if (lelph_launch_gs_bperm(!h->mixed, (const double2*)h->d_chat.p, (const long long*)h->d_chatoff.p,
                                   (const int*)h->d_gs_npw.p, (const int*)h->d_gs_npad.p,
                                   (const long long*)h->d_gs_permoff.p, (const int*)h->d_gs_perm.p,
-                                  (const long long*)h->d_gs_bpoff.p, 0, d.nkpts_BZ, nbox_per_k, h->gs_npad_max,
+                                  (const long long*)h->d_gs_bpoff.p, 0, d.nkpts_BZ, nset_per_k, h->gs_npad_max,
                                   h->d_gs_bp.p, h->st))
             return fail(h, LELPH_GPU_ERR_UNSUPPORTED, "G-space route: coefficient permutation grid");
         h->stats.kernel_launches += 2;
@@ -1413,7 +1769,7 @@ extern "C" int lelph_gpu_prepare(lelph_gpu* h)
         lelph_launch_scatter(0, d.nkpts_BZ, (const KPointSym*)h->d_ksym.p, (const int*)h->d_miller.p,
                              (const long long*)h->d_pwoff.p, (const int*)h->d_npw.p, npw_max,
                              (const double2*)h->d_coef.p, (const long long*)h->d_coefoff.p, g, 1, h->d_psi64.p, (double2*)h->d_chat.p,
-                             (const long long*)h->d_chatoff.p, h->st);
+                             (const long long*)h->d_chatoff.p, sub_tw, h->st);
         const long long nbox = (long long)d.nkpts_BZ * nbox_per_k;
         double2* psi = (double2*)h->d_psi64.p;
         lelph_launch_fft_contig_d(psi, nbox * g.Nx * g.Ny, h->plan[2], (const double2*)h->d_tw64[2].p, +1, h->st);
@@ -1464,7 +1820,7 @@ extern "C" int lelph_gpu_prepare(lelph_gpu* h)
             lelph_launch_scatter(k0, nk, (const KPointSym*)h->d_ksym.p, (const int*)h->d_miller.p,
                                  (const long long*)h->d_pwoff.p, (const int*)h->d_npw.p, npw_max,
                                  (const double2*)h->d_coef.p, (const long long*)h->d_coefoff.p, g, 0, h->d_boxes32.p,
-                                 (double2*)h->d_chat.p, (const long long*)h->d_chatoff.p, h->st, mk,
+                                 (double2*)h->d_chat.p, (const long long*)h->d_chatoff.p, sub_tw, h->st, mk,
                                  proj_tc ? (float2*)h->d_chat.p : nullptr);
             h->stats.prep_scatter_ms += gs_tock(h);
             const long long nbox = (long long)nk * nbox_per_k;
@@ -1490,8 +1846,8 @@ extern "C" int lelph_gpu_prepare(lelph_gpu* h)
             CUDA_TRY(h, cudaMemcpyAsync(cnt.data(), h->d_colcnt.p, sizeof(int) * cnt.size(), cudaMemcpyDeviceToHost,
                                         h->st));
             CUDA_TRY(h, cudaStreamSynchronize(h->st));
-            h->stats.box_columns = 0;
-            for (int c : cnt) h->stats.box_columns += c;
+            h->box_columns = 0;
+            for (int c : cnt) h->box_columns += c;
             h->boxmask_ready = true;
             h->stats.kernel_launches += 1;
         }
@@ -1534,42 +1890,207 @@ extern "C" int lelph_gpu_prepare(lelph_gpu* h)
     return LELPH_GPU_OK;
 }
 
+extern "C" int lelph_gpu_prepare(lelph_gpu* h)
+{
+    if (!h) return LELPH_GPU_ERR_INVALID;
+    CUDA_TRY(h, cudaSetDevice(h->device));
+    // the grid that the runs so far used; before the first one, that of the batch
+    // runs when q slots are loaded for them, else that of the one-call stage
+    // (which loads its own slot)
+    if (!h->ran)
+    {
+        bool slots = false;
+        for (const QSlot& q : h->qslots) slots = slots || q.set;
+        const int rc = use_grid(h, slots ? 0 : 1);
+        if (rc) return rc;
+    }
+    else if (!h->set_up)
+    {
+        const int rc = grid_setup(h);
+        if (rc) return rc;
+    }
+    return prepare_grid(h);
+}
+
+// Geometry of the dV windows of one q.
+struct WinGeom
+{
+    int N[3];         // the reference's FFT box
+    int n[3], sa[3];  // one copy of the product grid, shifts (GeomDev)
+    int dmin[3], dmax[3];  // every needed difference D lies in [dmin, dmax]
+    int sphere;
+    float q[3], gm[6], cut2;  // |D + q|^2 <= cut2 for the needed differences
+};
+
 // dV on the product grid for one (q slot, umklapp G0): with dVhat the
 // normalised forward transform of dV on the reference box,
-//   dV_G0(r') = sum_d dVhat(d + G0) e^{i d.r'},  d over one period of the product grid
-// (signed representatives), so that (1/M) sum_r' dV_G0 psi_k conj(psi_kq) equals
-// the reference's sum_{G1,G'} c_k(G1) conj(c_kq(G')) dVhat(G' - G1) exactly.
-template <typename T2>
-__global__ void k_dv_window(const T2* __restrict__ dvhat, int ncomp, int Nx, int Ny, int Nz,
-                            const int* __restrict__ ulms, int nu, int3 dmin, GeomDev g, double invN,
-                            T2* __restrict__ out)
+//   dV_G0(r') = sum_d dVhat(d + G0) e^{i d.r'},  one d per class of the grid's reciprocal lattice,
+// so that (1/M) sum_r' dV_G0 psi_k conj(psi_kq) equals the reference's
+// sum_{G1,G'} c_k(G1) conj(c_kq(G')) dVhat(G' - G1) exactly, provided that every
+// needed difference D = d + G0 is the representative of its class.
+// * box rule (wg.sphere = 0, one copy): the signed representative in
+//   [dmin - G0, dmin - G0 + n) per axis;
+// * sphere rule: a residue t of one copy holds nsub classes, d = t + (m_i n_i)
+//   with sum sa_i m_i = c mod nsub; of each, the D nearest to -q (the needed ones
+//   lie within 2 Gc of it and every other member of the class beyond, see
+//   pick_grid), and nothing where that lies outside.  Copy j of the grid
+//   receives sum_c dVhat(D_c) e^{i d_c.delta_j}.
+// One thread per residue finds the representatives once and applies them to
+// its share of the components (grid y).  The inverse transform per copy follows.
+template <typename T2, int P>
+__global__ void __launch_bounds__(256) k_dv_window(const T2* __restrict__ dvhat, int ncomp, WinGeom wg,
+                                                   const int* __restrict__ ulms, const T2* __restrict__ sub_tw,
+                                                   double invN, T2* __restrict__ out)
 {
-    const long long M = (long long)g.Nx * g.Ny * g.Nz;
-    const int c = blockIdx.y;   // (mode, component)
-    const int u = blockIdx.z;   // umklapp index
-    const int ux = ulms[3 * u], uy = ulms[3 * u + 1], uz = ulms[3 * u + 2];
-    const T2* src = dvhat + (size_t)c * ((size_t)Nx * Ny * Nz);
-    T2* dst = out + ((size_t)u * ncomp + c) * M;
-    // grid residue x stands for the difference D' = G'' - G1 in [dmin - G0, dmin - G0 + M); value dVhat(D' + G0)
-    const int lx = dmin.x - ux, ly = dmin.y - uy, lz = dmin.z - uz;
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < M; r += (long long)gridDim.x * blockDim.x)
+    const int Ns = wg.n[0] * wg.n[1] * wg.n[2];
+    const size_t NN = (size_t)wg.N[0] * wg.N[1] * wg.N[2];
+    const int u = blockIdx.z;  // umklapp index
+    const int um[3] = {ulms[3 * u], ulms[3 * u + 1], ulms[3 * u + 2]};
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < Ns; r += gridDim.x * blockDim.x)
     {
-        int x = (int)(r / ((long long)g.Ny * g.Nz));
-        int rem = (int)(r - (long long)x * g.Ny * g.Nz);
-        int y = rem / g.Nz, z = rem - (rem / g.Nz) * g.Nz;
-        int dx = lx + (((x - lx) % g.Nx) + g.Nx) % g.Nx;
-        int dy = ly + (((y - ly) % g.Ny) + g.Ny) % g.Ny;
-        int dz = lz + (((z - lz) % g.Nz) + g.Nz) % g.Nz;
-        int ix = ((dx + ux) % Nx + Nx) % Nx;
-        int iy = ((dy + uy) % Ny + Ny) % Ny;
-        int iz = ((dz + uz) % Nz + Nz) % Nz;
-        const T2 v = src[((size_t)ix * Ny + iy) * Nz + iz];
-        const decltype(v.x) s = (decltype(v.x))invN;  // the operand type's 1/N
-        dst[r] = mk2<T2>(v.x * s, v.y * s);
+        int t[3];
+        t[0] = r / (wg.n[1] * wg.n[2]);
+        const int rem = r - t[0] * (wg.n[1] * wg.n[2]);
+        t[1] = rem / wg.n[2];
+        t[2] = rem - t[1] * wg.n[2];
+        // first D >= dmin of the residue on each axis (d = D - G0), and its m
+        int D0[3], m0[3];
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+        {
+            const int lo = wg.dmin[x] - um[x];
+            int e = (t[x] - lo) % wg.n[x];
+            if (e < 0) e += wg.n[x];
+            D0[x] = lo + e + um[x];
+            m0[x] = (lo + e - t[x]) / wg.n[x];  // exact
+        }
+        int src[P];
+        T2 ph[P];
+#pragma unroll
+        for (int c = 0; c < P; ++c)
+        {
+            int D[3] = {D0[0], D0[1], D0[2]};
+            bool any = true;
+            if (wg.sphere)
+            {
+                float best = wg.cut2;
+                any = false;
+                for (int Dx = D0[0], mx = m0[0]; Dx <= wg.dmax[0]; Dx += wg.n[0], ++mx)
+                    for (int Dy = D0[1], my = m0[1]; Dy <= wg.dmax[1]; Dy += wg.n[1], ++my)
+                        for (int Dz = D0[2], mz = m0[2]; Dz <= wg.dmax[2]; Dz += wg.n[2], ++mz)
+                        {
+                            if (P > 1)
+                            {
+                                int cl = (wg.sa[0] * mx + wg.sa[1] * my + wg.sa[2] * mz) % P;
+                                if (cl < 0) cl += P;
+                                if (cl != c) continue;
+                            }
+                            const float vx = Dx + wg.q[0], vy = Dy + wg.q[1], vz = Dz + wg.q[2];
+                            const float s = wg.gm[0] * vx * vx + wg.gm[1] * vy * vy + wg.gm[2] * vz * vz +
+                                            2.f * (wg.gm[3] * vx * vy + wg.gm[4] * vx * vz + wg.gm[5] * vy * vz);
+                            if (s <= best)
+                            {
+                                best = s;
+                                any = true;
+                                D[0] = Dx;
+                                D[1] = Dy;
+                                D[2] = Dz;
+                            }
+                        }
+            }
+            src[c] = -1;
+            ph[c] = mk2<T2>(1.0, 0.0);
+            if (any)
+            {
+                int i3[3];
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+                {
+                    i3[x] = D[x] % wg.N[x];
+                    if (i3[x] < 0) i3[x] += wg.N[x];
+                }
+                src[c] = (i3[0] * wg.N[1] + i3[1]) * wg.N[2] + i3[2];
+                if (P > 1)
+                {
+                    const T2* tw = sub_tw;
+#pragma unroll
+                    for (int x = 0; x < 3; ++x)
+                    {
+                        const int L = P * wg.n[x];
+                        int e = wg.sa[x] * (D[x] - um[x]) % L;
+                        if (e < 0) e += L;
+                        ph[c] = cmul(ph[c], tw[e]);
+                        tw += L;
+                    }
+                }
+            }
+        }
+        for (int c = blockIdx.y; c < ncomp; c += gridDim.y)
+        {
+            const T2* s = dvhat + (size_t)c * NN;
+            T2* dst = out + ((size_t)u * ncomp + c) * P * Ns + r;
+            T2 v[P];
+#pragma unroll
+            for (int l = 0; l < P; ++l)
+            {
+                v[l] = mk2<T2>(0.0, 0.0);
+                if (src[l] >= 0)
+                {
+                    const T2 w = s[src[l]];
+                    const decltype(w.x) sc = (decltype(w.x))invN;  // the operand type's 1/N
+                    v[l] = mk2<T2>(w.x * sc, w.y * sc);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < P; ++j)
+            {
+                T2 a = v[0];
+#pragma unroll
+                for (int l = 1; l < P; ++l) a = cadd(a, v[l]);
+                dst[(size_t)j * Ns] = a;
+                if (j + 1 < P)
+                {
+#pragma unroll
+                    for (int l = 0; l < P; ++l) v[l] = cmul(v[l], ph[l]);
+                }
+            }
+        }
     }
 }
 
+template <typename T2>
+static void launch_dv_window(const T2* dvhat, int ncomp, const WinGeom& wg, int nsub, const int* ulms, int nu,
+                             const T2* sub_tw, double invN, T2* out, cudaStream_t st)
+{
+    const dim3 grid(64, (unsigned)((ncomp + 3) / 4), (unsigned)nu);
+    if (nsub == 1) k_dv_window<T2, 1><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, ulms, sub_tw, invN, out);
+    else if (nsub == 2) k_dv_window<T2, 2><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, ulms, sub_tw, invN, out);
+    else if (nsub == 3) k_dv_window<T2, 3><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, ulms, sub_tw, invN, out);
+    else k_dv_window<T2, 4><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, ulms, sub_tw, invN, out);
+}
+
 // Load q slot `slot`: eigVec and dV (host); dVscf == nullptr loads zeros.
+static WinGeom win_geom(const lelph_gpu* h, const QSlot& q)
+{
+    WinGeom wg{};
+    double gm[6];
+    recip_metric(h, gm);
+    const int n[3] = {h->g.Nx, h->g.Ny, h->g.Nz};
+    for (int x = 0; x < 3; ++x)
+    {
+        wg.N[x] = h->Nbox[x];
+        wg.n[x] = n[x];
+        wg.sa[x] = h->g.sa[x];
+        wg.dmin[x] = q.dmin[x];
+        wg.dmax[x] = (int)std::ceil(-q.q[x] + 2.0 * h->Rc[x] + 1e-9);
+        wg.q[x] = (float)q.q[x];
+    }
+    for (int i = 0; i < 6; ++i) wg.gm[i] = (float)gm[i];
+    wg.sphere = h->sphere_window;
+    wg.cut2 = (float)(4.0 * h->Gc * h->Gc * (1.0 + 1e-4));
+    return wg;
+}
+
 static int set_q_common(lelph_gpu* h, int slot, const double qpt_crys[3], const double* eigVec,
                         const double* dVscf)
 {
@@ -1631,7 +2152,7 @@ static int set_q_common(lelph_gpu* h, int slot, const double qpt_crys[3], const 
         CUDA_TRY(h, cudaMemsetAsync((double2*)h->d_dvr.p + (size_t)slot * dvn, 0, sizeof(double2) * dvn, h->st));
     CUDA_TRY(h, cudaStreamSynchronize(h->st));
     q.set = true;
-    h->windows_ok = false;
+    h->windows_ok = h->other.windows_ok = false;
     return LELPH_GPU_OK;
 }
 
@@ -1941,7 +2462,7 @@ extern "C" int lelph_gpu_set_q_induced(lelph_gpu* h, int slot, const double qpt_
     h->stats.kernel_launches += 1;
     CUDA_TRY(h, cudaGetLastError());
     CUDA_TRY(h, cudaStreamSynchronize(h->st));
-    h->windows_ok = false;
+    h->windows_ok = h->other.windows_ok = false;
     return LELPH_GPU_OK;
 }
 
@@ -1991,7 +2512,7 @@ extern "C" int lelph_gpu_set_q_dvscf_qe(lelph_gpu* h, int slot, const double qpt
         CUDA_TRY(h, cudaGetLastError());
     }
     CUDA_TRY(h, cudaStreamSynchronize(h->st));
-    h->windows_ok = false;
+    h->windows_ok = h->other.windows_ok = false;
     return LELPH_GPU_OK;
 }
 
@@ -2002,7 +2523,8 @@ static int build_windows(lelph_gpu* h)
     const lelph_gpu_desc& d = h->d;
     const GeomDev& g = h->g;
     const long long NN = (long long)h->Nbox[0] * h->Nbox[1] * h->Nbox[2];
-    const long long M = (long long)g.Nx * g.Ny * g.Nz;
+    const long long M = lelph_grid_points(g);
+    const int P = g.nsub;
     const int ncomp = d.nmodes * d.nmag;
     h->win_base.assign(h->qslots.size(), -1);
     int nwin = 0, umax = 0;
@@ -2071,15 +2593,13 @@ static int build_windows(lelph_gpu* h)
                                        (const float2*)h->d_twN32[1].p, -1, h->st);
             lelph_launch_fft_strided_f(tN, (long long)ncomp, h->Nbox[1] * h->Nbox[2], h->planN[0],
                                        (const float2*)h->d_twN32[0].p, -1, h->st);
-            const int3 dm = make_int3(h->qslots[s].dmin[0], h->qslots[s].dmin[1], h->qslots[s].dmin[2]);
-            k_dv_window<float2><<<dim3(64, ncomp, nu), 256, 0, h->st>>>(tN, ncomp, h->Nbox[0], h->Nbox[1], h->Nbox[2],
-                                                                        (const int*)h->d_tmp.p + uoff[s], nu, dm, g,
-                                                                        1.0 / (double)NN, tM);
-            lelph_launch_fft_contig_f(tM, (long long)nu * ncomp * g.Nx * g.Ny, h->plan[2],
+            launch_dv_window<float2>(tN, ncomp, win_geom(h, h->qslots[s]), P, (const int*)h->d_tmp.p + uoff[s], nu,
+                                     (const float2*)h->d_subtw32.p, 1.0 / (double)NN, tM, h->st);
+            lelph_launch_fft_contig_f(tM, (long long)nu * ncomp * P * g.Nx * g.Ny, h->plan[2],
                                       (const float2*)h->d_tw32[2].p, +1, h->st);
-            lelph_launch_fft_strided_f(tM, (long long)nu * ncomp * g.Nx, g.Nz, h->plan[1],
+            lelph_launch_fft_strided_f(tM, (long long)nu * ncomp * P * g.Nx, g.Nz, h->plan[1],
                                        (const float2*)h->d_tw32[1].p, +1, h->st);
-            lelph_launch_fft_strided_f(tM, (long long)nu * ncomp, g.Ny * g.Nz, h->plan[0],
+            lelph_launch_fft_strided_f(tM, (long long)nu * ncomp * P, g.Ny * g.Nz, h->plan[0],
                                        (const float2*)h->d_tw32[0].p, +1, h->st);
             if (h->gspace)
             {
@@ -2113,16 +2633,14 @@ static int build_windows(lelph_gpu* h)
                                    (const double2*)h->d_twN[1].p, -1, h->st);
         lelph_launch_fft_strided_d(tN, (long long)ncomp, h->Nbox[1] * h->Nbox[2], h->planN[0],
                                    (const double2*)h->d_twN[0].p, -1, h->st);
-        const int3 dm = make_int3(h->qslots[s].dmin[0], h->qslots[s].dmin[1], h->qslots[s].dmin[2]);
-        k_dv_window<double2><<<dim3(64, ncomp, nu), 256, 0, h->st>>>(tN, ncomp, h->Nbox[0], h->Nbox[1], h->Nbox[2],
-                                                             (const int*)h->d_tmp.p + uoff[s], nu, dm, g,
-                                                             1.0 / (double)NN, tM);
+        launch_dv_window<double2>(tN, ncomp, win_geom(h, h->qslots[s]), P, (const int*)h->d_tmp.p + uoff[s], nu,
+                                  (const double2*)h->d_subtw64.p, 1.0 / (double)NN, tM, h->st);
         // inverse transform on the product grid
-        lelph_launch_fft_contig_d(tM, (long long)nu * ncomp * g.Nx * g.Ny, h->plan[2], (const double2*)h->d_tw64[2].p,
+        lelph_launch_fft_contig_d(tM, (long long)nu * ncomp * P * g.Nx * g.Ny, h->plan[2], (const double2*)h->d_tw64[2].p,
                                   +1, h->st);
-        lelph_launch_fft_strided_d(tM, (long long)nu * ncomp * g.Nx, g.Nz, h->plan[1], (const double2*)h->d_tw64[1].p,
+        lelph_launch_fft_strided_d(tM, (long long)nu * ncomp * P * g.Nx, g.Nz, h->plan[1], (const double2*)h->d_tw64[1].p,
                                    +1, h->st);
-        lelph_launch_fft_strided_d(tM, (long long)nu * ncomp, g.Ny * g.Nz, h->plan[0], (const double2*)h->d_tw64[0].p,
+        lelph_launch_fft_strided_d(tM, (long long)nu * ncomp * P, g.Ny * g.Nz, h->plan[0], (const double2*)h->d_tw64[0].p,
                                    +1, h->st);
         const size_t base = (size_t)h->win_base[s] * ncomp * M;
         CUDA_TRY(h, cudaMemcpyAsync((double2*)h->d_win64.p + base, tM, sizeof(double2) * (size_t)nu * ncomp * M,
@@ -2146,12 +2664,13 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
     const GeomDev& g = h->g;
     const bool f64 = !h->mixed;
     const size_t e = f64 ? sizeof(double2) : sizeof(float2);
-    const long long M = (long long)g.Nx * g.Ny * g.Nz;
+    const long long M = lelph_grid_points(g);
     const int nb = d.nbnds, ns = d.nspinor, nm = d.nmodes;
-    const int nbox = d.nspin * nb * ns;
+    const int nset = d.nspin * nb * ns, nbox = nset * g.nsub;
+    const int nplane = g.nsub * g.Nx;  // (y, z) planes of a box, every copy
     const int nrows = nm * nb;
     const int npw_max = *std::max_element(h->npw.begin(), h->npw.end());
-    int rc = ensure(h, h->d_gs_psi, e * (size_t)nbox * M);
+    int rc = ensure(h, h->d_gs_psi, e * (size_t)nset * M);
     if (rc) return rc;
     // modes per pass: the plane-pass output and the GEMM operand of a block of
     // modes stay within ~2 GB
@@ -2159,9 +2678,9 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
     // arrays, TF32 hi and lo, and the k+q coefficients split the same way)
     const bool tc = !f64 && h->gs_tc;
     const size_t na = tc ? 2 : 1;
-    const size_t per_mode = e * (size_t)nb * ns * ((size_t)g.Nx * h->gs_ncol_max + na * h->gs_npad_max);
+    const size_t per_mode = e * (size_t)nb * ns * ((size_t)nplane * h->gs_ncol_max + na * h->gs_npad_max);
     const int nub = (int)std::max<size_t>(1, std::min<size_t>((size_t)nm, (2ull << 30) / per_mode));
-    rc = ensure(h, h->d_gs_out1, e * (size_t)nub * nb * ns * g.Nx * h->gs_ncol_max);
+    rc = ensure(h, h->d_gs_out1, e * (size_t)nub * nb * ns * nplane * h->gs_ncol_max);
     if (rc) return rc;
     const size_t a_cap = (size_t)nub * nb * ns * h->gs_npad_max;  // complex elements of one A array
     void* prev_A = h->d_gs_A.p;
@@ -2188,7 +2707,7 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
     const void* tw[3];
     for (int x = 0; x < 3; ++x) tw[x] = f64 ? h->d_tw64[x].p : h->d_tw32[x].p;
     const void* winb = f64 ? h->d_win64.p : h->d_win32.p;
-    GsGeom gg{g.Nx, g.Ny, g.Nz, nb, ns, d.nmag, 0};
+    GsGeom gg{g.Nx, g.Ny, g.Nz, g.nsub, nb, ns, d.nmag, 0, f64 || h->plan[0].allct};
     int cur = -1;
     for (int oi = 0; oi < n; ++oi)
     {
@@ -2197,11 +2716,12 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
         if (P.kbz_k != cur)
         {
             cur = P.kbz_k;
-            CUDA_TRY(h, cudaMemsetAsync(h->d_gs_psi.p, 0, e * (size_t)nbox * M, h->st));
+            CUDA_TRY(h, cudaMemsetAsync(h->d_gs_psi.p, 0, e * (size_t)nset * M, h->st));
             lelph_launch_scatter(cur, 1, (const KPointSym*)h->d_ksym.p, (const int*)h->d_miller.p,
                                  (const long long*)h->d_pwoff.p, (const int*)h->d_npw.p, npw_max,
                                  (const double2*)h->d_coef.p, (const long long*)h->d_coefoff.p, g, f64, h->d_gs_psi.p,
-                                 (double2*)h->d_chat.p, (const long long*)h->d_chatoff.p, h->st);
+                                 (double2*)h->d_chat.p, (const long long*)h->d_chatoff.p,
+                                 (const double2*)h->d_subtw64.p, h->st);
             if (f64)
             {
                 double2* bx = (double2*)h->d_gs_psi.p;
@@ -2260,8 +2780,9 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
                 h->stats.gs_plane_ms += gs_tock(h);
                 bad |= lelph_launch_gs_xpass(gg, f64, h->d_gs_out1.p, nmb * nb * ns, ncol, h->plan[0], tw[0],
                                              (const int*)h->d_gs_cst.p + h->gs_cst_off[kq],
-                                             (const int*)h->d_gs_kcx.p + h->gs_perm_off[kq], npad, h->d_gs_A.p,
-                                             h->st, A_lo);
+                                             (const int*)h->d_gs_kcx.p + h->gs_perm_off[kq],
+                                             (const char*)h->d_gs_shph.p + e * (size_t)h->gs_perm_off[kq], npad,
+                                             h->d_gs_A.p, h->st, A_lo);
                 h->stats.gs_xpass_ms += gs_tock(h);
                 if (tc)
                     bad |= lelph_launch_gs_gemm_tc(tm, nmb * nb, nb, Ktot, kchunk, nu0 * nb, nrows,
@@ -2283,16 +2804,22 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
     return LELPH_GPU_OK;
 }
 
+// which: the product grid (GridState): 0 for batch runs, 1 for the one-call stage
 static int run_impl(lelph_gpu* h, int n, const int* qslot, const int* kbz, int non_loc, int kminusq, int out_type,
-                    void* g_out, bool out_device)
+                    void* g_out, bool out_device, int which = 0)
 {
     if (!h || n < 0 || (n > 0 && (!qslot || !kbz || !g_out))) return LELPH_GPU_ERR_INVALID;
     if (out_type != LELPH_GPU_OUT_C128 && out_type != LELPH_GPU_OUT_C64) return fail(h, LELPH_GPU_ERR_INVALID, "out_type");
     if (n == 0) return LELPH_GPU_OK;
     CUDA_TRY(h, cudaSetDevice(h->device));
+    {
+        const int rc = use_grid(h, which);
+        if (rc) return rc;
+    }
+    h->ran = true;
     if (!h->prepared)
     {
-        int rc = lelph_gpu_prepare(h);
+        int rc = prepare_grid(h);
         if (rc) return rc;
     }
     if (!h->windows_ok)
@@ -2365,7 +2892,7 @@ static int run_impl(lelph_gpu* h, int n, const int* qslot, const int* kbz, int n
     if (h->mixed && !h->gspace && (h->tmapV_base != h->d_win32.p || h->tmapV_rows != h->nwin))
     {
         // dV windows, tile-major: blocks (window, 32-point block) of (mode, component) rows x 64 floats
-        const long long M = (long long)g.Nx * g.Ny * g.Nz;
+        const long long M = lelph_grid_points(g);
         rc = make_tmap3(h, &h->tmapV, h->d_win32.p, true, 64, (unsigned long long)d.nmodes * d.nmag,
                         (unsigned long long)h->nwin * (M / 32), (unsigned)(g.mt_modes * d.nmag),
                         (unsigned)(g.kpts / 32), false);
@@ -2486,7 +3013,7 @@ extern "C" int lelph_gpu_compute_elphq(lelph_gpu* h, const double qpt_crys[3], c
     if (rc) return rc;
     std::vector<int> qs(h->d.nkpts_BZ, 0), ks(h->d.nkpts_BZ);
     for (int i = 0; i < h->d.nkpts_BZ; ++i) ks[i] = i;
-    return lelph_gpu_run(h, h->d.nkpts_BZ, qs.data(), ks.data(), non_loc, kminusq, LELPH_GPU_OUT_C128, elph_out);
+    return run_impl(h, h->d.nkpts_BZ, qs.data(), ks.data(), non_loc, kminusq, LELPH_GPU_OUT_C128, elph_out, false, 1);
 }
 
 extern "C" int lelph_gpu_elph_q_rotate(lelph_gpu* h, const double* Dl, const double* g, const double* Dr,
@@ -2902,7 +3429,7 @@ extern "C" int lelph_gpu_compute_elphq_star(lelph_gpu* h, const double qpt_crys[
     {
         std::vector<int> qs(nk, 0), ks(nk);
         for (int i = 0; i < nk; ++i) ks[i] = i;
-        rc = run_impl(h, nk, qs.data(), ks.data(), non_loc, kminusq, out_type, h->d_gstar.p, true);
+        rc = run_impl(h, nk, qs.data(), ks.data(), non_loc, kminusq, out_type, h->d_gstar.p, true, 1);
         if (rc) return rc;
     }
     if (nstar > 1)
@@ -3071,7 +3598,7 @@ double tune_candidate(const lelph_gpu_desc& dc, const double* q, const double* e
         // that would take more than half of the device memory (as the automatic route does)
         const double per_kpt = h->mixed ? 24.0 * h->g.nbp * dc.nspin * dc.nspinor
                                         : 16.0 * dc.nspin * dc.nbnds * dc.nspinor;
-        const double resident = per_kpt * (double)h->g.Nx * h->g.Ny * h->g.Nz * dc.nkpts_BZ;
+        const double resident = per_kpt * (double)h->box_grid[0] * h->box_grid[1] * h->box_grid[2] * dc.nkpts_BZ;
         size_t fr = 0, tot = 0;
         if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || resident > 0.5 * (double)tot) goto done;
     }
@@ -3310,7 +3837,7 @@ extern "C" int lelph_gpu_run_device_noalloc(lelph_gpu* h, int n, const int* qslo
     const int batch = (int)std::min<size_t>({(size_t)n, room / per_pair, (size_t)max_pairs});
     if (h->mixed && (h->tmapV_base != h->d_win32.p || h->tmapV_rows != h->nwin))
     {
-        const long long M = (long long)g.Nx * g.Ny * g.Nz;
+        const long long M = lelph_grid_points(g);
         rc = make_tmap3(h, &h->tmapV, h->d_win32.p, true, 64, (unsigned long long)d.nmodes * d.nmag,
                         (unsigned long long)h->nwin * (M / 32), (unsigned)(g.mt_modes * d.nmag),
                         (unsigned)(g.kpts / 32), false);

@@ -12,6 +12,7 @@ struct FftPlan1D
 {
     int L;
     int nstage;
+    int allct;  // FP32 passes: every compile-time length, not only the original ones (lelph_fft_fixed)
     int radix[LELPH_MAX_RADIX_STAGES];
 };
 
@@ -40,13 +41,24 @@ struct PairInfo
     int dvslot;  // dV window of (q slot, G0) on the product grid
 };
 
+// The product grid is the union of nsub interleaved copies of an Nx x Ny x Nz
+// grid, copy j shifted by j (sa_i / (nsub N_i)) of the cell along axis i: its
+// reciprocal lattice is { (m_i N_i) : sum_i sa_i m_i = 0 mod nsub } (nsub = 1: a
+// plain grid; nsub = 2 and sa = (1, 1, 1): body-centred sampling).  A box of the
+// grid holds the nsub copies one after the other, each [x][y][z].
 struct GeomDev
 {
-    int Nx, Ny, Nz;
+    int Nx, Ny, Nz;  // one copy
+    int nsub;        // interleaved copies, 1 .. LELPH_MAX_SUB
+    int sa[3];
     int nspin, nspinor, nbnds, nbp, nmag, nmodes;
     int mt_modes;  // whole modes per 128-row tile of the tensor-core sandwich: min(nmodes, max(1, 128/nbnds))
     int kpts;      // grid points per pipeline stage of the tensor-core sandwich (64, or 32 for wide tiles)
 };
+
+#define LELPH_MAX_SUB 4
+__host__ __device__ inline long long lelph_sub_points(const GeomDev& g) { return (long long)g.Nx * g.Ny * g.Nz; }
+__host__ __device__ inline long long lelph_grid_points(const GeomDev& g) { return g.nsub * lelph_sub_points(g); }
 
 // Partial sums of the tensor-core sandwich, laid out
 // [pair * nspin + spin][mode tile][K chunk][128 rows][2 nbp] (FP32).  A mode
@@ -89,6 +101,10 @@ struct BoxMask
 };
 
 // FFT (fft_gather.cu)
+// a length with a compile-time transform (FP32 passes).  The plain product grid
+// uses the original lengths only, so that the mixed form's results on it keep
+// their digits; interleaved grids use all of them.
+bool lelph_fft_fixed(int L, int all);
 void lelph_launch_fft_contig_d(double2* data, long long nlines, const FftPlan1D& p, const double2* tw, int sign,
                                cudaStream_t st);
 void lelph_launch_fft_contig_f(float2* data, long long nlines, const FftPlan1D& p, const float2* tw, int sign,
@@ -108,11 +124,13 @@ void lelph_launch_col_lists(const uint8_t* col, int nk, int ncol, int* list, int
 void lelph_launch_clear_cols(float2* boxes, int nk, int nbox_per_k, long long N, int Nz, int ncol, const int* list,
                              const int* cnt, cudaStream_t st);
 
-// sphere -> box scatter with su2, fractional-translation phase and conj
+// sphere -> box scatter with su2, fractional-translation phase and conj; sub_tw: per axis i
+// the table e^{+2 pi i t / (nsub N_i)}, t < nsub N_i (x, y, z in sequence), for the copies' shifts
 void lelph_launch_scatter(int k0, int nk, const KPointSym* ksym_dev, const int* miller, const long long* pw_off,
                           const int* npw, int npw_max, const double2* coef, const long long* coef_off,
                           const GeomDev& g, int box_fp64, void* boxes, double2* chat, const long long* chat_off,
-                          cudaStream_t st, const BoxMask& mk = BoxMask(), float2* chat32 = nullptr);
+                          const double2* sub_tw, cudaStream_t st, const BoxMask& mk = BoxMask(),
+                          float2* chat32 = nullptr);
 
 // debugging / parity: box index of each rotated plane wave of one full-BZ k
 void lelph_launch_gmap(const KPointSym* ks, int kbz, const int* miller, const long long* pw_off, const int* npw,
@@ -121,8 +139,10 @@ void lelph_launch_gmap(const KPointSym* ks, int kbz, const int* miller, const lo
 // G-space route of the local sandwich (gspace.cu)
 struct GsGeom
 {
-    int Nx, Ny, Nz;  // product grid
+    int Nx, Ny, Nz;  // one copy of the product grid; the boxes hold nsub * Nx planes
+    int nsub;
     int nb, nspinor, nmag, spin;
+    int allct;  // every compile-time plane and line length (FftPlan1D)
 };
 size_t lelph_gs_plane_smem(const GsGeom& gg, int fp64);
 size_t lelph_gs_xpass_smem(const GsGeom& gg, int fp64);
@@ -132,11 +152,12 @@ bool lelph_gs_plane_fixed(const GsGeom& gg, int fp64);
 int lelph_launch_gs_plane(const GsGeom& gg, int fp64, const void* psi, const void* win, int nu0, int nub,
                           const FftPlan1D& py, const FftPlan1D& pz, const void* twy, const void* twz, const int* cols,
                           int ncol, const int* cols2, const int* zl, int nzl, void* out, cudaStream_t st);
-// x pass: A [rb][npad] (rb = row-box index of the block) in the sphere's sorted order;
+// x pass: A [rb][npad] (rb = row-box index of the block) in the sphere's sorted order, the
+// copies of the grid summed with their phases (shph[K] = that of copy 1, its powers the others');
 // with A_lo (FP32 only) A receives the TF32-rounded values and A_lo the rounded remainders
 int lelph_launch_gs_xpass(const GsGeom& gg, int fp64, const void* in, int nrb, int ncol, const FftPlan1D& px,
-                          const void* twx, const int* cst, const int* kcx, int npad, void* A, cudaStream_t st,
-                          void* A_lo = nullptr);
+                          const void* twx, const int* cst, const int* kcx, const void* shph, int npad, void* A,
+                          cudaStream_t st, void* A_lo = nullptr);
 // tensor-core GEMM of the mixed form (gspace_tc.cu): tmaps = CUtensorMap[4] of
 // A hi, A lo (nrows x 2 Ktot FP32, box 32 x 128), B hi, B lo (2 nb x 2 Ktot,
 // box 32 x NT); B from lelph_launch_gs_bsplit

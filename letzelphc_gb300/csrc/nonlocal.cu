@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(256) k_finish(const PairInfo* __restrict__ pai
         }
         __syncthreads();
     }
-    const double invN = 1.0 / ((double)gd.Nx * gd.Ny * gd.Nz);
+    const double invN = 1.0 / (double)lelph_grid_points(gd);
     const int nrows = gd.nmodes * nb;
     const int NT = 2 * gd.nbp;
     // pre-factor -2 pi i e2 (src/nonloc/Vbare_nloc.c:547)
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(NJ <= 12 ? 256 : 128, (NJ <= 12 && sizeof(T) =
         }
         __syncthreads();
     }
-    const double invN = 1.0 / ((double)gd.Nx * gd.Ny * gd.Nz);
+    const double invN = 1.0 / (double)lelph_grid_points(gd);
     const float invN_hi = (float)invN, invN_lo = (float)(invN - (double)invN_hi);  // 1/M as a float pair
     const int NT = 2 * gd.nbp;
     const double2 pre = make_double2(0.0, -2.0 * LELPH_PI_T * LELPH_E2);

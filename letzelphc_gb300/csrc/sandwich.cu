@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(256) k_local_fp64(const PairInfo* __restrict__
     const int nrows = gd.nmodes * gd.nbnds;
     const int row0 = blockIdx.x * F64_TM;
     const int col0 = blockIdx.y * F64_TN;
-    const long long N = (long long)gd.Nx * gd.Ny * gd.Nz;
+    const long long N = lelph_grid_points(gd);
     const long long Ktot = (long long)gd.nspinor * N;
     const size_t box = (size_t)N;
     // psi layout [kbz][spin][band][spinor][r]
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(TC_THREADS(KP, NDR), 1)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int NT = 2 * gd.nbp;
-    const long long N = (long long)gd.Nx * gd.Ny * gd.Nz;
+    const long long N = lelph_grid_points(gd);
     constexpr int TC_GROUP = 64 / KP;
     constexpr int NATOM = KP / 32;
     const int nstage = chunk_pts / KP;

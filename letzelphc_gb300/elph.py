@@ -75,7 +75,7 @@ EXPORTS = [
     "lelph_gpu_last_error", "lelph_gpu_destroy", "lelph_gpu_run_device_noalloc",
     "lelph_gpu_set_local_pseudo", "lelph_gpu_dvlocq", "lelph_gpu_set_q_induced", "lelph_gpu_rotate_dvscf",
     "lelph_gpu_dmats", "lelph_gpu_compute_elphq_star", "lelph_gpu_set_q_dvscf_qe",
-    "lelph_gpu_debug_partials_extent", "lelph_gpu_set_wait_limit", "lelph_gpu_tune",
+    "lelph_gpu_debug_partials_extent", "lelph_gpu_set_wait_limit", "lelph_gpu_tune", "lelph_gpu_grid",
 ]
 
 _lib = None
@@ -114,6 +114,7 @@ def load_library(path: str = LIB_PATH):
     L.lelph_gpu_debug_gvec_map.argtypes = [vp, C.c_int, _ip, _ip]
     L.lelph_gpu_set_profiling.argtypes = [vp, C.c_int]
     L.lelph_gpu_stats_get.argtypes = [vp, C.POINTER(Stats)]
+    L.lelph_gpu_grid.argtypes = [vp, _ip]
     L.lelph_gpu_stream.argtypes = [vp]
     L.lelph_gpu_stream.restype = vp
     L.lelph_gpu_strerror.argtypes = [C.c_int]
@@ -424,6 +425,14 @@ class LelphGPU:
         out = {f: getattr(st, f) for f, _ in Stats._fields_}
         out["product_grid"] = tuple(out["product_grid"])
         return out
+
+    def grid(self):
+        """Product grid in use: {"n": one copy's sizes, "copies": interleaved
+        copies, "shift": a, "points": of all copies}."""
+        out = (C.c_int * 7)()
+        self._check(self._L.lelph_gpu_grid(self.h, out))
+        n = tuple(out[:3])
+        return {"n": n, "copies": out[3], "shift": tuple(out[4:]), "points": n[0] * n[1] * n[2] * out[3]}
 
     def stream(self):
         return self._L.lelph_gpu_stream(self.h)
