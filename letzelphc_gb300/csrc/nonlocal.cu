@@ -309,138 +309,6 @@ void lelph_launch_projections(int k0, int nk, const KPointSym* ksym_dev, const d
 
 // ------------------------------------------------------------------ finish
 
-#define FIN_MN 32
-#define FIN_MAXJ 48  // 3 * natom
-
-// grid: (ceil(nb*nb/32), npairs*nspin); 256 threads.
-// gout layout per pair: (nmodes, nspin, nb_k, nb_kq) complex.
-__global__ void __launch_bounds__(256) k_finish(const PairInfo* __restrict__ pairs, int mode_fp64,
-                                                const double2* __restrict__ glocal,
-                                                const float* __restrict__ partials, int nchunks,
-                                                const float* __restrict__ mode_scale,
-                                                const float* __restrict__ band_scale,
-                                                const double2* __restrict__ proj, const double2* __restrict__ eig,
-                                                int non_loc, NonlocalDesc nl, GeomDev gd, int out_c64,
-                                                void* __restrict__ gout)
-{
-    __shared__ double2 out_s[FIN_MAXJ][FIN_MN];
-    const int zp = blockIdx.y;
-    const int pair = zp / gd.nspin, spin = zp - pair * gd.nspin;
-    const PairInfo P = pairs[pair];
-    const int nb = gd.nbnds, ns = gd.nspinor;
-    const int nsets = gd.nspin * nb * ns;
-    const int mn0 = blockIdx.x * FIN_MN;
-    const int nj = 3 * nl.natom;
-    if (non_loc)
-    {
-        for (int e = threadIdx.x; e < nj * FIN_MN; e += blockDim.x)
-        {
-            int j = e / FIN_MN, t = e - j * FIN_MN;
-            int mn = mn0 + t;
-            double2 acc = make_double2(0.0, 0.0);
-            if (mn < nb * nb)
-            {
-                int m = mn / nb, n = mn - m * nb;  // m: band of k, n: band of k+q
-                int a = j / 3, x = j - 3 * a;
-                int it = nl.atom_type[a];
-                const double2* PK = proj + (((size_t)P.kbz_kq * nl.natom + a) * nl.nproj_max) * 4 * nsets;
-                const double2* PKp = proj + (((size_t)P.kbz_k * nl.natom + a) * nl.nproj_max) * 4 * nsets;
-                int pbase = 0;
-                for (int lidx = 0; lidx < nl.nltimesj; ++lidx)
-                {
-                    int l = (int)rint(nl.PP_table[(lidx * nl.ntype + it) * 3] - 1.0);
-                    if (l < 0) continue;
-                    int twoj = (int)rint(nl.PP_table[(lidx * nl.ntype + it) * 3 + 1]);
-                    double soc_fac = 1.0;
-                    if (twoj != 0 && !nl.is_soc) soc_fac = (twoj + 1.0) / (4.0 * l + 2.0);
-                    int foff = nl.fcoef ? nl.fcoef_off[lidx * nl.ntype + it] : -1;
-                    int tl = 2 * l + 1;
-                    for (int im1 = 0; im1 < tl; ++im1)
-                        for (int im2 = 0; im2 < tl; ++im2)
-                        {
-                            if (foff < 0 && im1 != im2) continue;
-                            int p1 = pbase + im1, p2 = pbase + im2;
-                            for (int s1 = 0; s1 < ns; ++s1)
-                                for (int s2 = 0; s2 < ns; ++s2)
-                                {
-                                    double2 f;
-                                    if (foff >= 0)
-                                    {
-                                        const double* fc = nl.fcoef + 2 * ((size_t)foff + (im1 * tl + im2) * ns * ns +
-                                                                           s1 * ns + s2);
-                                        f = make_double2(fc[0], fc[1]);
-                                    }
-                                    else
-                                    {
-                                        f = make_double2(s1 == s2 ? soc_fac : 0.0, 0.0);
-                                    }
-                                    if (f.x == 0.0 && f.y == 0.0) continue;
-                                    int setK = (spin * nb + n) * ns + s1;
-                                    int setKp = (spin * nb + m) * ns + s2;
-                                    double2 K0 = PK[((size_t)p1 * 4 + 0) * nsets + setK];
-                                    double2 Kx = PK[((size_t)p1 * 4 + 1 + x) * nsets + setK];
-                                    double2 Kp0 = cconj(PKp[((size_t)p2 * 4 + 0) * nsets + setKp]);
-                                    double2 Kpx = PKp[((size_t)p2 * 4 + 1 + x) * nsets + setKp];
-                                    Kpx = make_double2(-Kpx.x, Kpx.y);  // -conj
-                                    double2 t2 = cadd(cmul(Kx, Kp0), cmul(K0, Kpx));
-                                    acc = cadd(acc, cmul(f, t2));
-                                }
-                        }
-                    pbase += tl;
-                }
-            }
-            out_s[j][t] = acc;
-        }
-        __syncthreads();
-    }
-    const double invN = 1.0 / (double)lelph_grid_points(gd);
-    const int nrows = gd.nmodes * nb;
-    const int NT = 2 * gd.nbp;
-    // pre-factor -2 pi i e2 (src/nonloc/Vbare_nloc.c:547)
-    const double2 pre = make_double2(0.0, -2.0 * LELPH_PI_T * LELPH_E2);
-    const double2* E = eig + (size_t)P.qslot * gd.nmodes * gd.nmodes;
-    for (int e = threadIdx.x; e < gd.nmodes * FIN_MN; e += blockDim.x)
-    {
-        int nu = e / FIN_MN, t = e - nu * FIN_MN;
-        int mn = mn0 + t;
-        if (mn >= nb * nb) continue;
-        int m = mn / nb, n = mn - m * nb;
-        int row = nu * nb + m;
-        double2 v;
-        if (mode_fp64)
-        {
-            v = glocal[((size_t)zp * nrows + row) * nb + n];
-        }
-        else
-        {
-            int mt = nu / gd.mt_modes, rr = (nu - mt * gd.mt_modes) * nb + m;
-            const float* pp = partials + lelph_tc_partial_offset(gd, nchunks, zp, mt, 0, rr);
-            double re = 0.0, im = 0.0;
-            for (int c = 0; c < nchunks; ++c)
-            {
-                re += (double)pp[(size_t)c * 128 * NT + n];
-                im += (double)pp[(size_t)c * 128 * NT + gd.nbp + n];
-            }
-            double sc = (double)mode_scale[(size_t)P.dvslot * gd.nmodes + nu] *
-                        (double)band_scale[((size_t)P.kbz_k * gd.nspin + spin) * nb + m] *
-                        (double)band_scale[((size_t)P.kbz_kq * gd.nspin + spin) * nb + n];
-            double f = invN / sc;
-            v = make_double2(re * f, im * f);
-        }
-        if (non_loc)
-        {
-            double2 s = make_double2(0.0, 0.0);
-            for (int j = 0; j < nj; ++j) s = cadd(s, cmul(E[(size_t)nu * gd.nmodes + j], out_s[j][t]));
-            v = cadd(v, cmul(pre, s));
-        }
-        size_t oidx = ((((size_t)pair * gd.nmodes + nu) * gd.nspin + spin) * nb + m) * nb + n;
-        if (out_c64)
-            reinterpret_cast<float2*>(gout)[oidx] = make_float2((float)v.x, (float)v.y);
-        else
-            reinterpret_cast<double2*>(gout)[oidx] = v;
-    }
-}
-
 // Knuth's TwoSum: s + x is added into s, its rounding error into e.  The
 // _rn intrinsics keep the compiler from contracting or reassociating.
 __device__ __forceinline__ void ff_two_sum(float& s, float& e, float x)
@@ -896,6 +764,302 @@ static size_t finish_tile_smem(const NonlocalDesc& nl, const GeomDev& g, size_t 
            (size_t)nl.ntype * 8 * sizeof(double);
 }
 
+// ------------------------------------------- finish for large projection sets
+// Arithmetic of the nonlocal term in k_finish_atoms: FP64 (plain form), or
+// pairs of floats holding about 46 bits (mixed form, where FP64 used to run:
+// GB300 issues 1/64 of FP32's rate in FP64).  A pair (h, l) stands for h + l.
+struct FinD
+{
+    typedef double R;
+    typedef double2 C;  // storage: (re, im)
+    struct Acc
+    {
+        double x = 0, y = 0;
+    };
+    __device__ static C load(double2 v) { return v; }
+    __device__ static double2 get(const Acc& a) { return make_double2(a.x, a.y); }
+    __device__ static C store(const Acc& a) { return make_double2(a.x, a.y); }
+    __device__ static C conj(C a) { return make_double2(a.x, -a.y); }
+    __device__ static C neg(C a) { return make_double2(-a.x, -a.y); }
+    // acc += a b
+    __device__ static void mac(Acc& s, C a, C b)
+    {
+        s.x = fma(a.x, b.x, s.x);
+        s.x = fma(-a.y, b.y, s.x);
+        s.y = fma(a.x, b.y, s.y);
+        s.y = fma(a.y, b.x, s.y);
+    }
+};
+struct FinF
+{
+    typedef float4 C;  // (re.h, re.l, im.h, im.l)
+    struct Acc
+    {
+        float xh = 0, xl = 0, yh = 0, yl = 0;
+    };
+    __device__ static C load(double2 v)
+    {
+        const float rh = (float)v.x, ih = (float)v.y;
+        return make_float4(rh, (float)(v.x - (double)rh), ih, (float)(v.y - (double)ih));
+    }
+    __device__ static double2 get(const Acc& a)
+    {
+        return make_double2((double)a.xh + (double)a.xl, (double)a.yh + (double)a.yl);
+    }
+    __device__ static C store(const Acc& a)
+    {
+        // renormalised: the error parts of a long sum may exceed half an ulp of h
+        const float rh = __fadd_rn(a.xh, a.xl), ih = __fadd_rn(a.yh, a.yl);
+        return make_float4(rh, __fadd_rn(__fsub_rn(a.xh, rh), a.xl), ih, __fadd_rn(__fsub_rn(a.yh, ih), a.yl));
+    }
+    __device__ static C conj(C a) { return make_float4(a.x, a.y, -a.z, -a.w); }
+    __device__ static C neg(C a) { return make_float4(-a.x, -a.y, -a.z, -a.w); }
+    // (sh, sl) += (ah + al)(bh + bl): the product's rounding error by FMA, the sum's by TwoSum
+    __device__ static void macr(float& sh, float& sl, float ah, float al, float bh, float bl)
+    {
+        const float p = __fmul_rn(ah, bh);
+        float e = __fmaf_rn(ah, bh, -p);
+        e = __fmaf_rn(ah, bl, e);
+        e = __fmaf_rn(al, bh, e);
+        ff_two_sum(sh, sl, p);
+        sl = __fadd_rn(sl, e);
+    }
+    __device__ static void mac(Acc& s, C a, C b)
+    {
+        macr(s.xh, s.xl, a.x, a.y, b.x, b.y);
+        macr(s.xh, s.xl, -a.z, -a.w, b.z, b.w);
+        macr(s.yh, s.yl, a.x, a.y, b.z, b.w);
+        macr(s.yh, s.yl, a.z, a.w, b.x, b.y);
+    }
+};
+
+// Finish where the pair's projection sets overflow shared memory (spinors with
+// d projectors, many atoms): one CTA per (16 bands of k+q x TM bands of k, pair,
+// spin) walks the atoms, with one atom's projections of the tile's bands in
+// shared memory at a time.  The channel coefficients are folded into the k
+// role as in k_finish_pair (Z and W_x), each thread owns one (m, n) and keeps
+// the 3 natom displacement sums in registers, then applies the mode transform
+// and adds the local term in FP64, as the kernel it replaces did (that one
+// formed every term with its coefficient from global memory in FP64: 31.8 ms
+// for 64 pairs of 64 spinor bands, 24 modes and 8 x 17 projectors; this one
+// 2.5 ms).
+#define FA_N 16
+#define FA_FC 28  // coefficients of one slot: (2 l + 1) ns^2, l <= 3
+template <int NJ, int TM, typename A>
+__global__ void __launch_bounds__(FA_N * TM, 2) k_finish_atoms(const PairInfo* __restrict__ pairs, int mode_fp64,
+                                                            const double2* __restrict__ glocal,
+                                                            const float* __restrict__ partials, int nchunks,
+                                                            const float* __restrict__ mode_scale,
+                                                            const float* __restrict__ band_scale,
+                                                            const double2* __restrict__ proj,
+                                                            const double2* __restrict__ eig, int non_loc,
+                                                            NonlocalDesc nl, GeomDev gd, int out_c64,
+                                                            void* __restrict__ gout)
+{
+    typedef typename A::C C2;
+    extern __shared__ __align__(16) unsigned char fasm[];
+    const int nb = gd.nbnds, ns = gd.nspinor;
+    const int ntn = (nb + FA_N - 1) / FA_N;
+    const int tm = blockIdx.x / ntn, tn = blockIdx.x - tm * ntn;
+    const int zp = blockIdx.y;
+    const int pair = zp / gd.nspin, spin = zp - pair * gd.nspin;
+    const PairInfo P = pairs[pair];
+    const int nsets = gd.nspin * nb * ns;
+    const int np = nl.nproj_max;
+    const int nj = 3 * nl.natom;
+    const int cn = FA_N * ns, cm = TM * ns;               // sets of the tile in either role
+    C2* sK = reinterpret_cast<C2*>(fasm);                 // [np * 4][max(cn, cm)]: raw k role, then k+q role
+    C2* sZ = sK + (size_t)np * 4 * (cn > cm ? cn : cm);   // [np * 4][cm]: Z, W_x
+    C2* sF = sZ + (size_t)np * 4 * cm;                    // [np][FA_FC]: f(p1, ., ., .) of the atom's slots
+    int* sch = reinterpret_cast<int*>(sF + np * FA_FC);   // slot -> channel: [type][np][4] = l, first slot, foff, lidx
+    const int m0 = tm * TM, n0 = tn * FA_N;
+    const int ml = threadIdx.x / FA_N, nlc = threadIdx.x - ml * FA_N;
+    const int m = m0 + ml, n = n0 + nlc;                  // m: band of k, n: band of k+q
+    typename A::Acc out[NJ];
+    if (non_loc)
+    {
+        for (int it = threadIdx.x; it < nl.ntype; it += blockDim.x)
+        {
+            int pb = 0;
+            for (int lidx = 0; lidx < nl.nltimesj; ++lidx)
+            {
+                const int l = (int)rint(nl.PP_table[(lidx * nl.ntype + it) * 3] - 1.0);
+                if (l < 0) continue;
+                for (int i = 0; i < 2 * l + 1; ++i)
+                {
+                    int* ch = sch + (it * np + pb + i) * 4;
+                    ch[0] = l;
+                    ch[1] = pb;
+                    ch[2] = nl.fcoef ? nl.fcoef_off[lidx * nl.ntype + it] : -1;
+                    ch[3] = lidx;
+                }
+                pb += 2 * l + 1;
+            }
+            for (; pb < np; ++pb) sch[(it * np + pb) * 4] = -1;
+        }
+#pragma unroll
+        for (int a = 0; a < NJ / 3; ++a)
+        {
+            if (a >= nl.natom) break;
+            const int it = nl.atom_type[a];
+            const double2* PK = proj + ((size_t)P.kbz_kq * nl.natom + a) * np * 4 * nsets + (size_t)spin * nb * ns;
+            const double2* PKp = proj + ((size_t)P.kbz_k * nl.natom + a) * np * 4 * nsets + (size_t)spin * nb * ns;
+            __syncthreads();  // the previous atom's tiles are consumed (and sch written)
+            for (int e = threadIdx.x; e < np * FA_FC; e += blockDim.x)
+            {
+                const int p1 = e / FA_FC, i = e - p1 * FA_FC;
+                const int* ch = sch + (it * np + p1) * 4;
+                const int row = (2 * ch[0] + 1) * ns * ns;  // coefficients of one slot
+                if (ch[0] >= 0 && ch[2] >= 0 && i < row)
+                {
+                    const double* f = nl.fcoef + 2 * ((size_t)ch[2] + (size_t)(p1 - ch[1]) * row + i);
+                    sF[e] = A::load(make_double2(f[0], f[1]));
+                }
+            }
+            for (int e = threadIdx.x; e < np * 4 * cm; e += blockDim.x)
+            {
+                const int r = e / cm, c = e - r * cm, b = m0 * ns + c;
+                sK[e] = A::load(b < nb * ns ? PKp[(size_t)r * nsets + b] : make_double2(0.0, 0.0));
+            }
+            __syncthreads();
+            // Z(p1, s1; m) = sum_{p2, s2} f(p1, p2, s1, s2) conj(Pi_0(p2, m, s2)), W_x = - the same of Pi_x
+            for (int e = threadIdx.x; e < np * 4 * cm; e += blockDim.x)
+            {
+                const int r = e / cm, c = e - r * cm;
+                const int p1 = r >> 2, comp = r & 3;
+                const int mm = c / ns, s1 = c - mm * ns;
+                const int* ch = sch + (it * np + p1) * 4;
+                const int l = ch[0];
+                typename A::Acc z;
+                if (l >= 0)
+                {
+                    const int tl = 2 * l + 1, pb = ch[1];
+                    if (ch[2] >= 0)
+                    {
+                        const C2* f = sF + p1 * FA_FC + s1 * ns;
+                        for (int p2 = 0; p2 < tl; ++p2)
+                            for (int s2 = 0; s2 < ns; ++s2)
+                                A::mac(z, f[p2 * ns * ns + s2], A::conj(sK[(size_t)((pb + p2) * 4 + comp) * cm + mm * ns + s2]));
+                    }
+                    else
+                    {
+                        const int twoj = (int)rint(nl.PP_table[(ch[3] * nl.ntype + it) * 3 + 1]);
+                        const double soc = (twoj != 0 && !nl.is_soc) ? (twoj + 1.0) / (4.0 * l + 2.0) : 1.0;
+                        A::mac(z, A::load(make_double2(soc, 0.0)), A::conj(sK[e]));
+                    }
+                }
+                const C2 v = A::store(z);
+                sZ[e] = comp ? A::neg(v) : v;
+            }
+            __syncthreads();
+            for (int e = threadIdx.x; e < np * 4 * cn; e += blockDim.x)
+            {
+                const int r = e / cn, c = e - r * cn, b = n0 * ns + c;
+                sK[e] = A::load(b < nb * ns ? PK[(size_t)r * nsets + b] : make_double2(0.0, 0.0));
+            }
+            __syncthreads();
+            const C2* kq = sK + nlc * ns;
+            const C2* kk = sZ + ml * ns;
+            typename A::Acc a0, a1, a2;
+            for (int p = 0; p < np; ++p)
+            {
+                if (sch[(it * np + p) * 4] < 0) break;
+                for (int sp = 0; sp < ns; ++sp)
+                {
+                    const C2* q = kq + (size_t)p * 4 * cn + sp;
+                    const C2* z = kk + (size_t)p * 4 * cm + sp;
+                    const C2 K0 = q[0], Z = z[0];
+                    A::mac(a0, q[cn], Z);
+                    A::mac(a0, K0, z[cm]);
+                    A::mac(a1, q[2 * cn], Z);
+                    A::mac(a1, K0, z[2 * cm]);
+                    A::mac(a2, q[3 * cn], Z);
+                    A::mac(a2, K0, z[3 * cm]);
+                }
+            }
+            out[3 * a] = a0;
+            out[3 * a + 1] = a1;
+            out[3 * a + 2] = a2;
+        }
+        // the eigenvectors take the tiles' place
+        __syncthreads();
+        const double2* E = eig + (size_t)P.qslot * gd.nmodes * gd.nmodes;
+        for (int e = threadIdx.x; e < gd.nmodes * nj; e += blockDim.x)
+            sK[e] = A::load(E[(e / nj) * gd.nmodes + (e % nj)]);
+        __syncthreads();
+    }
+    if (m >= nb || n >= nb) return;
+    const double invN = 1.0 / (double)lelph_grid_points(gd);
+    const double2 pre = make_double2(0.0, -2.0 * LELPH_PI_T * LELPH_E2);
+    const int nrows = gd.nmodes * nb, NT = 2 * gd.nbp;
+    const float bsc = mode_fp64 ? 1.f
+                                : band_scale[((size_t)P.kbz_k * gd.nspin + spin) * nb + m] *
+                                      band_scale[((size_t)P.kbz_kq * gd.nspin + spin) * nb + n];
+    C2 ov[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) ov[j] = A::store(out[j]);
+    for (int nu = 0; nu < gd.nmodes; ++nu)
+    {
+        double2 v;
+        if (mode_fp64)
+            v = glocal[((size_t)zp * nrows + nu * nb + m) * nb + n];
+        else
+        {
+            // K-chunk partials, compensated FP32 sums (about twice FP32's precision), unscaled by
+            // the exact inverse of the power-of-two operand scales
+            const int mt = nu / gd.mt_modes;
+            const float* pp = partials + lelph_tc_partial_offset(gd, nchunks, zp, mt, 0, (nu - mt * gd.mt_modes) * nb + m);
+            float sr = 0.f, er = 0.f, si = 0.f, ei = 0.f;
+#pragma unroll 4
+            for (int c = 0; c < nchunks; ++c)
+            {
+                ff_two_sum(sr, er, pp[(size_t)c * 128 * NT + n]);
+                ff_two_sum(si, ei, pp[(size_t)c * 128 * NT + gd.nbp + n]);
+            }
+            const double f = invN * (double)(1.0f / (mode_scale[(size_t)P.dvslot * gd.nmodes + nu] * bsc));
+            v = make_double2(((double)sr + (double)er) * f, ((double)si + (double)ei) * f);
+        }
+        if (non_loc)
+        {
+            typename A::Acc s;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+                if (j < nj) A::mac(s, sK[nu * nj + j], ov[j]);
+            v = cadd(v, cmul(pre, A::get(s)));
+        }
+        const size_t oidx = ((((size_t)pair * gd.nmodes + nu) * gd.nspin + spin) * nb + m) * nb + n;
+        if (out_c64)
+            reinterpret_cast<float2*>(gout)[oidx] = make_float2((float)v.x, (float)v.y);
+        else
+            reinterpret_cast<double2*>(gout)[oidx] = v;
+    }
+}
+
+template <int NJ, int TM, typename A>
+static int launch_finish_atoms(const PairInfo* pairs, int npairs, int mode_fp64, const double2* glocal,
+                               const float* partials, int nchunks, const float* mode_scale, const float* band_scale,
+                               const double2* proj, const double2* eig, int non_loc, const NonlocalDesc& nl,
+                               const GeomDev& g, int out_c64, void* gout, cudaStream_t st)
+{
+    const size_t e = sizeof(typename A::C);
+    const size_t rows = (size_t)nl.nproj_max * 4;
+    size_t smem = e * (rows * g.nspinor * ((FA_N > TM ? FA_N : TM) + TM) + (size_t)nl.nproj_max * FA_FC) +
+                  sizeof(int) * 4 * (size_t)nl.ntype * nl.nproj_max;
+    smem = std::max(smem, e * (size_t)g.nmodes * 3 * nl.natom);
+    if (smem > 220 * 1024) return -1;
+    static bool attr = false;
+    if (!attr)
+    {
+        cudaFuncSetAttribute(k_finish_atoms<NJ, TM, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+        attr = true;
+    }
+    const dim3 grid((unsigned)(((g.nbnds + FA_N - 1) / FA_N) * ((g.nbnds + TM - 1) / TM)),
+                    (unsigned)(npairs * g.nspin));
+    k_finish_atoms<NJ, TM, A><<<grid, FA_N * TM, smem, st>>>(pairs, mode_fp64, glocal, partials, nchunks, mode_scale,
+                                                             band_scale, proj, eig, non_loc, nl, g, out_c64, gout);
+    return 0;
+}
+
 void lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const double2* glocal,
                          const float* partials, int nchunks, const float* mode_scale, const float* band_scale,
                          const double2* proj, const double2* eig, int non_loc, const NonlocalDesc& nl,
@@ -956,7 +1120,20 @@ void lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const
                                                                  gout);
         return;
     }
-    dim3 grid((g.nbnds * g.nbnds + FIN_MN - 1) / FIN_MN, npairs * g.nspin);
-    k_finish<<<grid, 256, 0, st>>>(pairs, mode_fp64, glocal, partials, nchunks, mode_scale, band_scale, proj, eig,
-                                   non_loc, nl, g, out_c64, gout);
+    // larger sets: one atom's projections at a time (up to 8 atoms: 24 sums a thread; up to 16: 48
+    // sums, half as many threads)
+#define FINA(NJ, TM, A)                                                                                            \
+    launch_finish_atoms<NJ, TM, A>(pairs, npairs, mode_fp64, glocal, partials, nchunks, mode_scale, band_scale, proj, \
+                                   eig, non_loc, nl, g, out_c64, gout, st)
+    if (nj <= 24)
+    {
+        if (t64) FINA(24, 16, FinD);
+        else FINA(24, 16, FinF);
+    }
+    else
+    {
+        if (t64) FINA(48, 8, FinD);
+        else FINA(48, 8, FinF);
+    }
+#undef FINA
 }
