@@ -76,6 +76,7 @@ struct GridState
     bool sphere_window = false;   // dV windows hold the differences nearest to -q (see k_dv_window)
     DevBuf d_subtw64, d_subtw32;  // e^{+2 pi i t / (nsub N_i)} per axis (interleaved grids)
     DevBuf d_psi64, d_bsplit, d_psi32;
+    DevBuf d_epsi, d_edv;  // plain form, real-space route: scale exponents of psi64 and of the windows
     CUtensorMap tmapB, tmapP, tmapV;
     void* tmapV_base = nullptr;
     int tmapV_rows = 0;
@@ -101,7 +102,7 @@ struct GridState
     std::vector<DevBuf*> buffers()
     {
         return {&d_tw64[0], &d_tw64[1], &d_tw64[2], &d_tw32[0], &d_tw32[1], &d_tw32[2], &d_subtw64, &d_subtw32,
-                &d_psi64, &d_bsplit, &d_psi32, &d_win64, &d_win32, &d_winscale, &d_colmask, &d_collist, &d_colcnt,
+                &d_psi64, &d_bsplit, &d_psi32, &d_epsi, &d_edv, &d_win64, &d_win32, &d_winscale, &d_colmask, &d_collist, &d_colcnt,
                 &d_gs_perm, &d_gs_kcx, &d_gs_cols, &d_gs_cst, &d_gs_npw, &d_gs_npad, &d_gs_permoff, &d_gs_bpoff,
                 &d_gs_bp, &d_gs_shph, &d_gs_zl, &d_gs_cols2};
     }
@@ -1775,7 +1776,11 @@ static int prepare_grid(lelph_gpu* h)
         lelph_launch_fft_contig_d(psi, nbox * g.Nx * g.Ny, h->plan[2], (const double2*)h->d_tw64[2].p, +1, h->st);
         lelph_launch_fft_strided_d(psi, nbox * g.Nx, g.Nz, h->plan[1], (const double2*)h->d_tw64[1].p, +1, h->st);
         lelph_launch_fft_strided_d(psi, nbox, g.Ny * g.Nz, h->plan[0], (const double2*)h->d_tw64[0].p, +1, h->st);
-        h->stats.kernel_launches += 4;
+        const long long nbk = (long long)d.nkpts_BZ * d.nspin * d.nbnds;
+        rc = ensure(h, h->d_epsi, sizeof(int) * (size_t)nbk);
+        if (rc) return rc;
+        lelph_launch_oz_exponents(psi, nbk, d.nspinor * lelph_grid_points(g), OZ_GUARD_PSI, (int*)h->d_epsi.p, h->st);
+        h->stats.kernel_launches += 5;
     }
     else
     {
@@ -2565,6 +2570,8 @@ static int build_windows(lelph_gpu* h)
     {
         rc = ensure(h, h->d_win64, sizeof(double2) * (size_t)nwin * ncomp * M);
         if (rc) return rc;
+        rc = ensure(h, h->d_edv, sizeof(int) * (size_t)nwin * d.nmodes);
+        if (rc) return rc;
     }
     else
     {
@@ -2646,6 +2653,13 @@ static int build_windows(lelph_gpu* h)
         CUDA_TRY(h, cudaMemcpyAsync((double2*)h->d_win64.p + base, tM, sizeof(double2) * (size_t)nu * ncomp * M,
                                     cudaMemcpyDeviceToDevice, h->st));
         h->stats.kernel_launches += 7;
+        CUDA_TRY(h, cudaGetLastError());
+    }
+    if (!h->mixed && !h->gspace)
+    {
+        lelph_launch_oz_exponents((const double2*)h->d_win64.p, (long long)nwin * d.nmodes, d.nmag * M,
+                                  oz_guard_dv(d.nmag), (int*)h->d_edv.p, h->st);
+        h->stats.kernel_launches += 1;
         CUDA_TRY(h, cudaGetLastError());
     }
     h->windows_ok = true;
@@ -2941,8 +2955,21 @@ static int run_impl(lelph_gpu* h, int n, const int* qslot, const int* kbz, int n
             if (rc) return rc;
         }
         else if (!h->mixed)
-            lelph_launch_local_fp64(dp, nb, (const double2*)h->d_psi64.p, (const double2*)h->d_win64.p, g,
-                                    (double2*)h->d_glocal.p, (unsigned*)h->d_status.p, h->st);
+        {
+            // chunk partials in at most 1 GB
+            const int nch = lelph_local_fp64_chunks(nb, g, 1ull << 30);
+            if (nch > 1)
+            {
+                rc = ensure(h, h->d_partials, per_pair * nb * nch);
+                if (rc) return rc;
+            }
+            const int more = lelph_launch_local_fp64(dp, nb, (const double2*)h->d_psi64.p, (const int*)h->d_epsi.p,
+                                                     (const double2*)h->d_win64.p, (const int*)h->d_edv.p, g, nch,
+                                                     (double2*)h->d_partials.p, (double2*)h->d_glocal.p,
+                                                     (unsigned*)h->d_status.p, h->wait_ns, h->st);
+            if (more < 0) return fail(h, LELPH_GPU_ERR_UNSUPPORTED, "FP64 sandwich: launch configuration");
+            h->stats.kernel_launches += more;
+        }
         else
             lelph_launch_local_tc(dp, nb, &h->tmapB, &h->tmapP, &h->tmapV, g, h->ab_bf16, h->chunk_pts, h->nchunks,
                                   (float*)h->d_partials.p, (unsigned*)h->d_status.p, h->st, h->wait_ns);
@@ -3867,8 +3894,13 @@ extern "C" int lelph_gpu_run_device_noalloc(lelph_gpu* h, int n, const int* qslo
             CUDA_TRY(h, cudaMemcpyAsync(dpairs + c0, stage, sizeof(PairInfo) * nc, cudaMemcpyHostToDevice, h->st));
         }
         if (!h->mixed)
-            lelph_launch_local_fp64(dpairs, nb, (const double2*)h->d_psi64.p, (const double2*)h->d_win64.p, g,
-                                    (double2*)work, (unsigned*)h->d_status.p, h->st);
+        {
+            // one K chunk: the scratch holds the local blocks alone
+            if (lelph_launch_local_fp64(dpairs, nb, (const double2*)h->d_psi64.p, (const int*)h->d_epsi.p,
+                                        (const double2*)h->d_win64.p, (const int*)h->d_edv.p, g, 1, nullptr,
+                                        (double2*)work, (unsigned*)h->d_status.p, h->wait_ns, h->st) < 0)
+                return fail(h, LELPH_GPU_ERR_UNSUPPORTED, "FP64 sandwich: launch configuration");
+        }
         else
             lelph_launch_local_tc(dpairs, nb, &h->tmapB, &h->tmapP, &h->tmapV, g, h->ab_bf16, h->chunk_pts,
                                   h->nchunks, (float*)work, (unsigned*)h->d_status.p, h->st, h->wait_ns);

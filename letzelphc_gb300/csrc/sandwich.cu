@@ -13,8 +13,8 @@
 // M = (mode, band of k), N = band of k+q, K = (spinor, grid point), whose A
 // operand is generated on the fly from dV and psi_k.
 //
-// * k_local_fp64: the plain form, FP64 SIMT.
-// * k_local_tc:   the mixed form on the 5th-generation tensor cores: psi(r)
+// * k_local_oz (sandwich_f64.cu): the plain (FP64) form.
+// * k_local_tc: the mixed form on the 5th-generation tensor cores: psi(r)
 //   in FP32, A = dV psi_k formed in registers and written to tensor memory
 //   as 16-bit (hi, lo) pairs, B = psi_k+q split likewise in shared memory,
 //   three products A_hi B_hi + A_hi B_lo + A_lo B_hi accumulated in FP32 in
@@ -27,127 +27,6 @@
 
 #include "lelph_common.cuh"
 #include "lelph_internal.h"
-
-// ================================================================ FP64 form
-
-#define F64_TM 64
-#define F64_TN 32
-#define F64_KP 16
-
-// grid: (ceil(nrows/64), ceil(nb/32), npairs*nspin); 256 threads
-__global__ void __launch_bounds__(256) k_local_fp64(const PairInfo* __restrict__ pairs,
-                                                    const double2* __restrict__ psi, const double2* __restrict__ dV,
-                                                    GeomDev gd, double2* __restrict__ glocal)
-{
-    __shared__ double2 As[F64_TM][F64_KP + 1];
-    __shared__ double2 Bs[F64_TN][F64_KP + 1];
-    const int zp = blockIdx.z;
-    const int pair = zp / gd.nspin;
-    const int spin = zp - pair * gd.nspin;
-    const PairInfo P = pairs[pair];
-    const int nrows = gd.nmodes * gd.nbnds;
-    const int row0 = blockIdx.x * F64_TM;
-    const int col0 = blockIdx.y * F64_TN;
-    const long long N = lelph_grid_points(gd);
-    const long long Ktot = (long long)gd.nspinor * N;
-    const size_t box = (size_t)N;
-    // psi layout [kbz][spin][band][spinor][r]
-    const double2* psik = psi + ((size_t)P.kbz_k * gd.nspin + spin) * gd.nbnds * gd.nspinor * box;
-    const double2* psikq = psi + ((size_t)P.kbz_kq * gd.nspin + spin) * gd.nbnds * gd.nspinor * box;
-    const double2* dvq = dV + (size_t)P.dvslot * gd.nmodes * gd.nmag * box;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double2 acc[4][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) acc[i][j] = make_double2(0.0, 0.0);
-    __syncthreads();
-    for (long long k0 = 0; k0 < Ktot; k0 += F64_KP)
-    {
-        // A tile: 64 rows x 16 points
-        for (int e = threadIdx.x; e < F64_TM * F64_KP; e += blockDim.x)
-        {
-            int rr = e / F64_KP, p = e - rr * F64_KP;
-            int row = row0 + rr;
-            long long kc = k0 + p;
-            double2 a = make_double2(0.0, 0.0);
-            if (row < nrows && kc < Ktot)
-            {
-                int nu = row / gd.nbnds, m = row - nu * gd.nbnds;
-                int s = (int)(kc / N);
-                int r = (int)(kc - (long long)s * N);
-                const double2* dvn = dvq + (size_t)nu * gd.nmag * box;
-                const double2* pm = psik + (size_t)m * gd.nspinor * box;
-                if (gd.nmag == 4)
-                {
-                    a = cadd(cmul(dvn[(size_t)(2 * s) * box + r], pm[r]),
-                             cmul(dvn[(size_t)(2 * s + 1) * box + r], pm[box + r]));
-                }
-                else
-                {
-                    int comp = (gd.nmag == 2) ? spin : 0;
-                    a = cmul(dvn[(size_t)comp * box + r], pm[(size_t)s * box + r]);
-                }
-            }
-            As[rr][p] = a;
-        }
-        for (int e = threadIdx.x; e < F64_TN * F64_KP; e += blockDim.x)
-        {
-            int cc = e / F64_KP, p = e - cc * F64_KP;
-            int n = col0 + cc;
-            long long kc = k0 + p;
-            double2 b = make_double2(0.0, 0.0);
-            if (n < gd.nbnds && kc < Ktot)
-            {
-                int s = (int)(kc / N);
-                int r = (int)(kc - (long long)s * N);
-                b = cconj(psikq[((size_t)n * gd.nspinor + s) * box + r]);
-            }
-            Bs[cc][p] = b;
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int p = 0; p < F64_KP; ++p)
-        {
-            double2 av[4], bv[2];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) av[i] = As[ty * 4 + i][p];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) bv[j] = Bs[tx * 2 + j][p];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-                {
-                    acc[i][j].x = fma(av[i].x, bv[j].x, acc[i][j].x);
-                    acc[i][j].x = fma(-av[i].y, bv[j].y, acc[i][j].x);
-                    acc[i][j].y = fma(av[i].x, bv[j].y, acc[i][j].y);
-                    acc[i][j].y = fma(av[i].y, bv[j].x, acc[i][j].y);
-                }
-        }
-        __syncthreads();
-    }
-    const double invN = 1.0 / (double)N;
-    double2* go = glocal + (size_t)zp * nrows * gd.nbnds;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-        {
-            int row = row0 + ty * 4 + i, n = col0 + tx * 2 + j;
-            if (row < nrows && n < gd.nbnds)
-                go[(size_t)row * gd.nbnds + n] = make_double2(acc[i][j].x * invN, acc[i][j].y * invN);
-        }
-}
-
-void lelph_launch_local_fp64(const PairInfo* pairs, int npairs, const double2* psi, const double2* dV,
-                             const GeomDev& g, double2* glocal, unsigned* status, cudaStream_t st)
-{
-    (void)status;
-    int nrows = g.nmodes * g.nbnds;
-    dim3 grid((nrows + F64_TM - 1) / F64_TM, (g.nbnds + F64_TN - 1) / F64_TN, npairs * g.nspin);
-    k_local_fp64<<<grid, 256, 0, st>>>(pairs, psi, dV, g, glocal);
-}
 
 // ============================================================= mixed form
 //
