@@ -91,13 +91,25 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 
 // try_wait with a suspend-time hint: the thread sleeps until the phase
 // completes (or the hint expires) instead of spinning on the issue slots
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity, uint32_t hint_ns = 20000u)
 {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(hint_ns)
+        : "memory");
+    return ok != 0;
+}
+
+// whether the phase has completed, without waiting
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
     return ok != 0;
 }
@@ -107,11 +119,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity,
                                                   unsigned long long limit_ns = LELPH_WAIT_LIMIT_NS)
 {
-    if (mbar_try_wait(bar, parity)) return true;
+    // a limit shorter than the hint bounds the suspended time too
+    const uint32_t hint = limit_ns < 20000ull ? (uint32_t)limit_ns : 20000u;
+    if (mbar_try_wait(bar, parity, hint)) return true;
     unsigned long long t0 = gtimer_ns();
     while (true)
     {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait(bar, parity, hint)) return true;
         if (gtimer_ns() - t0 > limit_ns) return false;
     }
 }
@@ -152,6 +166,14 @@ __device__ __forceinline__ void prefetch_tmap(const void* tmap)
 }
 
 // ---------------------------------------------------------------- tcgen05
+
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols)
 {

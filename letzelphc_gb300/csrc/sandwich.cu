@@ -169,23 +169,13 @@ struct ProdFrag
     float4 dv[SUB / 2][NC];
 };
 
-// pp[c] points at the lane's psi row (128-byte swizzled half tile), dvp[c] at
-// the row's dV (16 points of the half); j0 is the first point of the SUB.
-template <int SUB, int NC>
-__device__ __forceinline__ void prod_load(ProdFrag<SUB, NC>& f, const uint8_t* const* pp, const float4* const* dvp,
-                                          uint32_t swz, int j0)
+// 16-byte shared-memory load by 32-bit address.  Volatile, so that it stays
+// behind the stage's barrier wait and in its place between the stores.
+__device__ __forceinline__ float4 lds128(uint32_t a)
 {
-#pragma unroll
-    for (int jj = 0; jj < SUB / 2; ++jj)
-    {
-        const int j = j0 / 2 + jj;  // 16-byte chunk = 2 points
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-        {
-            f.ps[jj][c] = *reinterpret_cast<const float4*>(pp[c] + ((((uint32_t)j) ^ swz) << 4));
-            f.dv[jj][c] = dvp[c][j];
-        }
-    }
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
 }
 
 // A operand of the SUB points: a = sum_c dV^{c} psi^{c}, split and stored to
@@ -236,66 +226,45 @@ __device__ __forceinline__ void prod_store(const ProdFrag<SUB, NC>& f, uint32_t 
     }
 }
 
-// A producer's share of one pipeline stage: points h*KP/PQ .. (h+1)*KP/PQ - 1,
-// in 16-point psi blocks of 16/SUB pieces of SUB points each.  The pieces are
-// software-pipelined: the shared-memory loads of piece t+1 are issued before
-// piece t is formed and stored, so that their latency overlaps the work.
-template <int BF16, int KP, int SUB, int NC, int PF>
-__device__ __forceinline__ void produce_stage(const uint8_t* st, const TcSmemLayout& L, const float4* zero_dv,
-                                              bool in_tile, int h, int m, int ml, int nmag, int comp0, int comp1,
-                                              int nsp, uint32_t swz, uint32_t col_base)
+// A producer's share of one pipeline stage: points h*KP/PQ .. (h+1)*KP/PQ - 1 in
+// pieces of SUB points, NC dV components.  Shared-memory addresses of a stage
+// (32 bits): psi of the share's first 16-point block (blocks p_half apart,
+// components p_comp apart) and the row's dV at the share's first point.
+template <int KP, int SUB, int NC>
+struct ProdShare
 {
-    constexpr int NATOM = KP / 32;
-    constexpr int PPW = KP / tc_pq<KP>();  // points of this warp
+    static constexpr int PPW = KP / tc_pq<KP>();
     static_assert(PPW % 16 == 0, "a producer warp forms whole 16-point blocks");
-    constexpr int NBW = PPW / 16;    // 16-point blocks of this warp
-    constexpr int PER_BLOCK = 16 / SUB;
-    constexpr int NPIECE = NBW * PER_BLOCK;
-    const uint8_t* pp[NBW][2];
-    const float4* dvp[NBW][2];
-#pragma unroll
-    for (int b = 0; b < NBW; ++b)
+    static constexpr int NPIECE = PPW / SUB, SUBP = SUB;
+    static constexpr bool PRE = NC == 1;
+    typedef ProdFrag<SUB, NC> Frag;
+    static_assert(NPIECE % 2 == 0, "the fragments alternate");
+    uint32_t psi, dv;          // addresses in this stage
+    uint32_t p_half, p_comp;   // strides
+    uint32_t dv_block;         // the next 32 points' dV (0: the zero block)
+    uint32_t dv_comp;
+
+    // xo[j]: the lane's row and swizzled 16-byte chunk j (two points) in a psi block
+    __device__ __forceinline__ void load(ProdFrag<SUB, NC>& f, const uint32_t* xo, int t) const
     {
-        const int p0 = h * PPW + 16 * b;  // first point of the block in the stage
-        const int pb = p0 >> 4;                // 16-point psi block
-        const float* dvs = reinterpret_cast<const float*>(st + L.dv + (uint32_t)(p0 >> 5) * L.dv_block);
-        pp[b][0] = st + L.p + (0 * 2 * NATOM + pb) * L.p_half + (uint32_t)m * 128;
-        pp[b][1] = st + L.p + ((nsp - 1) * 2 * NATOM + pb) * L.p_half + (uint32_t)m * 128;
-        dvp[b][0] = in_tile ? reinterpret_cast<const float4*>(dvs + ((size_t)(ml * nmag + comp0) * 32 + (p0 & 31)) * 2)
-                            : zero_dv;
-        dvp[b][1] = in_tile ? reinterpret_cast<const float4*>(dvs + ((size_t)(ml * nmag + comp1) * 32 + (p0 & 31)) * 2)
-                            : zero_dv;
-    }
-    if (PF)
-    {
-        ProdFrag<SUB, NC> f[2];
-        prod_load<SUB, NC>(f[0], pp[0], dvp[0], swz, 0);
+        const int p0 = t * SUB;                 // point in the share
+        const int j0 = (p0 & 15) / 2;
+        const uint32_t pb = psi + (uint32_t)(p0 >> 4) * p_half;
+        const uint32_t db = dv + (uint32_t)(p0 >> 5) * dv_block + (dv_block ? (uint32_t)(p0 & 31) * 8u : 0u);
 #pragma unroll
-        for (int t = 0; t < NPIECE; ++t)
-        {
-            if (t + 1 < NPIECE)
+        for (int jj = 0; jj < SUB / 2; ++jj)
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
             {
-                const int bn = (t + 1) / PER_BLOCK;
-                prod_load<SUB, NC>(f[(t + 1) & 1], pp[bn], dvp[bn], swz, ((t + 1) % PER_BLOCK) * SUB);
+                f.ps[jj][c] = lds128(pb + c * p_comp + xo[j0 + jj]);
+                f.dv[jj][c] = lds128(db + c * dv_comp + 16u * (uint32_t)jj);
             }
-            const int b = t / PER_BLOCK, j0 = (t % PER_BLOCK) * SUB;
-            const uint32_t col_hi = col_base + (uint32_t)(h * PPW + 16 * b + j0);
-            prod_store<BF16, SUB, NC>(f[t & 1], col_hi, col_hi + KP);
-        }
     }
-    else
+    template <int BF16> __device__ __forceinline__ static void store(const ProdFrag<SUB, NC>& f, uint32_t col)
     {
-#pragma unroll
-        for (int t = 0; t < NPIECE; ++t)
-        {
-            ProdFrag<SUB, NC> f;
-            const int b = t / PER_BLOCK, j0 = (t % PER_BLOCK) * SUB;
-            prod_load<SUB, NC>(f, pp[b], dvp[b], swz, j0);
-            const uint32_t col_hi = col_base + (uint32_t)(h * PPW + 16 * b + j0);
-            prod_store<BF16, SUB, NC>(f, col_hi, col_hi + KP);
-        }
+        prod_store<BF16, SUB, NC>(f, col, col + KP);
     }
-}
+};
 
 // One pipeline stage of the merged split product (NT <= 64): per 16-wide K
 // step k, A_hi [B_hi; B_lo] (N = 2 NT) into dacc and A_lo B_hi (N = NT) into
@@ -397,6 +366,11 @@ __device__ __forceinline__ void umma_stage_merged<32>(uint32_t dacc, uint32_t da
 // the MMA warp cycles through NACC TMEM accumulators, and the drain warps
 // add each finished accumulator into round-to-nearest FP32 registers, which
 // are written out per K chunk and reduced in FP64 by the finish kernel.
+template <int H> struct TcHalf
+{
+    static constexpr int value = H;
+};
+
 struct TcUnit
 {
     int chunk, mt, zp, spin;
@@ -438,9 +412,8 @@ __global__ void __launch_bounds__(TC_THREADS(KP, NDR), 1)
     const int NST = (int)L.nst, NA = (int)L.na, NACC = (int)L.nacc;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acce + TC_NACC_MAX);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    const float4* zero_dv = reinterpret_cast<const float4*>(sm + L.bar_off + 512);  // 256 zero bytes
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int NT = 2 * gd.nbp;
     const long long N = lelph_grid_points(gd);
     constexpr int TC_GROUP = 64 / KP;
@@ -475,7 +448,7 @@ __global__ void __launch_bounds__(TC_THREADS(KP, NDR), 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
     if (warp == 0)
     {
@@ -547,83 +520,92 @@ __global__ void __launch_bounds__(TC_THREADS(KP, NDR), 1)
     }
     else if (warp == 1)
     {
-        if (lane == 0)
+        // The whole warp runs the loop and one elected lane issues: with the loop
+        // warp-uniform, the descriptors live in uniform registers and a stage's MMAs
+        // issue at the tensor pipe's rate (768 cycles for 16) whatever the producers
+        // on this sub-partition do.  Issued under a lane test, each MMA needed moves from
+        // vector registers, which waited for issue slots (1140 cycles beside them).
+        // With the producers' overlap below: 4096 pairs of the 4-atom cell 35.3 -> 31.5
+        // ms, slab 6.3 -> 5.5, collinear spins 1.43 -> 1.23.  What bounds it now is
+        // shared memory: a 64-point stage moves about 1400 cycles' worth through it (psi
+        // and dV reads 640, TMA writes 390, B reads of the MMAs 384).
+        const uint32_t idesc = umma_idesc_f16(BF16 ? 1u : 0u, 128u, (uint32_t)NT);
+        const uint32_t idesc2 = umma_idesc_f16(BF16 ? 1u : 0u, 128u, (uint32_t)(2 * NT));
+        const bool merged = L.merged != 0;
+        int s = 0, a = 0, b = 0;
+        uint32_t pha = 0, phb = 0;
+        bool stop = false;
+        uint64_t* last_commit = nullptr;  // the A-slot barrier of the latest commit, and its phase parity
+        uint32_t last_par = 0;
+        for (int u = blockIdx.x; u < nunits && !stop; u += gridDim.x)
         {
-            const uint32_t idesc = umma_idesc_f16(BF16 ? 1u : 0u, 128u, (uint32_t)NT);
-            const uint32_t idesc2 = umma_idesc_f16(BF16 ? 1u : 0u, 128u, (uint32_t)(2 * NT));
-            const bool merged = L.merged != 0;
-            int s = 0, a = 0, b = 0;
-            uint32_t pha = 0, phb = 0;
-            bool stop = false;
-            uint64_t* last_commit = nullptr;  // the A-slot barrier of the latest commit, and its phase parity
-            uint32_t last_par = 0;
-            for (int u = blockIdx.x; u < nunits && !stop; u += gridDim.x)
+            for (int it = 0; it < nstage; ++it)
             {
-                for (int it = 0; it < nstage; ++it)
+                const bool first = (it % TC_GROUP) == 0;
+                const bool last = (it % TC_GROUP) == TC_GROUP - 1 || it == nstage - 1;
+                // one barrier per stage: the producers arrive on aready[a] only after
+                // they saw the stage's TMA tiles land (full[s]), which orders B for the
+                // MMAs too
+                bool ok = true;
+                if (first) ok = mbar_wait_bounded(&acce[b], phb ^ 1u, wait_ns);
+                ok = ok && mbar_wait_bounded(&aready[a], pha, wait_ns);
+                if (__any_sync(0xffffffffu, !ok))
                 {
-                    const bool first = (it % TC_GROUP) == 0;
-                    const bool last = (it % TC_GROUP) == TC_GROUP - 1 || it == nstage - 1;
-                    // MMA issue blocks per instruction, so this thread checks one barrier
-                    // per stage: the producers arrive on aready[a] only after they saw the
-                    // stage's TMA tiles land (full[s]), which orders B for the MMAs too
-                    bool ok = true;
-                    if (first) ok = mbar_wait_bounded(&acce[b], phb ^ 1u, wait_ns);
-                    ok = ok && mbar_wait_bounded(&aready[a], pha, wait_ns);
-                    if (!ok)
+                    if (lane == 0)
                     {
                         *abort_flag = 1;
                         atomicOr(status, LELPH_DEV_ERR_TIMEOUT);
-                        stop = true;
-                        break;
                     }
-                    tc_fence_after();
-                    const uint32_t base = smem_u32(sm + s * L.stage_bytes);
-                    const uint32_t dacc = tmem + (uint32_t)b * L.accw;
-                    const uint32_t ahi = tmem + L.a_col0 + (uint32_t)a * (2u * KP);
+                    stop = true;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t base = smem_u32(sm) + (uint32_t)s * L.stage_bytes;
+                const uint32_t dacc = tmem + (uint32_t)b * L.accw;
+                const uint32_t ahi = tmem + L.a_col0 + (uint32_t)a * (2u * KP);
+                if (elect_one())
+                {
                     if (merged)
                     {
                         // rows [0, NT) of each atom's 2*NT-row tile are B_hi, [NT, 2NT) B_lo
                         const uint64_t d0 = umma_desc_sw128(base + L.b_hi);
                         const uint64_t d1 = d0 + (uint64_t)(L.b_atom >> 4);
-                        umma_stage_merged<KP>(dacc, dacc + (uint32_t)NT, ahi, d0, d1, idesc2, idesc,
-                                              first ? 0u : 1u);
+                        umma_stage_merged<KP>(dacc, dacc + (uint32_t)NT, ahi, d0, d1, idesc2, idesc, first ? 0u : 1u);
                     }
                     else
 #pragma unroll
-                    for (int k = 0; k < KP / 8; ++k)
-                    {
-                        const uint32_t atom = base + (uint32_t)(k >> 2) * L.b_atom + 32u * (uint32_t)(k & 3);
-                        const uint64_t bh = umma_desc_sw128(atom + L.b_hi);
-                        const uint32_t en = (first && k == 0) ? 0u : 1u;
+                        for (int k = 0; k < KP / 8; ++k)
                         {
+                            const uint32_t atom = base + (uint32_t)(k >> 2) * L.b_atom + 32u * (uint32_t)(k & 3);
+                            const uint64_t bh = umma_desc_sw128(atom + L.b_hi);
                             const uint64_t bl = umma_desc_sw128(atom + L.b_lo);
-                            umma_f16_ta(dacc, ahi + 8 * k, bh, idesc, en);
+                            umma_f16_ta(dacc, ahi + 8 * k, bh, idesc, (first && k == 0) ? 0u : 1u);
                             umma_f16_ta(dacc, ahi + 8 * k, bl, idesc, 1u);
                             umma_f16_ta(dacc, ahi + KP + 8 * k, bh, idesc, 1u);
                         }
-                    }
                     umma_commit(&empty[s]);
                     umma_commit(&afree[a]);
-                    last_commit = &afree[a];
-                    last_par = pha;
                     if (last) umma_commit(&accf[b]);
-                    s = (s + 1 == NST) ? 0 : s + 1;
-                    if (++a == NA)
-                    {
-                        a = 0;
-                        pha ^= 1u;
-                    }
-                    if (last && ++b == NACC)
-                    {
-                        b = 0;
-                        phb ^= 1u;
-                    }
+                }
+                __syncwarp();
+                last_commit = &afree[a];
+                last_par = pha;
+                s = (s + 1 == NST) ? 0 : s + 1;
+                if (++a == NA)
+                {
+                    a = 0;
+                    pha ^= 1u;
+                }
+                if (last && ++b == NACC)
+                {
+                    b = 0;
+                    phb ^= 1u;
                 }
             }
-            // every MMA this thread issued completes before the tensor memory is
-            // released, also when a wait above gave up (the commit tracks them all)
-            if (last_commit) mbar_wait_bounded(last_commit, last_par);
         }
+        // every MMA this warp issued completes before the tensor memory is
+        // released, also when a wait above gave up (the commit tracks them all)
+        if (last_commit) mbar_wait_bounded(last_commit, last_par);
     }
     else if (warp < 2 + 4 * tc_pq<KP>())
     {
@@ -634,64 +616,110 @@ __global__ void __launch_bounds__(TC_THREADS(KP, NDR), 1)
         const int MT = gd.mt_modes;
         const int row = 32 * q + lane;
         const int ml = row / gd.nbnds, m = row - ml * gd.nbnds;
-        const uint32_t swz = (uint32_t)(m & 7);
         const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
-        int s = 0, a = 0;
-        uint32_t ph = 0, pha = 0;
-        bool stop = false;
-        for (int u = blockIdx.x; u < nunits && !stop; u += gridDim.x)
-        {
-            const TcUnit w = tc_unit(u, nchunks, mtiles, gd.nspin, pairs);
+        uint32_t xo[8];  // the row's 16-byte chunks in a 128-byte swizzled 16-point psi block
+#pragma unroll
+        for (int j = 0; j < 8; ++j) xo[j] = (uint32_t)m * 128u + (((uint32_t)j ^ (uint32_t)(m & 7)) << 4);
+        const uint32_t sm32 = smem_u32(sm);
+        long long left = 0;  // stages of this CTA
+        for (int u = blockIdx.x; u < nunits; u += gridDim.x) left += nstage;
+        auto run = [&](auto share_type) {
+            typedef decltype(share_type) Share;
+            typedef typename Share::Frag Frag;
+            Share sh;
+            sh.p_half = L.p_half;
+            sh.p_comp = 2 * NATOM * L.p_half;
             // rows of modes past nmodes read the TMA zero fill of the dV tile; rows
             // past the tile's MT*nb read the zero block
             const bool in_tile = ml < MT;
-            // a K chunk never straddles spinor components (chunk_pts divides N)
-            const int sp = (int)(((long long)w.chunk * chunk_pts) / N);
-            int comp0, comp1;
-            if (gd.nmag == 4)
+            sh.dv_block = in_tile ? L.dv_block : 0u;
+            sh.dv_comp = in_tile ? 256u : 0u;
+            const int p0 = h * Share::PPW;  // the share's first point
+            const uint32_t psi0 = sm32 + L.p + (uint32_t)(p0 >> 4) * L.p_half;
+            const uint32_t dv0 = sm32 + L.dv + (uint32_t)(p0 >> 5) * L.dv_block + (uint32_t)(p0 & 31) * 8u +
+                                 (uint32_t)(ml * gd.nmag) * 256u;
+            int u = blockIdx.x, it = 0;
+            uint32_t dvc = 0;  // the unit's first dV component (nmag 4: the next one follows)
+            auto unit = [&]() {
+                // a K chunk never straddles spinor components (chunk_pts divides N)
+                const int zp = u / nchunks / mtiles;
+                const int sp = (int)(((long long)(u % nchunks) * chunk_pts) / N);
+                dvc = 256u * (uint32_t)(gd.nmag == 4 ? 2 * sp : (gd.nmag == 2 ? zp % gd.nspin : 0));
+            };
+            auto stage_at = [&](int s) {
+                sh.psi = psi0 + (uint32_t)s * L.stage_bytes;
+                sh.dv = in_tile ? dv0 + (uint32_t)s * L.stage_bytes + dvc : sm32 + L.bar_off + 512;  // 256 zero bytes
+            };
+            if (left > 0) unit();
+            int s = 0, a = 0;
+            uint32_t ph = 0, pha = 0;
+            Frag f[2];
+            bool ok = true, have = false;  // have: piece 0 of the stage is loaded
+            for (; left > 0; --left)
             {
-                comp0 = 2 * sp;
-                comp1 = 2 * sp + 1;
-            }
-            else
-            {
-                comp0 = (gd.nmag == 2) ? w.spin : 0;
-                comp1 = comp0;
-            }
-            for (int it = 0; it < nstage; ++it, s = (s + 1 == NST) ? 0 : s + 1, ph ^= (s == 0) ? 1u : 0u,
-                     a = (a + 1 == NA) ? 0 : a + 1, pha ^= (a == 0) ? 1u : 0u)
-            {
-                bool ok = mbar_wait_bounded(&afree[a], pha ^ 1u, wait_ns) && mbar_wait_bounded(&full[s], ph, wait_ns);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok && lane == 0)
+                if (!Share::PRE) ok = mbar_wait_bounded(&afree[a], pha ^ 1u, wait_ns);
+                if (!have)
                 {
-                    *abort_flag = 1;
-                    atomicOr(status, LELPH_DEV_ERR_TIMEOUT);
+                    ok = ok && mbar_wait_bounded(&full[s], ph, wait_ns);
+                    stage_at(s);
+                    if (__all_sync(0xffffffffu, ok)) sh.load(f[0], xo, 0);
+                    else ok = false;
                 }
-                if (__any_sync(0xffffffffu, !ok || *abort_flag != 0))
+                if (Share::PRE) ok = ok && mbar_wait_bounded(&afree[a], pha ^ 1u, wait_ns);
+                if (__any_sync(0xffffffffu, !ok))
                 {
-                    stop = true;
+                    if (lane == 0)
+                    {
+                        *abort_flag = 1;
+                        atomicOr(status, LELPH_DEV_ERR_TIMEOUT);
+                    }
                     break;
                 }
                 tc_fence_after();
-                const uint8_t* st = sm + s * L.stage_bytes;
-                const uint32_t col_base = lane_base + L.a_col0 + (uint32_t)a * (2u * KP);
-                if (gd.nmag == 4)
-                    produce_stage<BF16, KP, 4, 2, (tc_pq<KP>() <= 2)>(st, L, zero_dv, in_tile, h, m, ml, gd.nmag, comp0, comp1, nsp,
-                                                     swz, col_base);
-                else
-                    produce_stage<BF16, KP, 8, 1, (tc_pq<KP>() <= 2)>(st, L, zero_dv, in_tile, h, m, ml, gd.nmag, comp0, comp1, nsp,
-                                                     swz, col_base);
+                const uint32_t col = lane_base + L.a_col0 + (uint32_t)a * (2u * KP) + (uint32_t)p0;
+#pragma unroll
+                for (int t = 0; t < Share::NPIECE; ++t)
+                {
+                    // the loads of the next piece are issued before this one is formed and stored
+                    if (t + 1 < Share::NPIECE) sh.load(f[(t + 1) & 1], xo, t + 1);
+                    Share::template store<BF16>(f[t & 1], col + (uint32_t)(t * Share::SUBP));
+                }
+                // the next stage's first piece, when its tiles are there already: its latency and
+                // that of the stores' completion overlap (not with two components, nmag 4: the
+                // larger fragments made that 4 % slower)
+                const int s1 = s, a1 = a;
+                s = (s + 1 == NST) ? 0 : s + 1;
+                ph ^= (s == 0) ? 1u : 0u;
+                a = (a + 1 == NA) ? 0 : a + 1;
+                pha ^= (a == 0) ? 1u : 0u;
+                have = false;
+                if (left > 1)
+                {
+                    if (++it == nstage)
+                    {
+                        it = 0;
+                        u += gridDim.x;
+                        unit();
+                    }
+                    if (Share::PRE) have = __all_sync(0xffffffffu, mbar_test_wait(&full[s], ph));
+                    if (have)
+                    {
+                        stage_at(s);
+                        sh.load(f[0], xo, 0);
+                    }
+                }
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0)
                 {
-                    mbar_arrive(&aready[a]);
-                    mbar_arrive(&empty[s]);
+                    mbar_arrive(&aready[a1]);
+                    mbar_arrive(&empty[s1]);
                 }
             }
-        }
+        };
+        if (gd.nmag == 4) run(ProdShare<KP, 4, 2>());
+        else run(ProdShare<KP, 8, 1>());
     }
     else if (warp < 2 + 4 * tc_pq<KP>() + ndrain)
     {
