@@ -13,7 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT_DIR, "liblelph_gpu.so")
-SOURCES = ["fft_gather.cu", "sandwich.cu", "sandwich_f64.cu", "nonlocal.cu", "dvloc.cu", "rotate_dv.cu", "dmats.cu", "qstar.cu",
+SOURCES = ["fft_gather.cu", "fft_box.cu", "sandwich.cu", "sandwich_f64.cu", "nonlocal.cu", "dvloc.cu", "rotate_dv.cu", "dmats.cu", "qstar.cu",
            "dvscf.cu", "gspace.cu", "gspace_tc.cu", "projections_tc.cu", "lelph_gpu.cu",
            "ndb_elph.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

@@ -478,7 +478,8 @@ __global__ void __launch_bounds__(256) k_scatter(int k0, const KPointSym* __rest
                                                  const long long* __restrict__ coef_off, GeomDev gd,
                                                  T2* __restrict__ boxes, double2* __restrict__ chat,
                                                  float2* __restrict__ chat32, const long long* __restrict__ chat_off,
-                                                 const double2* __restrict__ sub_tw, BoxMask mk)
+                                                 const double2* __restrict__ sub_tw, float2* __restrict__ copies,
+                                                 long long copy_stride, BoxMask mk)
 {
     const int kslot = blockIdx.y;
     const int kbz = k0 + kslot;
@@ -521,7 +522,7 @@ __global__ void __launch_bounds__(256) k_scatter(int k0, const KPointSym* __rest
     // e^{i G.delta} of the shift of copy 1 (its powers: the other copies'), from exact
     // tables of the rational angles
     double2 sh = make_double2(1.0, 0.0);
-    if (nsub > 1 && bxb)
+    if (nsub > 1 && (bxb || copies))
     {
         const double2* tw = sub_tw;
         const int Ga[3] = {gd.sa[0] * G0, gd.sa[1] * G1, gd.sa[2] * G2}, Na[3] = {gd.Nx, gd.Ny, gd.Nz};
@@ -556,7 +557,16 @@ __global__ void __launch_bounds__(256) k_scatter(int k0, const KPointSym* __rest
             if (s.trev) w.y = -w.y;
             if (chb32) chb32[co + (size_t)sp * npw + g] = make_float2((float)w.x, (float)w.y);
             else chb[co + (size_t)sp * npw + g] = w;
-            if (bxb)
+            if (copies)
+            {
+                float2* cp = copies + chat_off[kbz] + co + (size_t)sp * npw + g;
+                for (int j = 1; j < nsub; ++j, cp += copy_stride)
+                {
+                    w = cmul(w, sh);
+                    *cp = make_float2((float)w.x, (float)w.y);
+                }
+            }
+            else if (bxb)
             {
                 T2* b = bxb + ((size_t)set * gd.nspinor + sp) * nsub * N + bidx;
                 *b = mk2<T2>(w.x, w.y);
@@ -828,15 +838,18 @@ void lelph_launch_fft_x_to_split(const float2* boxes, int nbox_k, int k0, const 
 void lelph_launch_scatter(int k0, int nk, const KPointSym* ksym_dev, const int* miller, const long long* pw_off,
                           const int* npw, int npw_max, const double2* coef, const long long* coef_off,
                           const GeomDev& g, int box_fp64, void* boxes, double2* chat, const long long* chat_off,
-                          const double2* sub_tw, cudaStream_t st, const BoxMask& mk, float2* chat32)
+                          const double2* sub_tw, cudaStream_t st, const BoxMask& mk, float2* chat32, float2* copies,
+                          long long copy_stride)
 {
     dim3 grid((unsigned)((npw_max + 255) / 256), nk);
     if (box_fp64)
         k_scatter<double2><<<grid, 256, 0, st>>>(k0, ksym_dev, miller, pw_off, npw, coef, coef_off, g,
-                                                 (double2*)boxes, chat, chat32, chat_off, sub_tw, mk);
+                                                 (double2*)boxes, chat, chat32, chat_off, sub_tw, copies,
+                                                 copy_stride, mk);
     else
         k_scatter<float2><<<grid, 256, 0, st>>>(k0, ksym_dev, miller, pw_off, npw, coef, coef_off, g,
-                                                (float2*)boxes, chat, chat32, chat_off, sub_tw, mk);
+                                                (float2*)boxes, chat, chat32, chat_off, sub_tw, copies,
+                                                copy_stride, mk);
 }
 
 void lelph_launch_gmap(const KPointSym* ks, int kbz, const int* miller, const long long* pw_off, const int* npw,

@@ -89,6 +89,7 @@ struct GridState
     DevBuf d_collist, d_colcnt;  // occupied z-columns of every k as lists
     bool boxmask_ready = false;  // occupancy and lists built (geometry only: they stay valid)
     long long box_columns = 0;
+    DevBuf d_boxpos, d_copies;  // whole boxes in shared memory (fft_box.cu): positions, coefficients of the copies
     // G-space route: every full-BZ k's sphere (its k+q role) sorted by
     // ((y, z) column, x) on the product grid, and the k+q coefficients stored
     // in that order (Bp)
@@ -102,7 +103,8 @@ struct GridState
     std::vector<DevBuf*> buffers()
     {
         return {&d_tw64[0], &d_tw64[1], &d_tw64[2], &d_tw32[0], &d_tw32[1], &d_tw32[2], &d_subtw64, &d_subtw32,
-                &d_psi64, &d_bsplit, &d_psi32, &d_epsi, &d_edv, &d_win64, &d_win32, &d_winscale, &d_colmask, &d_collist, &d_colcnt,
+                &d_psi64, &d_bsplit, &d_psi32, &d_epsi, &d_edv, &d_win64, &d_win32, &d_winscale, &d_colmask, &d_collist, &d_colcnt, &d_boxpos,
+                &d_copies,
                 &d_gs_perm, &d_gs_kcx, &d_gs_cols, &d_gs_cst, &d_gs_npw, &d_gs_npad, &d_gs_permoff, &d_gs_bpoff,
                 &d_gs_bp, &d_gs_shph, &d_gs_zl, &d_gs_cols2};
     }
@@ -169,6 +171,7 @@ struct lelph_gpu : GridState
     DevBuf d_dvraw;  // QE-layout dV_scf of the last ingest and eig pats^H
     bool dm_coef32_ready = false;
     long long coef_total = 0;  // complex coefficients of every iBZ k
+    long long chat_total = 0;  // and of every full-BZ k
     std::unordered_map<long long, int> khash;  // full-BZ k-points by wrapped, quantised coordinates
     bool dm_gtab_ready = false;
     long long dm_first = 0, dm_count = 0;
@@ -1611,6 +1614,7 @@ extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
         chtot += (long long)nsets * h->npw[h->ksym[i].ik];
     }
 
+    h->chat_total = chtot;
     // ---- device
     if (cudaSetDevice(h->device) != cudaSuccess) return bad(LELPH_GPU_ERR_CUDA, "cudaSetDevice");
     if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1724,6 +1728,23 @@ extern "C" int lelph_gpu_set_wavefunctions(lelph_gpu* h, const double* const* wf
 
 static int build_windows(lelph_gpu* h);
 
+// Occupied z-columns of every k as lists, from the column mask.
+static int build_col_lists(lelph_gpu* h, size_t ncol)
+{
+    const int nk = h->d.nkpts_BZ;
+    lelph_launch_col_lists((const uint8_t*)h->d_colmask.p, nk, (int)ncol, (int*)h->d_collist.p, (int*)h->d_colcnt.p,
+                           h->st);
+    CUDA_TRY(h, cudaGetLastError());
+    std::vector<int> cnt(nk);
+    CUDA_TRY(h, cudaMemcpyAsync(cnt.data(), h->d_colcnt.p, sizeof(int) * cnt.size(), cudaMemcpyDeviceToHost, h->st));
+    CUDA_TRY(h, cudaStreamSynchronize(h->st));
+    h->box_columns = 0;
+    for (int c : cnt) h->box_columns += c;
+    h->boxmask_ready = true;
+    h->stats.kernel_launches += 1;
+    return LELPH_GPU_OK;
+}
+
 // The q-independent stage on the active grid.
 static int prepare_grid(lelph_gpu* h)
 {
@@ -1781,6 +1802,51 @@ static int prepare_grid(lelph_gpu* h)
         if (rc) return rc;
         lelph_launch_oz_exponents(psi, nbk, d.nspinor * lelph_grid_points(g), OZ_GUARD_PSI, (int*)h->d_epsi.p, h->st);
         h->stats.kernel_launches += 5;
+    }
+    else if (h->sphere_window && chat_f32 && lelph_box_fft_supported(g))
+    {
+        // boxes that fit in shared memory: the coefficients of every copy of the grid, then one
+        // kernel from them to the operands.  (The plain grid keeps the multi-pass transforms,
+        // whose digits its results have.)
+        const size_t ncol = (size_t)g.Nx * g.Ny;
+        const long long chtot = h->chat_total;
+        rc = ensure(h, h->d_copies, sizeof(float2) * (size_t)std::max(1LL, (g.nsub - 1) * chtot));
+        if (rc) return rc;
+        gs_tick(h);
+        if (!h->boxmask_ready)
+        {
+            rc = ensure(h, h->d_colmask, (ncol + g.Nx) * d.nkpts_BZ);
+            if (!rc) rc = ensure(h, h->d_collist, sizeof(int) * ncol * d.nkpts_BZ);
+            if (!rc) rc = ensure(h, h->d_colcnt, sizeof(int) * d.nkpts_BZ);
+            if (!rc) rc = ensure(h, h->d_boxpos, sizeof(int) * (size_t)(chtot / nset_per_k));
+            if (rc) return rc;
+            CUDA_TRY(h, cudaMemsetAsync(h->d_colmask.p, 0, (ncol + g.Nx) * d.nkpts_BZ, h->st));
+            BoxMask mk;
+            mk.col = (uint8_t*)h->d_colmask.p;
+            mk.xpl = mk.col + ncol * d.nkpts_BZ;
+            lelph_launch_box_pos((const KPointSym*)h->d_ksym.p, d.nkpts_BZ, (const int*)h->d_miller.p,
+                                 (const long long*)h->d_pwoff.p, (const int*)h->d_npw.p, npw_max,
+                                 (const long long*)h->d_chatoff.p, g, (int*)h->d_boxpos.p, mk, h->st);
+            rc = build_col_lists(h, ncol);
+            if (rc) return rc;
+            h->stats.kernel_launches += 1;
+        }
+        lelph_launch_scatter(0, d.nkpts_BZ, (const KPointSym*)h->d_ksym.p, (const int*)h->d_miller.p,
+                             (const long long*)h->d_pwoff.p, (const int*)h->d_npw.p, npw_max,
+                             (const double2*)h->d_coef.p, (const long long*)h->d_coefoff.p, g, 0, nullptr,
+                             (double2*)h->d_chat.p, (const long long*)h->d_chatoff.p, sub_tw, h->st, BoxMask(),
+                             (float2*)h->d_chat.p, g.nsub > 1 ? (float2*)h->d_copies.p : nullptr, chtot);
+        h->stats.prep_scatter_ms += gs_tock(h);
+        if (lelph_launch_box_fft_split((const float2*)h->d_chat.p, (const float2*)h->d_copies.p, chtot,
+                                       (const KPointSym*)h->d_ksym.p, d.nkpts_BZ, (const int*)h->d_npw.p,
+                                       (const long long*)h->d_chatoff.p, (const int*)h->d_boxpos.p,
+                                       (const int*)h->d_collist.p, (const int*)h->d_colcnt.p,
+                                       (const uint8_t*)h->d_colmask.p, g, (const float*)h->d_band_scale.p, h->ab_bf16,
+                                       (uint16_t*)h->d_bsplit.p, (float2*)h->d_psi32.p, h->st))
+            return fail(h, LELPH_GPU_ERR_UNSUPPORTED, "wavefunction box launch configuration");
+        h->stats.prep_xsplit_ms += gs_tock(h);
+        h->stats.kernel_launches += 2;
+        CUDA_TRY(h, cudaGetLastError());
     }
     else
     {
@@ -1845,16 +1911,8 @@ static int prepare_grid(lelph_gpu* h)
         }
         if (!masks)
         {
-            lelph_launch_col_lists(col_all, d.nkpts_BZ, (int)ncol, (int*)h->d_collist.p, (int*)h->d_colcnt.p, h->st);
-            CUDA_TRY(h, cudaGetLastError());
-            std::vector<int> cnt(d.nkpts_BZ);
-            CUDA_TRY(h, cudaMemcpyAsync(cnt.data(), h->d_colcnt.p, sizeof(int) * cnt.size(), cudaMemcpyDeviceToHost,
-                                        h->st));
-            CUDA_TRY(h, cudaStreamSynchronize(h->st));
-            h->box_columns = 0;
-            for (int c : cnt) h->box_columns += c;
-            h->boxmask_ready = true;
-            h->stats.kernel_launches += 1;
+            rc = build_col_lists(h, ncol);
+            if (rc) return rc;
         }
     }
     NonlocalDesc nl = nl_desc(h);

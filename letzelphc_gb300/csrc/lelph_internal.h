@@ -124,13 +124,25 @@ void lelph_launch_col_lists(const uint8_t* col, int nk, int ncol, int* list, int
 void lelph_launch_clear_cols(float2* boxes, int nk, int nbox_per_k, long long N, int Nz, int ncol, const int* list,
                              const int* cnt, cudaStream_t st);
 
-// sphere -> box scatter with su2, fractional-translation phase and conj; sub_tw: per axis i
+// whole wavefunction boxes in shared memory (fft_box.cu): positions and occupancy
+// (geometry only), then coefficients -> operands of the tensor-core sandwich
+bool lelph_box_fft_supported(const GeomDev& g);
+void lelph_launch_box_pos(const KPointSym* ks, int nk, const int* miller, const long long* pw_off, const int* npw,
+                          int npw_max, const long long* chat_off, const GeomDev& g, int* pos, const BoxMask& mk,
+                          cudaStream_t st);
+int lelph_launch_box_fft_split(const float2* coef0, const float2* coefs, long long copy_stride, const KPointSym* ks,
+                               int nk, const int* npw, const long long* chat_off, const int* pos, const int* collist,
+                               const int* colcnt, const uint8_t* colmask, const GeomDev& g, const float* band_scale,
+                               int ab_bf16, uint16_t* Bsplit, float2* psi32, cudaStream_t st);
+
+// sphere -> box scatter with su2, fractional-translation phase and conj (boxes may be null); copies: the FP32
+// coefficients of the grid's copies 1 .. nsub-1 in chat32's layout, copy_stride apart; sub_tw: per axis i
 // the table e^{+2 pi i t / (nsub N_i)}, t < nsub N_i (x, y, z in sequence), for the copies' shifts
 void lelph_launch_scatter(int k0, int nk, const KPointSym* ksym_dev, const int* miller, const long long* pw_off,
                           const int* npw, int npw_max, const double2* coef, const long long* coef_off,
                           const GeomDev& g, int box_fp64, void* boxes, double2* chat, const long long* chat_off,
                           const double2* sub_tw, cudaStream_t st, const BoxMask& mk = BoxMask(),
-                          float2* chat32 = nullptr);
+                          float2* chat32 = nullptr, float2* copies = nullptr, long long copy_stride = 0);
 
 // debugging / parity: box index of each rotated plane wave of one full-BZ k
 void lelph_launch_gmap(const KPointSym* ks, int kbz, const int* miller, const long long* pw_off, const int* npw,
