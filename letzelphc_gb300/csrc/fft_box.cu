@@ -9,7 +9,9 @@
 // bounds it is writing those (24 bytes a point); the multi-pass form
 // (fft_gather.cu: scatter into cleared boxes, z, y and x passes over HBM) moved
 // every box four more times.
-// FB_MEASURED
+// Measured for 512 k x 32 bands x 2 copies of 24^3: scatter 1.7 + z, y 3.8 + x pass
+// 2.1 ms -> 1.2 (unfolding, FP64 pipe) + 2.8 ms (10.9 GB written: 58 % of the
+// measured copy bandwidth); 432 k x 13 bands of 20^3: 0.81 -> 0.37 ms.
 #include <cuda_runtime.h>
 #include <stdint.h>
 

@@ -151,7 +151,7 @@ struct lelph_gpu : GridState
     DevBuf d_dvr, d_eig, d_maxabs;                 // per q slot: dV_scf on the reference box (FP64), eigVec
     DevBuf d_wtmpN, d_wtmpM;
     DevBuf d_pairs, d_glocal, d_partials, d_gout, d_status, d_tmp;
-    std::vector<int> ulms_all;  // every q slot's umklapp list, the host side of one upload
+    std::vector<char> win_tab;  // window tables of every q slot, the host side of one upload
     int Nbox[3] = {0, 0, 0};
     double Rc[3] = {0, 0, 0};  // largest |k+G| component (crystal units) over every rotated sphere
     double Gc = 0;             // largest |k+G| (cartesian, no 2 pi)
@@ -1984,6 +1984,11 @@ struct WinGeom
     int sphere;
     float q[3], gm[6], cut2;  // |D + q|^2 <= cut2 for the needed differences
 };
+// One window: its q slot (in the group of a launch) and umklapp vector.
+struct WinItem
+{
+    int slot, ulm[3];
+};
 
 // dV on the product grid for one (q slot, umklapp G0): with dVhat the
 // normalised forward transform of dV on the reference box,
@@ -2001,14 +2006,18 @@ struct WinGeom
 // One thread per residue finds the representatives once and applies them to
 // its share of the components (grid y).  The inverse transform per copy follows.
 template <typename T2, int P>
-__global__ void __launch_bounds__(256) k_dv_window(const T2* __restrict__ dvhat, int ncomp, WinGeom wg,
-                                                   const int* __restrict__ ulms, const T2* __restrict__ sub_tw,
+__global__ void __launch_bounds__(256) k_dv_window(const T2* __restrict__ dvhat, int ncomp,
+                                                   const WinGeom* __restrict__ geoms,
+                                                   const WinItem* __restrict__ items, const T2* __restrict__ sub_tw,
                                                    double invN, T2* __restrict__ out)
 {
+    const int u = blockIdx.z;  // window
+    const WinItem item = items[u];
+    const WinGeom wg = geoms[item.slot];
     const int Ns = wg.n[0] * wg.n[1] * wg.n[2];
     const size_t NN = (size_t)wg.N[0] * wg.N[1] * wg.N[2];
-    const int u = blockIdx.z;  // umklapp index
-    const int um[3] = {ulms[3 * u], ulms[3 * u + 1], ulms[3 * u + 2]};
+    dvhat += (size_t)item.slot * ncomp * NN;
+    const int um[3] = {item.ulm[0], item.ulm[1], item.ulm[2]};
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < Ns; r += gridDim.x * blockDim.x)
     {
         int t[3];
@@ -2122,14 +2131,15 @@ __global__ void __launch_bounds__(256) k_dv_window(const T2* __restrict__ dvhat,
 }
 
 template <typename T2>
-static void launch_dv_window(const T2* dvhat, int ncomp, const WinGeom& wg, int nsub, const int* ulms, int nu,
+static void launch_dv_window(const T2* dvhat, int ncomp, const WinGeom* wg, int nsub, const WinItem* items, int nwin,
                              const T2* sub_tw, double invN, T2* out, cudaStream_t st)
 {
-    const dim3 grid(64, (unsigned)((ncomp + 3) / 4), (unsigned)nu);
-    if (nsub == 1) k_dv_window<T2, 1><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, ulms, sub_tw, invN, out);
-    else if (nsub == 2) k_dv_window<T2, 2><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, ulms, sub_tw, invN, out);
-    else if (nsub == 3) k_dv_window<T2, 3><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, ulms, sub_tw, invN, out);
-    else k_dv_window<T2, 4><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, ulms, sub_tw, invN, out);
+    // residues of a window over 64 CTAs, fewer where many windows fill the chip
+    const dim3 grid(nwin >= 16 ? 16u : 64u, (unsigned)((ncomp + 3) / 4), (unsigned)nwin);
+    if (nsub == 1) k_dv_window<T2, 1><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
+    else if (nsub == 2) k_dv_window<T2, 2><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
+    else if (nsub == 3) k_dv_window<T2, 3><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
+    else k_dv_window<T2, 4><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
 }
 
 // Load q slot `slot`: eigVec and dV (host); dVscf == nullptr loads zeros.
@@ -2590,14 +2600,13 @@ static int build_windows(lelph_gpu* h)
     const int P = g.nsub;
     const int ncomp = d.nmodes * d.nmag;
     h->win_base.assign(h->qslots.size(), -1);
-    int nwin = 0, umax = 0;
+    int nwin = 0;
     for (size_t s = 0; s < h->qslots.size(); ++s)
         if (h->qslots[s].set)
         {
             h->win_base[s] = nwin;
             int nu = (int)h->qslots[s].ulms.size() / 3;
             nwin += nu;
-            umax = std::max(umax, nu);
         }
     h->nwin = nwin;
     if (nwin == 0)
@@ -2605,25 +2614,61 @@ static int build_windows(lelph_gpu* h)
         h->windows_ok = true;
         return LELPH_GPU_OK;
     }
-    int rc = ensure(h, h->d_wtmpN, sizeof(double2) * ncomp * NN);
-    if (rc) return rc;
-    rc = ensure(h, h->d_wtmpM, sizeof(double2) * (size_t)umax * ncomp * M);
-    if (rc) return rc;
-    // the umklapp lists of every slot, uploaded in one copy (a pageable copy
-    // may wait for the stream, so one per slot would stall the queue per slot)
-    h->ulms_all.clear();
-    std::vector<size_t> uoff(h->qslots.size(), 0);
-    for (size_t s = 0; s < h->qslots.size(); ++s)
-        if (h->qslots[s].set)
+    // Groups of neighbouring slots share the launches: their transforms are batches
+    // of lines, and one launch per pass instead of one per pass and slot matters (8 slots
+    // of the 4-atom cell: 88 launches, 1.4 ms -> 11, 0.9 ms; 3 of a 2-atom cell, 0.33 -> 0.17).  A group's scratch stays
+    // within 512 MB on the reference box and 1 GB on the product grid, or one slot's.
+    const size_t esz = h->mixed ? sizeof(float2) : sizeof(double2);
+    struct Group
+    {
+        int s0, ns, w0, nw;
+    };
+    std::vector<Group> groups;
+    size_t needN = 0, needM = 0;
+    h->win_tab.clear();
+    std::vector<size_t> tab_off;
+    for (int s = 0; s < (int)h->qslots.size();)
+    {
+        const int nu0 = h->qslots[s].set ? (int)h->qslots[s].ulms.size() / 3 : 0;
+        if (nu0 == 0)
         {
-            uoff[s] = h->ulms_all.size();
-            h->ulms_all.insert(h->ulms_all.end(), h->qslots[s].ulms.begin(), h->qslots[s].ulms.end());
+            ++s;
+            continue;
         }
-    rc = ensure(h, h->d_tmp, sizeof(int) * h->ulms_all.size() + 16);
+        Group gr{s, 0, h->win_base[s], 0};
+        while (s < (int)h->qslots.size() && h->qslots[s].set && !h->qslots[s].ulms.empty())
+        {
+            const int nu = (int)h->qslots[s].ulms.size() / 3;
+            if (gr.ns > 0 && ((size_t)(gr.ns + 1) * ncomp * NN * esz > (512ull << 20) ||
+                              (size_t)(gr.nw + nu) * ncomp * M * esz > (1ull << 30) || gr.nw + nu > 32768))
+                break;
+            ++gr.ns;
+            gr.nw += nu;
+            ++s;
+        }
+        needN = std::max(needN, (size_t)(gr.ns * ncomp * NN) * esz);
+        needM = std::max(needM, (size_t)(gr.nw * ncomp * M) * esz);
+        // geometries, then windows
+        tab_off.push_back(h->win_tab.size());
+        h->win_tab.resize(h->win_tab.size() + sizeof(WinGeom) * gr.ns + sizeof(WinItem) * gr.nw);
+        WinGeom* wg = reinterpret_cast<WinGeom*>(h->win_tab.data() + tab_off.back());
+        WinItem* wi = reinterpret_cast<WinItem*>(wg + gr.ns);
+        for (int i = 0; i < gr.ns; ++i)
+        {
+            const QSlot& q = h->qslots[gr.s0 + i];
+            wg[i] = win_geom(h, q);
+            for (size_t e = 0; e < q.ulms.size(); e += 3) *wi++ = WinItem{i, {q.ulms[e], q.ulms[e + 1], q.ulms[e + 2]}};
+        }
+        groups.push_back(gr);
+    }
+    int rc = ensure(h, h->d_wtmpN, needN);
     if (rc) return rc;
-    if (!h->ulms_all.empty())
-        CUDA_TRY(h, cudaMemcpyAsync(h->d_tmp.p, h->ulms_all.data(), sizeof(int) * h->ulms_all.size(),
-                                    cudaMemcpyHostToDevice, h->st));
+    rc = ensure(h, h->d_wtmpM, needM);
+    if (rc) return rc;
+    // the tables of every group, uploaded in one copy
+    rc = ensure(h, h->d_tmp, h->win_tab.size() + 16);
+    if (rc) return rc;
+    CUDA_TRY(h, cudaMemcpyAsync(h->d_tmp.p, h->win_tab.data(), h->win_tab.size(), cudaMemcpyHostToDevice, h->st));
     if (!h->mixed)
     {
         rc = ensure(h, h->d_win64, sizeof(double2) * (size_t)nwin * ncomp * M);
@@ -2637,79 +2682,77 @@ static int build_windows(lelph_gpu* h)
         if (rc) return rc;
         rc = ensure(h, h->d_winscale, sizeof(float) * (size_t)nwin * d.nmodes);
         if (rc) return rc;
-        rc = ensure(h, h->d_maxabs, sizeof(unsigned) * (size_t)umax * d.nmodes);
+        rc = ensure(h, h->d_maxabs, sizeof(unsigned) * (size_t)nwin * d.nmodes);
         if (rc) return rc;
     }
-    for (size_t s = 0; s < h->qslots.size(); ++s)
+    for (size_t ig = 0; ig < groups.size(); ++ig)
     {
-        if (!h->qslots[s].set) continue;
-        const int nu = (int)h->qslots[s].ulms.size() / 3;
-        if (nu == 0) continue;
+        const Group& gr = groups[ig];
+        const WinGeom* wg = reinterpret_cast<const WinGeom*>((const char*)h->d_tmp.p + tab_off[ig]);
+        const WinItem* wi = reinterpret_cast<const WinItem*>(wg + gr.ns);
+        const long long nbN = (long long)gr.ns * ncomp, nbM = (long long)gr.nw * ncomp * P;
+        const double2* dv = (const double2*)h->d_dvr.p + (size_t)gr.s0 * ncomp * NN;
         if (h->mixed)
         {
-            // mixed form: FP32 transforms (the windows end up as FP32 tiles);
-            // the scratch arrays of the FP64 path hold the FP32 data
+            // mixed form: FP32 transforms (the windows end up as FP32 tiles)
             float2* tN = (float2*)h->d_wtmpN.p;
             float2* tM = (float2*)h->d_wtmpM.p;
-            lelph_launch_dm_c64((const double2*)h->d_dvr.p + (size_t)s * ncomp * NN, (long long)ncomp * NN, tN, h->st);
-            lelph_launch_fft_contig_f(tN, (long long)ncomp * h->Nbox[0] * h->Nbox[1], h->planN[2],
-                                      (const float2*)h->d_twN32[2].p, -1, h->st);
-            lelph_launch_fft_strided_f(tN, (long long)ncomp * h->Nbox[0], h->Nbox[2], h->planN[1],
-                                       (const float2*)h->d_twN32[1].p, -1, h->st);
-            lelph_launch_fft_strided_f(tN, (long long)ncomp, h->Nbox[1] * h->Nbox[2], h->planN[0],
-                                       (const float2*)h->d_twN32[0].p, -1, h->st);
-            launch_dv_window<float2>(tN, ncomp, win_geom(h, h->qslots[s]), P, (const int*)h->d_tmp.p + uoff[s], nu,
-                                     (const float2*)h->d_subtw32.p, 1.0 / (double)NN, tM, h->st);
-            lelph_launch_fft_contig_f(tM, (long long)nu * ncomp * P * g.Nx * g.Ny, h->plan[2],
-                                      (const float2*)h->d_tw32[2].p, +1, h->st);
-            lelph_launch_fft_strided_f(tM, (long long)nu * ncomp * P * g.Nx, g.Nz, h->plan[1],
-                                       (const float2*)h->d_tw32[1].p, +1, h->st);
-            lelph_launch_fft_strided_f(tM, (long long)nu * ncomp * P, g.Ny * g.Nz, h->plan[0],
-                                       (const float2*)h->d_tw32[0].p, +1, h->st);
+            lelph_launch_dm_c64(dv, nbN * NN, tN, h->st);
+            lelph_launch_fft_contig_f(tN, nbN * h->Nbox[0] * h->Nbox[1], h->planN[2], (const float2*)h->d_twN32[2].p,
+                                      -1, h->st);
+            lelph_launch_fft_strided_f(tN, nbN * h->Nbox[0], h->Nbox[2], h->planN[1], (const float2*)h->d_twN32[1].p,
+                                       -1, h->st);
+            lelph_launch_fft_strided_f(tN, nbN, h->Nbox[1] * h->Nbox[2], h->planN[0], (const float2*)h->d_twN32[0].p,
+                                       -1, h->st);
+            launch_dv_window<float2>(tN, ncomp, wg, P, wi, gr.nw, (const float2*)h->d_subtw32.p, 1.0 / (double)NN, tM,
+                                     h->st);
+            lelph_launch_fft_contig_f(tM, nbM * g.Nx * g.Ny, h->plan[2], (const float2*)h->d_tw32[2].p, +1, h->st);
+            lelph_launch_fft_strided_f(tM, nbM * g.Nx, g.Nz, h->plan[1], (const float2*)h->d_tw32[1].p, +1, h->st);
+            lelph_launch_fft_strided_f(tM, nbM, g.Ny * g.Nz, h->plan[0], (const float2*)h->d_tw32[0].p, +1, h->st);
             if (h->gspace)
             {
                 // the G-space route reads the windows as plain FP32 boxes
-                CUDA_TRY(h, cudaMemcpyAsync((float2*)h->d_win32.p + (size_t)h->win_base[s] * ncomp * M, tM,
-                                            sizeof(float2) * (size_t)nu * ncomp * M, cudaMemcpyDeviceToDevice, h->st));
-                h->stats.kernel_launches += 7;
+                CUDA_TRY(h, cudaMemcpyAsync((float2*)h->d_win32.p + (size_t)gr.w0 * ncomp * M, tM,
+                                            sizeof(float2) * (size_t)gr.nw * ncomp * M, cudaMemcpyDeviceToDevice, h->st));
+                h->stats.kernel_launches += 8;
                 CUDA_TRY(h, cudaGetLastError());
                 continue;
             }
+            const int nwm = gr.nw * d.nmodes;
             unsigned* mx = (unsigned*)h->d_maxabs.p;
-            float* sc = (float*)h->d_winscale.p + (size_t)h->win_base[s] * d.nmodes;
-            CUDA_TRY(h, cudaMemsetAsync(mx, 0, sizeof(unsigned) * nu * d.nmodes, h->st));
-            k_dv_maxabs<float2><<<dim3(64, nu * d.nmodes), 256, 0, h->st>>>(tM, nu * d.nmodes, d.nmag, M, mx);
-            k_mode_scale<<<(nu * d.nmodes + 63) / 64, 64, 0, h->st>>>(mx, nu * d.nmodes, sc);
-            k_dv_convert<float2><<<1024, 256, 0, h->st>>>(tM, (float2*)h->d_win32.p, nu, (int)ncomp, M,
-                                                          h->win_base[s], d.nmag, sc);
+            float* sc = (float*)h->d_winscale.p + (size_t)gr.w0 * d.nmodes;
+            CUDA_TRY(h, cudaMemsetAsync(mx, 0, sizeof(unsigned) * nwm, h->st));
+            // (grid.y <= 65535: a group holds at most 32768 windows, launched in slices)
+            for (int r0 = 0; r0 < nwm; r0 += 32768)
+            {
+                const int nr = std::min(32768, nwm - r0);
+                k_dv_maxabs<float2><<<dim3(nr >= 512 ? 8 : 64, nr), 256, 0, h->st>>>(tM + (size_t)r0 * d.nmag * M, nr,
+                                                                                     d.nmag, M, mx + r0);
+            }
+            k_mode_scale<<<(nwm + 63) / 64, 64, 0, h->st>>>(mx, nwm, sc);
+            k_dv_convert<float2><<<2048, 256, 0, h->st>>>(tM, (float2*)h->d_win32.p, gr.nw, (int)ncomp, M, gr.w0,
+                                                          d.nmag, sc);
             h->stats.kernel_launches += 11;
             CUDA_TRY(h, cudaGetLastError());
             continue;
         }
         // plain form: FP64 transforms
         double2* tN = (double2*)h->d_wtmpN.p;
-        double2* tM = (double2*)h->d_wtmpM.p;
-        CUDA_TRY(h, cudaMemcpyAsync(tN, (const double2*)h->d_dvr.p + (size_t)s * ncomp * NN,
-                                    sizeof(double2) * ncomp * NN, cudaMemcpyDeviceToDevice, h->st));
+        double2* tM = (double2*)h->d_win64.p + (size_t)gr.w0 * ncomp * M;  // in place
+        CUDA_TRY(h, cudaMemcpyAsync(tN, dv, sizeof(double2) * nbN * NN, cudaMemcpyDeviceToDevice, h->st));
         // forward transform on the reference box (FFTW_FORWARD, unnormalised)
-        lelph_launch_fft_contig_d(tN, (long long)ncomp * h->Nbox[0] * h->Nbox[1], h->planN[2],
-                                  (const double2*)h->d_twN[2].p, -1, h->st);
-        lelph_launch_fft_strided_d(tN, (long long)ncomp * h->Nbox[0], h->Nbox[2], h->planN[1],
-                                   (const double2*)h->d_twN[1].p, -1, h->st);
-        lelph_launch_fft_strided_d(tN, (long long)ncomp, h->Nbox[1] * h->Nbox[2], h->planN[0],
-                                   (const double2*)h->d_twN[0].p, -1, h->st);
-        launch_dv_window<double2>(tN, ncomp, win_geom(h, h->qslots[s]), P, (const int*)h->d_tmp.p + uoff[s], nu,
-                                  (const double2*)h->d_subtw64.p, 1.0 / (double)NN, tM, h->st);
+        lelph_launch_fft_contig_d(tN, nbN * h->Nbox[0] * h->Nbox[1], h->planN[2], (const double2*)h->d_twN[2].p, -1,
+                                  h->st);
+        lelph_launch_fft_strided_d(tN, nbN * h->Nbox[0], h->Nbox[2], h->planN[1], (const double2*)h->d_twN[1].p, -1,
+                                   h->st);
+        lelph_launch_fft_strided_d(tN, nbN, h->Nbox[1] * h->Nbox[2], h->planN[0], (const double2*)h->d_twN[0].p, -1,
+                                   h->st);
+        launch_dv_window<double2>(tN, ncomp, wg, P, wi, gr.nw, (const double2*)h->d_subtw64.p, 1.0 / (double)NN, tM,
+                                  h->st);
         // inverse transform on the product grid
-        lelph_launch_fft_contig_d(tM, (long long)nu * ncomp * P * g.Nx * g.Ny, h->plan[2], (const double2*)h->d_tw64[2].p,
-                                  +1, h->st);
-        lelph_launch_fft_strided_d(tM, (long long)nu * ncomp * P * g.Nx, g.Nz, h->plan[1], (const double2*)h->d_tw64[1].p,
-                                   +1, h->st);
-        lelph_launch_fft_strided_d(tM, (long long)nu * ncomp * P, g.Ny * g.Nz, h->plan[0], (const double2*)h->d_tw64[0].p,
-                                   +1, h->st);
-        const size_t base = (size_t)h->win_base[s] * ncomp * M;
-        CUDA_TRY(h, cudaMemcpyAsync((double2*)h->d_win64.p + base, tM, sizeof(double2) * (size_t)nu * ncomp * M,
-                                    cudaMemcpyDeviceToDevice, h->st));
+        lelph_launch_fft_contig_d(tM, nbM * g.Nx * g.Ny, h->plan[2], (const double2*)h->d_tw64[2].p, +1, h->st);
+        lelph_launch_fft_strided_d(tM, nbM * g.Nx, g.Nz, h->plan[1], (const double2*)h->d_tw64[1].p, +1, h->st);
+        lelph_launch_fft_strided_d(tM, nbM, g.Ny * g.Nz, h->plan[0], (const double2*)h->d_tw64[0].p, +1, h->st);
         h->stats.kernel_launches += 7;
         CUDA_TRY(h, cudaGetLastError());
     }
