@@ -20,8 +20,11 @@
 // a third of that time.  The SIMT kernel that this replaces did the whole
 // contraction on the FP64 pipe (8 nb flops per element instead of 6).
 // Measured, SIMT -> this: 64 pairs of 384 rows x 32 bands x 27,648 points, 176 ->
-// 12.5 ms; 64 pairs of 48 x 8 x 5,832, 12.6 -> 0.40 ms; error against 64 bits
-// (norm) 5.5e-15 -> 1.9e-15 and 3.4e-15 -> 0.9e-15.
+// 11.3 ms; 64 pairs of 48 x 8 x 5,832, 12.6 -> 0.36 ms; error against 64 bits
+// (norm) 5.5e-15 -> 1.9e-15 and 3.4e-15 -> 0.9e-15.  (With 16 warps instead of 32:
+// 12.5 and 0.41 ms; the FP64 pipe is busy 40 % of the time, the rest is latency
+// between the barriers.  Forming part of the next stage's products between the digit
+// stores: no change; two rows at a time in straight-line code: 3 % slower.)
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -32,13 +35,14 @@
 #include "tc_operands.cuh"
 
 #define OZ_S 7        // digits
-#define OZ_THREADS 512
+#define OZ_THREADS 1024
 #define OZ_WARPS (OZ_THREADS / 32)
 #define OZ_ROWS 128   // (mode, band of k) rows of a tile
 #define OZ_BANDS 32   // bands of k+q of a tile
 #define OZ_PTS 32     // grid points of a stage (one 128-byte K atom of (re, im) digits)
 #define OZ_RPW (OZ_ROWS / OZ_WARPS)
 #define OZ_BPW (OZ_BANDS / OZ_WARPS)
+#define OZ_COLS (2 * OZ_BANDS / (OZ_WARPS / 4))  // accumulator columns of a thread (its row of the tile)
 
 struct OzRow
 {
@@ -213,13 +217,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             }
         }
     };
-    // this thread's 16 columns of its row: levels 0..3 exactly, 4..6 in FP32
+    // this thread's OZ_COLS columns of its row: levels 0..3 exactly, 4..6 in FP32
     const int cg = warp >> 2;
-    const bool mine = cg * 16 < NT;
-    long long H[16];
-    float L[16];
+    const bool mine = cg * OZ_COLS < NT;
+    long long H[OZ_COLS];
+    float L[OZ_COLS];
 #pragma unroll
-    for (int c = 0; c < 16; ++c)
+    for (int c = 0; c < OZ_COLS; ++c)
     {
         H[c] = 0;
         L[c] = 0.f;
@@ -227,23 +231,23 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     auto drain = [&]() {
         if (mine)
         {
-            const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(cg * 16);
-            float v[16];
+            const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(cg * OZ_COLS);
+            float v[OZ_COLS];
 #pragma unroll
             for (int l = 0; l < 4; ++l)
             {
-                tmem_ld16(ta + (uint32_t)(l * NT), v);
+                tmem_ld8(ta + (uint32_t)(l * NT), v);
 #pragma unroll
-                for (int c = 0; c < 16; ++c)
+                for (int c = 0; c < OZ_COLS; ++c)
                     H[c] += (long long)__float2int_rn(v[c]) * (long long)(1 << (27 - 9 * l));
             }
 #pragma unroll
             for (int l = 4; l < OZ_S; ++l)
             {
-                tmem_ld16(ta + (uint32_t)(l * NT), v);
+                tmem_ld8(ta + (uint32_t)(l * NT), v);
                 const float w = l == 4 ? 1.f : (l == 5 ? 0x1p-9f : 0x1p-18f);
 #pragma unroll
-                for (int c = 0; c < 16; ++c) L[c] = fmaf(v[c], w, L[c]);
+                for (int c = 0; c < OZ_COLS; ++c) L[c] = fmaf(v[c], w, L[c]);
             }
         }
         tc_fence_before();
@@ -307,9 +311,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             const bool bad = ss.badrow[r] != 0;
             double* o = out + (size_t)blockIdx.z * chunk_stride + 2 * ((size_t)zp * nrows + R) * nb;
 #pragma unroll
-            for (int c = 0; c < 16; ++c)
+            for (int c = 0; c < OZ_COLS; ++c)
             {
-                const int col = cg * 16 + c, im = col >= nbp, b = im ? col - nbp : col;
+                const int col = cg * OZ_COLS + c, im = col >= nbp, b = im ? col - nbp : col;
                 if (b >= nbt) continue;
                 // (H 2^27 + L 2^18) units of 2^(54 - 124) of the two scales' product
                 double v = fma((double)H[c], 0x1p27, (double)L[c] * 0x1p18);
