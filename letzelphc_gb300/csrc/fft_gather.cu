@@ -721,9 +721,9 @@ static void launch_strided(T2* data, long long nouter, int inner, const FftPlan1
 }
 
 void lelph_launch_fft_contig_d(double2* data, long long nlines, const FftPlan1D& p, const double2* tw, int sign,
-                               cudaStream_t st)
+                               cudaStream_t st, const BoxMask& mk)
 {
-    launch_contig<double2, double>(data, nlines, p, tw, sign, st, BoxMask());
+    launch_contig<double2, double>(data, nlines, p, tw, sign, st, mk);
 }
 void lelph_launch_fft_contig_f(float2* data, long long nlines, const FftPlan1D& p, const float2* tw, int sign,
                                cudaStream_t st, const BoxMask& mk)
@@ -731,9 +731,9 @@ void lelph_launch_fft_contig_f(float2* data, long long nlines, const FftPlan1D& 
     launch_contig<float2, float>(data, nlines, p, tw, sign, st, mk);
 }
 void lelph_launch_fft_strided_d(double2* data, long long nouter, int inner, const FftPlan1D& p, const double2* tw,
-                                int sign, cudaStream_t st)
+                                int sign, cudaStream_t st, const BoxMask& mk)
 {
-    launch_strided<double2, double>(data, nouter, inner, p, tw, sign, st, BoxMask());
+    launch_strided<double2, double>(data, nouter, inner, p, tw, sign, st, mk);
 }
 void lelph_launch_fft_strided_f(float2* data, long long nouter, int inner, const FftPlan1D& p, const float2* tw,
                                 int sign, cudaStream_t st, const BoxMask& mk)

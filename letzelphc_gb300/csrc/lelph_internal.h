@@ -106,11 +106,11 @@ struct BoxMask
 // their digits; interleaved grids use all of them.
 bool lelph_fft_fixed(int L, int all);
 void lelph_launch_fft_contig_d(double2* data, long long nlines, const FftPlan1D& p, const double2* tw, int sign,
-                               cudaStream_t st);
+                               cudaStream_t st, const BoxMask& mk = BoxMask());
 void lelph_launch_fft_contig_f(float2* data, long long nlines, const FftPlan1D& p, const float2* tw, int sign,
                                cudaStream_t st, const BoxMask& mk = BoxMask());
 void lelph_launch_fft_strided_d(double2* data, long long nouter, int inner, const FftPlan1D& p, const double2* tw,
-                                int sign, cudaStream_t st);
+                                int sign, cudaStream_t st, const BoxMask& mk = BoxMask());
 void lelph_launch_fft_strided_f(float2* data, long long nouter, int inner, const FftPlan1D& p, const float2* tw,
                                 int sign, cudaStream_t st, const BoxMask& mk = BoxMask());
 // x-pass of the mixed form writing the split tensor-core operand directly
