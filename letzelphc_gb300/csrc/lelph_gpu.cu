@@ -2836,6 +2836,16 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
     for (int x = 0; x < 3; ++x) tw[x] = f64 ? h->d_tw64[x].p : h->d_tw32[x].p;
     const void* winb = f64 ? h->d_win64.p : h->d_win32.p;
     GsGeom gg{g.Nx, g.Ny, g.Nz, g.nsub, nb, ns, d.nmag, 0, f64 || h->plan[0].allct};
+    // psi(r) of a k: z pass on its occupied columns, y pass on its occupied x planes
+    const size_t ncolbox = (size_t)g.Nx * g.Ny;
+    rc = ensure(h, h->d_colmask, ncolbox + g.Nx);
+    if (rc) return rc;
+    BoxMask mk;
+    mk.col = (uint8_t*)h->d_colmask.p;
+    mk.xpl = mk.col + ncolbox;
+    mk.Nx = g.Nx;
+    mk.Ny = g.Ny;
+    mk.nbox_per_k = nbox;
     int cur = -1;
     for (int oi = 0; oi < n; ++oi)
     {
@@ -2845,23 +2855,28 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
         {
             cur = P.kbz_k;
             CUDA_TRY(h, cudaMemsetAsync(h->d_gs_psi.p, 0, e * (size_t)nset * M, h->st));
+            CUDA_TRY(h, cudaMemsetAsync(h->d_colmask.p, 0, ncolbox + g.Nx, h->st));
             lelph_launch_scatter(cur, 1, (const KPointSym*)h->d_ksym.p, (const int*)h->d_miller.p,
                                  (const long long*)h->d_pwoff.p, (const int*)h->d_npw.p, npw_max,
                                  (const double2*)h->d_coef.p, (const long long*)h->d_coefoff.p, g, f64, h->d_gs_psi.p,
                                  (double2*)h->d_chat.p, (const long long*)h->d_chatoff.p,
-                                 (const double2*)h->d_subtw64.p, h->st);
+                                 (const double2*)h->d_subtw64.p, h->st, mk);
             if (f64)
             {
                 double2* bx = (double2*)h->d_gs_psi.p;
-                lelph_launch_fft_contig_d(bx, (long long)nbox * g.Nx * g.Ny, h->plan[2], (const double2*)tw[2], +1, h->st);
-                lelph_launch_fft_strided_d(bx, (long long)nbox * g.Nx, g.Nz, h->plan[1], (const double2*)tw[1], +1, h->st);
+                lelph_launch_fft_contig_d(bx, (long long)nbox * g.Nx * g.Ny, h->plan[2], (const double2*)tw[2], +1, h->st,
+                                          mk);
+                lelph_launch_fft_strided_d(bx, (long long)nbox * g.Nx, g.Nz, h->plan[1], (const double2*)tw[1], +1, h->st,
+                                           mk);
                 lelph_launch_fft_strided_d(bx, nbox, g.Ny * g.Nz, h->plan[0], (const double2*)tw[0], +1, h->st);
             }
             else
             {
                 float2* bx = (float2*)h->d_gs_psi.p;
-                lelph_launch_fft_contig_f(bx, (long long)nbox * g.Nx * g.Ny, h->plan[2], (const float2*)tw[2], +1, h->st);
-                lelph_launch_fft_strided_f(bx, (long long)nbox * g.Nx, g.Nz, h->plan[1], (const float2*)tw[1], +1, h->st);
+                lelph_launch_fft_contig_f(bx, (long long)nbox * g.Nx * g.Ny, h->plan[2], (const float2*)tw[2], +1, h->st,
+                                          mk);
+                lelph_launch_fft_strided_f(bx, (long long)nbox * g.Nx, g.Nz, h->plan[1], (const float2*)tw[1], +1, h->st,
+                                           mk);
                 lelph_launch_fft_strided_f(bx, nbox, g.Ny * g.Nz, h->plan[0], (const float2*)tw[0], +1, h->st);
             }
             h->stats.kernel_launches += 4;
