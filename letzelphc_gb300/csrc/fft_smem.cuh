@@ -221,6 +221,44 @@ __device__ __forceinline__ void dft_base(T2* v, int sign)
     if constexpr (R == 5) dft5<T2, T>(v, sign);
 }
 
+// cos and sin of 2 pi m / n at compile time (Taylor series on the first octant)
+__host__ __device__ constexpr double ct_taylor(double x, int k0)
+{
+    double s = 0, t = k0 ? x : 1.0;
+    for (int k = k0; k < k0 + 26; k += 2)
+    {
+        s += t;
+        t *= -x * x / ((k + 1.0) * (k + 2.0));
+    }
+    return s;
+}
+__host__ __device__ constexpr double ct_trig(int m, int n, bool sine)
+{
+    m %= n;
+    // angle in units of 2 pi / (8 n): octant and remainder
+    const int a = 8 * m, o = a / n, r = a - o * n;
+    const double p4 = 0.785398163397448309615660845819875721;
+    const double x = p4 * (o % 2 ? n - r : r) / n;  // distance to the nearer axis
+    const bool swap = o == 1 || o == 2 || o == 5 || o == 6;
+    const double v = ct_taylor(x, sine != swap ? 1 : 0);
+    const bool neg = sine ? o >= 4 : (o >= 2 && o < 6);
+    return neg ? -v : v;
+}
+
+template <int R>
+struct CtTwiddles
+{
+    float c[R]{}, s[R]{};
+    __host__ __device__ constexpr CtTwiddles()
+    {
+        for (int m = 0; m < R; ++m)
+        {
+            c[m] = (float)ct_trig(m, R, false);
+            s[m] = (float)ct_trig(m, R, true);
+        }
+    }
+};
+
 // DFT of R = R1 R2 points in registers: R2 DFTs of R1 points over the
 // stride-R2 subsets, twiddles w_R^(n2 k1) (w_R^m = tw[m L / R], tw holding
 // e^{+2 pi i t / L}), then R1 DFTs of R2 points; X[k1 + R1 k2].
@@ -247,9 +285,23 @@ __device__ __forceinline__ void dft_ct(T2* v, int sign, const T2* __restrict__ t
                 T2 x = u[k1];
                 if (n2 * k1 != 0)
                 {
-                    T2 w = tw[n2 * k1 * (L / R)];
-                    if (sign < 0) w.y = -w.y;
-                    x = cmul(x, w);
+                    // FP32: the same rounded values as constants (a table read per butterfly
+                    // takes a twentieth of the shared-memory pipe of the plane passes),
+                    // quarter turns without a product
+                    if constexpr (sizeof(T) == sizeof(float))
+                    {
+                        constexpr CtTwiddles<R> ct{};
+                        if (4 * n2 * k1 == R)
+                            x = sign < 0 ? mk2<T2>(x.y, -x.x) : mk2<T2>(-x.y, x.x);
+                        else
+                            x = cmul(x, mk2<T2>(ct.c[n2 * k1], sign < 0 ? -ct.s[n2 * k1] : ct.s[n2 * k1]));
+                    }
+                    else
+                    {
+                        T2 w = tw[n2 * k1 * (L / R)];
+                        if (sign < 0) w.y = -w.y;
+                        x = cmul(x, w);
+                    }
                 }
                 t[n2 * R1 + k1] = x;
             }

@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_plane(const T2* __restrict__ 
 // ------------------------------------------- plane pass, compile-time sizes
 // The same transform for square planes of the common product-grid sizes with
 // the compile-time Stockham schedule (ct_fft, fft_smem.cuh).  The z lines sit
-// at a padded stride (Nz + 1), so consecutive threads, taking consecutive
+// at an odd stride, so consecutive threads, taking consecutive
 // lines, hit distinct banks; the second (y) transform runs only on the z
 // lines that hold a column of the k+q sphere (their list zl; the result is
 // compact, element y of line l at l + y nzl).
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_plane_ct(const T2* __restrict
                                                             T2* __restrict__ out)
 {
     static_assert(ct_smooth(NY) && ct_smooth(NZ), "2, 3, 5-smooth plane");
-    constexpr int NZP = NZ + 1;       // padded z-line stride
+    constexpr int NZP = NZ | 1;       // z-line stride, odd
     constexpr int NP = NY * NZP;
     extern __shared__ __align__(16) unsigned char gsc_smem[];
     T2* a = reinterpret_cast<T2*>(gsc_smem);
@@ -123,13 +123,13 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_plane_ct(const T2* __restrict
             const T2* d0 = dv + (size_t)(2 * s) * M;
             const T2* d1 = d0 + M;
             for (int e = threadIdx.x; e < NPL; e += GS_THREADS)
-                a[e + e / NZ] = cadd(cmul(d0[e], pm[e]), cmul(d1[e], pm[M + e]));
+                a[e + e / NZ * (NZP - NZ)] = cadd(cmul(d0[e], pm[e]), cmul(d1[e], pm[M + e]));
         }
         else
         {
             const T2* d0 = dv + (size_t)(gg.nmag == 2 ? gg.spin : 0) * M;
             const T2* p0 = pm + (size_t)s * M;
-            for (int e = threadIdx.x; e < NPL; e += GS_THREADS) a[e + e / NZ] = cmul(d0[e], p0[e]);
+            for (int e = threadIdx.x; e < NPL; e += GS_THREADS) a[e + e / NZ * (NZP - NZ)] = cmul(d0[e], p0[e]);
         }
         __syncthreads();
         // z lines (line y at y NZP), then the y transform of the sphere's z lines
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(GS_THREADS, 3) k_gs_plane_ct1(const float2* __
                                                                const int* __restrict__ zl, int nzl,
                                                                float2* __restrict__ out)
 {
-    constexpr int NZP = NZ + 1;
+    constexpr int NZP = NZ | 1;
     constexpr int NP = NY * NZP;
     constexpr int NPL = NY * NZ;
     constexpr int PER = (NPL + GS_THREADS - 1) / GS_THREADS;
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(GS_THREADS, 3) k_gs_plane_ct1(const float2* __
         for (int i = 0; i < PER; ++i)
         {
             const int e = threadIdx.x + i * GS_THREADS;
-            if (e < NPL) a[e + e / NZ] = cmul(d0[e], ps[i]);
+            if (e < NPL) a[e + e / NZ * (NZP - NZ)] = cmul(d0[e], ps[i]);
         }
         __syncthreads();
         float2* r = ct_fft<float2, float, NZ, 0, 1, true, NY>(a, b, NY, 1, NZP, nullptr, 1, NZP, tz, -1);
@@ -601,11 +601,149 @@ __global__ void __launch_bounds__(GS_THREADS, 3) k_gs_plane_ct1(const float2* __
     }
 }
 
+// Stages STAGE .. LAST - 1 of ct_fft (the caller runs the last one itself).
+template <int L, int STAGE, int LAST, int NS>
+__device__ __forceinline__ float2* ct_fft_head(float2* a, float2* b, int nlines, int es_s, int ls_s, const int* loff,
+                                               int es, int ls, const float2* tw)
+{
+    if constexpr (STAGE == LAST)
+        return a;
+    else
+    {
+        constexpr int R = ct_radix_at(L, STAGE);
+        ct_pass<float2, float, L, R, NS, true, 0>(a, b, nlines, es_s, ls_s, loff, es, ls, tw, -1);
+        __syncthreads();
+        return ct_fft_head<L, STAGE + 1, LAST, NS * R>(b, a, nlines, es, ls, nullptr, es, ls, tw);
+    }
+}
+
+// The same for the interleaved grids, with the plane's ends fused: the y
+// transform goes first, so that its first stage takes element y = j + r Ny/R of
+// line z for thread j Nz + z - consecutive threads on consecutive points of the
+// plane in global memory - and forms dV psi in registers (psi held there for all
+// NUC modes); the z transform then runs on the sphere's y lines (yl), and its
+// last stage writes the sphere's columns to global memory through their map
+// (cmap[z nyl + line] = column or -1; the columns are sorted by (z, y), so
+// neighbouring lines write neighbouring columns).  Shared-memory bandwidth bounds
+// it: 8 -> 5 transfers per point, two barriers fewer per mode.
+// 48 x 48 planes take 160 threads (144 butterflies of 16 points; five CTAs an SM):
+// 31.1 ms for 8 pairs of 48 modes x 200 bands x 64 planes, 33.9 with 256, 42.8 with
+// 128; the LSU pipe is busy 75 % of the time.
+// Measured against k_gs_plane_ct1 (1152 products): 24 x 24 planes 4.3 -> 3.1 ms,
+// 30 x 30 7.5 -> 5.8, 40 x 40 10.9 -> 7.7, 48 x 48 12.2 -> 10.4, 60 x 60 34.3 -> 29.9.
+template <int NY, int NZ, int NUC, int NT>
+__global__ void __launch_bounds__(NT, NT == 160 ? 5 : 3) k_gs_plane_yz(const float2* __restrict__ psi,
+                                                              const float2* __restrict__ win, GsGeom gg, int nu0,
+                                                              int nub, const float2* __restrict__ twy,
+                                                              const float2* __restrict__ twz,
+                                                              const int* __restrict__ cmap, int ncol,
+                                                              const int* __restrict__ yl, int nyl,
+                                                              float2* __restrict__ out)
+{
+    constexpr int NZP = NZ | 1;
+    constexpr int NPL = NY * NZ;
+    constexpr int R0 = ct_radix_at(NY, 0);
+    constexpr int LR0 = NY / R0;
+    constexpr int NW = LR0 * NZ;  // butterflies of the first stage
+    constexpr int ITEMS = (NW + NT - 1) / NT;
+    constexpr int SL = ct_nstage(NZ) - 1;  // last z stage: radix RL on stride NSL
+    constexpr int RL = ct_radix_at(NZ, SL);
+    constexpr int NSL = NZ / RL;
+    static_assert(ct_nstage(NY) >= 2 && SL >= 1, "at least two stages per direction");
+    extern __shared__ __align__(16) unsigned char gsy_smem[];
+    float2* a = reinterpret_cast<float2*>(gsy_smem);
+    float2* b = a + NY * NZP;
+    float2* ty = b + NY * NZP;
+    float2* tz = ty + NY;
+    int* syl = reinterpret_cast<int*>(tz + NZ);
+    short* smap = reinterpret_cast<short*>(syl + NY);
+    const int m = blockIdx.y, x = blockIdx.z;
+    const int nl0 = blockIdx.x * NUC, nl1 = min(nub, nl0 + NUC);
+    for (int t = threadIdx.x; t < NY; t += blockDim.x) ty[t] = twy[t];
+    for (int t = threadIdx.x; t < NZ; t += blockDim.x) tz[t] = twz[t];
+    for (int t = threadIdx.x; t < nyl; t += blockDim.x) syl[t] = yl[t] * NZP;
+    for (int t = threadIdx.x; t < nyl * NZ; t += blockDim.x) smap[t] = (short)cmap[t];
+    const long long M = (long long)gg.nsub * gg.Nx * NPL;
+    const size_t xoff = (size_t)x * NPL;
+    const float2* pm = psi + (size_t)m * M + xoff;
+    const int comp = gg.nmag == 2 ? gg.spin : 0;
+    const RecipDiv dl = recip_div(nyl);
+    float2 ps[ITEMS][R0];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+    {
+        const int w = threadIdx.x + i * NT;
+#pragma unroll
+        for (int r = 0; r < R0; ++r) ps[i][r] = w < NW ? pm[w + r * NW] : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    for (int nul = nl0; nul < nl1; ++nul)
+    {
+        const float2* d0 = win + ((size_t)(nu0 + nul) * gg.nmag + comp) * M + xoff;
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i)
+        {
+            const int w = threadIdx.x + i * NT;
+            if (w < NW)
+            {
+                const int j = w / NZ, z = w - j * NZ;
+                float2 v[R0];
+#pragma unroll
+                for (int r = 0; r < R0; ++r) v[r] = d0[w + r * NW];
+#pragma unroll
+                for (int r = 0; r < R0; ++r) v[r] = cmul(v[r], ps[i][r]);
+                dft_ct<float2, float, R0, NY>(v, -1, ty);
+#pragma unroll
+                for (int r = 0; r < R0; ++r) a[(j * R0 + r) * NZP + z] = v[r];
+            }
+        }
+        __syncthreads();
+        float2* r = ct_fft<float2, float, NY, 1, R0, true, NZ>(a, b, NZ, NZP, 1, nullptr, NZP, 1, ty, -1);
+        float2* o = r == a ? b : a;
+        r = ct_fft_head<NZ, 0, SL, 1>(r, o, nyl, 1, 0, syl, nyl, 1, tz);
+        float2* dst = out + ((size_t)(nul * gg.nb + m) * gg.nsub * gg.Nx + x) * ncol;
+        for (int w = threadIdx.x; w < nyl * NSL; w += NT)
+        {
+            int line;
+            const int j = div_rem(w, dl, line);
+            float2 v[RL];
+#pragma unroll
+            for (int q = 0; q < RL; ++q) v[q] = r[(j + q * NSL) * nyl + line];
+            if (j != 0)
+            {
+#pragma unroll
+                for (int q = 1; q < RL; ++q)
+                {
+                    float2 t = tz[q * j];
+                    t.y = -t.y;
+                    v[q] = cmul(v[q], t);
+                }
+            }
+            dft_ct<float2, float, RL, NZ>(v, -1, tz);
+#pragma unroll
+            for (int q = 0; q < RL; ++q)
+            {
+                const int c = smap[(j + q * NSL) * nyl + line];
+                if (c >= 0) dst[c] = v[q];
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Planes that k_gs_plane_yz takes: FP32, one spinor component, interleaved grids
+// (the plain grid keeps the order of the transforms, and with it the digits that
+// the one-call stage returns), compile-time sizes whose psi fits the registers.
+bool lelph_gs_plane_yz(const GsGeom& gg, int fp64)
+{
+    return !fp64 && gg.nspinor == 1 && gg.allct && lelph_gs_plane_fixed(gg, 0) && gg.Ny <= 64;
+}
+
 template <typename T2, typename T, int N>
 static int gs_plane_ct(const GsGeom& gg, const void* psi, const void* win, int nu0, int nub, const void* twy,
                        const void* twz, const int* cols2, int ncol, const int* zl, int nzl, void* out, cudaStream_t st)
 {
-    const size_t smem = sizeof(T2) * (2 * (size_t)N * (N + 1) + 2 * N) + sizeof(int) * N;
+    const size_t smem = sizeof(T2) * (2 * (size_t)N * (N | 1) + 2 * N) + sizeof(int) * N;
     // (planes up to 64 x 64: the psi and window planes of a thread fit its registers)
     if constexpr (sizeof(T2) == sizeof(float2) && N * N <= 4096)
     {
@@ -613,6 +751,25 @@ static int gs_plane_ct(const GsGeom& gg, const void* psi, const void* win, int n
         {
             constexpr int NUC = 8;
             dim3 g1((unsigned)((nub + NUC - 1) / NUC), (unsigned)gg.nb, (unsigned)(gg.nsub * gg.Nx));
+            if (lelph_gs_plane_yz(gg, 0))
+            {
+                const size_t s2 = sizeof(float2) * (2 * (size_t)N * (N | 1) + 2 * N) + sizeof(int) * N +
+                                  sizeof(short) * ((size_t)nzl * N);
+                constexpr int NT = N <= 48 ? 160 : 256;  // psi of a plane in at most 32 registers
+                static bool attr2 = false;
+                if (!attr2)
+                {
+                    if (cudaFuncSetAttribute(k_gs_plane_yz<N, N, NUC, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(sizeof(float2) * (2 * (size_t)N * (N | 1) + 2 * N) +
+                                                   sizeof(int) * N + sizeof(short) * (size_t)N * N)) != cudaSuccess)
+                        return -1;
+                    attr2 = true;
+                }
+                k_gs_plane_yz<N, N, NUC, NT><<<g1, NT, s2, st>>>((const float2*)psi, (const float2*)win, gg, nu0, nub,
+                                                                     (const float2*)twy, (const float2*)twz, cols2, ncol,
+                                                                     zl, nzl, (float2*)out);
+                return 0;
+            }
             static bool attr1 = false;
             if (!attr1)
             {
@@ -726,6 +883,16 @@ static int gs_xpass_ct(int nrb, int ncol, int nsub, const void* twx, const int* 
     return 0;
 }
 
+bool lelph_gs_xpass_fixed(const GsGeom& gg)
+{
+    switch (gg.Nx)
+    {
+    case 36: case 48: case 60: case 64: case 72: case 80: case 96: return true;
+    case 16: case 20: case 24: case 30: case 32: case 40: case 45: case 54: return gg.allct != 0;
+    default: return false;
+    }
+}
+
 int lelph_launch_gs_xpass(const GsGeom& gg, int fp64, const void* in, int nrb, int ncol, const FftPlan1D& px,
                           const void* twx, const int* cst, const int* kcx, const void* shph, int npad, void* A,
                           cudaStream_t st, void* A_lo)
@@ -739,9 +906,11 @@ int lelph_launch_gs_xpass(const GsGeom& gg, int fp64, const void* in, int nrb, i
                                                           A_lo, st)                                         \
                     : gs_xpass_ct<float2, float, N, 64>(nrb, ncol, gg.nsub, twx, cst, kcx, shph, npad, in, A, A_lo, \
                                                         st);
-    if (gg.allct || gg.Nx == 36 || gg.Nx == 48 || gg.Nx == 60 || gg.Nx == 64 || gg.Nx == 72 || gg.Nx == 80 || gg.Nx == 96)
+    if (lelph_gs_xpass_fixed(gg))
     switch (gg.Nx)
     {
+        GS_XC(16)
+        GS_XC(20)
         GS_XC(24)
         GS_XC(30)
         GS_XC(32)
@@ -749,6 +918,7 @@ int lelph_launch_gs_xpass(const GsGeom& gg, int fp64, const void* in, int nrb, i
         GS_XC(40)
         GS_XC(45)
         GS_XC(48)
+        GS_XC(54)
         GS_XC(60)
         GS_XC(64)
         GS_XC(72)

@@ -94,7 +94,7 @@ struct GridState
     // ((y, z) column, x) on the product grid, and the k+q coefficients stored
     // in that order (Bp)
     std::vector<int> gs_npad, gs_ncol, gs_nzl;
-    std::vector<long long> gs_perm_off, gs_col_off, gs_cst_off, gs_bp_off, gs_zl_off;
+    std::vector<long long> gs_perm_off, gs_col_off, gs_cst_off, gs_bp_off, gs_zl_off, gs_c2_off;
     int gs_npad_max = 0, gs_ncol_max = 0;
     long long gs_bp_total = 0;
     DevBuf d_gs_perm, d_gs_kcx, d_gs_cols, d_gs_cst, d_gs_npw, d_gs_npad, d_gs_permoff, d_gs_bpoff, d_gs_bp;
@@ -820,6 +820,8 @@ static int gs_tables(lelph_gpu* h)
     const lelph_gpu_desc& d = h->d;
     const GeomDev& g = h->g;
     const int nk = d.nkpts_BZ;
+    const GsGeom gg{g.Nx, g.Ny, g.Nz, g.nsub, d.nbnds, d.nspinor, d.nmag, 0, !h->mixed || h->plan[0].allct};
+    const bool yz = lelph_gs_plane_yz(gg, !h->mixed);
     std::vector<std::vector<int>> perm(nk), kcx(nk), cols(nk), cst(nk), zls(nk), cols2(nk);
     std::vector<std::vector<double2>> shph(nk);
     std::vector<int> bad(nk, 0);
@@ -837,7 +839,7 @@ static int gs_tables(lelph_gpu* h)
                 G[r] = (ks.W[3 * r] * n[0] + ks.W[3 * r + 1] * n[1] + ks.W[3 * r + 2] * n[2]) % N3[r];
                 if (G[r] < 0) G[r] += N3[r];
             }
-            v[p] = {((long long)G[1] * g.Nz + G[2]) * g.Nx + G[0], p};
+            v[p] = {(yz ? (long long)G[2] * g.Ny + G[1] : (long long)G[1] * g.Nz + G[2]) * g.Nx + G[0], p};
         }
         std::sort(v.begin(), v.end());
         std::vector<int>& pm = perm[k];
@@ -884,6 +886,23 @@ static int gs_tables(lelph_gpu* h)
         // z lines of the sphere's columns, and each column's place in the
         // result of the y transform run on those lines only
         std::vector<int>& zl = zls[k];
+        std::vector<int>& c2 = cols2[k];
+        if (yz)
+        {
+            // the fused plane pass: y lines of the columns, and the map (z, line) -> column
+            std::vector<int> ypos(g.Ny, -1);
+            for (int c : cl) ypos[c % g.Ny] = 1;
+            for (int y = 0; y < g.Ny; ++y)
+                if (ypos[y] > 0)
+                {
+                    ypos[y] = (int)zl.size();
+                    zl.push_back(y);
+                }
+            c2.assign((size_t)g.Nz * zl.size(), -1);
+            for (size_t c = 0; c < cl.size(); ++c)
+                c2[(size_t)(cl[c] / g.Ny) * zl.size() + ypos[cl[c] % g.Ny]] = (int)c;
+            return;
+        }
         std::vector<int> zpos(g.Nz, -1);
         for (int c : cl) zpos[c % g.Nz] = 1;
         for (int z = 0; z < g.Nz; ++z)
@@ -892,7 +911,6 @@ static int gs_tables(lelph_gpu* h)
                 zpos[z] = (int)zl.size();
                 zl.push_back(z);
             }
-        std::vector<int>& c2 = cols2[k];
         c2.resize(cl.size());
         for (size_t c = 0; c < cl.size(); ++c) c2[c] = (cl[c] / g.Nz) * (int)zl.size() + zpos[cl[c] % g.Nz];
     };
@@ -913,8 +931,9 @@ static int gs_tables(lelph_gpu* h)
     h->gs_bp_off.resize(nk);
     h->gs_nzl.resize(nk);
     h->gs_zl_off.resize(nk);
+    h->gs_c2_off.resize(nk);
     std::vector<int> npw_k(nk);
-    long long po = 0, co = 0, so = 0, bo = 0, zo = 0;
+    long long po = 0, co = 0, so = 0, bo = 0, zo = 0, c2o = 0;
     h->gs_npad_max = h->gs_ncol_max = 0;
     for (int k = 0; k < nk; ++k)
     {
@@ -932,18 +951,20 @@ static int gs_tables(lelph_gpu* h)
         h->gs_nzl[k] = (int)zls[k].size();
         h->gs_zl_off[k] = zo;
         zo += h->gs_nzl[k];
+        h->gs_c2_off[k] = c2o;
+        c2o += (long long)cols2[k].size();
         h->gs_npad_max = std::max(h->gs_npad_max, h->gs_npad[k]);
         h->gs_ncol_max = std::max(h->gs_ncol_max, h->gs_ncol[k]);
     }
     h->gs_bp_total = bo;
-    std::vector<int> pall(po, 0), kall(po, 0), call(co), sall(so), c2all(co), zall(std::max(1LL, zo));
+    std::vector<int> pall(po, 0), kall(po, 0), call(co), sall(so), c2all(c2o), zall(std::max(1LL, zo));
     for (int k = 0; k < nk; ++k)
     {
         std::copy(perm[k].begin(), perm[k].end(), pall.begin() + h->gs_perm_off[k]);
         std::copy(kcx[k].begin(), kcx[k].end(), kall.begin() + h->gs_perm_off[k]);
         std::copy(cols[k].begin(), cols[k].end(), call.begin() + h->gs_col_off[k]);
         std::copy(cst[k].begin(), cst[k].end(), sall.begin() + h->gs_cst_off[k]);
-        std::copy(cols2[k].begin(), cols2[k].end(), c2all.begin() + h->gs_col_off[k]);
+        std::copy(cols2[k].begin(), cols2[k].end(), c2all.begin() + h->gs_c2_off[k]);
         std::copy(zls[k].begin(), zls[k].end(), zall.begin() + h->gs_zl_off[k]);
     }
     int rc;
@@ -1197,6 +1218,11 @@ static void pick_grid(const lelph_gpu* h, const double gm[6], const int ext[3], 
         {
             GsGeom gg{g.n[0], g.n[1], g.n[2], g.nsub, d.nbnds, d.nspinor, d.nmag, 0, !h->mixed || g.sphere};
             if (!lelph_gs_plane_fixed(gg, !h->mixed)) w *= 1.4;
+            // an x pass of run-time length takes three times as long (a fifth of the route)
+            if (!lelph_gs_xpass_fixed(gg)) w *= 1.3;
+            // butterflies of 15 x 3 points: 45 x 45 planes took 0.235 ns a point and mode, 48 x 48 ones 0.211
+            // (half of the route)
+            if (g.n[1] % 4 != 0) w *= 1.05;
         }
         return w;
     };
@@ -2917,7 +2943,7 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
                 gs_tick(h);
                 bad |= lelph_launch_gs_plane(gg, f64, psi, win, nu0, nmb, h->plan[1], h->plan[2], tw[1], tw[2],
                                              (const int*)h->d_gs_cols.p + h->gs_col_off[kq], ncol,
-                                             (const int*)h->d_gs_cols2.p + h->gs_col_off[kq],
+                                             (const int*)h->d_gs_cols2.p + h->gs_c2_off[kq],
                                              (const int*)h->d_gs_zl.p + h->gs_zl_off[kq], h->gs_nzl[kq],
                                              h->d_gs_out1.p, h->st);
                 h->stats.gs_plane_ms += gs_tock(h);

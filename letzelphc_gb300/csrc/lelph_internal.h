@@ -161,6 +161,9 @@ size_t lelph_gs_xpass_smem(const GsGeom& gg, int fp64);
 // plane pass of modes nu0 .. nu0+nub-1: out [(nu - nu0) nb + m][s][x][ncol]; square planes of the
 // sizes lelph_gs_plane_fixed accepts run the compile-time kernel (cols2, zl: pruned y transform)
 bool lelph_gs_plane_fixed(const GsGeom& gg, int fp64);
+bool lelph_gs_xpass_fixed(const GsGeom& gg);
+// planes of the fused y, z kernel: columns sorted by (z, y), cols2 the map (z, y line) -> column, zl the y lines
+bool lelph_gs_plane_yz(const GsGeom& gg, int fp64);
 int lelph_launch_gs_plane(const GsGeom& gg, int fp64, const void* psi, const void* win, int nu0, int nub,
                           const FftPlan1D& py, const FftPlan1D& pz, const void* twy, const void* twz, const int* cols,
                           int ncol, const int* cols2, const int* zl, int nzl, void* out, cudaStream_t st);
