@@ -55,7 +55,8 @@ template <typename T> static constexpr size_t pj_smem_bytes()
 {
     typedef typename cplx_of<T>::type C2;
     constexpr int G = PjCfg<T>::G;
-    return sizeof(C2) * (PJ_ROWS * (G + 1) + G * (PJ_SETS + 1) + 4 * G) + sizeof(T) * (16 * G + 3 * G);
+    constexpr int BR = sizeof(T) == 8 ? PJ_ROWS / 4 : PJ_ROWS;  // rows of beta kept
+    return sizeof(C2) * (BR * (G + 1) + G * (PJ_SETS + 1) + 4 * G) + sizeof(T) * (16 * G + 3 * G);
 }
 
 // grid: (nk, row blocks, set blocks x gsplit); 256 threads, 4 rows x 2 sets per
@@ -67,6 +68,10 @@ template <typename T> static constexpr size_t pj_smem_bytes()
 // FP32 and the chunk sums in FP64; the K vectors, Y_lm and the structure-factor
 // phases e^{-i 2pi K.tau} are evaluated in FP64 (the mixed form reduces the
 // phase angle to one turn in FP64 and takes sine and cosine in FP32).
+// T = double: the FP64 pipe bounds it, so a thread's four rows, which are one
+// (atom, projector) with its four components, share u = beta_0 conj(c^): 12 FP64
+// operations a point and set instead of 24 (1 and K_x times u), and only beta_0 is
+// formed.  64 k x 64 rows x 32 sets x 2500 plane waves: 4.5 -> 2.2 ms.
 template <typename T>
 __global__ void __launch_bounds__(256) k_projections(int k0, const KPointSym* __restrict__ ks,
                                                      const double* __restrict__ gvec,
@@ -79,10 +84,11 @@ __global__ void __launch_bounds__(256) k_projections(int k0, const KPointSym* __
 {
     typedef typename cplx_of<T>::type C2;
     constexpr int PG = PjCfg<T>::G;
-    constexpr int PARTS = 256 / PG;
+    constexpr bool D = std::is_same<T, double>::value;
+    constexpr int BR = D ? PJ_ROWS / 4 : PJ_ROWS;  // rows of beta_s: every row, or x = 0 of every four
     extern __shared__ __align__(16) unsigned char pj_smem[];
-    C2* beta_s = reinterpret_cast<C2*>(pj_smem);   // [PJ_ROWS][PG + 1]
-    C2* ch_s = beta_s + PJ_ROWS * (PG + 1);          // [PG][PJ_SETS + 1]
+    C2* beta_s = reinterpret_cast<C2*>(pj_smem);   // [BR][PG + 1]
+    C2* ch_s = beta_s + BR * (PG + 1);          // [PG][PJ_SETS + 1]
     C2* ph_s = ch_s + PG * (PJ_SETS + 1);            // [4][PG]
     T* ylm_s = reinterpret_cast<T*>(ph_s + 4 * PG);  // [16][PG]
     T* kx_s = ylm_s + 16 * PG;                       // [3][PG]
@@ -192,7 +198,6 @@ __global__ void __launch_bounds__(256) k_projections(int k0, const KPointSym* __
                 }
             }
         }
-        (void)PARTS;
         for (int e = threadIdx.x; e < ns * PG; e += blockDim.x)
         {
             const int ss = e / PG, gg = e - ss * PG;
@@ -201,9 +206,9 @@ __global__ void __launch_bounds__(256) k_projections(int k0, const KPointSym* __
         }
         __syncthreads();
         // beta_x(G) = F e^{-i 2pi K.tau} Y_lm (1 | K_x sign)  (src/nonloc/Vbare_nloc.c:318-363)
-        for (int e = threadIdx.x; e < PJ_ROWS * PG; e += blockDim.x)
+        for (int e = threadIdx.x; e < BR * PG; e += blockDim.x)
         {
-            const int rr = e / PG, gg = e - rr * PG;
+            const int br = e / PG, gg = e - br * PG, rr = D ? 4 * br : br;
             C2 b;
             b.x = 0;
             b.y = 0;
@@ -213,14 +218,36 @@ __global__ void __launch_bounds__(256) k_projections(int k0, const KPointSym* __
                 const C2 ph = ph_s[rinfo[rr][0] * PG + gg];
                 T fy = f * ylm_s[rinfo[rr][1] * PG + gg];
                 const int x = rinfo[rr][3];
-                if (x > 0) fy *= kx_s[(x - 1) * PG + gg] * rsign[rr];
+                if (!D && x > 0) fy *= kx_s[(x - 1) * PG + gg] * rsign[rr];
                 b.x = fy * ph.x;
                 b.y = fy * ph.y;
             }
-            beta_s[rr * (PG + 1) + gg] = b;
+            beta_s[br * (PG + 1) + gg] = b;
         }
         __syncthreads();
         // Pi += beta conj(c^) over the chunk
+        if constexpr (D)
+        {
+#pragma unroll 4
+            for (int gg = 0; gg < ng; ++gg)
+            {
+                const C2 b0 = beta_s[tr * (PG + 1) + gg];
+                const T K[3] = {kx_s[gg], kx_s[PG + gg], kx_s[2 * PG + gg]};
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                {
+                    const C2 u = cmul(b0, ch_s[gg * (PJ_SETS + 1) + tsx * 2 + j]);
+                    acc[0][j] = cadd(acc[0][j], u);
+#pragma unroll
+                    for (int x = 0; x < 3; ++x)
+                    {
+                        acc[1 + x][j].x = fma(K[x], u.x, acc[1 + x][j].x);
+                        acc[1 + x][j].y = fma(K[x], u.y, acc[1 + x][j].y);
+                    }
+                }
+            }
+        }
+        else
 #pragma unroll 8
         for (int gg = 0; gg < PG; ++gg)
         {
@@ -256,8 +283,13 @@ __global__ void __launch_bounds__(256) k_projections(int k0, const KPointSym* __
             const int rr = tr * 4 + i, ss = tsx * 2 + j;
             if (rr < nr && ss < ns)
             {
-                double2 v = std::is_same<T, float>::value ? acc64[i][j]
-                                                          : make_double2((double)acc[i][j].x, (double)acc[i][j].y);
+                double2 v = D ? make_double2((double)acc[i][j].x, (double)acc[i][j].y) : acc64[i][j];
+                if (D && i > 0)
+                {
+                    const double sg = (double)rsign[rr];  // the sign of the K_x rows
+                    v.x *= sg;
+                    v.y *= sg;
+                }
                 double2* o = proj + ((size_t)kbz * rows_tot + r0 + rr) * nsets + s0 + ss;
                 if (gsplit == 1)
                     *o = v;
