@@ -7,6 +7,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <chrono>
@@ -228,6 +230,33 @@ void run_workers(int nthr, F&& work)
     work(0);
     for (int w : here) work(w);
     for (auto& t : pool) t.join();
+}
+
+// Has the kernel back a large host result with memory while the GPU still computes
+// it.  A freshly allocated destination has no pages yet, and the copy that faults
+// them in runs at a tenth of the link (67 MB: 3.8 ms instead of 0.36).  The bytes
+// keep their values; where the call is refused the copy faults them as before.
+// (Writing to the pages from threads instead: 24 ms, each read maps the zero page
+// first.)  Below 8 MB the allocator hands out memory that it already holds.
+void back_pages(void* p, size_t bytes)
+{
+#ifdef MADV_POPULATE_WRITE
+    if (bytes < (8u << 20)) return;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return;  // pinned memory is resident; device memory is not ours
+    const long ps = sysconf(_SC_PAGESIZE);
+    const size_t page = ps > 0 ? (size_t)ps : 4096;
+    const size_t b0 = (size_t)p / page * page, b1 = ((size_t)p + bytes + page - 1) / page * page;
+    (void)madvise((void*)b0, b1 - b0, MADV_POPULATE_WRITE);
+#else
+    (void)p;
+    (void)bytes;
+#endif
 }
 
 int ensure(lelph_gpu* h, DevBuf& b, size_t bytes)
@@ -3086,6 +3115,7 @@ static int run_impl(lelph_gpu* h, int n, const int* qslot, const int* kbz, int n
     rc = ensure(h, fp64_local ? h->d_glocal : h->d_partials, per_pair * batch);
     if (rc) return rc;
     auto copy_batch = [&](int q0, int qn, int ev) -> int {
+        back_pages((char*)g_out + esz * gsz * q0, esz * gsz * qn);
         CUDA_TRY(h, cudaStreamWaitEvent(h->st_copy, h->evc[ev], 0));
         CUDA_TRY(h, cudaMemcpyAsync((char*)g_out + esz * gsz * q0, (const char*)gdev + esz * gsz * q0,
                                     esz * gsz * qn, cudaMemcpyDeviceToHost, h->st_copy));
@@ -3159,7 +3189,10 @@ static int run_impl(lelph_gpu* h, int n, const int* qslot, const int* kbz, int n
         CUDA_TRY(h, cudaStreamSynchronize(h->st_copy));
     }
     else if (!out_device)
+    {
+        back_pages(g_out, esz * gsz * n);
         CUDA_TRY(h, cudaMemcpyAsync(g_out, gdev, esz * gsz * n, cudaMemcpyDeviceToHost, h->st));
+    }
     rc = check_status(h);
     if (rc) return rc;
     for (int b = 0; b < ib; ++b)
@@ -3574,7 +3607,11 @@ extern "C" int lelph_gpu_dmats(lelph_gpu* h, int nsym, const double* Rmat, const
     h->dm_R.assign(Rmat, Rmat + 9 * (size_t)nsym);
     h->dm_tau.assign(tau, tau + 3 * (size_t)nsym);
     h->dm_trev.assign(time_rev, time_rev + nsym);
-    if (Dmats) CUDA_TRY(h, cudaMemcpyAsync(Dmats, h->d_dmats.p, dbytes, cudaMemcpyDeviceToHost, h->st));
+    if (Dmats)
+    {
+        back_pages(Dmats, dbytes);
+        CUDA_TRY(h, cudaMemcpyAsync(Dmats, h->d_dmats.p, dbytes, cudaMemcpyDeviceToHost, h->st));
+    }
     CUDA_TRY(h, cudaStreamSynchronize(h->st));
     return LELPH_GPU_OK;
 }
@@ -3702,6 +3739,7 @@ extern "C" int lelph_gpu_compute_elphq_star(lelph_gpu* h, const double qpt_crys[
         CUDA_TRY(h, cudaGetLastError());
         h->stats.qstar_ms += tstop(h);
     }
+    back_pages(out, total);
     CUDA_TRY(h, cudaMemcpyAsync(out, h->d_gstar.p, total, cudaMemcpyDeviceToHost, h->st));
     CUDA_TRY(h, cudaStreamSynchronize(h->st));
     return LELPH_GPU_OK;
