@@ -262,7 +262,10 @@ struct CtTwiddles
 // DFT of R = R1 R2 points in registers: R2 DFTs of R1 points over the
 // stride-R2 subsets, twiddles w_R^(n2 k1) (w_R^m = tw[m L / R], tw holding
 // e^{+2 pi i t / L}), then R1 DFTs of R2 points; X[k1 + R1 k2].
-template <typename T2, typename T, int R, int L>
+// CTW (FP32): the twiddles as constants of the same value instead of table reads, and
+// quarter turns without a product.  (Only where digits may move: with c == s the
+// compiler shares the products of a 45-degree twiddle and rounds them differently.)
+template <typename T2, typename T, int R, int L, bool CTW = false>
 __device__ __forceinline__ void dft_ct(T2* v, int sign, const T2* __restrict__ tw)
 {
     constexpr int R1 = ct_split(R);
@@ -285,10 +288,7 @@ __device__ __forceinline__ void dft_ct(T2* v, int sign, const T2* __restrict__ t
                 T2 x = u[k1];
                 if (n2 * k1 != 0)
                 {
-                    // FP32: the same rounded values as constants (a table read per butterfly
-                    // takes a twentieth of the shared-memory pipe of the plane passes),
-                    // quarter turns without a product
-                    if constexpr (sizeof(T) == sizeof(float))
+                    if constexpr (CTW)
                     {
                         constexpr CtTwiddles<R> ct{};
                         if (4 * n2 * k1 == R)
@@ -324,7 +324,7 @@ __device__ __forceinline__ void dft_ct(T2* v, int sign, const T2* __restrict__ t
 // of destination line l at dst[l*ls_d + e*es_d].  LINE_FAST: consecutive
 // threads take consecutive lines (lines interleaved in memory), else
 // consecutive elements of a line.
-template <typename T2, typename T, int L, int R, int NS, bool LINE_FAST, int NLC>
+template <typename T2, typename T, int L, int R, int NS, bool LINE_FAST, int NLC, bool CTW = false>
 __device__ __forceinline__ void ct_pass(const T2* __restrict__ src, T2* __restrict__ dst, int nlines, int es_s,
                                         int ls_s, const int* __restrict__ loff, int es_d, int ls_d,
                                         const T2* __restrict__ tw, int sign)
@@ -364,7 +364,7 @@ __device__ __forceinline__ void ct_pass(const T2* __restrict__ src, T2* __restri
                 v[r] = cmul(v[r], t);
             }
         }
-        dft_ct<T2, T, R, L>(v, sign, tw);
+        dft_ct<T2, T, R, L, CTW>(v, sign, tw);
         T2* dp = dst + line * ls_d;
         const int base = jq * NS * R + k;
 #pragma unroll
@@ -374,7 +374,7 @@ __device__ __forceinline__ void ct_pass(const T2* __restrict__ src, T2* __restri
 
 // All passes; the first reads the source layout, the rest the destination
 // layout.  Returns the buffer holding the result.
-template <typename T2, typename T, int L, int STAGE, int NS, bool LINE_FAST, int NLC>
+template <typename T2, typename T, int L, int STAGE, int NS, bool LINE_FAST, int NLC, bool CTW = false>
 __device__ __forceinline__ T2* ct_fft(T2* a, T2* b, int nlines, int es_s, int ls_s, const int* loff, int es, int ls,
                                       const T2* tw, int sign)
 {
@@ -383,8 +383,8 @@ __device__ __forceinline__ T2* ct_fft(T2* a, T2* b, int nlines, int es_s, int ls
     else
     {
         constexpr int R = ct_radix_at(L, STAGE);
-        ct_pass<T2, T, L, R, NS, LINE_FAST, NLC>(a, b, nlines, es_s, ls_s, loff, es, ls, tw, sign);
+        ct_pass<T2, T, L, R, NS, LINE_FAST, NLC, CTW>(a, b, nlines, es_s, ls_s, loff, es, ls, tw, sign);
         __syncthreads();
-        return ct_fft<T2, T, L, STAGE + 1, NS * R, LINE_FAST, NLC>(b, a, nlines, es, ls, nullptr, es, ls, tw, sign);
+        return ct_fft<T2, T, L, STAGE + 1, NS * R, LINE_FAST, NLC, CTW>(b, a, nlines, es, ls, nullptr, es, ls, tw, sign);
     }
 }

@@ -227,7 +227,9 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_xpass(const T2* __restrict__ 
 // every copy), every load of the tile issued before the first is used (the
 // generic pass waits on each), the x transform with the compile-time
 // schedule, consecutive threads on consecutive lines (conflict-free).
-template <typename T2, typename T, int NX, int CB>
+// CTW: constant twiddles on the FP32 interleaved grids (12.6 -> 12.1 ms for 8 pairs of
+// 48 modes x 200 bands on 32 x 48 x 48 points, two copies)
+template <typename T2, typename T, int NX, int CB, bool CTW>
 __global__ void __launch_bounds__(GS_THREADS) k_gs_xpass_ct(const T2* __restrict__ in, int ncol,
                                                             const T2* __restrict__ twx, const int* __restrict__ cst,
                                                             const int* __restrict__ kcx,
@@ -261,7 +263,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_xpass_ct(const T2* __restrict
         if (e < NE) a[e] = v[i];
     }
     __syncthreads();
-    T2* r = ct_fft<T2, T, NX, 0, 1, true, CB>(a, b, CB, CB, 1, nullptr, CB, 1, tx, -1);
+    T2* r = ct_fft<T2, T, NX, 0, 1, true, CB, CTW>(a, b, CB, CB, 1, nullptr, CB, 1, tx, -1);
     const int k0 = cst[c0], k1 = cst[min(c0 + cb, ncol)];
     T2* dst = A + (size_t)rb * npad;
     T2* dlo = A_lo ? A_lo + (size_t)rb * npad : nullptr;
@@ -611,7 +613,7 @@ __device__ __forceinline__ float2* ct_fft_head(float2* a, float2* b, int nlines,
     else
     {
         constexpr int R = ct_radix_at(L, STAGE);
-        ct_pass<float2, float, L, R, NS, true, 0>(a, b, nlines, es_s, ls_s, loff, es, ls, tw, -1);
+        ct_pass<float2, float, L, R, NS, true, 0, true>(a, b, nlines, es_s, ls_s, loff, es, ls, tw, -1);
         __syncthreads();
         return ct_fft_head<L, STAGE + 1, LAST, NS * R>(b, a, nlines, es, ls, nullptr, es, ls, tw);
     }
@@ -625,7 +627,8 @@ __device__ __forceinline__ float2* ct_fft_head(float2* a, float2* b, int nlines,
 // last stage writes the sphere's columns to global memory through their map
 // (cmap[z nyl + line] = column or -1; the columns are sorted by (z, y), so
 // neighbouring lines write neighbouring columns).  Shared-memory bandwidth bounds
-// it: 8 -> 5 transfers per point, two barriers fewer per mode.
+// it: 8 -> 5 transfers per point, two barriers fewer per mode, and the twiddles
+// inside a radix are constants (their table reads took a twentieth of the pipe).
 // 48 x 48 planes take 160 threads (144 butterflies of 16 points; five CTAs an SM):
 // 31.1 ms for 8 pairs of 48 modes x 200 bands x 64 planes, 33.9 with 256, 42.8 with
 // 128; the LSU pipe is busy 75 % of the time.
@@ -692,7 +695,7 @@ __global__ void __launch_bounds__(NT, NT == 160 ? 5 : 3) k_gs_plane_yz(const flo
                 for (int r = 0; r < R0; ++r) v[r] = d0[w + r * NW];
 #pragma unroll
                 for (int r = 0; r < R0; ++r) v[r] = cmul(v[r], ps[i][r]);
-                dft_ct<float2, float, R0, NY>(v, -1, ty);
+                dft_ct<float2, float, R0, NY, true>(v, -1, ty);
 #pragma unroll
                 for (int r = 0; r < R0; ++r) a[(j * R0 + r) * NZP + z] = v[r];
             }
@@ -719,7 +722,7 @@ __global__ void __launch_bounds__(NT, NT == 160 ? 5 : 3) k_gs_plane_yz(const flo
                     v[q] = cmul(v[q], t);
                 }
             }
-            dft_ct<float2, float, RL, NZ>(v, -1, tz);
+            dft_ct<float2, float, RL, NZ, true>(v, -1, tz);
 #pragma unroll
             for (int q = 0; q < RL; ++q)
             {
@@ -863,7 +866,7 @@ int lelph_launch_gs_plane(const GsGeom& gg, int fp64, const void* psi, const voi
     return 0;
 }
 
-template <typename T2, typename T, int NX, int CB>
+template <typename T2, typename T, int NX, int CB, bool CTW>
 static int gs_xpass_ct(int nrb, int ncol, int nsub, const void* twx, const int* cst, const int* kcx,
                        const void* shph, int npad, const void* in, void* A, void* A_lo, cudaStream_t st)
 {
@@ -871,14 +874,14 @@ static int gs_xpass_ct(int nrb, int ncol, int nsub, const void* twx, const int* 
     static bool attr = false;
     if (!attr)
     {
-        if (cudaFuncSetAttribute(k_gs_xpass_ct<T2, T, NX, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(k_gs_xpass_ct<T2, T, NX, CB, CTW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem) != cudaSuccess)
             return -1;
         attr = true;
     }
     const int cb = CB / nsub;
     dim3 grid((unsigned)((ncol + cb - 1) / cb), (unsigned)nrb);
-    k_gs_xpass_ct<T2, T, NX, CB><<<grid, GS_THREADS, smem, st>>>((const T2*)in, ncol, (const T2*)twx, cst, kcx,
+    k_gs_xpass_ct<T2, T, NX, CB, CTW><<<grid, GS_THREADS, smem, st>>>((const T2*)in, ncol, (const T2*)twx, cst, kcx,
                                                                 (const T2*)shph, nsub, npad, (T2*)A, (T2*)A_lo);
     return 0;
 }
@@ -902,10 +905,12 @@ int lelph_launch_gs_xpass(const GsGeom& gg, int fp64, const void* in, int nrb, i
     if (smem > 220 * 1024 || nrb > 65535) return -1;
 #define GS_XC(N)                                                                                            \
     case N:                                                                                                 \
-        return fp64 ? gs_xpass_ct<double2, double, N, 32>(nrb, ncol, gg.nsub, twx, cst, kcx, shph, npad, in, A,   \
+        return fp64 ? gs_xpass_ct<double2, double, N, 32, false>(nrb, ncol, gg.nsub, twx, cst, kcx, shph, npad, in, A,   \
                                                           A_lo, st)                                         \
-                    : gs_xpass_ct<float2, float, N, 64>(nrb, ncol, gg.nsub, twx, cst, kcx, shph, npad, in, A, A_lo, \
-                                                        st);
+                    : gg.allct ? gs_xpass_ct<float2, float, N, 64, true>(nrb, ncol, gg.nsub, twx, cst, kcx, shph,  \
+                                                                        npad, in, A, A_lo, st)              \
+                    : gs_xpass_ct<float2, float, N, 64, false>(nrb, ncol, gg.nsub, twx, cst, kcx, shph, npad, in,  \
+                                                               A, A_lo, st);
     if (lelph_gs_xpass_fixed(gg))
     switch (gg.Nx)
     {
