@@ -180,12 +180,12 @@ def g_elems(s, npairs):
     return npairs * s.nmodes * s.nspin * s.nbnds * s.nbnds
 
 
-def tensor_flops_per_pair(s, grid=None):
+def tensor_flops_per_pair(s, points=None):
     """Tensor-core work of the local sandwich per (k, q) pair: three real
     GEMMs (hi*hi, hi*lo, lo*hi) of (nmodes*nbnds) x (2*nbp) x (2*nspinor*M),
-    M the points of the product grid the library chose (the reference's box
-    when not given)."""
-    N = int(np.prod(grid if grid is not None else s.fft_dims))
+    M the points of the product grid the library chose, every interleaved
+    copy (the reference's box when not given)."""
+    N = int(points if points is not None else np.prod(s.fft_dims))
     nbp = (s.nbnds + 7) // 8 * 8
     M = s.nmodes * s.nbnds
     return 3 * 2.0 * M * (2 * nbp) * (2 * s.nspinor * N) * s.nspin
@@ -387,9 +387,10 @@ def run_profile_case(args):
         ctx.prepare()
         ctx.run_device(qs, ks, gdev.data_ptr(), out=OUT_C64)
         p1 = ctx.stats()
+        grid = ctx.grid()
     out = {"profile_case_pairs": n, "local_ms": p1["local_ms"] - p0["local_ms"],
            "prepare_ms": p1["prepare_ms"] - p0["prepare_ms"], "finish_ms": p1["finish_ms"] - p0["finish_ms"],
-           "tensor_flops": tensor_flops_per_pair(s, p1["product_grid"]) * n, "product_grid": p1["product_grid"]}
+           "tensor_flops": tensor_flops_per_pair(s, grid["points"]) * n, "product_grid": grid}
     out["local_tflops"] = out["tensor_flops"] / (out["local_ms"] * 1e-3) / 1e12
     print(json.dumps(out), flush=True)
     return 0
@@ -502,7 +503,8 @@ def run_ours(args):
     local_launches = p1["local_launches"] - p0["local_launches"]
     prep_ms = p1["prepare_ms"] - p0["prepare_ms"]
     fin_ms = p1["finish_ms"] - p0["finish_ms"]
-    flops = tensor_flops_per_pair(s, p1["product_grid"]) * npairs
+    grid = ctx.grid()
+    flops = tensor_flops_per_pair(s, grid["points"]) * npairs
     peaks = {}
     pk = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(pk):
@@ -520,7 +522,7 @@ def run_ours(args):
                 "frac": (achieved / peak) if achieved else None,
                 "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained (of measured)" if peaks else "fallback",
                 "flops_per_launch": flops_launch, "launches": live_n,
-                "product_grid": list(p1["product_grid"]), "reference_box": list(s.fft_dims),
+                "product_grid": grid, "reference_box": list(s.fft_dims),
                 "avg_launch_ms": live_ms,
                 "timing": "CUDA events around every k_local_tc launch on the library stream, over the timed steps "
                           f"({live_n} launches); {local_ms / max(1, local_launches):.2f} ms in the separately "
@@ -533,22 +535,33 @@ def run_ours(args):
     # HBM rooflines of the preparation's memory-bound kernels (per step, from the
     # library's per-role profiling events): algorithmic bytes / device time
     hbm = peaks.get("hbm_gbs") or 6800.0
-    Mp = int(np.prod(p1["product_grid"]))
+    Mp = grid["points"]
     nsets = s.nspin * s.nbnds * s.nspinor
     nbp = (s.nbnds + 7) // 8 * 8
     npw_k = np.array([len(s.gvec[int(ik)]) for ik in s.kmap[:, 0]], dtype=np.float64)
     box_bytes = s.nk_bz * nsets * Mp * 8.0            # FP32 boxes of every full-BZ k
     # after the first preparation only the occupied z-columns are zeroed
     ncols = p1.get("box_columns", 0)
-    clear_bytes = ncols * nsets * p1["product_grid"][2] * 8.0 if ncols else box_bytes
+    fused = p1["prep_fft_ms"] - p0["prep_fft_ms"] == 0  # boxes transformed in shared memory (k_box_fft_split)
+    clear_bytes = ncols * nsets * grid["copies"] * grid["n"][2] * 8.0 if ncols else box_bytes
+    split_bytes = s.nk_bz * s.nspin * s.nspinor * Mp * (2 * 2 * nbp * 4 + nbp * 8.0)
     prep_roles = {
+        "k_scatter": (p1["prep_scatter_ms"] - p0["prep_scatter_ms"],
+                      float((npw_k * (nsets * (16 + 8 * grid["copies"]) + 12)).sum()),
+                      "FP64 iBZ coefficients and Miller indices read, FP32 unfolded coefficients of every copy "
+                      "written"),
+        "k_box_fft_split": (p1["prep_xsplit_ms"] - p0["prep_xsplit_ms"],
+                            split_bytes + float((npw_k * (nsets * 8 * grid["copies"] + 4)).sum()),
+                            "FP32 coefficients of every copy and their box positions read, split k+q rows (hi, lo) "
+                            "and FP32 psi_k tiles written"),
+    } if fused else {
         "k_scatter (+ column clears)": (p1["prep_scatter_ms"] - p0["prep_scatter_ms"],
                                         float((npw_k * (nsets * (16 + 8 + 8) + 12)).sum()) + clear_bytes,
                                         "FP64 iBZ coefficients and Miller indices read, FP32 box entries and "
                                         "FP32 unfolded coefficients written, the occupied z-columns zeroed "
                                         f"({ncols} columns over the full-BZ k)"),
         "k_fft_x_split": (p1["prep_xsplit_ms"] - p0["prep_xsplit_ms"],
-                          box_bytes + s.nk_bz * s.nspin * s.nspinor * Mp * (2 * 2 * nbp * 4 + nbp * 8.0),
+                          box_bytes + split_bytes,
                           "FP32 boxes read (an upper bound: only occupied planes are read), split k+q rows "
                           "(hi, lo) and FP32 psi_k tiles written"),
         "k_fft_contig + k_fft_strided (z, y)": (p1["prep_fft_ms"] - p0["prep_fft_ms"], 4 * box_bytes,
@@ -1012,6 +1025,7 @@ def run_gspace(args):
     p1 = ctx.stats()
     ctx.set_profiling(False)
     st = ctx.stats()
+    grid = ctx.grid()
     ctx.close()
     d = {k: (p1[k] - p0[k]) / npairs for k in ("gs_plane_ms", "gs_xpass_ms", "gs_gemm_ms", "local_ms", "finish_ms")}
     npw = int(np.mean([len(g) for g in s.gvec]))
@@ -1044,7 +1058,7 @@ def run_gspace(args):
             "warmup": max(3, args.warmup), "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": args.precision, "data": "synthetic (seeded, configuration-4 shapes)",
             "config": {"workload": f"{nq} q x {len(kk)} k of the 16-atom cell ({npairs} pairs, "
-                                   f"product grid {list(st['product_grid'])}, npw ~{npw})",
+                                   f"product grid {grid['copies']} x {list(grid['n'])}, npw ~{npw})",
                        "route": {1: "real-space", 2: "G-space"}.get(st["route"]),
                        "timing": "CUDA events on the library stream, device-resident inputs and output"},
             "ms_per_pair": ms / npairs, "kernel_ms_per_pair": d, "clocks": clk,
@@ -1103,7 +1117,6 @@ def run_configs(args):
             ctx = LelphGPU(s, args.precision, device=local)
             st0 = ctx.stats()
             rec["route"] = {1: "real-space", 2: "G-space"}.get(st0["route"], st0["route"])
-            rec["product_grid"] = list(st0["product_grid"])
             for iq in range(nq):
                 ctx.set_q(iq, s.qpts[iq], s.eigVec[iq], s.dVscf[iq])
             gdev = torch.empty(len(blocks[0][0]) * gsz * 2, dtype=torch.float32, device="cuda")
@@ -1119,6 +1132,7 @@ def run_configs(args):
             for _ in range(1 if big else 2):
                 step(blocks[:1] if big else blocks)
             torch.cuda.synchronize()
+            rec["product_grid"] = ctx.grid()
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             reps = 1 if big else max(1, args.steps)
             e0.record(stream)
@@ -1248,6 +1262,7 @@ def run_batch(args):
     pp_full_ms = pp_ms * npairs / nsamp
     pp_full_wall = pp_wall * npairs / nsamp
     st = ctx.stats()
+    grid = ctx.grid()
     ctx.close()
     rate = lambda ms: elems / ((prep_ms + ms) * 1e-3)  # noqa: E731
     line = {"metric": METRIC, "unit": "g_elements/s", "n_gpus": 1, "dtype": args.precision,
@@ -1255,7 +1270,7 @@ def run_batch(args):
             "config": {"workload": "3-atom hexagonal slab, 36x36x216 grid, 12x12x1 k, 64 q, 9 modes, 40 bands, "
                                    "npw 1800-2600", "pairs": npairs, "g_elements": elems,
                        "route": {1: "real-space", 2: "G-space"}.get(st["route"], st["route"]),
-                       "product_grid": list(st["product_grid"])},
+                       "product_grid": grid},
             "prepare_ms": prep_ms,
             "batch": {"value": rate(batch_ms), "pairs_ms": batch_ms, "wall_ms": batch_wall, "calls": 1},
             "per_q": {"value": rate(perq_ms), "pairs_ms": perq_ms, "wall_ms": perq_wall, "calls": nq},
