@@ -623,21 +623,21 @@ __device__ __forceinline__ float2* ct_fft_head(float2* a, float2* b, int nlines,
 // transform goes first, so that its first stage takes element y = j + r Ny/R of
 // line z for thread j Nz + z - consecutive threads on consecutive points of the
 // plane in global memory - and forms dV psi in registers (psi held there for all
-// NUC modes); the z transform then runs on the sphere's y lines (yl), and its
+// nuc modes); the z transform then runs on the sphere's y lines (yl), and its
 // last stage writes the sphere's columns to global memory through their map
 // (cmap[z nyl + line] = column or -1; the columns are sorted by (z, y), so
 // neighbouring lines write neighbouring columns).  Shared-memory bandwidth bounds
 // it: 8 -> 5 transfers per point, two barriers fewer per mode, and the twiddles
 // inside a radix are constants (their table reads took a twentieth of the pipe).
 // 48 x 48 planes take 160 threads (144 butterflies of 16 points; five CTAs an SM):
-// 31.1 ms for 8 pairs of 48 modes x 200 bands x 64 planes, 33.9 with 256, 42.8 with
-// 128; the LSU pipe is busy 75 % of the time.
+// before the constants 31.1 ms for 8 pairs of 48 modes x 200 bands x 64 planes, 33.9
+// with 256, 42.8 with 128; the LSU pipe is busy 75 % of the time.  Now 28.5 ms.
 // Measured against k_gs_plane_ct1 (1152 products): 24 x 24 planes 4.3 -> 3.1 ms,
 // 30 x 30 7.5 -> 5.8, 40 x 40 10.9 -> 7.7, 48 x 48 12.2 -> 10.4, 60 x 60 34.3 -> 29.9.
-template <int NY, int NZ, int NUC, int NT>
+template <int NY, int NZ, int NT>
 __global__ void __launch_bounds__(NT, NT == 160 ? 5 : 3) k_gs_plane_yz(const float2* __restrict__ psi,
                                                               const float2* __restrict__ win, GsGeom gg, int nu0,
-                                                              int nub, const float2* __restrict__ twy,
+                                                              int nub, int nuc, const float2* __restrict__ twy,
                                                               const float2* __restrict__ twz,
                                                               const int* __restrict__ cmap, int ncol,
                                                               const int* __restrict__ yl, int nyl,
@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(NT, NT == 160 ? 5 : 3) k_gs_plane_yz(const flo
     int* syl = reinterpret_cast<int*>(tz + NZ);
     short* smap = reinterpret_cast<short*>(syl + NY);
     const int m = blockIdx.y, x = blockIdx.z;
-    const int nl0 = blockIdx.x * NUC, nl1 = min(nub, nl0 + NUC);
+    const int nl0 = blockIdx.x * nuc, nl1 = min(nub, nl0 + nuc);
     for (int t = threadIdx.x; t < NY; t += blockDim.x) ty[t] = twy[t];
     for (int t = threadIdx.x; t < NZ; t += blockDim.x) tz[t] = twz[t];
     for (int t = threadIdx.x; t < nyl; t += blockDim.x) syl[t] = yl[t] * NZP;
@@ -762,15 +762,21 @@ static int gs_plane_ct(const GsGeom& gg, const void* psi, const void* win, int n
                 static bool attr2 = false;
                 if (!attr2)
                 {
-                    if (cudaFuncSetAttribute(k_gs_plane_yz<N, N, NUC, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    if (cudaFuncSetAttribute(k_gs_plane_yz<N, N, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)(sizeof(float2) * (2 * (size_t)N * (N | 1) + 2 * N) +
                                                    sizeof(int) * N + sizeof(short) * (size_t)N * N)) != cudaSuccess)
                         return -1;
                     attr2 = true;
                 }
-                k_gs_plane_yz<N, N, NUC, NT><<<g1, NT, s2, st>>>((const float2*)psi, (const float2*)win, gg, nu0, nub,
-                                                                     (const float2*)twy, (const float2*)twz, cols2, ncol,
-                                                                     zl, nzl, (float2*)out);
+                // 16 modes per CTA where that leaves some ten waves (prologue and psi loads per
+                // mode halve: 28.5 against 29.1 ms for the case above), else 8 (24 x 24 planes, 72
+                // bands: 3.1 against 3.3 ms)
+                const long long cols = (long long)gg.nb * gg.nsub * gg.Nx;
+                const int nuc = cols * ((nub + 15) / 16) >= 12000 ? 16 : 8;
+                const dim3 g2((unsigned)((nub + nuc - 1) / nuc), (unsigned)gg.nb, (unsigned)(gg.nsub * gg.Nx));
+                k_gs_plane_yz<N, N, NT><<<g2, NT, s2, st>>>((const float2*)psi, (const float2*)win, gg, nu0, nub, nuc,
+                                                            (const float2*)twy, (const float2*)twz, cols2, ncol, zl,
+                                                            nzl, (float2*)out);
                 return 0;
             }
             static bool attr1 = false;

@@ -2862,7 +2862,11 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
     const bool tc = !f64 && h->gs_tc;
     const size_t na = tc ? 2 : 1;
     const size_t per_mode = e * (size_t)nb * ns * ((size_t)nplane * h->gs_ncol_max + na * h->gs_npad_max);
-    const int nub = (int)std::max<size_t>(1, std::min<size_t>((size_t)nm, (2ull << 30) / per_mode));
+    int nub = (int)std::max<size_t>(1, std::min<size_t>((size_t)nm, (2ull << 30) / per_mode));
+    // whole groups of the eight modes that a plane-pass CTA takes (17 -> 16 of the 16-atom
+    // cell's 48: its last CTA held one mode, and the GEMM's last row tile a quarter: 57.1 -> 56.0
+    // ms for 8 pairs)
+    if (nub > 8 && nub < nm) nub = nub / 8 * 8;
     rc = ensure(h, h->d_gs_out1, e * (size_t)nub * nb * ns * nplane * h->gs_ncol_max);
     if (rc) return rc;
     const size_t a_cap = (size_t)nub * nb * ns * h->gs_npad_max;  // complex elements of one A array

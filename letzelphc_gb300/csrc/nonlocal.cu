@@ -8,7 +8,7 @@
 // to modes with -2 pi i e2 eigVec (src/nonloc/Vbare_nloc.c:543-560).
 // The projections only depend on the full-BZ k-point, not on q, so here they
 // are computed once per k (k_projections) and the per-pair work reduces to
-// the small combination done in k_finish:
+// the small combination done in the finish kernels:
 //   role k+q : Pi[k+q]                      (= bandbufferK)
 //   role k   : conj(Pi[k]) for x = 0, -conj(Pi[k]) for x > 0   (= bandbufferKp)
 // with Pi[k][a][p][x][set] = sum_G beta_x(G) conj(c^(G)), c^ the unfolded

@@ -15,12 +15,13 @@ from letzelphc_gb300.elph import OUT_C64, LelphGPU
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("npw, box", [((700, 900), 48), (1500, 48), ((4000, 4500), 72), (5000, 72), (6500, 96),
-                                      (7600, 96), (9000, 96), ((11500, 12000), 96), (13500, 108), (24000, 128),
-                                      (32000, 144)])
-def test_planes_against_fp64(npw, box):
+@pytest.mark.parametrize("npw, box, nbnds", [
+    ((700, 900), 48, 3), (1500, 48, 3), ((4000, 4500), 72, 3), (5000, 72, 3), (6500, 96, 3), (7600, 96, 3),
+    (9000, 96, 3), ((11500, 12000), 96, 3), (13500, 108, 3), (24000, 128, 3), (32000, 144, 3),
+    (2500, 48, 260)])  # enough bands for 16 modes a CTA
+def test_planes_against_fp64(npw, box, nbnds):
     s = synth.make_system("planes", dict(kind="l12", a=10.0, fft=(box,) * 3, kgrid=(2, 2, 2),
-                                         qpts=[(0.5, 0.5, 0)], nbnds=3, npw=npw, ls=(0,)))
+                                         qpts=[(0.5, 0.5, 0)], nbnds=nbnds, npw=npw, ls=(0,)))
     got = {}
     for prec in ("fp64", "mixed"):
         with LelphGPU(s, prec, route="gspace") as ctx:
