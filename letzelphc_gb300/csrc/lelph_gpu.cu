@@ -2741,7 +2741,7 @@ static int build_windows(lelph_gpu* h)
     {
         rc = ensure(h, h->d_win64, sizeof(double2) * (size_t)nwin * ncomp * M);
         if (rc) return rc;
-        rc = ensure(h, h->d_edv, sizeof(int) * (size_t)nwin * d.nmodes);
+        rc = ensure(h, h->d_edv, sizeof(int) * (size_t)nwin * d.nmodes * 2);
         if (rc) return rc;
     }
     else
@@ -2826,7 +2826,9 @@ static int build_windows(lelph_gpu* h)
     }
     if (!h->mixed && !h->gspace)
     {
-        lelph_launch_oz_exponents((const double2*)h->d_win64.p, (long long)nwin * d.nmodes, d.nmag * M,
+        // one scale per component where each acts on a spin of its own, else one per mode
+        const int ne = d.nmag == 2 ? 2 : 1;
+        lelph_launch_oz_exponents((const double2*)h->d_win64.p, (long long)nwin * d.nmodes * ne, d.nmag / ne * M,
                                   oz_guard_dv(d.nmag), (int*)h->d_edv.p, h->st);
         h->stats.kernel_launches += 1;
         CUDA_TRY(h, cudaGetLastError());

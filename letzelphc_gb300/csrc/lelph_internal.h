@@ -192,7 +192,8 @@ int lelph_launch_gs_bperm(int fp64, const double2* chat, const long long* chat_o
                           int k0, int nk, int rows_per_k, int npad_max, void* Bp, cudaStream_t st);
 
 // local sandwich of the plain form (sandwich_f64.cu).  epsi: scale exponents of
-// psi per (k, spin, band), edv: of the dV windows per (window, mode), from
+// psi per (k, spin, band), edv: of the dV windows per (window, mode) -- nmag 2:
+// per (window, mode, component) --, from
 // lelph_launch_oz_exponents (guard OZ_GUARD_PSI, oz_guard_dv).  part: nchunks x
 // glocal's size (nchunks = lelph_local_fp64_chunks; 1: none needed).  Returns
 // the extra launches (>= 0), or -1.

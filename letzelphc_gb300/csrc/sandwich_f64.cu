@@ -116,7 +116,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             const int nu = R / nb, m = R - nu * nb;
             w.psi = psi + (((size_t)P.kbz_k * gd.nspin + spin) * nb + m) * gd.nspinor * M;
             w.dv = dV + ((size_t)P.dvslot * gd.nmodes + nu) * gd.nmag * M + (gd.nmag == 2 ? (size_t)spin * M : 0);
-            w.e = epsi[((size_t)P.kbz_k * gd.nspin + spin) * nb + m] + edv[(size_t)P.dvslot * gd.nmodes + nu];
+            w.e = epsi[((size_t)P.kbz_k * gd.nspin + spin) * nb + m] +
+                  (gd.nmag == 2 ? edv[2 * ((size_t)P.dvslot * gd.nmodes + nu) + spin]
+                                : edv[(size_t)P.dvslot * gd.nmodes + nu]);
         }
         ss.row[r] = w;
         ss.badrow[r] = 0;
@@ -338,8 +340,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 }
 
 // Exponent of the scale of each row of len complex numbers: with c the largest
-// |component| < 2^(E+1), e = -(E + guard), so that |z| 2^e < 2^(1.5 - guard).
+// |finite component| < 2^(E+1), e = -(E + guard), so that |z| 2^e < 2^(1.5 - guard).
 // The exponent fields alone are compared (integer instructions: no FP64 work).
+// Infinities and NaN do not count: the products that they enter are marked as
+// such, and the row's other products keep a scale that holds them.
 __global__ void __launch_bounds__(256) k_oz_exponents(const double2* __restrict__ x, long long len, int guard,
                                                       int* __restrict__ e)
 {
@@ -349,7 +353,9 @@ __global__ void __launch_bounds__(256) k_oz_exponents(const double2* __restrict_
     for (long long i = threadIdx.x; i < len; i += blockDim.x)
     {
         const double2 v = p[i];
-        m = max(m, max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu));
+        const unsigned a = (unsigned)__double2hiint(v.x) & 0x7fffffffu, b = (unsigned)__double2hiint(v.y) & 0x7fffffffu;
+        if (a < 0x7ff00000u) m = max(m, a);
+        if (b < 0x7ff00000u) m = max(m, b);
     }
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
@@ -358,7 +364,7 @@ __global__ void __launch_bounds__(256) k_oz_exponents(const double2* __restrict_
     {
         for (int w = 1; w < 8; ++w) m = max(m, sm[w]);
         const int ex = (int)(m >> 20);
-        e[blockIdx.x] = (ex == 0 || ex == 0x7ff) ? 0 : -(ex - 1023 + guard);
+        e[blockIdx.x] = ex == 0 ? 0 : -(ex - 1023 + guard);
     }
 }
 
