@@ -78,7 +78,7 @@ struct GridState
     bool sphere_window = false;   // dV windows hold the differences nearest to -q (see k_dv_window)
     DevBuf d_subtw64, d_subtw32;  // e^{+2 pi i t / (nsub N_i)} per axis (interleaved grids)
     DevBuf d_psi64, d_bsplit, d_psi32;
-    DevBuf d_epsi, d_edv;  // plain form, real-space route: scale exponents of psi64 and of the windows
+    DevBuf d_epsi, d_edv;  // plain form, real-space route: exponents of psi64 and of the windows
     CUtensorMap tmapB, tmapP, tmapV;
     void* tmapV_base = nullptr;
     int tmapV_rows = 0;
@@ -1865,10 +1865,10 @@ static int prepare_grid(lelph_gpu* h)
         lelph_launch_fft_contig_d(psi, nbox * g.Nx * g.Ny, h->plan[2], (const double2*)h->d_tw64[2].p, +1, h->st, mk);
         lelph_launch_fft_strided_d(psi, nbox * g.Nx, g.Nz, h->plan[1], (const double2*)h->d_tw64[1].p, +1, h->st, mk);
         lelph_launch_fft_strided_d(psi, nbox, g.Ny * g.Nz, h->plan[0], (const double2*)h->d_tw64[0].p, +1, h->st);
-        const long long nbk = (long long)d.nkpts_BZ * d.nspin * d.nbnds;
-        rc = ensure(h, h->d_epsi, sizeof(int) * (size_t)nbk);
+        const long long nrow = (long long)d.nkpts_BZ * nset_per_k, M = lelph_grid_points(g);
+        rc = ensure(h, h->d_epsi, lelph_oz_exponent_bytes(nrow, M));
         if (rc) return rc;
-        lelph_launch_oz_exponents(psi, nbk, d.nspinor * lelph_grid_points(g), OZ_GUARD_PSI, (int*)h->d_epsi.p, h->st);
+        lelph_launch_oz_exponents(psi, nrow, M, (short*)h->d_epsi.p, h->st);
         h->stats.kernel_launches += 5;
     }
     else if (h->sphere_window && chat_f32 && lelph_box_fft_supported(g))
@@ -2741,7 +2741,7 @@ static int build_windows(lelph_gpu* h)
     {
         rc = ensure(h, h->d_win64, sizeof(double2) * (size_t)nwin * ncomp * M);
         if (rc) return rc;
-        rc = ensure(h, h->d_edv, sizeof(int) * (size_t)nwin * d.nmodes * 2);
+        if (!h->gspace) rc = ensure(h, h->d_edv, lelph_oz_exponent_bytes((long long)nwin * ncomp, M));
         if (rc) return rc;
     }
     else
@@ -2826,10 +2826,7 @@ static int build_windows(lelph_gpu* h)
     }
     if (!h->mixed && !h->gspace)
     {
-        // one scale per component where each acts on a spin of its own, else one per mode
-        const int ne = d.nmag == 2 ? 2 : 1;
-        lelph_launch_oz_exponents((const double2*)h->d_win64.p, (long long)nwin * d.nmodes * ne, d.nmag / ne * M,
-                                  oz_guard_dv(d.nmag), (int*)h->d_edv.p, h->st);
+        lelph_launch_oz_exponents((const double2*)h->d_win64.p, (long long)nwin * ncomp, M, (short*)h->d_edv.p, h->st);
         h->stats.kernel_launches += 1;
         CUDA_TRY(h, cudaGetLastError());
     }
@@ -3154,8 +3151,8 @@ static int run_impl(lelph_gpu* h, int n, const int* qslot, const int* kbz, int n
                 rc = ensure(h, h->d_partials, per_pair * nb * nch);
                 if (rc) return rc;
             }
-            const int more = lelph_launch_local_fp64(dp, nb, (const double2*)h->d_psi64.p, (const int*)h->d_epsi.p,
-                                                     (const double2*)h->d_win64.p, (const int*)h->d_edv.p, g, nch,
+            const int more = lelph_launch_local_fp64(dp, nb, (const double2*)h->d_psi64.p, (const short*)h->d_epsi.p,
+                                                     (const double2*)h->d_win64.p, (const short*)h->d_edv.p, g, nch,
                                                      (double2*)h->d_partials.p, (double2*)h->d_glocal.p,
                                                      (unsigned*)h->d_status.p, h->wait_ns, h->st);
             if (more < 0) return fail(h, LELPH_GPU_ERR_UNSUPPORTED, "FP64 sandwich: launch configuration");
@@ -4095,8 +4092,8 @@ extern "C" int lelph_gpu_run_device_noalloc(lelph_gpu* h, int n, const int* qslo
         if (!h->mixed)
         {
             // one K chunk: the scratch holds the local blocks alone
-            if (lelph_launch_local_fp64(dpairs, nb, (const double2*)h->d_psi64.p, (const int*)h->d_epsi.p,
-                                        (const double2*)h->d_win64.p, (const int*)h->d_edv.p, g, 1, nullptr,
+            if (lelph_launch_local_fp64(dpairs, nb, (const double2*)h->d_psi64.p, (const short*)h->d_epsi.p,
+                                        (const double2*)h->d_win64.p, (const short*)h->d_edv.p, g, 1, nullptr,
                                         (double2*)work, (unsigned*)h->d_status.p, h->wait_ns, h->st) < 0)
                 return fail(h, LELPH_GPU_ERR_UNSUPPORTED, "FP64 sandwich: launch configuration");
         }

@@ -191,18 +191,16 @@ int lelph_launch_gs_bperm(int fp64, const double2* chat, const long long* chat_o
                           const int* npad_k, const long long* perm_off, const int* perm, const long long* bp_off,
                           int k0, int nk, int rows_per_k, int npad_max, void* Bp, cudaStream_t st);
 
-// local sandwich of the plain form (sandwich_f64.cu).  epsi: scale exponents of
-// psi per (k, spin, band), edv: of the dV windows per (window, mode) -- nmag 2:
-// per (window, mode, component) --, from
-// lelph_launch_oz_exponents (guard OZ_GUARD_PSI, oz_guard_dv).  part: nchunks x
+// local sandwich of the plain form (sandwich_f64.cu).  epsi: exponents of psi per
+// (k, spin, band, spinor), edv: of the dV windows per (window, mode, component),
+// each row of M points from lelph_launch_oz_exponents.  part: nchunks x
 // glocal's size (nchunks = lelph_local_fp64_chunks; 1: none needed).  Returns
 // the extra launches (>= 0), or -1.
-#define OZ_GUARD_PSI 2
-inline int oz_guard_dv(int nmag) { return nmag == 4 ? 3 : 2; }  // nmag 4: two components are added
-void lelph_launch_oz_exponents(const double2* x, long long nrows, long long len, int guard, int* e, cudaStream_t st);
+size_t lelph_oz_exponent_bytes(long long nrows, long long M);
+void lelph_launch_oz_exponents(const double2* x, long long nrows, long long M, short* e, cudaStream_t st);
 int lelph_local_fp64_chunks(int npairs, const GeomDev& g, size_t part_bytes);
-int lelph_launch_local_fp64(const PairInfo* pairs, int npairs, const double2* psi, const int* epsi, const double2* dV,
-                            const int* edv, const GeomDev& g, int nchunks, double2* part, double2* glocal,
+int lelph_launch_local_fp64(const PairInfo* pairs, int npairs, const double2* psi, const short* epsi, const double2* dV,
+                            const short* edv, const GeomDev& g, int nchunks, double2* part, double2* glocal,
                             unsigned* status, unsigned long long wait_ns, cudaStream_t st);
 
 // local sandwich of the mixed form (sandwich.cu)

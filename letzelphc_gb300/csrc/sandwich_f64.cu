@@ -12,8 +12,17 @@
 // i + j, weight 512^-(i+j); the 28 products with i + j <= 6 are formed, the rest
 // lie below 2^-63 of the scales' product.  Every 32 points the levels are
 // drained: 0 to 3 into 64-bit integers (exact), 4 to 6 -- 2^-36 and less of the
-// leading level -- into an FP32 sum.  An element's magnitude may lie 2^10 below
-// its row's largest before its rounding exceeds FP64's own.
+// leading level -- into an FP32 sum.
+//
+// The scales are those of the CTA's K chunk, from exponents kept per four points
+// of psi and of dV: a band's from its largest |psi|, a row's from the largest
+// |dV| |psi| at the same four points (not the product of the two maxima, which a
+// dV on one atom and a psi on another never reach).  An element about 2^6 below its
+// row's largest in the chunk is cut off at one FP64 rounding of its own; what is
+// smaller loses more, but below the rounding that the transforms of psi and dV leave
+// at every point.  (Measured against scales from the two maxima: error 8.4e-16 ->
+// 5.3e-16 on the 4-atom cell with its dV on one atom, 3.1e-8 -> 1.5e-8 where the bands
+// lie elsewhere and the elements are 1e-10 of max |dV|; the time is the same.)
 //
 // What bounds it: the FP64 products a (four operations an element; GB300 issues
 // about two per cycle and SM), then the integer work of the digits; the MMAs take
@@ -21,7 +30,7 @@
 // contraction on the FP64 pipe (8 nb flops per element instead of 6).
 // Measured, SIMT -> this: 64 pairs of 384 rows x 32 bands x 27,648 points, 176 ->
 // 11.3 ms; 64 pairs of 48 x 8 x 5,832, 12.6 -> 0.36 ms; error against 64 bits
-// (norm) 5.5e-15 -> 1.9e-15 and 3.4e-15 -> 0.9e-15.  (With 16 warps instead of 32:
+// (norm) 5.5e-15 -> 1.9e-15 and 3.4e-15 -> 0.86e-15.  (With 16 warps instead of 32:
 // 12.5 and 0.41 ms; the FP64 pipe is busy 40 % of the time, the rest is latency
 // between the barriers.  Forming part of the next stage's products between the digit
 // stores: no change; two rows at a time in straight-line code: 3 % slower.)
@@ -48,13 +57,12 @@ struct OzRow
 {
     const double2* psi;  // component 0 of the row's band of k (null: no such row)
     const double2* dv;   // component 0 of its mode's window
-    int e;               // exponent of the row's scale
 };
 struct OzSmem
 {
     OzRow row[OZ_ROWS];
     const double2* bpsi[OZ_BANDS];
-    int be[OZ_BANDS];
+    int re[OZ_ROWS], be[OZ_BANDS];               // exponents of the scales
     int badrow[OZ_ROWS], badband[OZ_BANDS];  // met an infinity or a NaN
     uint64_t bar;
     uint32_t tmem;
@@ -83,11 +91,20 @@ __device__ __forceinline__ uint32_t oz_digits(unsigned long long tr, unsigned lo
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+#define OZ_NO_EXP (-16384)  // four points without a normal finite number
+
+// the largest of the warp's packed 16-bit maxima, and the exponent of a scale from it
+__device__ __forceinline__ int oz_scale(unsigned mx, int guard)
+{
+    const int m = __reduce_max_sync(0xffffffffu, max((int)(short)(mx & 0xffffu), (int)(short)(mx >> 16)));
+    return m < OZ_NO_EXP / 2 ? 0 : -(m + guard);
+}
+
 // One CTA: one (pair, spin), 128 rows x up to 32 bands, one K chunk.
 // grid: (mode-row tiles x band tiles, pair * nspin, K chunks)
 __global__ void __launch_bounds__(OZ_THREADS, 1)
-    k_local_oz(const PairInfo* __restrict__ pairs, const double2* __restrict__ psi, const int* __restrict__ epsi,
-               const double2* __restrict__ dV, const int* __restrict__ edv, GeomDev gd, int ntn, int nstage_total,
+    k_local_oz(const PairInfo* __restrict__ pairs, const double2* __restrict__ psi, const short* __restrict__ epsi,
+               const double2* __restrict__ dV, const short* __restrict__ edv, GeomDev gd, int ntn, int nstage_total,
                int stages_per_chunk, double scale, long long chunk_stride, double* __restrict__ out,
                unsigned* __restrict__ status, unsigned long long wait_ns)
 {
@@ -110,15 +127,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     for (int r = threadIdx.x; r < OZ_ROWS; r += OZ_THREADS)
     {
         const int R = mt * OZ_ROWS + r;
-        OzRow w{nullptr, nullptr, 0};
+        OzRow w{nullptr, nullptr};
         if (R < nrows)
         {
             const int nu = R / nb, m = R - nu * nb;
             w.psi = psi + (((size_t)P.kbz_k * gd.nspin + spin) * nb + m) * gd.nspinor * M;
             w.dv = dV + ((size_t)P.dvslot * gd.nmodes + nu) * gd.nmag * M + (gd.nmag == 2 ? (size_t)spin * M : 0);
-            w.e = epsi[((size_t)P.kbz_k * gd.nspin + spin) * nb + m] +
-                  (gd.nmag == 2 ? edv[2 * ((size_t)P.dvslot * gd.nmodes + nu) + spin]
-                                : edv[(size_t)P.dvslot * gd.nmodes + nu]);
         }
         ss.row[r] = w;
         ss.badrow[r] = 0;
@@ -127,8 +141,52 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     {
         const size_t idx = ((size_t)P.kbz_kq * gd.nspin + spin) * nb + n0 + b;
         ss.bpsi[b] = b < nbt ? psi + idx * gd.nspinor * M : nullptr;
-        ss.be[b] = b < nbt ? epsi[idx] : 0;
         ss.badband[b] = 0;
+    }
+    const int st0 = blockIdx.z * stages_per_chunk;
+    const int nst = min(stages_per_chunk, nstage_total - st0);
+    // scales of the chunk: eight exponents (32 points) a 16-byte word
+    {
+        const long long k0 = (long long)st0 * OZ_PTS, k1 = min(Ktot, k0 + (long long)nst * OZ_PTS);
+        const size_t wpc = (size_t)((M + 31) / 32);  // words of a component
+        const uint4* const ep = reinterpret_cast<const uint4*>(epsi);
+        const uint4* const ed = reinterpret_cast<const uint4*>(edv);
+#pragma unroll 1
+        for (int r = warp; r < OZ_ROWS + OZ_BANDS; r += OZ_WARPS)
+        {
+            const bool row = r < OZ_ROWS;
+            const int R = mt * OZ_ROWS + r, b = r - OZ_ROWS;
+            if (row ? R >= nrows : b >= nbt) continue;
+            const int nu = row ? R / nb : 0, band = row ? R - nu * nb : n0 + b;
+            const uint4* p = ep + (((size_t)(row ? P.kbz_k : P.kbz_kq) * gd.nspin + spin) * nb + band) * gd.nspinor * wpc;
+            const uint4* d = ed + ((size_t)P.dvslot * gd.nmodes + nu) * gd.nmag * wpc;
+            unsigned mx = 0x80008000u;
+            for (int s = 0; s < gd.nspinor; ++s)
+            {
+                const int w0 = (int)((max(k0, s * M) - s * M) >> 5);
+                const int w1 = (int)((min(k1, (s + 1) * M) - s * M + 31) >> 5);
+                for (int w = w0 + lane; w < w1; w += 32)
+                    if (!row)
+                    {
+                        const uint4 x = p[s * wpc + w];
+                        mx = __vmaxs2(mx, __vmaxs2(__vmaxs2(x.x, x.y), __vmaxs2(x.z, x.w)));
+                    }
+                    else
+                        for (int c = 0; c < (gd.nmag == 4 ? 2 : 1); ++c)
+                        {
+                            const int dc = gd.nmag == 4 ? 2 * s + c : (gd.nmag == 2 ? spin : 0);
+                            const uint4 x = p[(gd.nmag == 4 ? c : s) * wpc + w], y = d[dc * wpc + w];
+                            mx = __viaddmax_s16x2(x.x, y.x, mx);
+                            mx = __viaddmax_s16x2(x.y, y.y, mx);
+                            mx = __viaddmax_s16x2(x.z, y.z, mx);
+                            mx = __viaddmax_s16x2(x.w, y.w, mx);
+                        }
+            }
+            // |re|, |im| < 2^(E+1) of either factor: |dV psi| < 2^(Ed+Ep+3), a sum of two (nmag 4)
+            // twice that; scaled below 1/2
+            const int e = oz_scale(mx, !row ? 2 : (gd.nmag == 4 ? 5 : 4));
+            if (lane == 0) (row ? ss.re[r] : ss.be[b]) = e;
+        }
     }
     if (threadIdx.x == 0)
     {
@@ -140,8 +198,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ss.tmem;
-    const int st0 = blockIdx.z * stages_per_chunk;
-    const int nst = min(stages_per_chunk, nstage_total - st0);
 
     long long ar[OZ_RPW], ai[OZ_RPW], br[OZ_BPW], bi[OZ_BPW];
     // fixed-point values of stage st: this lane's point of the warp's rows and bands
@@ -154,6 +210,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         for (int i = 0; i < OZ_RPW; ++i)
         {
             const OzRow w = ss.row[warp + i * OZ_WARPS];
+            const int we = ss.re[warp + i * OZ_WARPS];
             ar[i] = ai[i] = 0;
             if (w.psi && in)
             {
@@ -166,8 +223,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 else
                     a = cmul(w.dv[r], w.psi[kc]);
                 bool bad = false;
-                ar[i] = oz_fixed(a.x, w.e, bad);
-                ai[i] = oz_fixed(a.y, w.e, bad);
+                ar[i] = oz_fixed(a.x, we, bad);
+                ai[i] = oz_fixed(a.y, we, bad);
                 if (bad) ss.badrow[warp + i * OZ_WARPS] = 1;
             }
         }
@@ -319,7 +376,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 if (b >= nbt) continue;
                 // (H 2^27 + L 2^18) units of 2^(54 - 124) of the two scales' product
                 double v = fma((double)H[c], 0x1p27, (double)L[c] * 0x1p18);
-                v = scalbn(v, -70 - ss.row[r].e - ss.be[b]) * scale;
+                v = scalbn(v, -70 - ss.re[r] - ss.be[b]) * scale;
                 o[2 * (n0 + b) + im] = (bad || ss.badband[b]) ? __longlong_as_double(0x7ff8000000000000ll) : v;
             }
         }
@@ -339,38 +396,40 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     }
 }
 
-// Exponent of the scale of each row of len complex numbers: with c the largest
-// |finite component| < 2^(E+1), e = -(E + guard), so that |z| 2^e < 2^(1.5 - guard).
-// The exponent fields alone are compared (integer instructions: no FP64 work).
-// Infinities and NaN do not count: the products that they enter are marked as
-// such, and the row's other products keep a scale that holds them.
-__global__ void __launch_bounds__(256) k_oz_exponents(const double2* __restrict__ x, long long len, int guard,
-                                                      int* __restrict__ e)
+// Exponents of every four points of each row (component) of M complex numbers:
+// E of the largest |finite re or im| in [2^E, 2^(E+1)), OZ_NO_EXP where there is
+// none.  Infinities and NaN do not count: the products that they enter are marked
+// as such, and the row's other products keep a scale that holds them.  A row takes
+// M rounded up to 32 points.  The exponent fields alone are compared (integer
+// instructions: no FP64 work); reading the numbers bounds it.
+__global__ void __launch_bounds__(256) k_oz_exponents(const double2* __restrict__ x, long long nrows, long long M,
+                                                      short* __restrict__ e)
 {
-    __shared__ unsigned sm[8];
-    const double2* p = x + (size_t)blockIdx.x * len;
-    unsigned m = 0;
-    for (long long i = threadIdx.x; i < len; i += blockDim.x)
+    const long long per = (M + 31) / 32, ng = nrows * per;
+    const int lane = threadIdx.x & 31;
+    for (long long g = blockIdx.x * 8ll + (threadIdx.x >> 5); g < ng; g += gridDim.x * 8ll)
     {
-        const double2 v = p[i];
-        const unsigned a = (unsigned)__double2hiint(v.x) & 0x7fffffffu, b = (unsigned)__double2hiint(v.y) & 0x7fffffffu;
-        if (a < 0x7ff00000u) m = max(m, a);
-        if (b < 0x7ff00000u) m = max(m, b);
-    }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        for (int w = 1; w < 8; ++w) m = max(m, sm[w]);
-        const int ex = (int)(m >> 20);
-        e[blockIdx.x] = ex == 0 ? 0 : -(ex - 1023 + guard);
+        const long long row = g / per, r = (g - row * per) * 32 + lane;
+        unsigned m = 0;
+        if (r < M)
+        {
+            const double2 v = x[row * M + r];
+            const unsigned a = (unsigned)__double2hiint(v.x) & 0x7fffffffu, b = (unsigned)__double2hiint(v.y) & 0x7fffffffu;
+            if (a < 0x7ff00000u) m = a;
+            if (b < 0x7ff00000u) m = max(m, b);
+        }
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+        if ((lane & 3) == 0) e[g * 8 + (lane >> 2)] = (short)(m >> 20 ? (int)(m >> 20) - 1023 : OZ_NO_EXP);
     }
 }
 
-void lelph_launch_oz_exponents(const double2* x, long long nrows, long long len, int guard, int* e, cudaStream_t st)
+size_t lelph_oz_exponent_bytes(long long nrows, long long M) { return sizeof(short) * 8 * (size_t)nrows * ((M + 31) / 32); }
+
+void lelph_launch_oz_exponents(const double2* x, long long nrows, long long M, short* e, cudaStream_t st)
 {
-    if (nrows > 0) k_oz_exponents<<<(unsigned)nrows, 256, 0, st>>>(x, len, guard, e);
+    const long long blocks = (nrows * ((M + 31) / 32) + 7) / 8;
+    if (blocks > 0) k_oz_exponents<<<(unsigned)std::min<long long>(blocks, 152 * 64), 256, 0, st>>>(x, nrows, M, e);
 }
 
 // K chunks of a launch: enough CTAs for about sixteen rounds over the chip (the
@@ -388,8 +447,8 @@ int lelph_local_fp64_chunks(int npairs, const GeomDev& g, size_t part_bytes)
     return (int)std::max<long long>(1, std::min<long long>(n, 1024));
 }
 
-int lelph_launch_local_fp64(const PairInfo* pairs, int npairs, const double2* psi, const int* epsi, const double2* dV,
-                            const int* edv, const GeomDev& g, int nchunks, double2* part, double2* glocal,
+int lelph_launch_local_fp64(const PairInfo* pairs, int npairs, const double2* psi, const short* epsi, const double2* dV,
+                            const short* edv, const GeomDev& g, int nchunks, double2* part, double2* glocal,
                             unsigned* status, unsigned long long wait_ns, cudaStream_t st)
 {
     if (wait_ns == 0) wait_ns = LELPH_WAIT_LIMIT_NS;

@@ -3,7 +3,9 @@
 Each (mode, spin) has its own: a NaN or an infinity in the dV of one spin (with
 products dV psi above 1, which a scale of 1 would not hold), or a dV of one spin
 2^40 times the other's, leaves the other spin's matrix elements
-at the FP64 bar of the other tests (1e-10 of their own max|g|)."""
+at the FP64 bar of the other tests (1e-10 of their own max|g|).  A row's scale is
+that of the products it holds: components of dV 2^60 above the rest that meet only
+zeros of psi change nothing."""
 import dataclasses
 
 import numpy as np
@@ -49,3 +51,16 @@ def test_one_spin_does_not_touch_the_other(spin, bad):
         assert not np.isfinite(g[:, hit, spin]).any()
         rest = np.abs(g[:, ~hit, spin] - ref[:, ~hit, spin]).max()
         assert rest < TOL * np.abs(ref[:, ~hit, spin]).max()
+
+
+def test_scale_of_the_products_not_of_the_maxima():
+    s = synth.make_system("case", dict(LSDA, kind="diamond", a=10.26, nspin=1, nspinor=2, nmag=4, ls=(0,)))
+    w = [x.copy() for x in s.wfc]
+    for x in w:
+        x[:, :, 1] = 0
+    s = dataclasses.replace(s, wfc=w)
+    ref = O.compute_elphq(s, 0, non_loc=False)
+    dv = s.dVscf.copy()
+    dv[:, :, [1, 3]] *= 2.0 ** 60  # [up, down] and [down, down] multiply psi's second component
+    g = _gpu(dataclasses.replace(s, dVscf=dv))
+    assert np.abs(g - ref).max() < TOL * np.abs(ref).max()
