@@ -4092,10 +4092,12 @@ extern "C" int lelph_gpu_run_device_noalloc(lelph_gpu* h, int n, const int* qslo
         if (!h->mixed)
         {
             // one K chunk: the scratch holds the local blocks alone
-            if (lelph_launch_local_fp64(dpairs, nb, (const double2*)h->d_psi64.p, (const short*)h->d_epsi.p,
-                                        (const double2*)h->d_win64.p, (const short*)h->d_edv.p, g, 1, nullptr,
-                                        (double2*)work, (unsigned*)h->d_status.p, h->wait_ns, h->st) < 0)
-                return fail(h, LELPH_GPU_ERR_UNSUPPORTED, "FP64 sandwich: launch configuration");
+            const int more = lelph_launch_local_fp64(dpairs, nb, (const double2*)h->d_psi64.p,
+                                                     (const short*)h->d_epsi.p, (const double2*)h->d_win64.p,
+                                                     (const short*)h->d_edv.p, g, 1, nullptr, (double2*)work,
+                                                     (unsigned*)h->d_status.p, h->wait_ns, h->st);
+            if (more < 0) return fail(h, LELPH_GPU_ERR_UNSUPPORTED, "FP64 sandwich: launch configuration");
+            h->stats.kernel_launches += more;
         }
         else
             lelph_launch_local_tc(dpairs, nb, &h->tmapB, &h->tmapP, &h->tmapV, g, h->ab_bf16, h->chunk_pts,

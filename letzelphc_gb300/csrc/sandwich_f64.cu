@@ -51,6 +51,7 @@
 #define OZ_PTS 32     // grid points of a stage (one 128-byte K atom of (re, im) digits)
 #define OZ_RPW (OZ_ROWS / OZ_WARPS)
 #define OZ_BPW (OZ_BANDS / OZ_WARPS)
+#define OZ_SUM 60000   // stages that the 64-bit sums hold (a stage adds less than 2^47 + 2^41)
 #define OZ_COLS (2 * OZ_BANDS / (OZ_WARPS / 4))  // accumulator columns of a thread (its row of the tile)
 
 struct OzRow
@@ -100,12 +101,13 @@ __device__ __forceinline__ int oz_scale(unsigned mx, int guard)
     return m < OZ_NO_EXP / 2 ? 0 : -(m + guard);
 }
 
-// One CTA: one (pair, spin), 128 rows x up to 32 bands, one K chunk.
+// One CTA: one (pair, spin), 128 rows x up to 32 bands, one K chunk of the stages
+// stage0 .. nstage_total - 1; add: to what an earlier launch left in out.
 // grid: (mode-row tiles x band tiles, pair * nspin, K chunks)
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     k_local_oz(const PairInfo* __restrict__ pairs, const double2* __restrict__ psi, const short* __restrict__ epsi,
-               const double2* __restrict__ dV, const short* __restrict__ edv, GeomDev gd, int ntn, int nstage_total,
-               int stages_per_chunk, double scale, long long chunk_stride, double* __restrict__ out,
+               const double2* __restrict__ dV, const short* __restrict__ edv, GeomDev gd, int ntn, int stage0,
+               int nstage_total, int stages_per_chunk, int add, double scale, long long chunk_stride, double* __restrict__ out,
                unsigned* __restrict__ status, unsigned long long wait_ns)
 {
     extern __shared__ __align__(1024) uint8_t smraw[];
@@ -143,7 +145,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         ss.bpsi[b] = b < nbt ? psi + idx * gd.nspinor * M : nullptr;
         ss.badband[b] = 0;
     }
-    const int st0 = blockIdx.z * stages_per_chunk;
+    const int st0 = stage0 + blockIdx.z * stages_per_chunk;
     const int nst = min(stages_per_chunk, nstage_total - st0);
     // scales of the chunk: eight exponents (32 points) a 16-byte word
     {
@@ -377,6 +379,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 // (H 2^27 + L 2^18) units of 2^(54 - 124) of the two scales' product
                 double v = fma((double)H[c], 0x1p27, (double)L[c] * 0x1p18);
                 v = scalbn(v, -70 - ss.re[r] - ss.be[b]) * scale;
+                if (add) v += o[2 * (n0 + b) + im];
                 o[2 * (n0 + b) + im] = (bad || ss.badband[b]) ? __longlong_as_double(0x7ff8000000000000ll) : v;
             }
         }
@@ -455,9 +458,6 @@ int lelph_launch_local_fp64(const PairInfo* pairs, int npairs, const double2* ps
     const long long nst = (g.nspinor * lelph_grid_points(g) + OZ_PTS - 1) / OZ_PTS;
     const int nrows = g.nmodes * g.nbnds;
     const int ntm = (nrows + OZ_ROWS - 1) / OZ_ROWS, ntn = (g.nbnds + OZ_BANDS - 1) / OZ_BANDS;
-    const int per = (int)((nst + nchunks - 1) / nchunks);
-    nchunks = (int)((nst + per - 1) / per);
-    if (per > 60000) return -1;  // the 64-bit sums
     const int smem = OZ_S * (OZ_ROWS + 2 * OZ_BANDS) * 128 + (int)sizeof(OzSmem) + 1024;
     static bool attr = false;
     if (!attr)
@@ -468,15 +468,23 @@ int lelph_launch_local_fp64(const PairInfo* pairs, int npairs, const double2* ps
     }
     const double invM = 1.0 / (double)lelph_grid_points(g);
     const long long nel = (long long)npairs * g.nspin * nrows * g.nbnds;
-    // grid.y is limited to 65535 (pair, spin)s a launch
-    for (int z0 = 0; z0 < npairs * g.nspin; z0 += 65535 / g.nspin * g.nspin)
-    {
-        const int nz = std::min(npairs * g.nspin - z0, 65535 / g.nspin * g.nspin);
-        const dim3 grid((unsigned)(ntm * ntn), (unsigned)nz, (unsigned)nchunks);
-        double2* o = (nchunks > 1 ? part : glocal) + (size_t)z0 * nrows * g.nbnds;
-        k_local_oz<<<grid, OZ_THREADS, smem, st>>>(pairs + z0 / g.nspin, psi, epsi, dV, edv, g, ntn, (int)nst, per,
-                                                   nchunks > 1 ? 1.0 : invM, 2 * nel, (double*)o, status, wait_ns);
-    }
+    // chunks of more than OZ_SUM stages go in several launches, each adding to the last one's
+    // sums; grid.y is limited to 65535 (pair, spin)s a launch
+    const long long pass = std::min<long long>(nst, (long long)nchunks * OZ_SUM);
+    const int per = (int)((pass + nchunks - 1) / nchunks);
+    nchunks = (int)((pass + per - 1) / per);
+    int launches = 0;
+    for (long long s0 = 0; s0 < nst; s0 += pass)
+        for (int z0 = 0; z0 < npairs * g.nspin; z0 += 65535 / g.nspin * g.nspin, ++launches)
+        {
+            const int nz = std::min(npairs * g.nspin - z0, 65535 / g.nspin * g.nspin);
+            const int se = (int)std::min(nst, s0 + pass);
+            const dim3 grid((unsigned)(ntm * ntn), (unsigned)nz, (unsigned)((se - s0 + per - 1) / per));
+            double2* o = (nchunks > 1 ? part : glocal) + (size_t)z0 * nrows * g.nbnds;
+            k_local_oz<<<grid, OZ_THREADS, smem, st>>>(pairs + z0 / g.nspin, psi, epsi, dV, edv, g, ntn, (int)s0, se, per,
+                                                       s0 > 0, nchunks > 1 ? 1.0 : invM, 2 * nel, (double*)o, status,
+                                                       wait_ns);
+        }
     if (nchunks > 1) lelph_launch_gs_reduce(1, part, nel, nchunks, invM, glocal, st);
-    return nchunks > 1 ? 1 : 0;
+    return launches - 1 + (nchunks > 1 ? 1 : 0);
 }
