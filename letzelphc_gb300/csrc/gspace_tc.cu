@@ -339,14 +339,7 @@ static int gt_launch(const CUtensorMap* m, int nrows, int nb, int Ktot, int kchu
                      float2* part, unsigned* status, unsigned long long wait_ns, cudaStream_t st)
 {
     const GtLayout L = gt_layout(NT);
-    static bool attr = false;
-    if (!attr)
-    {
-        if (cudaFuncSetAttribute(k_gs_gemm_tc<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total) !=
-            cudaSuccess)
-            return -1;
-        attr = true;
-    }
+    if (lelph_smem_opt_in(k_gs_gemm_tc<NT>, L.total, L.total) != cudaSuccess) return -1;
     int nnt = 0;
     lelph_gs_tc_ntile(nb, &nnt);
     const int nrt = (nrows + 127) / 128;

@@ -100,6 +100,18 @@ struct BoxMask
     int Nx = 0, Ny = 0, nbox_per_k = 1;
 };
 
+// Dynamic shared memory above the default 48 KB has to be opted into, per kernel and
+// per context.  limit: the kernel's largest, so that host threads that launch it with
+// different sizes do not lower each other's.  Called before every such launch (under a
+// microsecond): a flag kept by the process would miss another device's context and one
+// created anew after cudaDeviceReset.
+template <typename K>
+inline cudaError_t lelph_smem_opt_in(K* kernel, size_t smem, size_t limit)
+{
+    if (smem <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+}
+
 // FFT (fft_gather.cu)
 // a length with a compile-time transform (FP32 passes).  The plain product grid
 // uses the original lengths only, so that the mixed form's results on it keep

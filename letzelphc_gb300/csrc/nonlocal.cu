@@ -321,15 +321,8 @@ void lelph_launch_projections(int k0, int nk, const KPointSym* ksym_dev, const d
     if (gsplit > 1)
         cudaMemsetAsync(proj + (size_t)k0 * rows * nsets, 0, sizeof(double2) * (size_t)nk * rows * nsets, st);
     dim3 grid(nk, rb, sb * gsplit);
-    static bool attr = false;
-    if (!attr)
-    {
-        cudaFuncSetAttribute(k_projections<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)pj_smem_bytes<float>());
-        cudaFuncSetAttribute(k_projections<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)pj_smem_bytes<double>());
-        attr = true;
-    }
+    lelph_smem_opt_in(k_projections<float>, pj_smem_bytes<float>(), pj_smem_bytes<float>());
+    lelph_smem_opt_in(k_projections<double>, pj_smem_bytes<double>(), pj_smem_bytes<double>());
     if (f32acc)
         k_projections<float><<<grid, 256, pj_smem_bytes<float>(), st>>>(k0, ksym_dev, gvec, pw_off, npw, Fk, fk_off,
                                                                         chat, chat_off, nl, g, gsplit, proj);
@@ -1079,12 +1072,7 @@ static int launch_finish_atoms(const PairInfo* pairs, int npairs, int mode_fp64,
                   sizeof(int) * 4 * (size_t)nl.ntype * nl.nproj_max;
     smem = std::max(smem, e * (size_t)g.nmodes * 3 * nl.natom);
     if (smem > 220 * 1024) return -1;
-    static bool attr = false;
-    if (!attr)
-    {
-        cudaFuncSetAttribute(k_finish_atoms<NJ, TM, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        attr = true;
-    }
+    if (lelph_smem_opt_in(k_finish_atoms<NJ, TM, A>, smem, 220 * 1024) != cudaSuccess) return -1;
     const dim3 grid((unsigned)(((g.nbnds + FA_N - 1) / FA_N) * ((g.nbnds + TM - 1) / TM)),
                     (unsigned)(npairs * g.nspin));
     k_finish_atoms<NJ, TM, A><<<grid, FA_N * TM, smem, st>>>(pairs, mode_fp64, glocal, partials, nchunks, mode_scale,
@@ -1105,20 +1093,15 @@ void lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const
     const int nj = 3 * nl.natom;
     if (smem <= 160 * 1024 && nj <= 24)
     {
-        static bool attr = false;
-        if (!attr)
-        {
-            cudaFuncSetAttribute(k_finish_pair<12, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-            cudaFuncSetAttribute(k_finish_pair<24, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-            cudaFuncSetAttribute(k_finish_pair<12, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-            cudaFuncSetAttribute(k_finish_pair<24, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-            attr = true;
-        }
         const int nz = npairs * g.nspin;
 #define FINL(NJ, T)                                                                                              \
-    k_finish_pair<NJ, T><<<nz, NJ <= 12 ? 256 : 128, smem, st>>>(pairs, mode_fp64, glocal, partials, nchunks,    \
-                                                                  mode_scale, band_scale, proj, eig, non_loc, nl, g, \
-                                                                  out_c64, gout)
+    do                                                                                                           \
+    {                                                                                                            \
+        lelph_smem_opt_in(k_finish_pair<NJ, T>, smem, 160 * 1024);                                               \
+        k_finish_pair<NJ, T><<<nz, NJ <= 12 ? 256 : 128, smem, st>>>(pairs, mode_fp64, glocal, partials, nchunks, \
+                                                                     mode_scale, band_scale, proj, eig, non_loc, \
+                                                                     nl, g, out_c64, gout);                      \
+    } while (0)
         if (t64)
         {
             if (nj <= 12) FINL(12, double);
@@ -1135,21 +1118,20 @@ void lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const
     const size_t tsm = finish_tile_smem(nl, g, t64 ? sizeof(double2) : sizeof(float2));
     if (mode_fp64 && nj <= 48 && tsm <= 200 * 1024)
     {
-        static bool tattr = false;
-        if (!tattr)
-        {
-            cudaFuncSetAttribute(k_finish_tile<48, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            cudaFuncSetAttribute(k_finish_tile<48, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            tattr = true;
-        }
         const int nt = (g.nbnds + FT_B - 1) / FT_B;
         dim3 tg((unsigned)(nt * nt), (unsigned)(npairs * g.nspin));
         if (t64)
+        {
+            lelph_smem_opt_in(k_finish_tile<48, double>, tsm, 200 * 1024);
             k_finish_tile<48, double><<<tg, FT_B * FT_B, tsm, st>>>(pairs, glocal, proj, eig, non_loc, nl, g, out_c64,
                                                                   gout);
+        }
         else
+        {
+            lelph_smem_opt_in(k_finish_tile<48, float>, tsm, 200 * 1024);
             k_finish_tile<48, float><<<tg, FT_B * FT_B, tsm, st>>>(pairs, glocal, proj, eig, non_loc, nl, g, out_c64,
                                                                  gout);
+        }
         return;
     }
     // larger sets: one atom's projections at a time (up to 8 atoms: 24 sums a thread; up to 16: 48
