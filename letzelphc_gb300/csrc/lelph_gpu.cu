@@ -3165,11 +3165,12 @@ static int run_impl(lelph_gpu* h, int n, const int* qslot, const int* kbz, int n
         h->stats.local_ms += tstop(h);
         h->stats.local_launches += 1;
         tstart(h);
-        lelph_launch_finish(dp, nb, !fp64_local ? 0 : (h->mixed ? 2 : 1), (const double2*)h->d_glocal.p,
-                            (const float*)h->d_partials.p,
-                            h->nchunks, (const float*)h->d_winscale.p, (const float*)h->d_band_scale.p,
-                            (const double2*)h->d_proj.p, (const double2*)h->d_eig.p, non_loc, nl, g,
-                            out_type == LELPH_GPU_OUT_C64, (char*)gdev + esz * gsz * p0, h->st);
+        if (lelph_launch_finish(dp, nb, !fp64_local ? 0 : (h->mixed ? 2 : 1), (const double2*)h->d_glocal.p,
+                                (const float*)h->d_partials.p,
+                                h->nchunks, (const float*)h->d_winscale.p, (const float*)h->d_band_scale.p,
+                                (const double2*)h->d_proj.p, (const double2*)h->d_eig.p, non_loc, nl, g,
+                                out_type == LELPH_GPU_OUT_C64, (char*)gdev + esz * gsz * p0, h->st))
+            return fail(h, LELPH_GPU_ERR_UNSUPPORTED, "finish: launch configuration");
         h->stats.finish_ms += tstop(h);
         h->stats.kernel_launches += h->gspace ? 1 : 2;  // gs_local counts its own launches
         CUDA_TRY(h, cudaGetLastError());
@@ -4102,10 +4103,11 @@ extern "C" int lelph_gpu_run_device_noalloc(lelph_gpu* h, int n, const int* qslo
         else
             lelph_launch_local_tc(dpairs, nb, &h->tmapB, &h->tmapP, &h->tmapV, g, h->ab_bf16, h->chunk_pts,
                                   h->nchunks, (float*)work, (unsigned*)h->d_status.p, h->st, h->wait_ns);
-        lelph_launch_finish(dpairs, nb, h->mixed ? 0 : 1, (const double2*)work, (const float*)work, h->nchunks,
-                            (const float*)h->d_winscale.p, (const float*)h->d_band_scale.p,
-                            (const double2*)h->d_proj.p, (const double2*)h->d_eig.p, non_loc, nl, g,
-                            out_type == LELPH_GPU_OUT_C64, (char*)g_out_dev + esz * gsz * p0, h->st);
+        if (lelph_launch_finish(dpairs, nb, h->mixed ? 0 : 1, (const double2*)work, (const float*)work, h->nchunks,
+                                (const float*)h->d_winscale.p, (const float*)h->d_band_scale.p,
+                                (const double2*)h->d_proj.p, (const double2*)h->d_eig.p, non_loc, nl, g,
+                                out_type == LELPH_GPU_OUT_C64, (char*)g_out_dev + esz * gsz * p0, h->st))
+            return fail(h, LELPH_GPU_ERR_UNSUPPORTED, "finish: launch configuration");
         h->stats.kernel_launches += 2;
         h->stats.local_launches += 1;
         CUDA_TRY(h, cudaGetLastError());

@@ -249,7 +249,8 @@ int lelph_launch_projections_tc(int k0, int nk, const KPointSym* ksym_dev, const
                                 const void* chat, int chat_f32, const long long* chat_off, const NonlocalDesc& nl,
                                 const GeomDev& g, double2* proj, unsigned* status, unsigned long long wait_ns,
                                 cudaStream_t st);
-void lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const double2* glocal,
+// 0, or -1 with nothing launched
+int lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const double2* glocal,
                          const float* partials, int nchunks, const float* mode_scale, const float* band_scale,
                          const double2* proj, const double2* eig, int non_loc, const NonlocalDesc& nl,
                          const GeomDev& g, int out_c64, void* gout, cudaStream_t st);

@@ -1080,7 +1080,7 @@ static int launch_finish_atoms(const PairInfo* pairs, int npairs, int mode_fp64,
     return 0;
 }
 
-void lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const double2* glocal,
+int lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const double2* glocal,
                          const float* partials, int nchunks, const float* mode_scale, const float* band_scale,
                          const double2* proj, const double2* eig, int non_loc, const NonlocalDesc& nl,
                          const GeomDev& g, int out_c64, void* gout, cudaStream_t st)
@@ -1113,7 +1113,7 @@ void lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const
             else FINL(24, float);
         }
 #undef FINL
-        return;
+        return 0;
     }
     const size_t tsm = finish_tile_smem(nl, g, t64 ? sizeof(double2) : sizeof(float2));
     if (mode_fp64 && nj <= 48 && tsm <= 200 * 1024)
@@ -1132,22 +1132,19 @@ void lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const
             k_finish_tile<48, float><<<tg, FT_B * FT_B, tsm, st>>>(pairs, glocal, proj, eig, non_loc, nl, g, out_c64,
                                                                  gout);
         }
-        return;
+        return 0;
     }
     // larger sets: one atom's projections at a time (up to 8 atoms: 24 sums a thread; up to 16: 48
     // sums, half as many threads)
 #define FINA(NJ, TM, A)                                                                                            \
-    launch_finish_atoms<NJ, TM, A>(pairs, npairs, mode_fp64, glocal, partials, nchunks, mode_scale, band_scale, proj, \
+    return launch_finish_atoms<NJ, TM, A>(pairs, npairs, mode_fp64, glocal, partials, nchunks, mode_scale, band_scale, proj, \
                                    eig, non_loc, nl, g, out_c64, gout, st)
     if (nj <= 24)
     {
         if (t64) FINA(24, 16, FinD);
-        else FINA(24, 16, FinF);
+        FINA(24, 16, FinF);
     }
-    else
-    {
-        if (t64) FINA(48, 8, FinD);
-        else FINA(48, 8, FinF);
-    }
+    if (t64) FINA(48, 8, FinD);
+    FINA(48, 8, FinF);
 #undef FINA
 }
