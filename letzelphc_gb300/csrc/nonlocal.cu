@@ -858,6 +858,8 @@ struct FinF
     }
 };
 
+__device__ __forceinline__ int pow2_exponent(float x) { return (int)((__float_as_uint(x) >> 23) & 255u) - 127; }
+
 // Finish where the pair's projection sets overflow shared memory (spinors with
 // d projectors, many atoms): one CTA per (16 bands of k+q x TM bands of k, pair,
 // spin) walks the atoms, with one atom's projections of the tile's bands in
@@ -1017,9 +1019,10 @@ __global__ void __launch_bounds__(FA_N * TM, 2) k_finish_atoms(const PairInfo* _
     const double invN = 1.0 / (double)lelph_grid_points(gd);
     const double2 pre = make_double2(0.0, -2.0 * LELPH_PI_T * LELPH_E2);
     const int nrows = gd.nmodes * nb, NT = 2 * gd.nbp;
-    const float bsc = mode_fp64 ? 1.f
-                                : band_scale[((size_t)P.kbz_k * gd.nspin + spin) * nb + m] *
-                                      band_scale[((size_t)P.kbz_kq * gd.nspin + spin) * nb + n];
+    // exponents of the power-of-two operand scales, added: their product may leave FP32's range
+    const int ebs = mode_fp64 ? 0
+                              : pow2_exponent(band_scale[((size_t)P.kbz_k * gd.nspin + spin) * nb + m]) +
+                                    pow2_exponent(band_scale[((size_t)P.kbz_kq * gd.nspin + spin) * nb + n]);
     C2 ov[NJ];
 #pragma unroll
     for (int j = 0; j < NJ; ++j) ov[j] = A::store(out[j]);
@@ -1041,7 +1044,8 @@ __global__ void __launch_bounds__(FA_N * TM, 2) k_finish_atoms(const PairInfo* _
                 ff_two_sum(sr, er, pp[(size_t)c * 128 * NT + n]);
                 ff_two_sum(si, ei, pp[(size_t)c * 128 * NT + gd.nbp + n]);
             }
-            const double f = invN * (double)(1.0f / (mode_scale[(size_t)P.dvslot * gd.nmodes + nu] * bsc));
+            const int es = ebs + pow2_exponent(mode_scale[(size_t)P.dvslot * gd.nmodes + nu]);
+            const double f = invN * __hiloint2double((1023 - es) << 20, 0);  // |es| <= 3 x 127
             v = make_double2(((double)sr + (double)er) * f, ((double)si + (double)ei) * f);
         }
         if (non_loc)
