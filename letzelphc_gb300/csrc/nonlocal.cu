@@ -793,6 +793,9 @@ static size_t finish_tile_smem(const NonlocalDesc& nl, const GeomDev& g, size_t 
 // Arithmetic of the nonlocal term in k_finish_atoms: FP64 (plain form), or
 // pairs of floats holding about 46 bits (mixed form, where FP64 used to run:
 // GB300 issues 1/64 of FP32's rate in FP64).  A pair (h, l) stands for h + l.
+// The mixed form with FP64 here instead: its results differ by 6e-14 (norm; nonlocal
+// term alone, 40 and 64 spinor bands, 20 bands of 16 atoms), its error against 64 bits is
+// the same 3.07e-7, and 64 pairs of 64 spinor bands take 22.6 ms instead of 20.3.
 struct FinD
 {
     typedef double R;
@@ -801,7 +804,9 @@ struct FinD
     {
         double x = 0, y = 0;
     };
+    static constexpr bool scaled = false;
     __device__ static C load(double2 v) { return v; }
+    __device__ static C times(C v, float) { return v; }
     __device__ static double2 get(const Acc& a) { return make_double2(a.x, a.y); }
     __device__ static C store(const Acc& a) { return make_double2(a.x, a.y); }
     __device__ static C conj(C a) { return make_double2(a.x, -a.y); }
@@ -817,6 +822,7 @@ struct FinD
 };
 struct FinF
 {
+    static constexpr bool scaled = true;  // projections times the band's operand scale: within FP32's range
     typedef float4 C;  // (re.h, re.l, im.h, im.l)
     struct Acc
     {
@@ -827,6 +833,7 @@ struct FinF
         const float rh = (float)v.x, ih = (float)v.y;
         return make_float4(rh, (float)(v.x - (double)rh), ih, (float)(v.y - (double)ih));
     }
+    __device__ static C times(C v, float p2) { return make_float4(v.x * p2, v.y * p2, v.z * p2, v.w * p2); }  // exact
     __device__ static double2 get(const Acc& a)
     {
         return make_double2((double)a.xh + (double)a.xl, (double)a.yh + (double)a.yl);
@@ -902,6 +909,12 @@ __global__ void __launch_bounds__(FA_N * TM, 2) k_finish_atoms(const PairInfo* _
     const int m0 = tm * TM, n0 = tn * FA_N;
     const int ml = threadIdx.x / FA_N, nlc = threadIdx.x - ml * FA_N;
     const int m = m0 + ml, n = n0 + nlc;                  // m: band of k, n: band of k+q
+    auto band_sc = [&](int k, int band) { return band_scale[((size_t)k * gd.nspin + spin) * nb + band]; };
+    // row r of set b (of this spin)
+    auto projection = [&](const double2* pi, int k, int r, int b) {
+        const C2 v = A::load(pi[(size_t)r * nsets + b]);
+        return A::scaled ? A::times(v, band_sc(k, b / ns)) : v;
+    };
     typename A::Acc out[NJ];
     if (non_loc)
     {
@@ -946,7 +959,7 @@ __global__ void __launch_bounds__(FA_N * TM, 2) k_finish_atoms(const PairInfo* _
             for (int e = threadIdx.x; e < np * 4 * cm; e += blockDim.x)
             {
                 const int r = e / cm, c = e - r * cm, b = m0 * ns + c;
-                sK[e] = A::load(b < nb * ns ? PKp[(size_t)r * nsets + b] : make_double2(0.0, 0.0));
+                sK[e] = b < nb * ns ? projection(PKp, P.kbz_k, r, b) : C2();
             }
             __syncthreads();
             // Z(p1, s1; m) = sum_{p2, s2} f(p1, p2, s1, s2) conj(Pi_0(p2, m, s2)), W_x = - the same of Pi_x
@@ -982,7 +995,7 @@ __global__ void __launch_bounds__(FA_N * TM, 2) k_finish_atoms(const PairInfo* _
             for (int e = threadIdx.x; e < np * 4 * cn; e += blockDim.x)
             {
                 const int r = e / cn, c = e - r * cn, b = n0 * ns + c;
-                sK[e] = A::load(b < nb * ns ? PK[(size_t)r * nsets + b] : make_double2(0.0, 0.0));
+                sK[e] = b < nb * ns ? projection(PK, P.kbz_kq, r, b) : C2();
             }
             __syncthreads();
             const C2* kq = sK + nlc * ns;
@@ -1017,12 +1030,11 @@ __global__ void __launch_bounds__(FA_N * TM, 2) k_finish_atoms(const PairInfo* _
     }
     if (m >= nb || n >= nb) return;
     const double invN = 1.0 / (double)lelph_grid_points(gd);
-    const double2 pre = make_double2(0.0, -2.0 * LELPH_PI_T * LELPH_E2);
     const int nrows = gd.nmodes * nb, NT = 2 * gd.nbp;
     // exponents of the power-of-two operand scales, added: their product may leave FP32's range
-    const int ebs = mode_fp64 ? 0
-                              : pow2_exponent(band_scale[((size_t)P.kbz_k * gd.nspin + spin) * nb + m]) +
-                                    pow2_exponent(band_scale[((size_t)P.kbz_kq * gd.nspin + spin) * nb + n]);
+    const int ebs = A::scaled || !mode_fp64 ? pow2_exponent(band_sc(P.kbz_k, m)) + pow2_exponent(band_sc(P.kbz_kq, n)) : 0;
+    const double2 pre = make_double2(0.0, A::scaled ? -2.0 * LELPH_PI_T * LELPH_E2 * __hiloint2double((1023 - ebs) << 20, 0)
+                                                    : -2.0 * LELPH_PI_T * LELPH_E2);
     C2 ov[NJ];
 #pragma unroll
     for (int j = 0; j < NJ; ++j) ov[j] = A::store(out[j]);
