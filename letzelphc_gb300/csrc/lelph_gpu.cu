@@ -72,6 +72,7 @@ struct GridState
     GeomDev g{};
     bool set_up = false;
     bool prepared = false;
+    bool used = false;  // a run has taken it (not only prepare)
     FftPlan1D plan[3];   // one copy of the product grid (g.Nx, g.Ny, g.Nz)
     FftPlan1D planN[3];  // the reference's FFT box
     DevBuf d_tw64[3], d_tw32[3];
@@ -1075,11 +1076,13 @@ static int grid_operands(lelph_gpu* h)
     const long long N = lelph_grid_points(g);
     size_t bb, pb;
     tc_operand_bytes(h, N, &bb, &pb);
-    if (h->two_grids && !h->d_bsplit.p && !h->other.prepared)
+    if (h->two_grids && !h->d_bsplit.p && !h->other.used)
     {
-        // buffers that hold nothing yet (made at creation, large enough for either grid)
+        // buffers that no run needs (made at creation or by a prepare before the first run), large
+        // enough for either grid
         std::swap(h->d_bsplit, h->other.d_bsplit);
         std::swap(h->d_psi32, h->other.d_psi32);
+        h->other.prepared = false;
         h->other.set_up = false;
     }
     int rc = ensure(h, h->d_bsplit, bb);
@@ -1176,6 +1179,24 @@ static int grid_setup(lelph_gpu* h)
     }
     h->set_up = true;
     return LELPH_GPU_OK;
+}
+
+// Frees what the inactive grid holds, and the boxes that its preparation may have gone
+// through; it is set up again when it is next used.
+static void release_other(lelph_gpu* h)
+{
+    GridState& s = h->other;
+    std::vector<DevBuf*> bufs = s.buffers();
+    if (std::none_of(bufs.begin(), bufs.end(), [](const DevBuf* b) { return b->p != nullptr; })) return;
+    bufs.push_back(&h->d_boxes32);
+    for (DevBuf* b : bufs)
+    {
+        if (b->p) cudaFree(b->p);
+        *b = DevBuf();
+    }
+    s.set_up = s.prepared = s.used = s.windows_ok = s.boxmask_ready = false;
+    s.tmapV_base = nullptr;
+    s.tmapV_rows = s.nwin = 0;
 }
 
 // Makes grid `which` the active one.
@@ -3017,7 +3038,9 @@ static int run_impl(lelph_gpu* h, int n, const int* qslot, const int* kbz, int n
         const int rc = use_grid(h, which);
         if (rc) return rc;
     }
-    h->ran = true;
+    h->ran = h->used = true;
+    // a grid that was only prepared, before q slots told which one runs take
+    if (h->two_grids && !h->other.used) release_other(h);
     if (!h->prepared)
     {
         int rc = prepare_grid(h);
