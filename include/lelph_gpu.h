@@ -178,7 +178,11 @@ int lelph_gpu_set_wavefunctions(lelph_gpu* h, const double* const* wfc);
 
 /* q-independent work: unfold every full-BZ wavefunction (rotation, SU(2),
  * fractional translation, time reversal), inverse-FFT it to the grid and
- * project it on the KB projectors.  Runs implicitly on first use. */
+ * project it on the KB projectors.  Runs implicitly on first use.  Mixed form:
+ * batch runs and the one-call stage may use different product grids (see
+ * lelph_gpu_grid); prepare takes that of the last run or, when a q slot was
+ * loaded since, that of the batch runs.  Before either it takes that of the
+ * one-call stage: for batch runs, load the q slots first. */
 int lelph_gpu_prepare(lelph_gpu* h);
 
 /* Load one q-point into a slot: q in crystal coordinates, eigVec
@@ -340,8 +344,9 @@ int lelph_gpu_stats_get(lelph_gpu* h, lelph_gpu_stats* s);
  * j a_i / (nsub N_i) of the cell along axis i (no counterpart in the
  * reference, which works on its FFT box).  Plain grid: nsub = 1.  The one-call
  * stage (compute_elphq, compute_elphq_star) of the mixed form keeps the plain
- * product grid, so that its complex128 results keep their digits; batch runs
- * take the smallest grid that is exact for the spheres. */
+ * product grid for either output type, and with it its digits; batch runs (run,
+ * run_device, and the allocation-free call where that grid is ready) take the
+ * smallest grid that is exact for the spheres. */
 int lelph_gpu_grid(lelph_gpu* h, int out[7]);
 /* the CUDA stream (cudaStream_t) every kernel of the context runs on */
 void* lelph_gpu_stream(lelph_gpu* h);

@@ -159,7 +159,7 @@ struct lelph_gpu : GridState
     double Rc[3] = {0, 0, 0};  // largest |k+G| component (crystal units) over every rotated sphere
     double Gc = 0;             // largest |k+G| (cartesian, no 2 pi)
     int box_grid[3] = {0, 0, 0};  // plain product grid; the one in use (g) may be interleaved
-    bool ran = false;             // a run has picked the active grid
+    int next = 1;                 // grid that prepare takes: of the last run, or of the one that set_q announces
     GridChoice choice[2];         // product grids: batch runs, one-call stage (GridState::which)
     bool two_grids = false;
     GridState other;              // the inactive one (two_grids)
@@ -2046,22 +2046,10 @@ extern "C" int lelph_gpu_prepare(lelph_gpu* h)
 {
     if (!h) return LELPH_GPU_ERR_INVALID;
     CUDA_TRY(h, cudaSetDevice(h->device));
-    // the grid that the runs so far used; before the first one, that of the batch
-    // runs when q slots are loaded for them, else that of the one-call stage
-    // (which loads its own slot)
-    if (!h->ran)
-    {
-        bool slots = false;
-        for (const QSlot& q : h->qslots) slots = slots || q.set;
-        const int rc = use_grid(h, slots ? 0 : 1);
-        if (rc) return rc;
-    }
-    else if (!h->set_up)
-    {
-        const int rc = grid_setup(h);
-        if (rc) return rc;
-    }
-    return prepare_grid(h);
+    // the grid of the last run, or of the batch run that a q slot loaded since is for; with
+    // neither, that of the one-call stage (which loads its own slot)
+    const int rc = use_grid(h, h->next);
+    return rc ? rc : prepare_grid(h);
 }
 
 // Geometry of the dV windows of one q.
@@ -2314,6 +2302,7 @@ static int set_q_common(lelph_gpu* h, int slot, const double qpt_crys[3], const 
         CUDA_TRY(h, cudaMemsetAsync((double2*)h->d_dvr.p + (size_t)slot * dvn, 0, sizeof(double2) * dvn, h->st));
     CUDA_TRY(h, cudaStreamSynchronize(h->st));
     q.set = true;
+    h->next = 0;
     h->windows_ok = h->other.windows_ok = false;
     return LELPH_GPU_OK;
 }
@@ -3038,7 +3027,8 @@ static int run_impl(lelph_gpu* h, int n, const int* qslot, const int* kbz, int n
         const int rc = use_grid(h, which);
         if (rc) return rc;
     }
-    h->ran = h->used = true;
+    h->next = which;
+    h->used = true;
     // a grid that was only prepared, before q slots told which one runs take
     if (h->two_grids && !h->other.used) release_other(h);
     if (!h->prepared)
@@ -4061,8 +4051,17 @@ extern "C" int lelph_gpu_run_device_noalloc(lelph_gpu* h, int n, const int* qslo
     if (out_type != LELPH_GPU_OUT_C128 && out_type != LELPH_GPU_OUT_C64) return fail(h, LELPH_GPU_ERR_INVALID, "out_type");
     if (n == 0) return LELPH_GPU_OK;
     CUDA_TRY(h, cudaSetDevice(h->device));
+    // the batch runs' grid where it is ready, else the one-call stage's
+    if (h->two_grids)
+    {
+        const GridState& batch = h->which == 0 ? static_cast<const GridState&>(*h) : h->other;
+        const bool ready = batch.set_up && batch.prepared && batch.windows_ok;
+        if (ready != (h->which == 0) && (ready || (h->other.set_up && h->other.prepared && h->other.windows_ok)))
+            std::swap(static_cast<GridState&>(*h), h->other);
+    }
     if (!h->prepared || !h->windows_ok)
         return fail(h, LELPH_GPU_ERR_STATE, "lelph_gpu_prepare must run (after the last set_q) before the allocation-free call");
+    h->used = true;
     if (h->gspace)
         return fail(h, LELPH_GPU_ERR_UNSUPPORTED,
                     "the G-space route builds psi(r) per k in device buffers; it has no allocation-free form");
