@@ -162,6 +162,8 @@ struct lelph_gpu : GridState
     int next = 1;                 // grid that prepare takes: of the last run, or of the one that set_q announces
     GridChoice choice[2];         // product grids: batch runs, one-call stage (GridState::which)
     bool two_grids = false;
+    size_t mem_total = 0;         // device memory, or the limit below
+    size_t mem_limit = 0;         // LELPH_DEVICE_LIMIT (bytes; 0: none): what the context may hold
     GridState other;              // the inactive one (two_grids)
     int nslots_alloc = 0;
     // local bare potential: V_loc(|G|) table and its spline slopes per species
@@ -260,6 +262,25 @@ void back_pages(void* p, size_t bytes)
 #endif
 }
 
+// Frees what the inactive grid holds; it is set up again when it is next used.  True if
+// there was anything.
+bool release_other(lelph_gpu* h)
+{
+    GridState& s = h->other;
+    bool any = false;
+    for (DevBuf* b : s.buffers())
+    {
+        any = any || b->p;
+        if (b->p) cudaFree(b->p);
+        *b = DevBuf();
+    }
+    if (!any) return false;
+    s.set_up = s.prepared = s.used = s.windows_ok = s.boxmask_ready = false;
+    s.tmapV_base = nullptr;
+    s.tmapV_rows = s.nwin = 0;
+    return true;
+}
+
 int ensure(lelph_gpu* h, DevBuf& b, size_t bytes)
 {
     if (b.n >= bytes && b.p) return LELPH_GPU_OK;
@@ -267,10 +288,26 @@ int ensure(lelph_gpu* h, DevBuf& b, size_t bytes)
     b.p = nullptr;
     b.n = 0;
     if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMalloc(&b.p, bytes);
+    auto get = [&]() {
+        if (h->mem_limit)
+        {
+            size_t held = 0;
+            for (const DevBuf* o : h->owned) held += o->n;
+            if (held + bytes > h->mem_limit) return cudaErrorMemoryAllocation;
+        }
+        return cudaMalloc(&b.p, bytes);
+    };
+    cudaError_t e = get();
     if (e != cudaSuccess)
     {
         cudaGetLastError();
+        // the inactive grid gives its memory up
+        if (h->two_grids && release_other(h)) e = get();
+    }
+    if (e != cudaSuccess)
+    {
+        cudaGetLastError();
+        b.p = nullptr;
         return fail(h, LELPH_GPU_ERR_ALLOC, "cudaMalloc of " + std::to_string(bytes) + " bytes failed");
     }
     b.n = bytes;
@@ -1067,8 +1104,7 @@ static void tc_operand_bytes(const lelph_gpu* h, long long N, size_t* bsplit, si
 }
 
 // The active grid's operand buffers and their tensor maps (mixed form,
-// real-space route).  Where the device has no room for a second grid's, the
-// inactive grid gives up its own and is prepared again when it is next used.
+// real-space route).
 static int grid_operands(lelph_gpu* h)
 {
     const lelph_gpu_desc& d = h->d;
@@ -1076,10 +1112,13 @@ static int grid_operands(lelph_gpu* h)
     const long long N = lelph_grid_points(g);
     size_t bb, pb;
     tc_operand_bytes(h, N, &bb, &pb);
-    if (h->two_grids && !h->d_bsplit.p && !h->other.used)
+    const GridState& o = h->other;
+    if (h->two_grids && !h->d_bsplit.p && o.d_bsplit.p &&
+        (!o.used || bb + pb + o.d_bsplit.n + o.d_psi32.n > h->mem_total / 8))
     {
-        // buffers that no run needs (made at creation or by a prepare before the first run), large
-        // enough for either grid
+        // buffers that no run needs (made at creation or by a prepare before the first run); or both
+        // grids' own would take more than an eighth of the device: then they share one set, and a
+        // switch prepares again
         std::swap(h->d_bsplit, h->other.d_bsplit);
         std::swap(h->d_psi32, h->other.d_psi32);
         h->other.prepared = false;
@@ -1087,20 +1126,6 @@ static int grid_operands(lelph_gpu* h)
     }
     int rc = ensure(h, h->d_bsplit, bb);
     if (!rc) rc = ensure(h, h->d_psi32, pb);
-    if (rc && h->two_grids && h->other.d_bsplit.p)
-    {
-        for (DevBuf* b : {&h->d_bsplit, &h->d_psi32})
-        {
-            if (b->p) cudaFree(b->p);
-            *b = DevBuf();
-        }
-        std::swap(h->d_bsplit, h->other.d_bsplit);
-        std::swap(h->d_psi32, h->other.d_psi32);
-        h->other.prepared = false;
-        h->other.set_up = false;
-        rc = ensure(h, h->d_bsplit, bb);
-        if (!rc) rc = ensure(h, h->d_psi32, pb);
-    }
     if (rc) return rc;
     CUDA_TRY(h, cudaMemsetAsync(h->d_bsplit.p, 0, bb, h->st));
     CUDA_TRY(h, cudaMemsetAsync(h->d_psi32.p, 0, pb, h->st));
@@ -1179,24 +1204,6 @@ static int grid_setup(lelph_gpu* h)
     }
     h->set_up = true;
     return LELPH_GPU_OK;
-}
-
-// Frees what the inactive grid holds, and the boxes that its preparation may have gone
-// through; it is set up again when it is next used.
-static void release_other(lelph_gpu* h)
-{
-    GridState& s = h->other;
-    std::vector<DevBuf*> bufs = s.buffers();
-    if (std::none_of(bufs.begin(), bufs.end(), [](const DevBuf* b) { return b->p != nullptr; })) return;
-    bufs.push_back(&h->d_boxes32);
-    for (DevBuf* b : bufs)
-    {
-        if (b->p) cudaFree(b->p);
-        *b = DevBuf();
-    }
-    s.set_up = s.prepared = s.used = s.windows_ok = s.boxmask_ready = false;
-    s.tmapV_base = nullptr;
-    s.tmapV_rows = s.nwin = 0;
 }
 
 // Makes grid `which` the active one.
@@ -1693,6 +1700,12 @@ extern "C" int lelph_gpu_create(const lelph_gpu_desc* desc, lelph_gpu** out)
     h->chat_total = chtot;
     // ---- device
     if (cudaSetDevice(h->device) != cudaSuccess) return bad(LELPH_GPU_ERR_CUDA, "cudaSetDevice");
+    {
+        size_t fr = 0;
+        if (cudaMemGetInfo(&fr, &h->mem_total) != cudaSuccess) return bad(LELPH_GPU_ERR_CUDA, "cudaMemGetInfo");
+        if (const char* e = getenv("LELPH_DEVICE_LIMIT")) h->mem_limit = (size_t)std::max(0ll, atoll(e));
+        if (h->mem_limit) h->mem_total = std::min(h->mem_total, h->mem_limit);
+    }
     if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->st_copy, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&h->evc[0], cudaEventDisableTiming) != cudaSuccess ||
@@ -3030,7 +3043,12 @@ static int run_impl(lelph_gpu* h, int n, const int* qslot, const int* kbz, int n
     h->next = which;
     h->used = true;
     // a grid that was only prepared, before q slots told which one runs take
-    if (h->two_grids && !h->other.used) release_other(h);
+    if (h->two_grids && !h->other.used && release_other(h))
+    {
+        // and the boxes that its preparation went through
+        if (h->d_boxes32.p) cudaFree(h->d_boxes32.p);
+        h->d_boxes32 = DevBuf();
+    }
     if (!h->prepared)
     {
         int rc = prepare_grid(h);

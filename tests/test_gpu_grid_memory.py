@@ -2,7 +2,10 @@
 
 A context that prepares before its q slots are loaded, and then runs, holds no more
 than one that never left the plain grid: what prepare made for the other grid is
-handed over or given back.  Results are the bits of the usual order's."""
+handed over or given back.  One that alternates between the two holds one set of
+operands where two would take more than an eighth of the memory it may hold, and
+gives the inactive grid's up when another allocation needs it.  Results are the bits
+of the usual order's throughout."""
 import numpy as np
 import pytest
 
@@ -42,3 +45,46 @@ def test_prepare_before_the_slots(route, monkeypatch):
         _run(ctx, s)
         assert usual <= ctx.stats()["device_bytes"]
     assert np.array_equal(g, ref) and np.array_equal(again, ref)
+
+
+def _alternate(ctx, s):
+    args = (s.qpts[0], s.eigVec[0], s.dVscf[0])
+    return [x for _ in range(2) for x in (ctx.compute_elphq(*args), _run(ctx, s))]
+
+
+def test_alternating_grids_share_one_set(monkeypatch):
+    s = synth.make_system("case", CELL)
+    with LelphGPU(s, "mixed", route="real") as ctx:
+        ref = _alternate(ctx, s)
+    monkeypatch.setenv("LELPH_PLAIN_GRID", "1")
+    with LelphGPU(s, "mixed", route="real") as ctx:
+        ctx.compute_elphq(s.qpts[0], s.eigVec[0], s.dVscf[0])
+        one = ctx.stats()["device_bytes"]
+        pts = ctx.grid()["points"]
+    monkeypatch.delenv("LELPH_PLAIN_GRID")
+    second = 24 * 8 * pts * s.nk_bz        # operands of 8 bands on the plain grid
+    limit = one + second // 2
+    monkeypatch.setenv("LELPH_DEVICE_LIMIT", str(limit))
+    with LelphGPU(s, "mixed", route="real") as ctx:
+        got = _alternate(ctx, s)
+        assert ctx.stats()["device_bytes"] <= limit
+    assert all(np.array_equal(a, b) for a, b in zip(got, ref))
+
+
+def test_the_inactive_grid_gives_way(monkeypatch):
+    s = synth.make_system("case", CELL)
+    args = (s.qpts[0], s.eigVec[0], s.dVscf[0])
+    with LelphGPU(s, "mixed", route="real") as ctx:
+        ref = _alternate(ctx, s)
+        held = ctx.stats()["device_bytes"]
+    nslots = 60
+    new = nslots * 16 * s.nmodes * int(np.prod(s.fft_dims))  # the slot arrays grow to this, beside the old ones
+    limit = held + new - (20 << 20)
+    monkeypatch.setenv("LELPH_DEVICE_LIMIT", str(limit))
+    with LelphGPU(s, "mixed", route="real") as ctx:
+        got = _alternate(ctx, s)
+        assert ctx.stats()["device_bytes"] >= held          # both sets are kept
+        ctx.set_q(nslots - 1, *args)
+        assert ctx.stats()["device_bytes"] < held + new - (60 << 20)  # one set (over 60 MB) and the old slots are gone
+        got += _alternate(ctx, s)
+    assert all(np.array_equal(a, b) for a, b in zip(got, ref + ref))
