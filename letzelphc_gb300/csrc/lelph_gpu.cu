@@ -1334,6 +1334,14 @@ static void pick_grid(const lelph_gpu* h, const double gm[6], const int ext[3], 
                         const long long M = t.points();
                         if ((double)M >= c.cost) break;  // ascending lengths: the rest cost more
                         if (M >= plain.points() || (tc && M % (d.tile_points == 64 ? 64 : 32) != 0)) continue;
+                        if (gspace)
+                        {
+                            // the limits that the plain grid was checked against
+                            const GsGeom gg{a, b, e, p, d.nbnds, d.nspinor, d.nmag, 0, 1};
+                            if (lelph_gs_plane_smem(gg, !h->mixed) > 220 * 1024 ||
+                                lelph_gs_xpass_smem(gg, !h->mixed) > 220 * 1024)
+                                continue;
+                        }
                         t.cost = weight(t);
                         if (t.cost >= c.cost || !exact(t.n, p, t.sa)) continue;
                         if (tc && M / tc_chunk_points(M, kp_of(M)) > nch_plain) continue;
