@@ -162,6 +162,18 @@ __device__ __forceinline__ void gs_store(float2* hi, float2* lo, int K, float2 v
     lo[K] = make_float2(tf32_rn(v.x - h.x), tf32_rn(v.y - h.y));
 }
 
+// Positions past the sphere, npw .. npad: they meet zero k+q coefficients, and whatever an
+// earlier pair or another buffer left there (a NaN) would not vanish in the product.
+template <typename T2>
+__device__ __forceinline__ void gs_pad(T2* hi, T2* lo, int npw, int npad)
+{
+    for (int K = npw + threadIdx.x; K < npad; K += blockDim.x)
+    {
+        hi[K] = mk2<T2>(0.0, 0.0);
+        if (lo) lo[K] = mk2<T2>(0.0, 0.0);
+    }
+}
+
 // Sphere point K: the copies' values summed with their phases e^{-i G.delta_j} = shph[K]^j.
 template <typename T2>
 __device__ __forceinline__ T2 gs_sum_copies(const T2* r, int cb, int nsub, const T2* __restrict__ shph, int K)
@@ -221,6 +233,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_xpass(const T2* __restrict__ 
         gs_store(dst, A_lo ? A_lo + (size_t)rb * npad : nullptr, K,
                  gs_sum_copies(r + x * GS_CB + (c - c0), cb, nsub, shph, K));
     }
+    if (c0 + cb >= ncol) gs_pad(dst, A_lo ? A_lo + (size_t)rb * npad : nullptr, cst[ncol], npad);
 }
 
 // x pass for the compile-time sizes: CB lines per CTA (CB / nsub columns of
@@ -273,6 +286,7 @@ __global__ void __launch_bounds__(GS_THREADS) k_gs_xpass_ct(const T2* __restrict
         const int c = w / NX, x = w - c * NX;
         gs_store(dst, dlo, K, gs_sum_copies(r + x * CB + (c - c0), cb, nsub, shph, K));
     }
+    if (c0 + cb >= ncol) gs_pad(dst, dlo, cst[ncol], npad);
 }
 
 // ---------------------------------------------------------------------- GEMM

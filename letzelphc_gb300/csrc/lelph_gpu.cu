@@ -2900,12 +2900,8 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
     rc = ensure(h, h->d_gs_out1, e * (size_t)nub * nb * ns * nplane * h->gs_ncol_max);
     if (rc) return rc;
     const size_t a_cap = (size_t)nub * nb * ns * h->gs_npad_max;  // complex elements of one A array
-    void* prev_A = h->d_gs_A.p;
     rc = ensure(h, h->d_gs_A, e * na * a_cap);
     if (rc) return rc;
-    // a row's positions past its sphere (npw .. npad) meet zero k+q coefficients
-    // and must hold finite values: clear a fresh buffer once
-    if (h->d_gs_A.p != prev_A) CUDA_TRY(h, cudaMemsetAsync(h->d_gs_A.p, 0, h->d_gs_A.n, h->st));
     int ntile_count = 0;
     const int NT = tc ? lelph_gs_tc_ntile(nb, &ntile_count) : 0;
     if (tc)
