@@ -173,7 +173,8 @@ int lelph_gpu_tune(const lelph_gpu_desc* desc, const double qpt_crys[3], const d
                    int npairs, const char* cache_path, lelph_gpu_tuning* out);
 
 /* Replace the plane-wave coefficients of every iBZ k-point
- * ([ik] -> (nspin, nbnds, nspinor, npw) complex); invalidates lelph_gpu_prepare. */
+ * ([ik] -> (nspin, nbnds, nspinor, npw) complex); invalidates lelph_gpu_prepare and
+ * the Dmats that lelph_gpu_dmats left on the device. */
 int lelph_gpu_set_wavefunctions(lelph_gpu* h, const double* const* wfc);
 
 /* q-independent work: unfold every full-BZ wavefunction (rotation, SU(2),

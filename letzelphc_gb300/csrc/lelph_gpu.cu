@@ -872,6 +872,7 @@ static int upload_wfc(lelph_gpu* h, const double* const* wfc)
     h->prepared = h->other.prepared = false;
     h->dm_coef32_ready = false;
     h->dm_coefT_ready = false;
+    h->dm_count = 0;  // the resident Dmats are those of the old wavefunctions
     return LELPH_GPU_OK;
 }
 
