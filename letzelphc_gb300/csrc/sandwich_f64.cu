@@ -94,6 +94,17 @@ __device__ __forceinline__ uint32_t oz_digits(unsigned long long tr, unsigned lo
 
 #define OZ_NO_EXP (-16384)  // four points without a normal finite number
 
+// Limits below the suspend hint of mbar_wait_bounded poll instead: a suspended wait sleeps
+// past them, and the MMAs of a stage (a microsecond) then always complete first.
+__device__ __forceinline__ bool oz_wait(uint64_t* bar, uint32_t parity, unsigned long long limit_ns)
+{
+    if (limit_ns >= 20000ull) return mbar_wait_bounded(bar, parity, limit_ns);
+    const unsigned long long t0 = gtimer_ns();
+    while (!mbar_test_wait(bar, parity))
+        if (gtimer_ns() - t0 > limit_ns) return false;
+    return true;
+}
+
 // the largest of the warp's packed 16-bit maxima, and the exponent of a scale from it
 __device__ __forceinline__ int oz_scale(unsigned mx, int guard)
 {
@@ -322,7 +333,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         if (st > 0)
         {
             // the MMAs of the previous stage: accumulators complete, operand tiles free
-            ok = mbar_wait_bounded(&ss.bar, (uint32_t)(st - 1) & 1u, wait_ns);
+            ok = oz_wait(&ss.bar, (uint32_t)(st - 1) & 1u, wait_ns);
             if (__syncthreads_or(!ok))
             {
                 ok = false;
@@ -359,7 +370,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     }
     if (ok)
     {
-        ok = mbar_wait_bounded(&ss.bar, (uint32_t)(nst - 1) & 1u, wait_ns);
+        ok = oz_wait(&ss.bar, (uint32_t)(nst - 1) & 1u, wait_ns);
         ok = !__syncthreads_or(!ok);
     }
     if (ok)
