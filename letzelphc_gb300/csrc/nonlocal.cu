@@ -46,6 +46,7 @@ __device__ __forceinline__ double ylm_real(int l, int m, double vx, double vy, d
 #define PJ_MAXP 24
 #define PJ_ROWS 64   // (atom, projector, component) rows per block
 #define PJ_SETS 32   // coefficient sets per block
+#define PJ_ATOMS 16  // atoms that a block's rows can belong to: 16 with one projector each
 
 template <typename T> struct PjCfg;
 template <> struct PjCfg<float> { static constexpr int G = 64; };
@@ -56,7 +57,7 @@ template <typename T> static constexpr size_t pj_smem_bytes()
     typedef typename cplx_of<T>::type C2;
     constexpr int G = PjCfg<T>::G;
     constexpr int BR = sizeof(T) == 8 ? PJ_ROWS / 4 : PJ_ROWS;  // rows of beta kept
-    return sizeof(C2) * (BR * (G + 1) + G * (PJ_SETS + 1) + 4 * G) + sizeof(T) * (16 * G + 3 * G);
+    return sizeof(C2) * (BR * (G + 1) + G * (PJ_SETS + 1) + PJ_ATOMS * G) + sizeof(T) * (16 * G + 3 * G);
 }
 
 // grid: (nk, row blocks, set blocks x gsplit); 256 threads, 4 rows x 2 sets per
@@ -89,8 +90,8 @@ __global__ void __launch_bounds__(256) k_projections(int k0, const KPointSym* __
     extern __shared__ __align__(16) unsigned char pj_smem[];
     C2* beta_s = reinterpret_cast<C2*>(pj_smem);   // [BR][PG + 1]
     C2* ch_s = beta_s + BR * (PG + 1);          // [PG][PJ_SETS + 1]
-    C2* ph_s = ch_s + PG * (PJ_SETS + 1);            // [4][PG]
-    T* ylm_s = reinterpret_cast<T*>(ph_s + 4 * PG);  // [16][PG]
+    C2* ph_s = ch_s + PG * (PJ_SETS + 1);            // [PJ_ATOMS][PG]
+    T* ylm_s = reinterpret_cast<T*>(ph_s + PJ_ATOMS * PG);  // [16][PG]
     T* kx_s = ylm_s + 16 * PG;                       // [3][PG]
     __shared__ int rinfo[PJ_ROWS][4];  // atom slot, lm index, (lidx*ntype+type), x
     __shared__ T rsign[PJ_ROWS];
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(256) k_projections(int k0, const KPointSym* __
     const double* G = gvec + 3 * pw_off[S.ik];
     const double* F = Fk + fk_off[S.ik];
     const double2* Cc = chat + chat_off[kbz];
-    const int natom_blk = min(4, nl.natom - a0);
+    const int natom_blk = (r0 + nr - 1) / (nl.nproj_max * 4) - a0 + 1;  // <= PJ_ATOMS: 64 rows, four or more an atom
     const int nlm = (nl.lmax + 1) * (nl.lmax + 1);
     for (int g0 = gs * PG; g0 < npw; g0 += gsplit * PG)
     {
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(256) k_projections(int k0, const KPointSym* __
         __syncthreads();
         {
             // K = S (k + G), cartesian (src/nonloc/Vbare_nloc.c:148-168); part 0
-            // tabulates Y_lm and K, parts 0..3 one structure-factor phase each
+            // tabulates Y_lm and K, every part the structure-factor phases of its atoms
             const int t = threadIdx.x % PG, part = threadIdx.x / PG;
             if (t < ng && (part == 0 || part < natom_blk))
             {
@@ -176,9 +177,9 @@ __global__ void __launch_bounds__(256) k_projections(int k0, const KPointSym* __
                     ylm_all(nl.lmax, K0, K1, K2, y);
                     for (int i = 0; i < nlm; ++i) ylm_s[i * PG + t] = (T)y[i];
                 }
-                if (part < natom_blk)
+                for (int ap = part; ap < natom_blk; ap += 256 / PG)
                 {
-                    const double* tau = nl.atom_pos + 3 * (a0 + part);
+                    const double* tau = nl.atom_pos + 3 * (a0 + ap);
                     double dot = K0 * tau[0] + K1 * tau[1] + K2 * tau[2];
                     if constexpr (std::is_same<T, float>::value)
                     {
@@ -187,13 +188,13 @@ __global__ void __launch_bounds__(256) k_projections(int k0, const KPointSym* __
                         const double turns = dot * (LELPH_PI_T / 3.14159265358979323846);
                         float sn, cs;
                         sincospif(2.0f * (float)(turns - rint(turns)), &sn, &cs);
-                        ph_s[part * PG + t] = mk2<C2>(cs, -sn);
+                        ph_s[ap * PG + t] = mk2<C2>(cs, -sn);
                     }
                     else
                     {
                         double sn, cs;
                         sincos(2.0 * LELPH_PI_T * dot, &sn, &cs);
-                        ph_s[part * PG + t] = mk2<C2>(cs, -sn);
+                        ph_s[ap * PG + t] = mk2<C2>(cs, -sn);
                     }
                 }
             }
