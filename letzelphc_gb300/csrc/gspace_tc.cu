@@ -16,8 +16,12 @@
 // scaling), three products hi hi + hi lo + lo hi per K step (kind::tf32,
 // K = 8), FP32 accumulation in tensor memory.  The accumulator loses low-order
 // bits on every accumulation, so each chain is one 32-element K stage (12
-// MMAs); drain warps add every finished chain into FP32 registers and write
-// one partial per K chunk, summed in FP64 by k_gs_reduce.
+// MMAs), and on the interleaved grids its eight small products (hi lo, lo hi)
+// come first: they lose next to nothing, and four accumulations instead of
+// twelve meet the full sum (error of the 16-atom cell with 200 bands 4.21e-7 ->
+// 3.94e-7, 54.7 ms either way).  The plain grid keeps the K order, whose digits
+// the one-call stage returns.  Drain warps add every finished chain into FP32
+// registers and write one partial per K chunk, summed in FP64 by k_gs_reduce.
 //
 // k_gs_gemm_tc: persistent, one CTA per SM over units (K chunk, 128-row
 // tile, N tile), N tile fastest so that the CTAs that share an A tile run
@@ -85,7 +89,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
     k_gs_gemm_tc(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CUtensorMap tmA_lo,
                  const __grid_constant__ CUtensorMap tmB_hi, const __grid_constant__ CUtensorMap tmB_lo, int nrows,
                  int nb, int kreal, int kchunk_real, int nrt, int nnt, int nunits, int rowoff, int nrows_total,
-                 float2* __restrict__ part, unsigned* __restrict__ status, unsigned long long wait_ns)
+                 int small_first, float2* __restrict__ part, unsigned* __restrict__ status, unsigned long long wait_ns)
 {
     extern __shared__ __align__(1024) uint8_t gt_raw[];
     // aligned by pointer arithmetic on the shared array itself (not through an
@@ -199,17 +203,27 @@ __global__ void __launch_bounds__(GT_THREADS, 1)
                     tc_fence_after();
                     const uint32_t base = smem_u32(sm + s * L.stage_bytes);
                     const uint32_t dacc = tmem + (uint32_t)b * L.acc_stride;
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
+                    auto desc = [&](uint32_t off, int kk) { return umma_desc_sw128(base + off + 32u * kk); };
+                    const uint32_t a_lo = L.a_bytes, b_hi = 2 * L.a_bytes, b_lo = b_hi + L.b_bytes;
+                    if (small_first)
                     {
-                        const uint64_t ah = umma_desc_sw128(base + 32u * kk);
-                        const uint64_t al = umma_desc_sw128(base + L.a_bytes + 32u * kk);
-                        const uint64_t bh = umma_desc_sw128(base + 2 * L.a_bytes + 32u * kk);
-                        const uint64_t bl = umma_desc_sw128(base + 2 * L.a_bytes + L.b_bytes + 32u * kk);
-                        umma_tf32(dacc, ah, bh, idesc, kk > 0 ? 1u : 0u);
-                        umma_tf32(dacc, ah, bl, idesc, 1u);
-                        umma_tf32(dacc, al, bh, idesc, 1u);
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                        {
+                            umma_tf32(dacc, desc(0, kk), desc(b_lo, kk), idesc, kk > 0 ? 1u : 0u);
+                            umma_tf32(dacc, desc(a_lo, kk), desc(b_hi, kk), idesc, 1u);
+                        }
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) umma_tf32(dacc, desc(0, kk), desc(b_hi, kk), idesc, 1u);
                     }
+                    else
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                        {
+                            umma_tf32(dacc, desc(0, kk), desc(b_hi, kk), idesc, kk > 0 ? 1u : 0u);
+                            umma_tf32(dacc, desc(0, kk), desc(b_lo, kk), idesc, 1u);
+                            umma_tf32(dacc, desc(a_lo, kk), desc(b_hi, kk), idesc, 1u);
+                        }
                     umma_commit(&empty[s]);
                     umma_commit(&accf[b]);
                     last_commit = &accf[b];
@@ -336,7 +350,7 @@ void lelph_launch_gs_bsplit(const float2* Bp, int nb, int Ktot, float* Bq, cudaS
 
 template <int NT>
 static int gt_launch(const CUtensorMap* m, int nrows, int nb, int Ktot, int kchunk, int rowoff, int nrows_total,
-                     float2* part, unsigned* status, unsigned long long wait_ns, cudaStream_t st)
+                     int small_first, float2* part, unsigned* status, unsigned long long wait_ns, cudaStream_t st)
 {
     const GtLayout L = gt_layout(NT);
     if (lelph_smem_opt_in(k_gs_gemm_tc<NT>, L.total, L.total) != cudaSuccess) return -1;
@@ -352,14 +366,14 @@ static int gt_launch(const CUtensorMap* m, int nrows, int nb, int Ktot, int kchu
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const int grid = (int)std::min<long long>(units, std::max(1, nsm));
     k_gs_gemm_tc<NT><<<grid, GT_THREADS, L.total, st>>>(m[0], m[1], m[2], m[3], nrows, nb, kreal, kch, nrt, nnt,
-                                                        (int)units, rowoff, nrows_total, part, status,
+                                                        (int)units, rowoff, nrows_total, small_first, part, status,
                                                         wait_ns ? wait_ns : LELPH_WAIT_LIMIT_NS);
     return 0;
 }
 
 int lelph_launch_gs_gemm_tc(const void* tmaps, int nrows, int nb, int Ktot, int kchunk, int rowoff,
-                            int nrows_total, float2* part, unsigned* status, unsigned long long wait_ns,
-                            cudaStream_t st)
+                            int nrows_total, int small_first, float2* part, unsigned* status,
+                            unsigned long long wait_ns, cudaStream_t st)
 {
     int nnt = 0;
     const int NT = lelph_gs_tc_ntile(nb, &nnt);
@@ -367,7 +381,7 @@ int lelph_launch_gs_gemm_tc(const void* tmaps, int nrows, int nb, int Ktot, int 
     switch (NT)
     {
 #define GT_CASE(N) \
-    case N: return gt_launch<N>(m, nrows, nb, Ktot, kchunk, rowoff, nrows_total, part, status, wait_ns, st);
+    case N: return gt_launch<N>(m, nrows, nb, Ktot, kchunk, rowoff, nrows_total, small_first, part, status, wait_ns, st);
         GT_CASE(16) GT_CASE(32) GT_CASE(48) GT_CASE(64) GT_CASE(80) GT_CASE(96) GT_CASE(112) GT_CASE(128)
         GT_CASE(144)
 #undef GT_CASE

@@ -2104,8 +2104,8 @@ struct WinItem
 //   receives sum_c dVhat(D_c) e^{i d_c.delta_j}.
 // One thread per residue finds the representatives once and applies them to
 // its share of the components (grid y).  The inverse transform per copy follows.
-template <typename T2, int P>
-__global__ void __launch_bounds__(256) k_dv_window(const T2* __restrict__ dvhat, int ncomp,
+template <typename TI, typename T2, int P>
+__global__ void __launch_bounds__(256) k_dv_window(const TI* __restrict__ dvhat, int ncomp,
                                                    const WinGeom* __restrict__ geoms,
                                                    const WinItem* __restrict__ items, const T2* __restrict__ sub_tw,
                                                    double invN, T2* __restrict__ out)
@@ -2198,7 +2198,7 @@ __global__ void __launch_bounds__(256) k_dv_window(const T2* __restrict__ dvhat,
         }
         for (int c = blockIdx.y; c < ncomp; c += gridDim.y)
         {
-            const T2* s = dvhat + (size_t)c * NN;
+            const TI* s = dvhat + (size_t)c * NN;
             T2* dst = out + ((size_t)u * ncomp + c) * P * Ns + r;
             T2 v[P];
 #pragma unroll
@@ -2207,8 +2207,8 @@ __global__ void __launch_bounds__(256) k_dv_window(const T2* __restrict__ dvhat,
                 v[l] = mk2<T2>(0.0, 0.0);
                 if (src[l] >= 0)
                 {
-                    const T2 w = s[src[l]];
-                    const decltype(w.x) sc = (decltype(w.x))invN;  // the operand type's 1/N
+                    const T2 w = mk2<T2>(s[src[l]].x, s[src[l]].y);
+                    const decltype(w.x) sc = (decltype(w.x))invN;  // the result type's 1/N
                     v[l] = mk2<T2>(w.x * sc, w.y * sc);
                 }
             }
@@ -2229,16 +2229,16 @@ __global__ void __launch_bounds__(256) k_dv_window(const T2* __restrict__ dvhat,
     }
 }
 
-template <typename T2>
-static void launch_dv_window(const T2* dvhat, int ncomp, const WinGeom* wg, int nsub, const WinItem* items, int nwin,
+template <typename TI, typename T2>
+static void launch_dv_window(const TI* dvhat, int ncomp, const WinGeom* wg, int nsub, const WinItem* items, int nwin,
                              const T2* sub_tw, double invN, T2* out, cudaStream_t st)
 {
     // residues of a window over 64 CTAs, fewer where many windows fill the chip
     const dim3 grid(nwin >= 16 ? 16u : 64u, (unsigned)((ncomp + 3) / 4), (unsigned)nwin);
-    if (nsub == 1) k_dv_window<T2, 1><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
-    else if (nsub == 2) k_dv_window<T2, 2><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
-    else if (nsub == 3) k_dv_window<T2, 3><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
-    else k_dv_window<T2, 4><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
+    if (nsub == 1) k_dv_window<TI, T2, 1><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
+    else if (nsub == 2) k_dv_window<TI, T2, 2><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
+    else if (nsub == 3) k_dv_window<TI, T2, 3><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
+    else k_dv_window<TI, T2, 4><<<grid, 256, 0, st>>>(dvhat, ncomp, wg, items, sub_tw, invN, out);
 }
 
 // Load q slot `slot`: eigVec and dV (host); dVscf == nullptr loads zeros.
@@ -2719,6 +2719,8 @@ static int build_windows(lelph_gpu* h)
     // of the 4-atom cell: 88 launches, 1.4 ms -> 11, 0.9 ms; 3 of a 2-atom cell, 0.33 -> 0.17).  A group's scratch stays
     // within 512 MB on the reference box and 1 GB on the product grid, or one slot's.
     const size_t esz = h->mixed ? sizeof(float2) : sizeof(double2);
+    const bool inv64 = h->mixed && h->gspace && h->sphere_window;
+    const size_t eszM = inv64 ? sizeof(double2) : esz;
     struct Group
     {
         int s0, ns, w0, nw;
@@ -2740,14 +2742,14 @@ static int build_windows(lelph_gpu* h)
         {
             const int nu = (int)h->qslots[s].ulms.size() / 3;
             if (gr.ns > 0 && ((size_t)(gr.ns + 1) * ncomp * NN * esz > (512ull << 20) ||
-                              (size_t)(gr.nw + nu) * ncomp * M * esz > (1ull << 30) || gr.nw + nu > 32768))
+                              (size_t)(gr.nw + nu) * ncomp * M * eszM > (1ull << 30) || gr.nw + nu > 32768))
                 break;
             ++gr.ns;
             gr.nw += nu;
             ++s;
         }
         needN = std::max(needN, (size_t)(gr.ns * ncomp * NN) * esz);
-        needM = std::max(needM, (size_t)(gr.nw * ncomp * M) * esz);
+        needM = std::max(needM, (size_t)(gr.nw * ncomp * M) * eszM);
         // geometries, then windows
         tab_off.push_back(h->win_tab.size());
         h->win_tab.resize(h->win_tab.size() + sizeof(WinGeom) * gr.ns + sizeof(WinItem) * gr.nw);
@@ -2804,8 +2806,23 @@ static int build_windows(lelph_gpu* h)
                                        -1, h->st);
             lelph_launch_fft_strided_f(tN, nbN, h->Nbox[1] * h->Nbox[2], h->planN[0], (const float2*)h->d_twN32[0].p,
                                        -1, h->st);
-            launch_dv_window<float2>(tN, ncomp, wg, P, wi, gr.nw, (const float2*)h->d_subtw32.p, 1.0 / (double)NN, tM,
-                                     h->st);
+            if (inv64)
+            {
+                // the inverse transform in FP64: the interleaved grid has about half the plain one's
+                // points to average its rounding over (16-atom cell, 200 bands: error 3.94e-7 -> 3.86e-7,
+                // the windows of a q 2.0 -> 5.0 ms; the forward one too: 10 ms.  FP32 on both and the
+                // GEMM in K order: 4.21e-7; the plain grid: 3.82e-7)
+                double2* tD = (double2*)h->d_wtmpM.p;
+                launch_dv_window(tN, ncomp, wg, P, wi, gr.nw, (const double2*)h->d_subtw64.p, 1.0 / (double)NN, tD, h->st);
+                lelph_launch_fft_contig_d(tD, nbM * g.Nx * g.Ny, h->plan[2], (const double2*)h->d_tw64[2].p, +1, h->st);
+                lelph_launch_fft_strided_d(tD, nbM * g.Nx, g.Nz, h->plan[1], (const double2*)h->d_tw64[1].p, +1, h->st);
+                lelph_launch_fft_strided_d(tD, nbM, g.Ny * g.Nz, h->plan[0], (const double2*)h->d_tw64[0].p, +1, h->st);
+                lelph_launch_dm_c64(tD, nbM * g.Nx * g.Ny * g.Nz, (float2*)h->d_win32.p + (size_t)gr.w0 * ncomp * M, h->st);
+                h->stats.kernel_launches += 9;
+                CUDA_TRY(h, cudaGetLastError());
+                continue;
+            }
+            launch_dv_window(tN, ncomp, wg, P, wi, gr.nw, (const float2*)h->d_subtw32.p, 1.0 / (double)NN, tM, h->st);
             lelph_launch_fft_contig_f(tM, nbM * g.Nx * g.Ny, h->plan[2], (const float2*)h->d_tw32[2].p, +1, h->st);
             lelph_launch_fft_strided_f(tM, nbM * g.Nx, g.Nz, h->plan[1], (const float2*)h->d_tw32[1].p, +1, h->st);
             lelph_launch_fft_strided_f(tM, nbM, g.Ny * g.Nz, h->plan[0], (const float2*)h->d_tw32[0].p, +1, h->st);
@@ -2847,7 +2864,7 @@ static int build_windows(lelph_gpu* h)
                                    h->st);
         lelph_launch_fft_strided_d(tN, nbN, h->Nbox[1] * h->Nbox[2], h->planN[0], (const double2*)h->d_twN[0].p, -1,
                                    h->st);
-        launch_dv_window<double2>(tN, ncomp, wg, P, wi, gr.nw, (const double2*)h->d_subtw64.p, 1.0 / (double)NN, tM,
+        launch_dv_window(tN, ncomp, wg, P, wi, gr.nw, (const double2*)h->d_subtw64.p, 1.0 / (double)NN, tM,
                                   h->st);
         // inverse transform on the product grid
         lelph_launch_fft_contig_d(tM, nbM * g.Nx * g.Ny, h->plan[2], (const double2*)h->d_tw64[2].p, +1, h->st);
@@ -3014,7 +3031,7 @@ static int gs_local(lelph_gpu* h, const PairInfo* pairs, int n, double2* glocal)
                                              h->d_gs_A.p, h->st, A_lo);
                 h->stats.gs_xpass_ms += gs_tock(h);
                 if (tc)
-                    bad |= lelph_launch_gs_gemm_tc(tm, nmb * nb, nb, Ktot, kchunk, nu0 * nb, nrows,
+                    bad |= lelph_launch_gs_gemm_tc(tm, nmb * nb, nb, Ktot, kchunk, nu0 * nb, nrows, h->sphere_window,
                                                    (float2*)h->d_gs_part.p, (unsigned*)h->d_status.p, h->wait_ns,
                                                    h->st);
                 else

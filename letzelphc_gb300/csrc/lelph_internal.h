@@ -193,8 +193,8 @@ int lelph_gs_tc_supported(int nb);
 size_t lelph_gs_tc_smem(int nb);
 void lelph_launch_gs_bsplit(const float2* Bp, int nb, int Ktot, float* Bq, cudaStream_t st);
 int lelph_launch_gs_gemm_tc(const void* tmaps, int nrows, int nb, int Ktot, int kchunk, int rowoff,
-                            int nrows_total, float2* part, unsigned* status, unsigned long long wait_ns,
-                            cudaStream_t st);
+                            int nrows_total, int small_first, float2* part, unsigned* status,
+                            unsigned long long wait_ns, cudaStream_t st);
 int lelph_launch_gs_gemm(int fp64, const void* A, const void* B, int nrows, int nb, int Ktot, int kchunk,
                          int rowoff, int nrows_total, void* part, cudaStream_t st);
 void lelph_launch_gs_reduce(int fp64, const void* part, long long nel, int nchunks, double invM, double2* glocal,
