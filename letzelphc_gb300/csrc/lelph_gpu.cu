@@ -2765,7 +2765,7 @@ static int build_windows(lelph_gpu* h)
     }
     int rc = ensure(h, h->d_wtmpN, needN);
     if (rc) return rc;
-    rc = ensure(h, h->d_wtmpM, needM);
+    if (h->mixed) rc = ensure(h, h->d_wtmpM, needM);  // the plain form transforms in place
     if (rc) return rc;
     // the tables of every group, uploaded in one copy
     rc = ensure(h, h->d_tmp, h->win_tab.size() + 16);
