@@ -26,35 +26,12 @@
 
 // ------------------------------------------------------ line FFT in registers
 
-// cos and sin of 2 pi m / L at compile time: reduction to an octant in exact
-// integer arithmetic, then the Taylor series (terms below 1e-19 after ten)
-__host__ __device__ constexpr double fb_series(double x, bool sine)
-{
-    double t = sine ? x : 1.0, s = t;
-    for (int k = sine ? 2 : 1; k < 24; k += 2)
-    {
-        t *= -x * x / (double)(k * (k + 1));
-        s += t;
-    }
-    return s;
-}
-__host__ __device__ constexpr double fb_cos(int m, int L)
-{
-    m %= L;
-    if (2 * m > L) m = L - m;                    // cos(2 pi - a) = cos a
-    if (4 * m > L) return -fb_cos(L - 2 * m, 2 * L);  // cos(pi - a) = -cos a
-    // a in [0, pi / 2]
-    if (8 * m <= L) return fb_series(6.283185307179586476925286766559 * m / L, false);
-    return fb_series(6.283185307179586476925286766559 * (L - 4 * m) / (4.0 * L), true);
-}
-__host__ __device__ constexpr double fb_sin(int m, int L) { return fb_cos(((4 * m - L) % (4 * L) + 4 * L) % (4 * L), 4 * L); }
-
 template <int M, int L>
 __device__ __forceinline__ float2 fb_twiddle(float2 x)
 {
     constexpr int m = M % L;
     if constexpr (m == 0) return x;
-    constexpr float c = (float)fb_cos(m, L), s = (float)fb_sin(m, L);
+    constexpr float c = (float)ct_trig(m, L, false), s = (float)ct_trig(m, L, true);
     return make_float2(x.x * c - x.y * s, x.x * s + x.y * c);
 }
 

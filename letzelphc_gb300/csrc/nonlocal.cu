@@ -799,7 +799,6 @@ static size_t finish_tile_smem(const NonlocalDesc& nl, const GeomDev& g, size_t 
 // the same 3.07e-7, and 64 pairs of 64 spinor bands take 22.6 ms instead of 20.3.
 struct FinD
 {
-    typedef double R;
     typedef double2 C;  // storage: (re, im)
     struct Acc
     {

@@ -366,11 +366,6 @@ __device__ __forceinline__ void umma_stage_merged<32>(uint32_t dacc, uint32_t da
 // the MMA warp cycles through NACC TMEM accumulators, and the drain warps
 // add each finished accumulator into round-to-nearest FP32 registers, which
 // are written out per K chunk and reduced in FP64 by the finish kernel.
-template <int H> struct TcHalf
-{
-    static constexpr int value = H;
-};
-
 struct TcUnit
 {
     int chunk, mt, zp, spin;
