@@ -3197,13 +3197,9 @@ static int run_impl(lelph_gpu* h, int n, const int* qslot, const int* kbz, int n
         }
         else if (!h->mixed)
         {
-            // chunk partials in at most 1 GB
-            const int nch = lelph_local_fp64_chunks(nb, g, 1ull << 30);
-            if (nch > 1)
-            {
-                rc = ensure(h, h->d_partials, per_pair * nb * nch);
-                if (rc) return rc;
-            }
+            // chunk partials in at most 1 GB; one chunk, which needs none, where there is no room
+            int nch = lelph_local_fp64_chunks(nb, g, 1ull << 30);
+            if (nch > 1 && ensure(h, h->d_partials, per_pair * nb * nch) != LELPH_GPU_OK) nch = 1;
             const int more = lelph_launch_local_fp64(dp, nb, (const double2*)h->d_psi64.p, (const short*)h->d_epsi.p,
                                                      (const double2*)h->d_win64.p, (const short*)h->d_edv.p, g, nch,
                                                      (double2*)h->d_partials.p, (double2*)h->d_glocal.p,
