@@ -2726,46 +2726,54 @@ static int build_windows(lelph_gpu* h)
         int s0, ns, w0, nw;
     };
     std::vector<Group> groups;
-    size_t needN = 0, needM = 0;
-    h->win_tab.clear();
     std::vector<size_t> tab_off;
-    for (int s = 0; s < (int)h->qslots.size();)
-    {
-        const int nu0 = h->qslots[s].set ? (int)h->qslots[s].ulms.size() / 3 : 0;
-        if (nu0 == 0)
+    auto make_groups = [&](size_t capN, size_t capM, size_t& needN, size_t& needM) {
+        groups.clear();
+        tab_off.clear();
+        h->win_tab.clear();
+        needN = needM = 0;
+        for (int s = 0; s < (int)h->qslots.size();)
         {
-            ++s;
-            continue;
+            const int nu0 = h->qslots[s].set ? (int)h->qslots[s].ulms.size() / 3 : 0;
+            if (nu0 == 0)
+            {
+                ++s;
+                continue;
+            }
+            Group gr{s, 0, h->win_base[s], 0};
+            while (s < (int)h->qslots.size() && h->qslots[s].set && !h->qslots[s].ulms.empty())
+            {
+                const int nu = (int)h->qslots[s].ulms.size() / 3;
+                if (gr.ns > 0 && ((size_t)(gr.ns + 1) * ncomp * NN * esz > capN ||
+                                  (size_t)(gr.nw + nu) * ncomp * M * eszM > capM || gr.nw + nu > 32768))
+                    break;
+                ++gr.ns;
+                gr.nw += nu;
+                ++s;
+            }
+            needN = std::max(needN, (size_t)(gr.ns * ncomp * NN) * esz);
+            needM = std::max(needM, (size_t)(gr.nw * ncomp * M) * eszM);
+            // geometries, then windows
+            tab_off.push_back(h->win_tab.size());
+            h->win_tab.resize(h->win_tab.size() + sizeof(WinGeom) * gr.ns + sizeof(WinItem) * gr.nw);
+            WinGeom* wg = reinterpret_cast<WinGeom*>(h->win_tab.data() + tab_off.back());
+            WinItem* wi = reinterpret_cast<WinItem*>(wg + gr.ns);
+            for (int i = 0; i < gr.ns; ++i)
+            {
+                const QSlot& q = h->qslots[gr.s0 + i];
+                wg[i] = win_geom(h, q);
+                for (size_t e = 0; e < q.ulms.size(); e += 3)
+                    *wi++ = WinItem{i, {q.ulms[e], q.ulms[e + 1], q.ulms[e + 2]}};
+            }
+            groups.push_back(gr);
         }
-        Group gr{s, 0, h->win_base[s], 0};
-        while (s < (int)h->qslots.size() && h->qslots[s].set && !h->qslots[s].ulms.empty())
-        {
-            const int nu = (int)h->qslots[s].ulms.size() / 3;
-            if (gr.ns > 0 && ((size_t)(gr.ns + 1) * ncomp * NN * esz > (512ull << 20) ||
-                              (size_t)(gr.nw + nu) * ncomp * M * eszM > (1ull << 30) || gr.nw + nu > 32768))
-                break;
-            ++gr.ns;
-            gr.nw += nu;
-            ++s;
-        }
-        needN = std::max(needN, (size_t)(gr.ns * ncomp * NN) * esz);
-        needM = std::max(needM, (size_t)(gr.nw * ncomp * M) * eszM);
-        // geometries, then windows
-        tab_off.push_back(h->win_tab.size());
-        h->win_tab.resize(h->win_tab.size() + sizeof(WinGeom) * gr.ns + sizeof(WinItem) * gr.nw);
-        WinGeom* wg = reinterpret_cast<WinGeom*>(h->win_tab.data() + tab_off.back());
-        WinItem* wi = reinterpret_cast<WinItem*>(wg + gr.ns);
-        for (int i = 0; i < gr.ns; ++i)
-        {
-            const QSlot& q = h->qslots[gr.s0 + i];
-            wg[i] = win_geom(h, q);
-            for (size_t e = 0; e < q.ulms.size(); e += 3) *wi++ = WinItem{i, {q.ulms[e], q.ulms[e + 1], q.ulms[e + 2]}};
-        }
-        groups.push_back(gr);
-    }
-    int rc = ensure(h, h->d_wtmpN, needN);
-    if (rc) return rc;
-    if (h->mixed) rc = ensure(h, h->d_wtmpM, needM);  // the plain form transforms in place
+        int rc = ensure(h, h->d_wtmpN, needN);
+        if (!rc && h->mixed) rc = ensure(h, h->d_wtmpM, needM);  // the plain form transforms in place
+        return rc;
+    };
+    size_t needN = 0, needM = 0;
+    int rc = make_groups(512ull << 20, 1ull << 30, needN, needM);
+    if (rc) rc = make_groups(0, 0, needN, needM);  // no room: a slot at a time
     if (rc) return rc;
     // the tables of every group, uploaded in one copy
     rc = ensure(h, h->d_tmp, h->win_tab.size() + 16);
