@@ -93,6 +93,7 @@ __device__ __forceinline__ uint32_t oz_digits(unsigned long long tr, unsigned lo
 }
 
 #define OZ_NO_EXP (-16384)  // four points without a normal finite number
+#define OZ_NO_EXP2 0xc000c000u  // two of them
 
 // Limits below the suspend hint of mbar_wait_bounded poll instead: a suspended wait sleeps
 // past them, and the MMAs of a stage (a microsecond) then always complete first.
@@ -103,13 +104,6 @@ __device__ __forceinline__ bool oz_wait(uint64_t* bar, uint32_t parity, unsigned
     while (!mbar_test_wait(bar, parity))
         if (gtimer_ns() - t0 > limit_ns) return false;
     return true;
-}
-
-// the largest of the warp's packed 16-bit maxima, and the exponent of a scale from it
-__device__ __forceinline__ int oz_scale(unsigned mx, int guard)
-{
-    const int m = __reduce_max_sync(0xffffffffu, max((int)(short)(mx & 0xffffu), (int)(short)(mx >> 16)));
-    return m < OZ_NO_EXP / 2 ? 0 : -(m + guard);
 }
 
 // One CTA: one (pair, spin), 128 rows x up to 32 bands, one K chunk of the stages
@@ -156,57 +150,75 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         ss.bpsi[b] = b < nbt ? psi + idx * gd.nspinor * M : nullptr;
         ss.badband[b] = 0;
     }
-    const int st0 = stage0 + blockIdx.z * stages_per_chunk;
-    const int nst = min(stages_per_chunk, nstage_total - st0);
-    // scales of the chunk: eight exponents (32 points) a 16-byte word
-    {
-        const long long k0 = (long long)st0 * OZ_PTS, k1 = min(Ktot, k0 + (long long)nst * OZ_PTS);
-        const size_t wpc = (size_t)((M + 31) / 32);  // words of a component
-        const uint4* const ep = reinterpret_cast<const uint4*>(epsi);
-        const uint4* const ed = reinterpret_cast<const uint4*>(edv);
-#pragma unroll 1
-        for (int r = warp; r < OZ_ROWS + OZ_BANDS; r += OZ_WARPS)
-        {
-            const bool row = r < OZ_ROWS;
-            const int R = mt * OZ_ROWS + r, b = r - OZ_ROWS;
-            if (row ? R >= nrows : b >= nbt) continue;
-            const int nu = row ? R / nb : 0, band = row ? R - nu * nb : n0 + b;
-            const uint4* p = ep + (((size_t)(row ? P.kbz_k : P.kbz_kq) * gd.nspin + spin) * nb + band) * gd.nspinor * wpc;
-            const uint4* d = ed + ((size_t)P.dvslot * gd.nmodes + nu) * gd.nmag * wpc;
-            unsigned mx = 0x80008000u;
-            for (int s = 0; s < gd.nspinor; ++s)
-            {
-                const int w0 = (int)((max(k0, s * M) - s * M) >> 5);
-                const int w1 = (int)((min(k1, (s + 1) * M) - s * M + 31) >> 5);
-                for (int w = w0 + lane; w < w1; w += 32)
-                    if (!row)
-                    {
-                        const uint4 x = p[s * wpc + w];
-                        mx = __vmaxs2(mx, __vmaxs2(__vmaxs2(x.x, x.y), __vmaxs2(x.z, x.w)));
-                    }
-                    else
-                        for (int c = 0; c < (gd.nmag == 4 ? 2 : 1); ++c)
-                        {
-                            const int dc = gd.nmag == 4 ? 2 * s + c : (gd.nmag == 2 ? spin : 0);
-                            const uint4 x = p[(gd.nmag == 4 ? c : s) * wpc + w], y = d[dc * wpc + w];
-                            mx = __viaddmax_s16x2(x.x, y.x, mx);
-                            mx = __viaddmax_s16x2(x.y, y.y, mx);
-                            mx = __viaddmax_s16x2(x.z, y.z, mx);
-                            mx = __viaddmax_s16x2(x.w, y.w, mx);
-                        }
-            }
-            // |re|, |im| < 2^(E+1) of either factor: |dV psi| < 2^(Ed+Ep+3), a sum of two (nmag 4)
-            // twice that; scaled below 1/2
-            const int e = oz_scale(mx, !row ? 2 : (gd.nmag == 4 ? 5 : 4));
-            if (lane == 0) (row ? ss.re[r] : ss.be[b]) = e;
-        }
-    }
     if (threadIdx.x == 0)
     {
         mbar_init(&ss.bar, 1);
         fence_barrier_init();
     }
     if (warp == 0) tmem_alloc(&ss.tmem, 512);
+    const int st0 = stage0 + blockIdx.z * stages_per_chunk;
+    const int nst = min(stages_per_chunk, nstage_total - st0);
+    // scales of the chunk: eight exponents (32 points) a 16-byte word, eight lanes a row or band,
+    // four words in flight.  Its latency is what the scales cost: 50 (pair, spin)s of 27 rows x 3
+    // bands x 4,608 points 211 -> 218 us, 27 pairs of 240 x 20 x 11,664 1275 -> 1293 (a warp a row
+    // 1308), 64 of 384 x 32 x 27,648 within 0.4 %
+    {
+        const long long k0 = (long long)st0 * OZ_PTS, k1 = min(Ktot, k0 + (long long)nst * OZ_PTS);
+        const unsigned wpc = (unsigned)((M + 31) / 32);  // words of a component
+        const int lo = (int)(k0 >= M ? 1 : 0), hi = (int)(k1 > M ? 1 : 0);
+        const int nrt = min(OZ_ROWS, nrows - mt * OZ_ROWS), total = nrt + nbt;
+        const int nc = gd.nmag == 4 ? 2 : 1;
+        for (int i0 = 4 * warp; i0 < total; i0 += 4 * OZ_WARPS)
+        {
+            const int i = i0 + (lane >> 3);
+            const bool row = i < nrt;
+            unsigned mx = 0x80008000u;
+            if (i < total)
+            {
+                const int R = mt * OZ_ROWS + i, nu = row ? R / nb : 0, band = row ? R - nu * nb : n0 + i - nrt;
+                const uint4* p = reinterpret_cast<const uint4*>(epsi) +
+                                 (size_t)(((row ? P.kbz_k : P.kbz_kq) * gd.nspin + spin) * nb + band) * (gd.nspinor * wpc);
+                const uint4* d = reinterpret_cast<const uint4*>(edv) +
+                                 (size_t)(P.dvslot * gd.nmodes + nu) * (gd.nmag * wpc) + (gd.nmag == 2 ? spin * wpc : 0u);
+                for (int s = lo; s <= hi; ++s)
+                {
+                    const unsigned w0 = s == lo ? (unsigned)((k0 - s * M) >> 5) : 0u;
+                    const unsigned w1 = s == hi ? (unsigned)((k1 - s * M + 31) >> 5) : wpc;
+                    for (int c = 0; c < (row ? nc : 1); ++c)
+                    {
+                        const uint4* pc = p + (row && nc == 2 ? c : s) * wpc;
+                        const uint4* dc = d + (nc == 2 ? (2 * s + c) * wpc : 0u);
+                        for (unsigned w = w0 + (lane & 7); w < w1; w += 32)
+                        {
+                            uint4 x[4], y[4];  // four words of each in flight
+#pragma unroll
+                            for (int u = 0; u < 4; ++u)
+                            {
+                                const bool in = w + 8 * u < w1;
+                                x[u] = in ? pc[w + 8 * u] : make_uint4(OZ_NO_EXP2, OZ_NO_EXP2, OZ_NO_EXP2, OZ_NO_EXP2);
+                                y[u] = in && row ? dc[w + 8 * u] : make_uint4(0u, 0u, 0u, 0u);
+                            }
+#pragma unroll
+                            for (int u = 0; u < 4; ++u)
+                            {
+                                mx = __viaddmax_s16x2(x[u].x, y[u].x, mx);
+                                mx = __viaddmax_s16x2(x[u].y, y[u].y, mx);
+                                mx = __viaddmax_s16x2(x[u].z, y[u].z, mx);
+                                mx = __viaddmax_s16x2(x[u].w, y[u].w, mx);
+                            }
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) mx = __vmaxs2(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const int m = max((int)(short)(mx & 0xffffu), (int)(short)(mx >> 16));
+            // |re|, |im| < 2^(E+1) of either factor: |dV psi| < 2^(Ed+Ep+3), a sum of two (nmag 4)
+            // twice that; scaled below 1/2
+            const int e = m < OZ_NO_EXP / 2 ? 0 : -(m + (!row ? 2 : 3 + nc));
+            if ((lane & 7) == 0 && i < total) (row ? ss.re[i] : ss.be[i - nrt]) = e;
+        }
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
