@@ -184,7 +184,7 @@ int lelph_launch_dvloc_g(const VlocDesc& vd, const double2* eig, double2* out, u
     const long long N = (long long)vd.Nx * vd.Ny * vd.Nz;
     const size_t smem = sizeof(double2) * (size_t)vd.nmodes * 3 * vd.natom + sizeof(double) * 3 * vd.natom +
                         sizeof(int) * vd.natom + 16;
-    lelph_smem_opt_in(k_dvloc_g, smem, 200 * 1024);
+    lelph_smem_opt_in<k_dvloc_g>(smem, 200 * 1024);
     k_dvloc_g<<<(unsigned)((N + 255) / 256), 256, smem, st>>>(vd, eig, out, status);
     return 0;
 }

@@ -643,7 +643,7 @@ static void launch_contig_l(T2* data, long long nlines, const FftPlan1D& p, cons
     int lpc = elems / p.L;
     if (lpc < 1) lpc = 1;
     size_t smem = (size_t)(2 * lpc * p.L + p.L) * sizeof(T2) + sizeof(int) * lpc;
-    lelph_smem_opt_in(k_fft_contig<T2, T, CTL>, smem, 200 * 1024);
+    lelph_smem_opt_in<k_fft_contig<T2, T, CTL>>(smem, 200 * 1024);
     long long nb = (nlines + lpc - 1) / lpc;
     k_fft_contig<T2, T, CTL><<<(unsigned)nb, 256, smem, st>>>(data, nlines, p, tw, sign, lpc, mk);
 }
@@ -663,12 +663,12 @@ static void launch_strided_l(T2* data, long long nouter, int inner, const FftPla
     {
         // cubic planes (inner = L): a compile-time line count
         constexpr int NLC = CTL;
-        lelph_smem_opt_in(k_fft_strided<T2, T, CTL, NLC>, smem, 200 * 1024);
+        lelph_smem_opt_in<k_fft_strided<T2, T, CTL, NLC>>(smem, 200 * 1024);
         k_fft_strided<T2, T, CTL, NLC><<<(unsigned)nb, 256, smem, st>>>(data, nouter, inner, ich, nchunk, p, tw, sign,
                                                                         mk);
         return;
     }
-    lelph_smem_opt_in(k_fft_strided<T2, T, CTL, 0>, smem, 200 * 1024);
+    lelph_smem_opt_in<k_fft_strided<T2, T, CTL, 0>>(smem, 200 * 1024);
     k_fft_strided<T2, T, CTL, 0><<<(unsigned)nb, 256, smem, st>>>(data, nouter, inner, ich, nchunk, p, tw, sign, mk);
 }
 
@@ -742,7 +742,7 @@ static void launch_x_split_n(unsigned nb, size_t smem, const float2* boxes, int 
                              const float* band_scale, uint16_t* Bsplit, float2* psi32, cudaStream_t st,
                              const BoxMask& mk)
 {
-    lelph_smem_opt_in(k_fft_x_split<BF16, CTL, NLC>, smem, 200 * 1024);
+    lelph_smem_opt_in<k_fft_x_split<BF16, CTL, NLC>>(smem, 200 * 1024);
     k_fft_x_split<BF16, CTL, NLC><<<nb, 256, smem, st>>>(boxes, nbox, k0, ich, nchunk, p, tw, sign, g, band_scale,
                                                          Bsplit, psi32, mk);
 }

@@ -773,7 +773,7 @@ static int gs_plane_ct(const GsGeom& gg, const void* psi, const void* win, int n
                 const size_t s2 = sizeof(float2) * (2 * (size_t)N * (N | 1) + 2 * N) + sizeof(int) * N +
                                   sizeof(short) * ((size_t)nzl * N);
                 constexpr int NT = N <= 48 ? 160 : 256;  // psi of a plane in at most 32 registers
-                if (lelph_smem_opt_in(k_gs_plane_yz<N, N, NT>, s2,
+                if (lelph_smem_opt_in<k_gs_plane_yz<N, N, NT>>(s2,
                                       sizeof(float2) * (2 * (size_t)N * (N | 1) + 2 * N) + sizeof(int) * N +
                                           sizeof(short) * (size_t)N * N) != cudaSuccess)
                     return -1;
@@ -788,14 +788,14 @@ static int gs_plane_ct(const GsGeom& gg, const void* psi, const void* win, int n
                                                             nzl, (float2*)out);
                 return 0;
             }
-            if (lelph_smem_opt_in(k_gs_plane_ct1<N, N, NUC>, smem, smem) != cudaSuccess) return -1;
+            if (lelph_smem_opt_in<k_gs_plane_ct1<N, N, NUC>>(smem, smem) != cudaSuccess) return -1;
             k_gs_plane_ct1<N, N, NUC><<<g1, GS_THREADS, smem, st>>>((const float2*)psi, (const float2*)win, gg, nu0, nub,
                                                                     (const float2*)twy, (const float2*)twz, cols2, ncol,
                                                                     zl, nzl, (float2*)out);
             return 0;
         }
     }
-    if (lelph_smem_opt_in(k_gs_plane_ct<T2, T, N, N>, smem, smem) != cudaSuccess) return -1;
+    if (lelph_smem_opt_in<k_gs_plane_ct<T2, T, N, N>>(smem, smem) != cudaSuccess) return -1;
     dim3 grid((unsigned)nub, (unsigned)gg.nb, (unsigned)(gg.nsub * gg.Nx));
     k_gs_plane_ct<T2, T, N, N><<<grid, GS_THREADS, smem, st>>>((const T2*)psi, (const T2*)win, gg, nu0,
                                                                (const T2*)twy, (const T2*)twz, cols2, ncol, zl, nzl,
@@ -848,7 +848,7 @@ int lelph_launch_gs_plane(const GsGeom& gg, int fp64, const void* psi, const voi
     dim3 grid((unsigned)nub, (unsigned)gg.nb, (unsigned)(gg.nsub * gg.Nx));
     if (fp64)
     {
-        if (lelph_smem_opt_in(k_gs_plane<double2, double>, smem, 220 * 1024) != cudaSuccess)
+        if (lelph_smem_opt_in<k_gs_plane<double2, double>>(smem, 220 * 1024) != cudaSuccess)
             return -1;
         k_gs_plane<double2, double><<<grid, GS_THREADS, smem, st>>>(
             (const double2*)psi, (const double2*)win, gg, nu0, py, pz, (const double2*)twy, (const double2*)twz,
@@ -856,7 +856,7 @@ int lelph_launch_gs_plane(const GsGeom& gg, int fp64, const void* psi, const voi
     }
     else
     {
-        if (lelph_smem_opt_in(k_gs_plane<float2, float>, smem, 220 * 1024) != cudaSuccess)
+        if (lelph_smem_opt_in<k_gs_plane<float2, float>>(smem, 220 * 1024) != cudaSuccess)
             return -1;
         k_gs_plane<float2, float><<<grid, GS_THREADS, smem, st>>>((const float2*)psi, (const float2*)win, gg, nu0,
                                                                   py, pz, (const float2*)twy, (const float2*)twz,
@@ -870,7 +870,7 @@ static int gs_xpass_ct(int nrb, int ncol, int nsub, const void* twx, const int* 
                        const void* shph, int npad, const void* in, void* A, void* A_lo, cudaStream_t st)
 {
     const size_t smem = sizeof(T2) * (2 * (size_t)NX * CB + NX);
-    if (lelph_smem_opt_in(k_gs_xpass_ct<T2, T, NX, CB, CTW>, smem, smem) != cudaSuccess) return -1;
+    if (lelph_smem_opt_in<k_gs_xpass_ct<T2, T, NX, CB, CTW>>(smem, smem) != cudaSuccess) return -1;
     const int cb = CB / nsub;
     dim3 grid((unsigned)((ncol + cb - 1) / cb), (unsigned)nrb);
     k_gs_xpass_ct<T2, T, NX, CB, CTW><<<grid, GS_THREADS, smem, st>>>((const T2*)in, ncol, (const T2*)twx, cst, kcx,
@@ -929,7 +929,7 @@ int lelph_launch_gs_xpass(const GsGeom& gg, int fp64, const void* in, int nrb, i
     dim3 grid((unsigned)((ncol + cb - 1) / cb), (unsigned)nrb);
     if (fp64)
     {
-        if (lelph_smem_opt_in(k_gs_xpass<double2, double>, smem, 220 * 1024) != cudaSuccess)
+        if (lelph_smem_opt_in<k_gs_xpass<double2, double>>(smem, 220 * 1024) != cudaSuccess)
             return -1;
         k_gs_xpass<double2, double><<<grid, GS_THREADS, smem, st>>>((const double2*)in, gg.Nx, ncol, px,
                                                                     (const double2*)twx, cst, kcx,
@@ -938,7 +938,7 @@ int lelph_launch_gs_xpass(const GsGeom& gg, int fp64, const void* in, int nrb, i
     }
     else
     {
-        if (lelph_smem_opt_in(k_gs_xpass<float2, float>, smem, 220 * 1024) != cudaSuccess)
+        if (lelph_smem_opt_in<k_gs_xpass<float2, float>>(smem, 220 * 1024) != cudaSuccess)
             return -1;
         k_gs_xpass<float2, float><<<grid, GS_THREADS, smem, st>>>((const float2*)in, gg.Nx, ncol, px,
                                                                   (const float2*)twx, cst, kcx,
@@ -980,7 +980,7 @@ int lelph_launch_gs_gemm(int fp64, const void* A, const void* B, int nrows, int 
     do                                                                                                           \
     {                                                                                                            \
         const int sm = (int)(sizeof(float) * 4 * GS_BK * (32 * TM + 2) + sizeof(float2) * 2 * GS_BK * (8 * TN + 1)); \
-        if (lelph_smem_opt_in(k_gs_gemm_f32x2<TM, TN>, sm, sm) != cudaSuccess) return -1;                        \
+        if (lelph_smem_opt_in<k_gs_gemm_f32x2<TM, TN>>(sm, sm) != cudaSuccess) return -1;                        \
         k_gs_gemm_f32x2<TM, TN><<<g2, GS_THREADS, sm, st>>>((const float2*)A, (const float2*)B, nrows, nb, Ktot,  \
                                                             kchunk, rowoff, nrows_total, (float2*)part);         \
     } while (0)

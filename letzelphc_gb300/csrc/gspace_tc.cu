@@ -353,7 +353,7 @@ static int gt_launch(const CUtensorMap* m, int nrows, int nb, int Ktot, int kchu
                      int small_first, float2* part, unsigned* status, unsigned long long wait_ns, cudaStream_t st)
 {
     const GtLayout L = gt_layout(NT);
-    if (lelph_smem_opt_in(k_gs_gemm_tc<NT>, L.total, L.total) != cudaSuccess) return -1;
+    if (lelph_smem_opt_in<k_gs_gemm_tc<NT>>(L.total, L.total) != cudaSuccess) return -1;
     int nnt = 0;
     lelph_gs_tc_ntile(nb, &nnt);
     const int nrt = (nrows + 127) / 128;

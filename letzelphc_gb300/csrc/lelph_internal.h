@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #define LELPH_MAX_RADIX_STAGES 12
 #define TC_KPTS_MAX 64  // largest pipeline stage of the tensor-core sandwich (grid points)
 
@@ -100,16 +102,25 @@ struct BoxMask
     int Nx = 0, Ny = 0, nbox_per_k = 1;
 };
 
-// Dynamic shared memory above the default 48 KB has to be opted into, per kernel and
-// per context.  limit: the kernel's largest, so that host threads that launch it with
-// different sizes do not lower each other's.  Called before every such launch (under a
-// microsecond): a flag kept by the process would miss another device's context and one
-// created anew after cudaDeviceReset.
-template <typename K>
-inline cudaError_t lelph_smem_opt_in(K* kernel, size_t smem, size_t limit)
+// Dynamic shared memory above the default 48 KB has to be opted into, per kernel and per
+// device: once on each device (a set of device numbers per kernel; two host threads may both
+// do it).  limit: the kernel's largest, so that threads that launch it with different sizes
+// do not lower each other's.  Opting in before every launch instead took 3 us of a 300 us
+// run of a small FP64 system.  A context created anew after cudaDeviceReset keeps the
+// attribute (checked: the runtime applies it again when it loads the kernel).
+template <auto K>
+inline cudaError_t lelph_smem_opt_in(size_t smem, size_t limit)
 {
     if (smem <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+    if (e == cudaSuccess && bit) done.fetch_or(bit, std::memory_order_release);
+    return e;
 }
 
 // FFT (fft_gather.cu)

@@ -322,8 +322,8 @@ void lelph_launch_projections(int k0, int nk, const KPointSym* ksym_dev, const d
     if (gsplit > 1)
         cudaMemsetAsync(proj + (size_t)k0 * rows * nsets, 0, sizeof(double2) * (size_t)nk * rows * nsets, st);
     dim3 grid(nk, rb, sb * gsplit);
-    lelph_smem_opt_in(k_projections<float>, pj_smem_bytes<float>(), pj_smem_bytes<float>());
-    lelph_smem_opt_in(k_projections<double>, pj_smem_bytes<double>(), pj_smem_bytes<double>());
+    lelph_smem_opt_in<k_projections<float>>(pj_smem_bytes<float>(), pj_smem_bytes<float>());
+    lelph_smem_opt_in<k_projections<double>>(pj_smem_bytes<double>(), pj_smem_bytes<double>());
     if (f32acc)
         k_projections<float><<<grid, 256, pj_smem_bytes<float>(), st>>>(k0, ksym_dev, gvec, pw_off, npw, Fk, fk_off,
                                                                         chat, chat_off, nl, g, gsplit, proj);
@@ -1088,7 +1088,7 @@ static int launch_finish_atoms(const PairInfo* pairs, int npairs, int mode_fp64,
                   sizeof(int) * 4 * (size_t)nl.ntype * nl.nproj_max;
     smem = std::max(smem, e * (size_t)g.nmodes * 3 * nl.natom);
     if (smem > 220 * 1024) return -1;
-    if (lelph_smem_opt_in(k_finish_atoms<NJ, TM, A>, smem, 220 * 1024) != cudaSuccess) return -1;
+    if (lelph_smem_opt_in<k_finish_atoms<NJ, TM, A>>(smem, 220 * 1024) != cudaSuccess) return -1;
     const dim3 grid((unsigned)(((g.nbnds + FA_N - 1) / FA_N) * ((g.nbnds + TM - 1) / TM)),
                     (unsigned)(npairs * g.nspin));
     k_finish_atoms<NJ, TM, A><<<grid, FA_N * TM, smem, st>>>(pairs, mode_fp64, glocal, partials, nchunks, mode_scale,
@@ -1113,7 +1113,7 @@ int lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const 
 #define FINL(NJ, T)                                                                                              \
     do                                                                                                           \
     {                                                                                                            \
-        lelph_smem_opt_in(k_finish_pair<NJ, T>, smem, 160 * 1024);                                               \
+        lelph_smem_opt_in<k_finish_pair<NJ, T>>(smem, 160 * 1024);                                               \
         k_finish_pair<NJ, T><<<nz, NJ <= 12 ? 256 : 128, smem, st>>>(pairs, mode_fp64, glocal, partials, nchunks, \
                                                                      mode_scale, band_scale, proj, eig, non_loc, \
                                                                      nl, g, out_c64, gout);                      \
@@ -1138,13 +1138,13 @@ int lelph_launch_finish(const PairInfo* pairs, int npairs, int mode_fp64, const 
         dim3 tg((unsigned)(nt * nt), (unsigned)(npairs * g.nspin));
         if (t64)
         {
-            lelph_smem_opt_in(k_finish_tile<48, double>, tsm, 200 * 1024);
+            lelph_smem_opt_in<k_finish_tile<48, double>>(tsm, 200 * 1024);
             k_finish_tile<48, double><<<tg, FT_B * FT_B, tsm, st>>>(pairs, glocal, proj, eig, non_loc, nl, g, out_c64,
                                                                   gout);
         }
         else
         {
-            lelph_smem_opt_in(k_finish_tile<48, float>, tsm, 200 * 1024);
+            lelph_smem_opt_in<k_finish_tile<48, float>>(tsm, 200 * 1024);
             k_finish_tile<48, float><<<tg, FT_B * FT_B, tsm, st>>>(pairs, glocal, proj, eig, non_loc, nl, g, out_c64,
                                                                  gout);
         }

@@ -482,7 +482,7 @@ int lelph_launch_local_fp64(const PairInfo* pairs, int npairs, const double2* ps
     const int nrows = g.nmodes * g.nbnds;
     const int ntm = (nrows + OZ_ROWS - 1) / OZ_ROWS, ntn = (g.nbnds + OZ_BANDS - 1) / OZ_BANDS;
     const int smem = OZ_S * (OZ_ROWS + 2 * OZ_BANDS) * 128 + (int)sizeof(OzSmem) + 1024;
-    if (lelph_smem_opt_in(k_local_oz, smem, smem) != cudaSuccess) return -1;
+    if (lelph_smem_opt_in<k_local_oz>(smem, smem) != cudaSuccess) return -1;
     const double invM = 1.0 / (double)lelph_grid_points(g);
     const long long nel = (long long)npairs * g.nspin * nrows * g.nbnds;
     // chunks of more than OZ_SUM stages go in several launches, each adding to the last one's
