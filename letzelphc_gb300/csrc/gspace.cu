@@ -645,7 +645,7 @@ __device__ __forceinline__ float2* ct_fft_head(float2* a, float2* b, int nlines,
 // inside a radix are constants (their table reads took a twentieth of the pipe).
 // 48 x 48 planes take 160 threads (144 butterflies of 16 points; five CTAs an SM):
 // before the constants 31.1 ms for 8 pairs of 48 modes x 200 bands x 64 planes, 33.9
-// with 256, 42.8 with 128; the LSU pipe is busy 75 % of the time.  Now 28.5 ms.
+// with 256, 42.8 with 128; the LSU pipe is busy 71 % of the time.  Now 28.5 ms.
 // Measured against k_gs_plane_ct1 (1152 products): 24 x 24 planes 4.3 -> 3.1 ms,
 // 30 x 30 7.5 -> 5.8, 40 x 40 10.9 -> 7.7, 48 x 48 12.2 -> 10.4, 60 x 60 34.3 -> 29.9.
 template <int NY, int NZ, int NT>

@@ -31,7 +31,7 @@
 // Measured, SIMT -> this: 64 pairs of 384 rows x 32 bands x 27,648 points, 176 ->
 // 11.3 ms; 64 pairs of 48 x 8 x 5,832, 12.6 -> 0.36 ms; error against 64 bits
 // (norm) 5.5e-15 -> 1.9e-15 and 3.4e-15 -> 0.86e-15.  (With 16 warps instead of 32:
-// 12.5 and 0.41 ms; the FP64 pipe is busy 40 % of the time, the rest is latency
+// 12.5 and 0.41 ms; the FP64 pipe is busy 45 % of the time, the rest is latency
 // between the barriers.  Forming part of the next stage's products between the digit
 // stores: no change; two rows at a time in straight-line code: 3 % slower.)
 #include <cuda_runtime.h>
