@@ -54,16 +54,19 @@
 #define OZ_SUM 60000   // stages that the 64-bit sums hold (a stage adds less than 2^47 + 2^41)
 #define OZ_COLS (2 * OZ_BANDS / (OZ_WARPS / 4))  // accumulator columns of a thread (its row of the tile)
 
+// (One 24-byte record a row: with the exponent in an array of its own the compiler ordered
+// the loads of two components, nmag 4, so that the kernel took 16 % longer.)
 struct OzRow
 {
     const double2* psi;  // component 0 of the row's band of k (null: no such row)
     const double2* dv;   // component 0 of its mode's window
+    int e;               // exponent of the row's scale
 };
 struct OzSmem
 {
     OzRow row[OZ_ROWS];
     const double2* bpsi[OZ_BANDS];
-    int re[OZ_ROWS], be[OZ_BANDS];               // exponents of the scales
+    int be[OZ_BANDS];                           // exponents of the bands' scales
     int badrow[OZ_ROWS], badband[OZ_BANDS];  // met an infinity or a NaN
     uint64_t bar;
     uint32_t tmem;
@@ -134,14 +137,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     for (int r = threadIdx.x; r < OZ_ROWS; r += OZ_THREADS)
     {
         const int R = mt * OZ_ROWS + r;
-        OzRow w{nullptr, nullptr};
+        const double2 *rp = nullptr, *rd = nullptr;
         if (R < nrows)
         {
             const int nu = R / nb, m = R - nu * nb;
-            w.psi = psi + (((size_t)P.kbz_k * gd.nspin + spin) * nb + m) * gd.nspinor * M;
-            w.dv = dV + ((size_t)P.dvslot * gd.nmodes + nu) * gd.nmag * M + (gd.nmag == 2 ? (size_t)spin * M : 0);
+            rp = psi + (((size_t)P.kbz_k * gd.nspin + spin) * nb + m) * gd.nspinor * M;
+            rd = dV + ((size_t)P.dvslot * gd.nmodes + nu) * gd.nmag * M + (gd.nmag == 2 ? (size_t)spin * M : 0);
         }
-        ss.row[r] = w;
+        ss.row[r].psi = rp;
+        ss.row[r].dv = rd;  // (e comes from the warp that finds it, below)
         ss.badrow[r] = 0;
     }
     for (int b = threadIdx.x; b < OZ_BANDS; b += OZ_THREADS)
@@ -216,7 +220,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             // |re|, |im| < 2^(E+1) of either factor: |dV psi| < 2^(Ed+Ep+3), a sum of two (nmag 4)
             // twice that; scaled below 1/2
             const int e = m < OZ_NO_EXP / 2 ? 0 : -(m + (!row ? 2 : 3 + nc));
-            if ((lane & 7) == 0 && i < total) (row ? ss.re[i] : ss.be[i - nrt]) = e;
+            if ((lane & 7) == 0 && i < total) (row ? ss.row[i].e : ss.be[i - nrt]) = e;
         }
     }
     tc_fence_before();
@@ -235,7 +239,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         for (int i = 0; i < OZ_RPW; ++i)
         {
             const OzRow w = ss.row[warp + i * OZ_WARPS];
-            const int we = ss.re[warp + i * OZ_WARPS];
             ar[i] = ai[i] = 0;
             if (w.psi && in)
             {
@@ -248,8 +251,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 else
                     a = cmul(w.dv[r], w.psi[kc]);
                 bool bad = false;
-                ar[i] = oz_fixed(a.x, we, bad);
-                ai[i] = oz_fixed(a.y, we, bad);
+                ar[i] = oz_fixed(a.x, w.e, bad);
+                ai[i] = oz_fixed(a.y, w.e, bad);
                 if (bad) ss.badrow[warp + i * OZ_WARPS] = 1;
             }
         }
@@ -401,7 +404,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 if (b >= nbt) continue;
                 // (H 2^27 + L 2^18) units of 2^(54 - 124) of the two scales' product
                 double v = fma((double)H[c], 0x1p27, (double)L[c] * 0x1p18);
-                v = scalbn(v, -70 - ss.re[r] - ss.be[b]) * scale;
+                v = scalbn(v, -70 - ss.row[r].e - ss.be[b]) * scale;
                 if (add) v += o[2 * (n0 + b) + im];
                 o[2 * (n0 + b) + im] = (bad || ss.badband[b]) ? __longlong_as_double(0x7ff8000000000000ll) : v;
             }
