@@ -154,18 +154,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         ss.bpsi[b] = b < nbt ? psi + idx * gd.nspinor * M : nullptr;
         ss.badband[b] = 0;
     }
-    if (threadIdx.x == 0)
-    {
-        mbar_init(&ss.bar, 1);
-        fence_barrier_init();
-    }
-    if (warp == 0) tmem_alloc(&ss.tmem, 512);
     const int st0 = stage0 + blockIdx.z * stages_per_chunk;
     const int nst = min(stages_per_chunk, nstage_total - st0);
     // scales of the chunk: eight exponents (32 points) a 16-byte word, eight lanes a row or band,
-    // four words in flight.  Its latency is what the scales cost: 50 (pair, spin)s of 27 rows x 3
-    // bands x 4,608 points 211 -> 218 us, 27 pairs of 240 x 20 x 11,664 1275 -> 1293 (a warp a row
-    // 1308), 64 of 384 x 32 x 27,648 within 0.4 %
+    // four words in flight.  What they cost: 50 (pair, spin)s of 27 rows x 3 bands x 4,608 points
+    // 211 -> 213 us, 27 pairs of 240 x 20 x 11,664 1278 -> 1296 (a warp a row 1308), 125 of 72 x 12
+    // with nmag 4 3082 -> 3134, 64 of 384 x 32 x 27,648 within 0.4 %.  (The tensor memory is
+    // allocated after them: before, its wait for the last CTA's added 3 us.)
     {
         const long long k0 = (long long)st0 * OZ_PTS, k1 = min(Ktot, k0 + (long long)nst * OZ_PTS);
         const unsigned wpc = (unsigned)((M + 31) / 32);  // words of a component
@@ -223,6 +218,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             if ((lane & 7) == 0 && i < total) (row ? ss.row[i].e : ss.be[i - nrt]) = e;
         }
     }
+    if (threadIdx.x == 0)
+    {
+        mbar_init(&ss.bar, 1);
+        fence_barrier_init();
+    }
+    if (warp == 0) tmem_alloc(&ss.tmem, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
