@@ -62,10 +62,10 @@ struct GridChoice
 // What a context holds on one product grid: psi(r) of every full-BZ k, the dV
 // windows of the q slots, and the tables of both.  The mixed form has two where
 // pick_grid finds a grid smaller than the plain one: batch runs (run,
-// run_device and the allocation-free form) use the smaller one, the one-call
-// entry points (compute_elphq, compute_elphq_star) the plain one, whose
-// complex128 results thereby keep their digits.  use_grid makes one of them
-// active (the base of lelph_gpu) and sets it up when it is first needed.
+// run_device, and the allocation-free form where it is ready) use the smaller
+// one, the one-call entry points (compute_elphq, compute_elphq_star) the plain
+// one, whose digits they thereby keep.  use_grid makes one of them active (the
+// base of lelph_gpu) and sets it up when it is first needed.
 struct GridState
 {
     int which = 0;  // 0: batch runs, 1: one-call stage
