@@ -22,7 +22,7 @@
 // smaller loses more, but below the rounding that the transforms of psi and dV leave
 // at every point.  (Measured against scales from the two maxima: error 8.4e-16 ->
 // 5.3e-16 on the 4-atom cell with its dV on one atom, 3.1e-8 -> 1.5e-8 where the bands
-// lie elsewhere and the elements are 1e-10 of max |dV|; the time is the same.)
+// lie elsewhere and the elements are 1e-10 of max |dV|; the time: at the prologue.)
 //
 // What bounds it: the FP64 products a (four operations an element; GB300 issues
 // about two per cycle and SM), then the integer work of the digits; the MMAs take
